@@ -97,6 +97,7 @@ BasisDev make_basis_dev(int p, const double* xi, const double* w, const double* 
     for (int k = 0; k < B.np; ++k) B.D[i][k] = D[i + (size_t)k * B.np];
   for (int i = 0; i < B.np; ++i)
     for (int k = 0; k < B.np; ++k) B.W2[i][k] = B.w[i] * (B.D[i][k] * B.D[i][k]);
+  B.fD = make_fix(B.D, B.np);
   // chebyshev_fixed!, elliptic.jl:373-378
   const double table[4] = {1.5, 2.0, 2.1, 2.2};
   const double lmax = table[std::min(p, 4) - 1], lmin = 1.0;

@@ -25,6 +25,10 @@ struct Tiling2D {
   static constexpr int TY = 4;
   static constexpr int TE = TX * TY;       // elements per tile
   static constexpr int NN = NP * NP;       // nodes per element
+  // Stride of an element in shared memory. A phase reads 8-byte nodes down its lines: with the 16 nodes of a P3
+  // element packed, a warp's 8 elements hit the same banks (8 wavefronts for 2); 18 spreads them over all banks and
+  // keeps the rows 16-byte aligned (128-bit accesses, also without conflicts). 5 does it for P1; 9 and 25 are odd.
+  static constexpr int SN = NP == 4 ? 18 : (NP == 2 ? 5 : NN);
   static constexpr int NT = TE * NP;       // threads per CTA (one per line)
   static constexpr int L = NP - 1;
 };
@@ -302,15 +306,22 @@ struct ApplyArgs2D {
   InstSum isum;
 };
 
-// Partner data across one face: its value and end-node derivative of x, and its stiffness coefficient.
-struct Partner1 { double x, d, k; };
+// Partner data across one face: its value and its flux k (D x) at the face node.
+struct Partner1 { double x, t; };
 
 // Shared memory of one tile's operator application: the tile's x, the x-phase
-// result and the end-node derivatives of every line.
-template <int NP>
+// sums (fixed point, with each row's exponent) and the end-node fluxes of
+// every line; f: the fields a solver epilogue's last phase reads, copied while
+// the first phases run (NF = 5: cky, cm, b, cinvM, d; 0: read from global memory
+// there, for the PCG epilogues, whose persistent form has no room for them).
+__host__ __device__ constexpr int apply_fields(int epi) { return epi == EPI_CHEB || epi == EPI_JACOBI ? 5 : 0; }
+template <int NP, int NF>
 struct ApplySmem {
-  double x[Tiling2D<NP>::TE][Tiling2D<NP>::NN], yx[Tiling2D<NP>::TE][Tiling2D<NP>::NN];
-  double gxf[Tiling2D<NP>::TE][NP][2], gyf[Tiling2D<NP>::TE][NP][2];
+  alignas(16) double f[NF ? NF : 1][NF ? Tiling2D<NP>::TE : 1][Tiling2D<NP>::SN];
+  alignas(16) double x[Tiling2D<NP>::TE][Tiling2D<NP>::SN];
+  alignas(16) long long yx[Tiling2D<NP>::TE][Tiling2D<NP>::SN];
+  int ex[Tiling2D<NP>::TE][NP];
+  double txf[Tiling2D<NP>::TE][NP][2], tyf[Tiling2D<NP>::TE][NP][2];
 };
 
 // y = A x on tile tl (of instance I) with the EPI epilogue, by the CTA's
@@ -319,14 +330,16 @@ struct ApplySmem {
 // 0 otherwise). k2_apply runs it on tile blockIdx.x; the persistent PCG kernel
 // on every tile of its CTA.
 template <int NP, int EPI>
-__device__ __forceinline__ double apply_tile(const ApplyArgs2D& a, const Tile2D tl, const Inst2D& I, ApplySmem<NP>& sm) {
+__device__ __forceinline__ double apply_tile(const ApplyArgs2D& a, const Tile2D tl, const Inst2D& I,
+                                             ApplySmem<NP, apply_fields(EPI)>& sm) {
   using TL = Tiling2D<NP>;
   constexpr int L = TL::L, TX = TL::TX, TY = TL::TY;
   constexpr bool PCG = EPI == EPI_PCG0 || EPI == EPI_PCG;
   auto& s_x = sm.x;
   auto& s_yx = sm.yx;
-  auto& s_gxf = sm.gxf;
-  auto& s_gyf = sm.gyf;
+  auto& s_ex = sm.ex;
+  auto& s_txf = sm.txf;
+  auto& s_tyf = sm.tyf;
   const ElemView vr = elem_view<NP>(tl, I, 0), vc = elem_view<NP>(tl, I, 1);
   const BasisDev& B = a.B;
   const double hw = B.hw;
@@ -338,63 +351,73 @@ __device__ __forceinline__ double apply_tile(const ApplyArgs2D& a, const Tile2D 
     return a.x[n];
   };
 
-  // ---- xi-phase part 1: row derivatives
-  double xr[NP], gx[NP];
+  constexpr int NF = apply_fields(EPI);
+  if (NF && vr.valid) {
+    const double* src[5] = {a.cky, a.cm, a.b, a.cinvM, a.d_in};
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+      if (src[f]) {
+#pragma unroll
+        for (int i = 0; i < NP; ++i) copy_async8(&sm.f[f][vr.e][vr.t * NP + i], src[f] + vr.base + vr.t * NP + i);
+      }
+      if (f == 0) copy_async_commit();
+    }
+  }
+  copy_async_commit();
+  auto field = [&](int f, const double* g, int e, long long base, int nd) { return NF ? sm.f[NF ? f : 0][NF ? e : 0][nd] : g[base + nd]; };
+
+  // ---- xi-phase part 1: row fluxes
+  double xr[NP], kx0, kxL;
+  FixFlux<NP> fr;
   if (vr.valid) {
     const int t = vr.t, e = vr.e;
+    double k[NP];
 #pragma unroll
     for (int i = 0; i < NP; ++i) { xr[i] = ldx(vr.base + t * NP + i); s_x[e][t * NP + i] = xr[i]; }
+#pragma unroll
+    for (int i = 0; i < NP; ++i) k[i] = a.ckx[vr.base + t * NP + i];
     if (form_p) {
 #pragma unroll
       for (int i = 0; i < NP; ++i) a.p_out[vr.base + t * NP + i] = xr[i];
     }
-#pragma unroll
-    for (int i = 0; i < NP; ++i) gx[i] = dot_row<NP>(B, i, xr);
-    s_gxf[e][t][0] = gx[0]; s_gxf[e][t][1] = gx[L];
+    flux_line<NP>(B, xr, k, fr);
+    s_txf[e][t][0] = fr.t0; s_txf[e][t][1] = fr.tL;
+    kx0 = k[0]; kxL = k[L];
     if (a.tape_x) {
 #pragma unroll
       for (int i = 0; i < NP; ++i) a.tape_x[vr.base + t * NP + i] = xr[i];
     }
-    if (a.tape_gx) {
-#pragma unroll
-      for (int i = 0; i < NP; ++i) a.tape_gx[vr.base + t * NP + i] = gx[i];
-    }
   }
+  if (NF) copy_async_wait<1>();
   __syncthreads();
-  double xc[NP], gy[NP];
+  double xc[NP], ky0, kyL;
+  FixFlux<NP> fc;
   if (vc.valid) {
     const int t = vc.t, e = vc.e;
+    double k[NP];
 #pragma unroll
-    for (int l = 0; l < NP; ++l) xc[l] = s_x[e][l * NP + t];
-#pragma unroll
-    for (int l = 0; l < NP; ++l) gy[l] = dot_row<NP>(B, l, xc);
-    s_gyf[e][t][0] = gy[0]; s_gyf[e][t][1] = gy[L];
-    if (a.tape_gy) {
-#pragma unroll
-      for (int l = 0; l < NP; ++l) a.tape_gy[vc.base + l * NP + t] = gy[l];
-    }
+    for (int l = 0; l < NP; ++l) { xc[l] = s_x[e][l * NP + t]; k[l] = field(0, a.cky, e, vc.base, l * NP + t); }
+    flux_line<NP>(B, xc, k, fc);
+    s_tyf[e][t][0] = fc.t0; s_tyf[e][t][1] = fc.tL;
+    ky0 = k[0]; kyL = k[L];
   }
   if (vr.valid) {
     // ---- xi-phase part 2: x faces of the row and the x-stiffness transpose
     const int t = vr.t, e = vr.e;
-    double kxr[NP];
-#pragma unroll
-    for (int i = 0; i < NP; ++i) kxr[i] = a.ckx[vr.base + t * NP + i];
     auto fetch = [&](int s) {
       Partner1 P;
       int it;
       const long long pb = neighbour<NP>(tl, I, vr.ex, vr.ey, s == 0 ? -1 : 1, 0, &it);
       const int pi = s == 0 ? L : 0;  // partner face node index along x
-      P.k = a.ckx[pb + t * NP + pi];
       if (it >= 0) {
         P.x = s_x[it][t * NP + pi];
-        P.d = s_gxf[it][t][s == 0 ? 1 : 0];
+        P.t = s_txf[it][t][s == 0 ? 1 : 0];
       } else {
         double pr[NP];
 #pragma unroll
         for (int k = 0; k < NP; ++k) pr[k] = ldx(pb + t * NP + k);
         P.x = s == 0 ? pr[L] : pr[0];
-        P.d = dot_end<NP>(B, s == 0, pr);
+        P.t = flux_end<NP>(B, s == 0, pr, a.ckx[pb + t * NP + pi]);
       }
       return P;
     };
@@ -403,20 +426,16 @@ __device__ __forceinline__ double apply_tile(const ApplyArgs2D& a, const Tile2D 
     const Partner1 pl = sf == 0 ? pA : pB, prt = sf == 0 ? pB : pA;
     // left face: own node (0,t) is the R side; right face: own node (L,t) is the L side
     const double jl = pl.x - xr[0];
-    const double Fl = fma(a.cpx[vr.base + t * NP], jl, hw * fma(pl.k, pl.d, kxr[0] * gx[0]));
+    const double Fl = fma(a.cpx[vr.base + t * NP], jl, hw * (pl.t + fr.t0));
     const double jr = xr[L] - prt.x;
-    const double Fr = fma(a.cpx[vr.base + t * NP + L], jr, hw * fma(kxr[L], gx[L], prt.k * prt.d));
-    double sx[NP];
+    const double Fr = fma(a.cpx[vr.base + t * NP + L], jr, hw * (fr.tL + prt.t));
+    FixSums<NP> sums;
+    row_sums<NP>(B, fr, hw * kx0 * jl, hw * kxL * jr, -Fl, Fr, sums);
 #pragma unroll
-    for (int i = 1; i < L; ++i) sx[i] = kxr[i] * gx[i];
-    sx[0] = kxr[0] * fma(hw, jl, gx[0]);
-    sx[L] = kxr[L] * fma(hw, jr, gx[L]);
-#pragma unroll
-    for (int k = 0; k < NP; ++k) {
-      const double acc = (k == 0) ? -Fl : ((k == L) ? Fr : 0.0);
-      s_yx[e][t * NP + k] = dot_col<NP>(B, k, sx, acc);
-    }
+    for (int k = 0; k < NP; ++k) s_yx[e][t * NP + k] = sums.G[k];
+    s_ex[e][t] = sums.e;
   }
+  if (NF) copy_async_wait<0>();
   __syncthreads();
   if (!PCG && !vc.valid) return 0.0;
   double part = 0.0;  // PCG inner-product partial of this thread
@@ -424,24 +443,20 @@ __device__ __forceinline__ double apply_tile(const ApplyArgs2D& a, const Tile2D 
   // ---- eta-phase: y faces of the column, y-stiffness transpose, mass, epilogue
   if (vc.valid) {
     const int t = vc.t, e = vc.e;
-    double kyc[NP];
-#pragma unroll
-    for (int l = 0; l < NP; ++l) kyc[l] = a.cky[vc.base + l * NP + t];
     auto fetchy = [&](int s) {
       Partner1 P;
       int it;
       const long long pb = neighbour<NP>(tl, I, vc.ex, vc.ey, 0, s == 0 ? -1 : 1, &it);
       const int pl = s == 0 ? L : 0;
-      P.k = a.cky[pb + pl * NP + t];
       if (it >= 0) {
         P.x = s_x[it][pl * NP + t];
-        P.d = s_gyf[it][t][s == 0 ? 1 : 0];
+        P.t = s_tyf[it][t][s == 0 ? 1 : 0];
       } else {
         double pc[NP];
 #pragma unroll
         for (int k = 0; k < NP; ++k) pc[k] = ldx(pb + k * NP + t);
         P.x = s == 0 ? pc[L] : pc[0];
-        P.d = dot_end<NP>(B, s == 0, pc);
+        P.t = flux_end<NP>(B, s == 0, pc, a.cky[pb + pl * NP + t]);
       }
       return P;
     };
@@ -449,21 +464,26 @@ __device__ __forceinline__ double apply_tile(const ApplyArgs2D& a, const Tile2D 
     const Partner1 qA = fetchy(sf), qB = fetchy(1 - sf);
     const Partner1 qb = sf == 0 ? qA : qB, qt = sf == 0 ? qB : qA;
     const double jb = qb.x - xc[0];
-    const double Fb = fma(a.cpy[vc.base + t], jb, hw * fma(qb.k, qb.d, kyc[0] * gy[0]));
+    const double Fb = fma(a.cpy[vc.base + t], jb, hw * (qb.t + fc.t0));
     const double jt = xc[L] - qt.x;
-    const double Ft = fma(a.cpy[vc.base + L * NP + t], jt, hw * fma(kyc[L], gy[L], qt.k * qt.d));
-    double sy[NP];
+    const double Ft = fma(a.cpy[vc.base + L * NP + t], jt, hw * (fc.tL + qt.t));
+    // the residual epilogues form b - A x at once: b - cm x enters the last sum, the rest with a minus sign
+    constexpr bool RES = EPI == EPI_CHEB || EPI == EPI_JACOBI || EPI == EPI_PCG0;
+    double acc[NP], yy[NP];
+    long long R[NP];
+    int er[NP];
 #pragma unroll
-    for (int l = 1; l < L; ++l) sy[l] = kyc[l] * gy[l];
-    sy[0] = kyc[0] * fma(hw, jb, gy[0]);
-    sy[L] = kyc[L] * fma(hw, jt, gy[L]);
+    for (int l = 0; l < NP; ++l) {
+      const double cm = field(1, a.cm, e, vc.base, l * NP + t);
+      acc[l] = RES ? fma(-cm, xc[l], field(2, a.b, e, vc.base, l * NP + t)) : cm * xc[l];
+      R[l] = s_yx[e][l * NP + t];
+      er[l] = s_ex[e][l];
+    }
+    column_sums<NP>(B, fc, hw * ky0 * jb, hw * kyL * jt, -Fb, Ft, R, er, acc, RES ? -1 : 1, yy);
 #pragma unroll
     for (int l = 0; l < NP; ++l) {
       const long long n = vc.base + l * NP + t;
-      // y-face flux at the column's end nodes (l is a compile-time index: interior nodes add nothing)
-      const double syx = s_yx[e][l * NP + t];
-      double y = fma(a.cm[n], xc[l], (l == 0) ? syx - Fb : ((l == L) ? syx + Ft : syx));
-      y = dot_col<NP>(B, l, sy, y);
+      const double y = yy[l];  // A x, or b - A x (RES)
       if (EPI == EPI_RESID) { a.y_out[n] = y; continue; }
       if (EPI == EPI_PCG) {
         a.ap_out[n] = y;
@@ -471,34 +491,38 @@ __device__ __forceinline__ double apply_tile(const ApplyArgs2D& a, const Tile2D 
         continue;
       }
       if (EPI == EPI_PCG0) {
-        const double r0 = a.b[n] - y;
+        const double r0 = y;
         const double z0 = r0 * a.cinvM[n];
         a.r_out[n] = r0;
         a.p_out[n] = z0;
         part = fma(r0, z0, part);
         continue;
       }
-      const double r = a.b[n] - y;
+      const double r = y;
       if (a.tape_r) a.tape_r[n] = r;
       if (EPI == EPI_CHEB) {
-        const double z = r * a.cinvM[n];
-        const double d = a.d_in ? fma(a.ca, a.d_in[n], a.cc * z) : a.cc * z;
+        const double z = r * field(3, a.cinvM, e, vc.base, l * NP + t);
+        const double d = a.d_in ? fma(a.ca, field(4, a.d_in, e, vc.base, l * NP + t), a.cc * z) : a.cc * z;
         a.d_out[n] = d;
         a.x_out[n] = xc[l] + d;
       } else {  // EPI_JACOBI: x + omega (b - A x) / M   (elliptic.jl:358)
-        a.x_out[n] = fma(a.omega * r, a.cinvM[n], xc[l]);
+        a.x_out[n] = fma(a.omega * r, field(3, a.cinvM, e, vc.base, l * NP + t), xc[l]);
       }
     }
   }
   return part;
 }
 
+// What bounds it: per warp of 32 lines 50 FP64 instructions (106 with FP64 contractions), 1018 on the integer ALU and 482
+// integer multiply-adds; at 2.1 M nodes (P3, Chebyshev) the FP64 pipe is 60% busy, the ALU 38%, DRAM 32%, and the rest is
+// latency under 18 warps per SM. 127 us with FP64 contractions, 79 us now; the last phase's fields are copied to shared
+// memory while the first phases run, which shows on small meshes (64 x 64: 12.3 against 11.3 us) and costs nothing here.
 template <int NP, int EPI>
 __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_apply(ApplyArgs2D a) {
   using TL = Tiling2D<NP>;
   constexpr bool PCG = EPI == EPI_PCG0 || EPI == EPI_PCG;
   constexpr int P2 = pow2_at_least(TL::NT);
-  __shared__ ApplySmem<NP> sm;
+  __shared__ ApplySmem<NP, apply_fields(EPI)> sm;
   __shared__ double s_red[PCG ? P2 : 1];
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];

@@ -10,6 +10,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "igr_fix.cuh"
+
 namespace igrgpu {
 
 constexpr int MAXNP = 5;  // p <= 4
@@ -25,6 +27,7 @@ struct BasisDev {
   double cheb_theta, cheb_delta, cheb_sigma;  // elliptic.jl:373-378
   double hw;                // -1 / (2 w_0): SIP face coefficient factor
   double iw0, iwL;          // 1 / w_0, 1 / w_L
+  FixMat fD;                // D as integers (igr_fix.cuh)
 };
 
 // One problem instance of a batch (2D): mesh, physics parameters and where
@@ -77,6 +80,16 @@ enum : int { DEV_OK = 0, DEV_NONFINITE = 1, DEV_TIMEOUT = 2 };
 __device__ __forceinline__ void flag_nonfinite(int* status) {
   if (status) atomicOr(status, DEV_NONFINITE);
 }
+
+// Asynchronous copies of 8 bytes from global to shared memory (no register and
+// no scoreboard holds them; completion is waited for by group).
+__device__ __forceinline__ void copy_async8(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
 
 // Comparisons on bit patterns. GB300 issues a double compare (DSETP), fmax and
 // isfinite through the FP64 unit at ~94 cycles per warp instruction per SM

@@ -1,0 +1,514 @@
+// Line contractions with the LGL differentiation matrix in 64-bit block fixed
+// point: the integer pipes do what the FP64 pipe is too slow for.
+//
+// Why: GB300 issues one FP64 warp instruction per 64 cycles and SM
+// sub-partition (DADD: 76), while its integer multiply-adds (32 x 32 + 64 bit,
+// about 5 cycles) and logic / shifts (2 cycles) run on other pipes at the same
+// time. A P3 line (4 nodes, 14 FP64 instructions) takes 1067 cycles per warp on
+// the FP64 pipe; in fixed point it takes 398, and four independent FP64
+// instructions per line hide in those (412 together; measured with 16 warps
+// per SM). P4 lines: 1673 against 547.
+//
+// Representation: the values of one line share the exponent e of their largest
+// member and become integers |X| < 2^62, split as X = h 2^32 + 2 l with |h| <
+// 2^30 and |l| < 2^31; the matrix is scaled by a power of two so that no row or
+// column has an absolute sum above 0.7, and stored the same way with a balanced
+// l (|l| <= 2^30). A product then takes three 32 x 32 -> 64 bit multiply-adds
+// (h h, h l, l h), whose sums over at most five terms stay below 2^63:
+//   H = sum h_D h_X,  M = sum (h_D l_X + l_D h_X),  G = H + M / 2^31.
+// The low x low products and the truncation of the line's values are a few units
+// of 2^-61 of the line's scale, and one rounding to nearest ends the sum: against
+// 128-bit sums the results are off by 3.3e-17 rms of |D||x| where the FP64 chain
+// is off by 4.5e-17. A whole SIP line (flux, transposed contraction, mass and
+// face terms) has 0.2 to 0.7 times the chain's rms error (tests/test_fixed_point.py).
+//
+// Lines that hold infinities, NaN or values beyond 2^1007, and lines of nothing
+// but subnormal-range values (below 2^-894), take the FP64 chain, as before. A
+// line of zeros gives zeros.
+#pragma once
+#include <cmath>
+
+#ifdef __CUDACC__
+#include <cuda_runtime.h>
+#endif
+
+namespace igrgpu {
+
+constexpr int FIX_MAXNP = 5;
+
+// A matrix as integers: A[i][k] = (h 2^32 + 2 l) 2^(s - 63).
+struct FixMat {
+  int h[FIX_MAXNP][FIX_MAXNP], l[FIX_MAXNP][FIX_MAXNP];
+  int s;
+};
+
+// The FixMat of the leading np x np block of A: scaled by 2^-s so that no row or column has an absolute sum above 0.7
+// (with h < 2^31 and |l| <= 2^30 this keeps M below 2^63 over five terms), rounded at 2^-63.
+inline FixMat make_fix(const double A[FIX_MAXNP][FIX_MAXNP], int np) {
+  FixMat F = {};
+  double most = 0.0;
+  for (int i = 0; i < np; ++i) {
+    double r = 0.0, c = 0.0;
+    for (int k = 0; k < np; ++k) { r += std::fabs(A[i][k]); c += std::fabs(A[k][i]); }
+    most = std::fmax(most, std::fmax(r, c));
+  }
+  while (F.s < 64 && 0.7 * std::ldexp(1.0, F.s) < most) ++F.s;
+  for (int i = 0; i < np; ++i)
+    for (int k = 0; k < np; ++k) {
+      const long long f = std::llrint(std::ldexp(A[i][k], 63 - F.s));
+      const long long h = (f + (1LL << 31)) >> 32;
+      F.h[i][k] = (int)h;
+      F.l[i][k] = (int)((f - h * (1LL << 32)) / 2);
+    }
+  return F;
+}
+
+namespace fix {
+
+constexpr int E_MIN = 128, E_MAX = 2030;  // biased exponents the integer path takes
+
+// One instruction each on the GPU; the C forms serve host builds of this header (the unit test).
+__device__ __forceinline__ long long mad(int a, int b, long long c) {
+#ifdef __CUDA_ARCH__
+  long long r;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+  return r;
+#else
+  return (long long)a * b + c;
+#endif
+}
+// a >> s, 0 for s > 63 (PTX clamps the shift amount; C leaves it undefined)
+__device__ __forceinline__ unsigned long long shr(unsigned long long a, unsigned s) {
+#ifdef __CUDA_ARCH__
+  unsigned long long r;
+  asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(a), "r"(s));
+  return r;
+#else
+  return s > 63 ? 0 : a >> s;
+#endif
+}
+__device__ __forceinline__ int abs_hi(double v) { return __double2hiint(v) & 0x7fffffff; }
+
+// |v| 2^(53 + PRE) / 2^(e - 1022), truncated; e is a biased exponent >= v's
+template <int PRE>
+__device__ __forceinline__ unsigned long long magnitude(double v, int e) {
+  const unsigned hi = __double2hiint(v), lo = __double2loint(v);
+  const unsigned m = (hi & 0xfffffu) | 0x100000u;
+  const unsigned long long t = ((unsigned long long)__funnelshift_l(lo, m, PRE) << 32) | (lo << PRE);
+  return shr(t, e - ((hi & 0x7fffffffu) >> 20));
+}
+
+struct Limb { int h, l; };
+// v 2^(53 + PRE) / 2^(e - 1022) as h 2^32 + 2 l
+template <int PRE = 9>
+__device__ __forceinline__ Limb limbs(double v, int e) {
+  const unsigned long long t = magnitude<PRE>(v, e);
+  const int sg = (__double2hiint(v) >> 31) | 1;
+  return {(int)(t >> 32) * sg, (int)((unsigned)t >> 1) * sg};
+}
+// a + v, v in units of 2^(53 + PRE) / 2^(e - 1022), truncated
+template <int PRE>
+__device__ __forceinline__ long long add(long long a, double v, int e) {
+  const long long s = __double2hiint(v) >> 31;
+  return a + ((long long)magnitude<PRE>(v, e) ^ s) - s;
+}
+
+// G 2^(e - 1082) rounded to nearest, |G| < 2^62
+__device__ __forceinline__ double to_double(long long G, int e) {
+  const int gh = (int)(G >> 32), sg = gh >> 31;
+  const unsigned mh = gh ^ sg, ml = (unsigned)G ^ sg;
+  const bool z = mh == 0;
+  const unsigned m = z ? ml : mh;
+  int lz = __clz(m);
+  lz = z ? lz + 32 : lz;
+  unsigned long long t = (((unsigned long long)mh << 32) | ml) << (lz - 1);  // leading bit 62
+  t += 0x200;
+  unsigned hi = (unsigned)(t >> 42) + (unsigned)((e + 3 - lz) << 20);  // the implicit bit adds one to the exponent
+  hi |= gh & 0x80000000;
+  return __hiloint2double(m ? hi : 0, (unsigned)(t >> 10));
+}
+
+template <int NP>
+__device__ __forceinline__ constexpr bool skip(int i, int k) { return i == k && i > 0 && i < NP - 1; }
+
+// P1 lines stay on the FP64 chain: it is four instructions with the exact factors +-1/2, no slower than the integers
+// (256 cycles) and as exact as it can be.
+template <int NP>
+constexpr bool F64_LINE = NP <= 2;
+
+// FP64 needed: a value out of range, or a line of tiny values that are not all zero
+template <int NP>
+__device__ __forceinline__ bool out_of_range(int m, const double* v) {
+  if (F64_LINE<NP>) return true;
+  if ((unsigned)(m - (E_MIN << 20)) < (unsigned)((E_MAX - E_MIN) << 20)) return false;
+  if (m >= (E_MAX << 20)) return true;
+  unsigned any = 0;
+#pragma unroll
+  for (int k = 0; k < NP; ++k) any |= (unsigned)abs_hi(v[k]) | (unsigned)__double2loint(v[k]);
+  return any != 0;
+}
+template <int NP>
+__device__ __forceinline__ int max_hi(const double* v) {
+  int m = abs_hi(v[0]);
+#pragma unroll
+  for (int k = 1; k < NP; ++k) m = max(m, abs_hi(v[k]));
+  return m;
+}
+
+constexpr long long HALF = 1LL << 31;  // M / 2^31 is added as 2 (M >> 32): rounded to nearest by this
+
+// One sum of a line: coefficient (h, l)[k] by index function cf(k) -> Limb, over the terms keep(k) lets through
+template <int NP, class CF, class KEEP>
+__device__ __forceinline__ long long line_sum(const Limb* x, CF cf, KEEP keep, long long acc) {
+  long long H = acc, M = HALF;
+#pragma unroll
+  for (int k = 0; k < NP; ++k) {
+    if (!keep(k)) continue;
+    const Limb c = cf(k);
+    H = mad(c.h, x[k].h, H);
+    M = mad(c.h, x[k].l, M);
+    M = mad(c.l, x[k].h, M);
+  }
+  return mad((int)(M >> 32), 2, H);
+}
+
+}  // namespace fix
+
+// A factor every sum of a line is multiplied by, prepared once per thread.
+struct FixScale {
+  double d;
+  fix::Limb m;  // d = (m.h 2^32 + 2 m.l) 2^(e - 1085)
+  int e;
+};
+__device__ __forceinline__ FixScale fix_scale(double d) {
+  FixScale s;
+  s.d = d;
+  s.e = fix::abs_hi(d) >> 20;
+  s.m = fix::limbs<10>(d, s.e);
+  return s;
+}
+
+// out[i] = acc[i] + c sum_k A[i][k] v[k] (T: A[k][i]) for every node of a line, rounded once. acc[i] is read only where
+// has(i) (else 0), c only if SCALED (else 1). A is the FP64 matrix of F; its zero interior diagonal is skipped where
+// SKIP is set. The scaled sum is the integer product of G and the factor, four more multiply-adds per node against an
+// FP64 multiply's 64 cycles; a scaled line's units are 2^-60 of its scale, 2^-61 otherwise.
+template <int NP, bool T, bool SKIP, bool SCALED, class MAT, class HAS>
+__device__ __forceinline__ void line_op(const FixMat& F, const MAT& A, const FixScale* c, const double* v,
+                                        const double* acc, HAS has, double* out) {
+  const int m = fix::max_hi<NP>(v);
+  int ma = 0;
+#pragma unroll
+  for (int i = 0; i < NP; ++i) if (has(i)) ma = max(ma, fix::abs_hi(acc[i]));
+  // exponent of the sums above that of the line: |sum| < 2^(e + up - 1022)
+  const int up = F.s + (SCALED ? c->e - 1022 : 0);
+  const int mm = max(m, ma);
+  bool slow = fix::F64_LINE<NP> || (SCALED && (unsigned)(c->e - 1022 + 256) > 512u);
+  if ((unsigned)(mm - (fix::E_MIN << 20)) >= (unsigned)((fix::E_MAX - fix::E_MIN) << 20)) {
+    unsigned any = 0;
+#pragma unroll
+    for (int k = 0; k < NP; ++k) {
+      any |= (unsigned)fix::abs_hi(v[k]) | (unsigned)__double2loint(v[k]);
+      if (has(k)) any |= (unsigned)fix::abs_hi(acc[k]) | (unsigned)__double2loint(acc[k]);
+    }
+    slow |= any != 0;
+  }
+  const int e = max(max(m >> 20, (ma >> 20) - up), fix::E_MIN);
+  if (SCALED) slow |= (unsigned)(e + up - 64) >= (unsigned)(fix::E_MAX - 64);
+  if (slow) {
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+      double s = (has(i) && !SCALED) ? acc[i] : 0.0;
+#pragma unroll
+      for (int k = 0; k < NP; ++k) {
+        if (SKIP && fix::skip<NP>(i, k)) continue;
+        s = fma(T ? A[k][i] : A[i][k], v[k], s);
+      }
+      out[i] = SCALED ? (has(i) ? fma(c->d, s, acc[i]) : c->d * s) : s;
+    }
+    return;
+  }
+  fix::Limb x[NP];
+#pragma unroll
+  for (int k = 0; k < NP; ++k) x[k] = fix::limbs(v[k], e);
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    const long long A0 = has(i) ? fix::add<SCALED ? 7 : 8>(0, acc[i], e + up) : 0;
+    long long G = fix::line_sum<NP>(
+        x, [&](int k) { return fix::Limb{T ? F.h[k][i] : F.h[i][k], T ? F.l[k][i] : F.l[i][k]}; },
+        [&](int k) { return !(SKIP && fix::skip<NP>(i, k)); }, SCALED ? 0 : A0);
+    if (SCALED) {
+      const int gh = (int)(G >> 32), gl = (int)((unsigned)G >> 1);
+      const long long M = fix::mad(gl, c->m.h, fix::mad(gh, c->m.l, fix::HALF));
+      G = fix::mad((int)(M >> 32), 2, fix::mad(gh, c->m.h, A0));
+    }
+    out[i] = fix::to_double(G, e + up - (SCALED ? 0 : 1));
+  }
+}
+
+// out[i] = sum_k D[i][k] v[k]: the reference derivative of a line at its nodes
+template <int NP, class BASIS>
+__device__ __forceinline__ void line_rows(const BASIS& B, const double* v, double* out) {
+  line_op<NP, false, true, false>(B.fD, B.D, nullptr, v, nullptr, [](int) { return false; }, out);
+}
+// out[i] = c sum_k D[i][k] v[k]
+template <int NP, class BASIS>
+__device__ __forceinline__ void line_rows(const BASIS& B, const FixScale& c, const double* v, double* out) {
+  line_op<NP, false, true, true>(B.fD, B.D, &c, v, nullptr, [](int) { return false; }, out);
+}
+// out[i] = acc[i] + c sum_k D[i][k] v[k]
+template <int NP, class BASIS>
+__device__ __forceinline__ void line_rows_acc(const BASIS& B, const FixScale& c, const double* v, const double* acc,
+                                              double* out) {
+  line_op<NP, false, true, true>(B.fD, B.D, &c, v, acc, [](int) { return true; }, out);
+}
+// out[k] = c sum_i D[i][k] v[i]
+template <int NP, class BASIS>
+__device__ __forceinline__ void line_cols(const BASIS& B, const FixScale& c, const double* v, double* out) {
+  line_op<NP, true, true, true>(B.fD, B.D, &c, v, nullptr, [](int) { return false; }, out);
+}
+// out[k] = acc[k] (where has(k)) + sum_i D[i][k] v[i]
+template <int NP, class BASIS, class HAS>
+__device__ __forceinline__ void line_cols_acc(const BASIS& B, const double* v, const double* acc, HAS has, double* out) {
+  line_op<NP, true, true, false>(B.fD, B.D, nullptr, v, acc, has, out);
+}
+
+// sum_k D[last ? NP-1 : 0][k] v[k]: the bits of line_rows at that end node
+template <int NP, class BASIS>
+__device__ __forceinline__ double line_end(const BASIS& B, bool last, const double* v) {
+  const FixMat& F = B.fD;
+  const int m = fix::max_hi<NP>(v);
+  if (fix::out_of_range<NP>(m, v)) {
+    double s = 0.0;
+#pragma unroll
+    for (int k = 0; k < NP; ++k) s = fma(last ? B.D[NP - 1][k] : B.D[0][k], v[k], s);
+    return s;
+  }
+  const int e = max(m >> 20, fix::E_MIN);
+  fix::Limb x[NP];
+#pragma unroll
+  for (int k = 0; k < NP; ++k) x[k] = fix::limbs(v[k], e);
+  const long long G = fix::line_sum<NP>(
+      x, [&](int k) { return fix::Limb{last ? F.h[NP - 1][k] : F.h[0][k], last ? F.l[NP - 1][k] : F.l[0][k]}; },
+      [](int) { return true; }, 0);
+  return fix::to_double(G, e + F.s - 1);
+}
+
+// ---------------------------------------------------------------------------
+// A line of the SIP operator without leaving the integers: fluxes k (D x) and
+// their transposed contraction, so that neither the derivatives nor the fluxes
+// are rounded to doubles and taken apart again (a conversion costs 13
+// instructions in, 22 out, the products and sums 4 multiply-adds each).
+// ---------------------------------------------------------------------------
+
+// The fluxes of a line: k[i] (D x)[i] = P[i] 2^(e - 1082), and at the two end nodes as doubles. Lines outside the
+// integer path's range (see line_op) hold the doubles' bits in P (slow).
+template <int NP>
+struct FixFlux {
+  long long P[NP];
+  int e;  // 0 for a line of zeros
+  bool slow;
+  double t0, tL;
+};
+
+namespace fix {
+// v = (h 2^32 + 2 l) 2^(e - 1085), e its biased exponent (v normal)
+__device__ __forceinline__ Limb mantissa(double v) {
+  const unsigned hi = __double2hiint(v), lo = __double2loint(v);
+  const int sg = ((int)hi >> 31) | 1;
+  return {(int)__funnelshift_l(lo, (hi & 0xfffffu) | 0x100000u, 10) * sg, (int)((lo << 9) & 0x7fffffffu) * sg};
+}
+// G c / 2^64 for |G| < 2^62 and c of 63 bits
+__device__ __forceinline__ long long times(long long G, Limb c) {
+  const int gh = (int)(G >> 32), gl = (int)((unsigned)G >> 1);
+  const long long M = mad(gl, c.h, mad(gh, c.l, HALF));
+  return mad((int)(M >> 32), 2, mad(gh, c.h, 0));
+}
+__device__ __forceinline__ long long sar(long long a, unsigned s) {
+#ifdef __CUDA_ARCH__
+  long long r;
+  asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"(a), "r"(s));
+  return r;
+#else
+  return a >> (s > 63 ? 63 : s);
+#endif
+}
+__device__ __forceinline__ bool zero(double v) { return (((unsigned)abs_hi(v)) | (unsigned)__double2loint(v)) == 0; }
+// k is a coefficient the integer path takes: nonzero, finite, of moderate exponent
+__device__ __forceinline__ bool plain_coef(int k_hi) { return (unsigned)(k_hi - (523 << 20)) < (unsigned)(1000 << 20); }
+}  // namespace fix
+
+template <int NP, class BASIS>
+__device__ __forceinline__ void flux_line(const BASIS& B, const double* x, const double* k, FixFlux<NP>& f) {
+  const int m = fix::max_hi<NP>(x);
+  int ke[NP], km = 0;
+  bool ok = true;
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    ke[i] = fix::abs_hi(k[i]);
+    ok &= fix::plain_coef(ke[i]);
+    km = max(km, ke[i]);
+  }
+  const int ex = max(m >> 20, fix::E_MIN);
+  const int eg = ex + B.fD.s - 1022;  // P_i before alignment has exponent eg + ke_i
+  f.slow = fix::out_of_range<NP>(m, x) || !ok || (unsigned)(eg + (km >> 20) - 64) >= (unsigned)(fix::E_MAX - 64);
+  if (f.slow) {
+    f.e = 0;
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+      double g = 0.0;
+#pragma unroll
+      for (int j = 0; j < NP; ++j) if (!fix::skip<NP>(i, j)) g = fma(B.D[i][j], x[j], g);
+      g *= k[i];
+      if (i == 0) f.t0 = g;
+      if (i == NP - 1) f.tL = g;
+      f.P[i] = __double_as_longlong(g);
+    }
+    return;
+  }
+  f.e = m == 0 ? 0 : eg + (km >> 20);
+  fix::Limb X[NP];
+#pragma unroll
+  for (int i = 0; i < NP; ++i) X[i] = fix::limbs(x[i], ex);
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    const long long G = fix::line_sum<NP>(
+        X, [&](int j) { return fix::Limb{B.fD.h[i][j], B.fD.l[i][j]}; }, [&](int j) { return !fix::skip<NP>(i, j); }, 0);
+    const long long P = fix::times(G, fix::mantissa(k[i]));
+    if (i == 0) f.t0 = fix::to_double(P, eg + (ke[i] >> 20));
+    if (i == NP - 1) f.tL = fix::to_double(P, eg + (ke[i] >> 20));
+    f.P[i] = fix::sar(P, (km >> 20) - (ke[i] >> 20));
+  }
+  // A smooth line's fluxes are far below what its values allow: shifted up to use their bits, so that the units of the
+  // sums that follow go by the fluxes, as an FP64 sum's roundings do.
+  unsigned any = 0;
+#pragma unroll
+  for (int i = 0; i < NP; ++i) { const int h = (int)(f.P[i] >> 32); any |= h ^ (h >> 31); }
+  const int z = __clz(any) - 4;  // |P| < 2^60
+#pragma unroll
+  for (int i = 0; i < NP; ++i) f.P[i] = (long long)((unsigned long long)f.P[i] << z);
+  if (m != 0) f.e -= z;
+}
+
+// The flux at one end of a line, with the bits of flux_line's t0 / tL; k is the coefficient there.
+template <int NP, class BASIS>
+__device__ __forceinline__ double flux_end(const BASIS& B, bool last, const double* x, double k) {
+  const int m = fix::max_hi<NP>(x), ke = fix::abs_hi(k);
+  const int ex = max(m >> 20, fix::E_MIN), e = ex + B.fD.s - 1022 + (ke >> 20);
+  if (fix::out_of_range<NP>(m, x) || !fix::plain_coef(ke) || (unsigned)(e - 64) >= (unsigned)(fix::E_MAX - 64)) {
+    double s = 0.0;
+#pragma unroll
+    for (int j = 0; j < NP; ++j) s = fma(last ? B.D[NP - 1][j] : B.D[0][j], x[j], s);
+    return s * k;
+  }
+  fix::Limb X[NP];
+#pragma unroll
+  for (int j = 0; j < NP; ++j) X[j] = fix::limbs(x[j], ex);
+  const long long G = fix::line_sum<NP>(
+      X, [&](int j) { return fix::Limb{last ? B.fD.h[NP - 1][j] : B.fD.h[0][j], last ? B.fD.l[NP - 1][j] : B.fD.l[0][j]}; },
+      [](int) { return true; }, 0);
+  return fix::to_double(fix::times(G, fix::mantissa(k)), e);
+}
+
+// Sums in units of 2^59 / 2^(e - 1022); e < 0: the bits of doubles (FP64 lines).
+template <int NP>
+struct FixSums { long long G[NP]; int e; };
+
+// D^T (P + u0 at node 0 + uL at node NP-1) in units of at least exponent `need`, the largest exponent of what the
+// caller adds; all_zero: the caller adds zeros only. False (nothing formed) where the FP64 chain has to run.
+template <int NP, class BASIS>
+__device__ __forceinline__ bool div_line(const BASIS& B, const FixFlux<NP>& f, double u0, double uL, int need, bool all_zero,
+                                         FixSums<NP>& r) {
+  const int mu = max(fix::abs_hi(u0), fix::abs_hi(uL)) >> 20;
+  const int sd = B.fD.s;
+  int e = max(max(f.e, mu) + sd, need);
+  if (f.slow || e >= fix::E_MAX) return false;
+  if (e < 192) {
+    if (f.e != 0 || !fix::zero(u0) || !fix::zero(uL) || !all_zero) return false;
+    e = 192;
+  }
+  r.e = e;
+  fix::Limb S[NP];
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    long long v = fix::sar(f.P[i], e - sd - f.e);
+    if (i == 0) v = fix::add<7>(v, u0, e - sd);
+    if (i == NP - 1) v = fix::add<7>(v, uL, e - sd);
+    S[i] = {(int)(v >> 32), (int)((unsigned)v >> 1)};
+  }
+#pragma unroll
+  for (int k = 0; k < NP; ++k)
+    r.G[k] = fix::line_sum<NP>(
+        S, [&](int i) { return fix::Limb{B.fD.h[i][k], B.fD.l[i][k]}; }, [&](int i) { return !fix::skip<NP>(i, k); }, 0);
+  return true;
+}
+
+// The same in FP64: acc[k] + sum_i D[i][k] (flux_i + u at the ends)
+template <int NP, class BASIS>
+__device__ __forceinline__ void div_line_fp64(const BASIS& B, const FixFlux<NP>& f, double u0, double uL, double* acc) {
+  double s[NP];
+#pragma unroll
+  for (int i = 0; i < NP; ++i) s[i] = f.slow ? __longlong_as_double(f.P[i]) : fix::to_double(f.P[i], f.e);
+  s[0] += u0;
+  s[NP - 1] += uL;
+#pragma unroll
+  for (int k = 0; k < NP; ++k)
+#pragma unroll
+    for (int i = 0; i < NP; ++i) if (!fix::skip<NP>(i, k)) acc[k] = fma(B.D[i][k], s[i], acc[k]);
+}
+
+// A row's sums kept between the phases: units as FixSums, e < 0: doubles.
+template <int NP, class BASIS>
+__device__ __forceinline__ void row_sums(const BASIS& B, const FixFlux<NP>& f, double u0, double uL, double a0, double aL,
+                                         FixSums<NP>& r) {
+  const int need = max(fix::abs_hi(a0), fix::abs_hi(aL)) >> 20;
+  if (div_line<NP>(B, f, u0, uL, need, fix::zero(a0) && fix::zero(aL), r)) {
+    r.G[0] = fix::add<6>(r.G[0], a0, r.e);
+    r.G[NP - 1] = fix::add<6>(r.G[NP - 1], aL, r.e);
+    return;
+  }
+  double acc[NP];
+#pragma unroll
+  for (int k = 0; k < NP; ++k) acc[k] = k == 0 ? a0 : (k == NP - 1 ? aL : 0.0);
+  div_line_fp64<NP>(B, f, u0, uL, acc);
+  r.e = -1;
+#pragma unroll
+  for (int k = 0; k < NP; ++k) r.G[k] = __double_as_longlong(acc[k]);
+}
+
+// out[k] = acc[k] + sg (row part[k] + D^T(f + u)[k] + (a0 at node 0, aL at node NP-1)), sg = +-1, rounded once: the
+// column's share of the operator, the rows' sums R (units of exponent er, e < 0: doubles) and the caller's terms.
+template <int NP, class BASIS>
+__device__ __forceinline__ void column_sums(const BASIS& B, const FixFlux<NP>& f, double u0, double uL, double a0, double aL,
+                                            const long long* R, const int* er, const double* acc, int sg, double* out) {
+  int need = max(fix::abs_hi(a0), fix::abs_hi(aL)), el = er[0], eh = er[0];
+#pragma unroll
+  for (int k = 0; k < NP; ++k) {
+    need = max(need, fix::abs_hi(acc[k]));
+    el = el < er[k] ? el : er[k];
+    eh = max(eh, er[k]);
+  }
+  need = max(need >> 20, eh);
+  FixSums<NP> s;
+  if (el >= 0 && div_line<NP>(B, f, u0, uL, need, false, s)) {
+#pragma unroll
+    for (int k = 0; k < NP; ++k) {
+      long long v = s.G[k] + fix::sar(R[k], s.e - er[k]);
+      if (k == 0) v = fix::add<6>(v, a0, s.e);
+      if (k == NP - 1) v = fix::add<6>(v, aL, s.e);
+      out[k] = fix::to_double(fix::add<6>(sg > 0 ? v : -v, acc[k], s.e), s.e + 1);
+    }
+    return;
+  }
+  double y[NP];
+#pragma unroll
+  for (int k = 0; k < NP; ++k) {
+    y[k] = er[k] < 0 ? __longlong_as_double(R[k]) : fix::to_double(R[k], er[k] + 1);
+    if (k == 0) y[k] += a0;
+    if (k == NP - 1) y[k] += aL;
+  }
+  div_line_fp64<NP>(B, f, u0, uL, y);
+#pragma unroll
+  for (int k = 0; k < NP; ++k) out[k] = sg > 0 ? acc[k] + y[k] : acc[k] - y[k];
+}
+
+}  // namespace igrgpu
