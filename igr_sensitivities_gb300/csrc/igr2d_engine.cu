@@ -320,19 +320,12 @@ struct StageBuf {
   // scal = per-instance rz_0..rz_n, pAp_0..pAp_{n-1}, alpha_0..alpha_{n-1},
   // beta_0..beta_{n-1} (pcg_scal_count).
   std::vector<double*> xk, rk;
-  std::vector<double*> gxk, gyk;  // taped reference derivatives of the iterates (optional)
   std::vector<double*> pk, apk;
   double* x0t = nullptr;
   double* scal = nullptr;
 };
 
 constexpr int STAGE_FIXED_FIELDS = 16;  // q(4) invr Sout b cm ckx cky cinvM cpx cpy cM wsx wsy
-// Taping the reference derivatives of the Jacobi / Chebyshev iterates saves
-// two line contractions per reverse apply but adds two fields per iteration to
-// the tape; on the 32 x 128^2 P3 Chebyshev-5 adjoint the smaller tape (more
-// instances per group) measured faster (3.77 vs 3.59 gradients/s), so the
-// reverse recomputes them.
-constexpr bool TAPE_ITERATE_DERIVATIVES = false;
 
 // Per-instance scalars of one PCG solve: rz (n + 1), pAp, alpha, beta (n each).
 static long long pcg_scal_count(int n_iter, int ni) { return (long long)(4 * n_iter + 1) * ni; }
@@ -345,7 +338,7 @@ static int pcg_scal_fields(const Solve2DOpts& o, long long NG, int ni) {
 int stage_fields2d(const Solve2DOpts& o, bool alpha_pos, long long NG, int ni) {
   if (!alpha_pos) return STAGE_FIXED_FIELDS;
   if (o.solver == SOLVER_PCG) return STAGE_FIXED_FIELDS + 1 + (o.n_iter + 1) + 2 * o.n_iter + pcg_scal_fields(o, NG, ni);
-  return STAGE_FIXED_FIELDS + (TAPE_ITERATE_DERIVATIVES ? 4 : 2) * o.n_iter;
+  return STAGE_FIXED_FIELDS + 2 * o.n_iter;
 }
 
 static StageBuf stage_from(double* base, long long NG, const Solve2DOpts& o, bool alpha_pos, bool taped, int ni) {
@@ -367,10 +360,6 @@ static StageBuf stage_from(double* base, long long NG, const Solve2DOpts& o, boo
     } else {
       for (int k = 0; k < o.n_iter; ++k) s.xk.push_back(nxt());
       for (int k = 0; k < o.n_iter; ++k) s.rk.push_back(nxt());
-      if (TAPE_ITERATE_DERIVATIVES) {
-        for (int k = 0; k < o.n_iter; ++k) s.gxk.push_back(nxt());
-        for (int k = 0; k < o.n_iter; ++k) s.gyk.push_back(nxt());
-      }
     }
   }
   return s;
@@ -677,8 +666,6 @@ static void stage_solve_b(Ctx& c, const Plan2D& P, const Solve2DOpts& o, StageBu
     if (taped) {
       a.tape_x = st.xk.empty() ? nullptr : st.xk[k];
       a.tape_r = st.rk.empty() ? nullptr : st.rk[k];
-      a.tape_gx = st.gxk.empty() ? nullptr : st.gxk[k];
-      a.tape_gy = st.gyk.empty() ? nullptr : st.gyk[k];
     }
     a.ca = ca[k + 1]; a.cc = cc[k + 1];
     a.omega = 2.0 / 3.0;
@@ -1494,8 +1481,6 @@ void adjoint2d(Ctx& c, const Plan2D& P, const double* const q0[4], int n_steps, 
         std::memset(&r, 0, sizeof(r));
         r.tiles = P.d_tiles; r.inst = P.d_inst; r.B = P.B;
         r.u = U[cur]; r.xk = st[s].xk[m];
-        r.gxk = st[s].gxk.empty() ? nullptr : st[s].gxk[m];
-        r.gyk = st[s].gyk.empty() ? nullptr : st[s].gyk[m];
         r.cm = st[s].cm; r.ckx = st[s].ckx; r.cky = st[s].cky; r.cpx = st[s].cpx; r.cpy = st[s].cpy; r.cinvM = st[s].cinvM;
         r.invr = st[s].invr;
         r.xb = Sb; r.bb = bb; r.Zm = Zm; r.Zs = Zs;

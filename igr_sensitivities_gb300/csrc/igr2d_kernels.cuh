@@ -290,7 +290,6 @@ struct ApplyArgs2D {
   const double* d_in;                    // Chebyshev d_k (null on the first iteration)
   double *d_out, *x_out;                 // d_{k+1}, x_{k+1}
   double *tape_x, *tape_r;               // optional tape of x_k and r_k = b - A x_k
-  double *tape_gx, *tape_gy;             // optional tape of the reference derivatives of x_k
   double *y_out;                         // EPI_RESID: raw y = A x
   double ca, cc, omega;                  // d_{k+1} = ca d_k + cc M^-1 r_k ; Jacobi omega
   // Jacobi-preconditioned CG (pcg_fixed!, elliptic.jl:329-347):

@@ -321,7 +321,6 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_hyp_rev(HypRevArgs2D a) {
 struct ApplyRevArgs2D {
   const Tile2D* tiles; const Inst2D* inst; BasisDev B;
   const double *u, *xk;               // residual adjoint and taped iterate
-  const double *gxk, *gyk;            // taped reference derivatives of x_k (null: recompute)
   const double *cm, *ckx, *cky, *cpx, *cpy, *cinvM, *invr;
   double *xb, *bb, *Zm, *Zs;
   int first;                          // first reverse apply of this solve: write Zm, Zs (else add)
@@ -343,18 +342,24 @@ struct ApplyRevArgs2D {
   InstSum isum;
 };
 
-// Partner data across one face for the reverse apply: values and end-node
-// derivatives of u and of x_k, the partner's stiffness coefficient and 1/rho.
-struct Partner2 { double u, v, du, dv, k, ir; };
+// Partner data across one face for the reverse apply: values of u and x_k, the flux of u at the face node and 1/rho.
+struct Partner2 { double u, v, t, ir; };
 
+// What bounds it: FP64 issue and latency, about evenly. The line contractions, fluxes, coefficient products and sums run
+// on the integer pipes (igr_fix.cuh); 8 x 128^2 P3, Chebyshev: 226 us with FP64 contractions, 138 us now. Eight CTAs per
+// SM for P3 (128 registers): 156 us with the 146 the compiler takes unbounded (7 CTAs), 135 us with nine, which costs
+// a single 64 x 64 instance 7% (17.9 against 16.7 us per launch, 18.9 before).
 template <int NP, int SREV>
-__global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_apply_rev(ApplyRevArgs2D a) {
+__global__ void __launch_bounds__(Tiling2D<NP>::NT, NP == 4 ? 8 : 1) k2_apply_rev(ApplyRevArgs2D a) {
   using TL = Tiling2D<NP>;
-  constexpr int TE = TL::TE, NN = TL::NN, L = TL::L, TX = TL::TX, TY = TL::TY;
+  constexpr int TE = TL::TE, SN = TL::SN, L = TL::L, TX = TL::TX, TY = TL::TY;
   constexpr bool PCG = SREV == SREV_PCG;
   constexpr int P2 = pow2_at_least(TL::NT);
-  __shared__ double s_u[TE][NN], s_v[TE][NN], s_yx[TE][NN], s_zr[TE][NN];
-  __shared__ double s_gxf[2][TE][NP][2], s_gyf[2][TE][NP][2];  // [u|v] face derivatives
+  __shared__ __align__(16) double s_u[TE][SN], s_v[TE][SN];
+  __shared__ __align__(16) long long s_yx[TE][SN], s_zr[TE][SN];  // row sums and products (fixed point)
+  __shared__ int s_ey[TE][NP], s_ez[TE][NP];                      // their exponents
+  __shared__ double s_tx[TE][NP][2], s_ty[TE][NP][2];             // end-node fluxes of u
+  __shared__ __align__(16) double s_f[3][TE][SN];                 // cky, cm, xb, copied while the row phase runs
   __shared__ double s_red[PCG ? P2 : 1];
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];
@@ -371,176 +376,168 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_apply_rev(ApplyRevArgs2D 
     if (PCG) return fma(pal, a.u[n], -ppb * xkv);
     return a.u[n];
   };
+  if (vr.valid) {
+    const double* src[3] = {a.cky, a.cm, a.xb};
+#pragma unroll
+    for (int f = 0; f < 3; ++f) {
+#pragma unroll
+      for (int i = 0; i < NP; ++i) copy_async8(&s_f[f][vr.e][vr.t * NP + i], src[f] + vr.base + vr.t * NP + i);
+      if (f == 0) copy_async_commit();
+    }
+  }
+  copy_async_commit();
 
-  double ur[NP], vr_[NP], gxu[NP], gxv[NP];
-  const bool taped_g = !PCG && a.gxk != nullptr;
+  // the ends of a row or column: values of u and x_k, the stiffness coefficient of u's jump terms
+  double ur0 = 0.0, urL = 0.0, vr0 = 0.0, vrL = 0.0, kx0 = 0.0, kxL = 0.0;
+  FixFlux<NP> fr;
+  FixDeriv<NP> dr;
   if (vr.valid) {
     const int t = vr.t, e = vr.e;
+    double u[NP], v[NP], k[NP];
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
       const long long n = vr.base + t * NP + i;
-      vr_[i] = a.xk[n]; ur[i] = ldu(n, vr_[i]);
-      s_u[e][t * NP + i] = ur[i]; s_v[e][t * NP + i] = vr_[i];
+      v[i] = a.xk[n]; u[i] = ldu(n, v[i]); k[i] = a.ckx[n];
+      s_u[e][t * NP + i] = u[i]; s_v[e][t * NP + i] = v[i];
     }
-#pragma unroll
-    for (int i = 0; i < NP; ++i) {
-      gxu[i] = dot_row<NP>(B, i, ur);
-      gxv[i] = taped_g ? a.gxk[vr.base + t * NP + i] : dot_row<NP>(B, i, vr_);
-    }
-    s_gxf[0][e][t][0] = gxu[0]; s_gxf[0][e][t][1] = gxu[L];
-    s_gxf[1][e][t][0] = gxv[0]; s_gxf[1][e][t][1] = gxv[L];
+    flux_line<NP>(B, u, k, fr);
+    deriv_line<NP>(B, v, dr);
+    s_tx[e][t][0] = fr.t0; s_tx[e][t][1] = fr.tL;
+    ur0 = u[0]; urL = u[L]; vr0 = v[0]; vrL = v[L]; kx0 = k[0]; kxL = k[L];
   }
+  copy_async_wait<1>();
   __syncthreads();
-  double uc[NP], vc_[NP], gyu[NP], gyv[NP];
+  double uc[NP], vc_[NP], ky0 = 0.0, kyL = 0.0;
+  FixFlux<NP> fc;
+  FixDeriv<NP> dc;
   if (vc.valid) {
     const int t = vc.t, e = vc.e;
+    double k[NP];
 #pragma unroll
-    for (int l = 0; l < NP; ++l) { uc[l] = s_u[e][l * NP + t]; vc_[l] = s_v[e][l * NP + t]; }
-#pragma unroll
-    for (int l = 0; l < NP; ++l) {
-      gyu[l] = dot_row<NP>(B, l, uc);
-      gyv[l] = taped_g ? a.gyk[vc.base + l * NP + t] : dot_row<NP>(B, l, vc_);
-    }
-    s_gyf[0][e][t][0] = gyu[0]; s_gyf[0][e][t][1] = gyu[L];
-    s_gyf[1][e][t][0] = gyv[0]; s_gyf[1][e][t][1] = gyv[L];
+    for (int l = 0; l < NP; ++l) { uc[l] = s_u[e][l * NP + t]; vc_[l] = s_v[e][l * NP + t]; k[l] = s_f[0][e][l * NP + t]; }
+    flux_line<NP>(B, uc, k, fc);
+    deriv_line<NP>(B, vc_, dc);
+    s_ty[e][t][0] = fc.t0; s_ty[e][t][1] = fc.tL;
+    ky0 = k[0]; kyL = k[L];
   }
+  // One face of a line: own end values (uo, vo, stiffness k, flux t0, derivative of x_k gv, 1/rho io, penalty p), the
+  // partner P; s = +1 when the own node is the left side, else -1 (jumps are left minus right). F: the flux terms
+  // (consistency + penalty, as added to the left side), us: the symmetry term hw k [u], z: the coefficient adjoint's
+  // face terms hw k ([u] gv + gu [x_k]) and, where the own 1/rho sets the penalty, p [u] [x_k].
+  auto face = [&](int s, double uo, double vo, double k, double t0, double gv, double io, double p, const Partner2& P,
+                  double& F, double& us, double& z) {
+    const double ju = s > 0 ? uo - P.u : P.u - uo, jv = s > 0 ? vo - P.v : P.v - vo;
+    const double pj = p * ju;
+    F = fma(hw, s > 0 ? t0 + P.t : P.t + t0, pj);
+    us = hw * k * ju;
+    const bool wins = s > 0 ? !gt_nonneg(P.ir, io) : gt_nonneg(io, P.ir);  // the right side wins only when strictly larger
+    z = fma(gv, us, jv * fma(hw, t0, wins ? pj : 0.0));
+  };
   if (vr.valid) {
     // ---- row of vr: x faces
     const int t = vr.t, e = vr.e;
-    double kxr[NP], zr[NP];
-#pragma unroll
-    for (int i = 0; i < NP; ++i) { kxr[i] = a.ckx[vr.base + t * NP + i]; zr[i] = kxr[i] * gxu[i] * gxv[i]; }
     auto fetch = [&](int s) {
       Partner2 P;
       int it;
       const long long pb = neighbour<NP>(tl, I, vr.ex, vr.ey, s == 0 ? -1 : 1, 0, &it);
       const int pi = s == 0 ? L : 0;
-      P.k = a.ckx[pb + t * NP + pi];
       P.ir = a.invr[pb + t * NP + pi];
       if (it >= 0) {
         P.u = s_u[it][t * NP + pi]; P.v = s_v[it][t * NP + pi];
-        P.du = s_gxf[0][it][t][s == 0 ? 1 : 0]; P.dv = s_gxf[1][it][t][s == 0 ? 1 : 0];
+        P.t = s_tx[it][t][s == 0 ? 1 : 0];
       } else {
         double pr[NP];
-        if (taped_g) {
+        P.v = a.xk[pb + t * NP + pi];
 #pragma unroll
-          for (int k = 0; k < NP; ++k) pr[k] = a.u[pb + t * NP + k];
-          P.v = a.xk[pb + t * NP + pi];
-          P.dv = a.gxk[pb + t * NP + pi];
-        } else {
-          double pw[NP];
-#pragma unroll
-          for (int k = 0; k < NP; ++k) { pw[k] = a.xk[pb + t * NP + k]; pr[k] = ldu(pb + t * NP + k, pw[k]); }
-          P.v = s == 0 ? pw[L] : pw[0];
-          P.dv = dot_end<NP>(B, s == 0, pw);
-        }
+        for (int k = 0; k < NP; ++k) pr[k] = ldu(pb + t * NP + k, PCG ? a.xk[pb + t * NP + k] : 0.0);
         P.u = s == 0 ? pr[L] : pr[0];
-        P.du = dot_end<NP>(B, s == 0, pr);
+        P.t = flux_end<NP>(B, s == 0, pr, a.ckx[pb + t * NP + pi]);
       }
       return P;
     };
     const int sf = first_side(vr.ext, TX);
     const Partner2 pA = fetch(sf), pB = fetch(1 - sf);
     const Partner2 pl = sf == 0 ? pA : pB, prt = sf == 0 ? pB : pA;
-    const double irl0 = a.invr[vr.base + t * NP], irlL = a.invr[vr.base + t * NP + L];
-    // left face (own R side, node 0)
-    const double jul = pl.u - ur[0], jvl = pl.v - vr_[0];
-    const double pl_ = a.cpx[vr.base + t * NP];
-    const double Fl = fma(pl_, jul, hw * fma(pl.k, pl.du, kxr[0] * gxu[0]));
-    zr[0] = fma(hw * kxr[0], fma(gxv[0], jul, gxu[0] * jvl), zr[0]);
-    if (gt_nonneg(irl0, pl.ir)) zr[0] = fma(pl_ * jvl, jul, zr[0]);  // R wins only when strictly larger
-    // right face (own L side, node L)
-    const double jur = ur[L] - prt.u, jvr = vr_[L] - prt.v;
-    const double pr_ = a.cpx[vr.base + t * NP + L];
-    const double Fr = fma(pr_, jur, hw * fma(kxr[L], gxu[L], prt.k * prt.du));
-    zr[L] = fma(hw * kxr[L], fma(gxv[L], jur, gxu[L] * jvr), zr[L]);
-    if (!gt_nonneg(prt.ir, irlL)) zr[L] = fma(pr_ * jvr, jur, zr[L]);
-    double sx[NP];
+    double Fl, Fr, us0, usL, z0, zL;
+    const long long n0 = vr.base + t * NP;
+    face(-1, ur0, vr0, kx0, fr.t0, deriv_at<NP>(dr, 0), a.invr[n0], a.cpx[n0], pl, Fl, us0, z0);
+    face(1, urL, vrL, kxL, fr.tL, deriv_at<NP>(dr, L), a.invr[n0 + L], a.cpx[n0 + L], prt, Fr, usL, zL);
+    FixSums<NP> sums;
+    row_products<NP>(fr, dr, z0, zL, sums);
 #pragma unroll
-    for (int i = 1; i < L; ++i) sx[i] = kxr[i] * gxu[i];
-    sx[0] = kxr[0] * fma(hw, jul, gxu[0]);
-    sx[L] = kxr[L] * fma(hw, jur, gxu[L]);
+    for (int k = 0; k < NP; ++k) s_zr[e][t * NP + k] = sums.G[k];
+    s_ez[e][t] = sums.e;
+    row_sums<NP>(B, fr, us0, usL, -Fl, Fr, sums);
 #pragma unroll
-    for (int k = 0; k < NP; ++k) {
-      const double acc = (k == 0) ? -Fl : ((k == L) ? Fr : 0.0);
-      s_yx[e][t * NP + k] = dot_col<NP>(B, k, sx, acc);
-      s_zr[e][t * NP + k] = zr[k];
-    }
+    for (int k = 0; k < NP; ++k) s_yx[e][t * NP + k] = sums.G[k];
+    s_ey[e][t] = sums.e;
   }
+  copy_async_wait<0>();
   __syncthreads();
   if (!PCG && !vc.valid) return;
   double part = 0.0;  // PCG: betab partial of this thread
   // ---- column of vc: y faces, transposes, outputs
   if (vc.valid) {
     const int t = vc.t, e = vc.e;
-    double kyc[NP], zc[NP];
-#pragma unroll
-    for (int l = 0; l < NP; ++l) { kyc[l] = a.cky[vc.base + l * NP + t]; zc[l] = kyc[l] * gyu[l] * gyv[l]; }
     auto fetchy = [&](int s) {
       Partner2 P;
       int it;
       const long long pb = neighbour<NP>(tl, I, vc.ex, vc.ey, 0, s == 0 ? -1 : 1, &it);
       const int pl = s == 0 ? L : 0;
-      P.k = a.cky[pb + pl * NP + t];
       P.ir = a.invr[pb + pl * NP + t];
       if (it >= 0) {
         P.u = s_u[it][pl * NP + t]; P.v = s_v[it][pl * NP + t];
-        P.du = s_gyf[0][it][t][s == 0 ? 1 : 0]; P.dv = s_gyf[1][it][t][s == 0 ? 1 : 0];
+        P.t = s_ty[it][t][s == 0 ? 1 : 0];
       } else {
         double pc[NP];
-        if (taped_g) {
+        P.v = a.xk[pb + pl * NP + t];
 #pragma unroll
-          for (int k = 0; k < NP; ++k) pc[k] = a.u[pb + k * NP + t];
-          P.v = a.xk[pb + pl * NP + t];
-          P.dv = a.gyk[pb + pl * NP + t];
-        } else {
-          double pw[NP];
-#pragma unroll
-          for (int k = 0; k < NP; ++k) { pw[k] = a.xk[pb + k * NP + t]; pc[k] = ldu(pb + k * NP + t, pw[k]); }
-          P.v = s == 0 ? pw[L] : pw[0];
-          P.dv = dot_end<NP>(B, s == 0, pw);
-        }
+        for (int k = 0; k < NP; ++k) pc[k] = ldu(pb + k * NP + t, PCG ? a.xk[pb + k * NP + t] : 0.0);
         P.u = s == 0 ? pc[L] : pc[0];
-        P.du = dot_end<NP>(B, s == 0, pc);
+        P.t = flux_end<NP>(B, s == 0, pc, a.cky[pb + pl * NP + t]);
       }
       return P;
     };
     const int sf = first_side(vc.eyt, TY);
     const Partner2 qA = fetchy(sf), qB = fetchy(1 - sf);
     const Partner2 qb = sf == 0 ? qA : qB, qt = sf == 0 ? qB : qA;
-    const double ic0 = a.invr[vc.base + t], icL = a.invr[vc.base + L * NP + t];
-    const double jub = qb.u - uc[0], jvb = qb.v - vc_[0];
-    const double pbot = a.cpy[vc.base + t];
-    const double Fb = fma(pbot, jub, hw * fma(qb.k, qb.du, kyc[0] * gyu[0]));
-    zc[0] = fma(hw * kyc[0], fma(gyv[0], jub, gyu[0] * jvb), zc[0]);
-    if (gt_nonneg(ic0, qb.ir)) zc[0] = fma(pbot * jvb, jub, zc[0]);
-    const double jut = uc[L] - qt.u, jvt = vc_[L] - qt.v;
-    const double ptop = a.cpy[vc.base + L * NP + t];
-    const double Ft = fma(ptop, jut, hw * fma(kyc[L], gyu[L], qt.k * qt.du));
-    zc[L] = fma(hw * kyc[L], fma(gyv[L], jut, gyu[L] * jvt), zc[L]);
-    if (!gt_nonneg(qt.ir, icL)) zc[L] = fma(ptop * jvt, jut, zc[L]);
-    double sy[NP];
+    double Fb, Ft, us0, usL, z0, zL;
+    const long long n0 = vc.base + t, nL = vc.base + L * NP + t;
+    face(-1, uc[0], vc_[0], ky0, fc.t0, deriv_at<NP>(dc, 0), a.invr[n0], a.cpy[n0], qb, Fb, us0, z0);
+    face(1, uc[L], vc_[L], kyL, fc.tL, deriv_at<NP>(dc, L), a.invr[nL], a.cpy[nL], qt, Ft, usL, zL);
+    // zscale is -1 (r = b - A x) or +1 (A p): applied through operand signs, not a multiply
+    const int zsg = a.zscale > 0 ? 1 : -1;
+    double acc[NP], out[NP];
+    long long R[NP];
+    int er[NP];
 #pragma unroll
-    for (int l = 1; l < L; ++l) sy[l] = kyc[l] * gyu[l];
-    sy[0] = kyc[0] * fma(hw, jub, gyu[0]);
-    sy[L] = kyc[L] * fma(hw, jut, gyu[L]);
+    for (int l = 0; l < NP; ++l) {
+      R[l] = s_zr[e][l * NP + t];
+      er[l] = s_ez[e][l];
+      acc[l] = a.first ? 0.0 : a.Zs[vc.base + l * NP + t];
+    }
+    column_products<NP>(fc, dc, z0, zL, R, er, acc, zsg, out);
+#pragma unroll
+    for (int l = 0; l < NP; ++l) a.Zs[vc.base + l * NP + t] = out[l];
+    // xb - A u (and, for PCG, + alpha_it xconst + pApb apk) in one sum
 #pragma unroll
     for (int l = 0; l < NP; ++l) {
       const long long n = vc.base + l * NP + t;
-      const double cmn = a.cm[n];
-      const double syx = s_yx[e][l * NP + t];  // y-face flux at the end nodes only (l is compile-time)
-      double w = fma(cmn, uc[l], (l == 0) ? syx - Fb : ((l == L) ? syx + Ft : syx));
-      w = dot_col<NP>(B, l, sy, w);
-      // zscale is -1 (r = b - A x) or +1 (A p): applied through operand signs, not a multiply
+      R[l] = s_yx[e][l * NP + t];
+      er[l] = s_ey[e][l];
+      acc[l] = fma(-s_f[1][e][l * NP + t], uc[l], s_f[2][e][l * NP + t]);
+      if (PCG) acc[l] = fma(ppb, a.apk[n], fma(pal, a.xconst[n], acc[l]));
+    }
+    column_sums<NP>(B, fc, us0, usL, -Fb, Ft, R, er, acc, -1, out);
+#pragma unroll
+    for (int l = 0; l < NP; ++l) {
+      const long long n = vc.base + l * NP + t;
+      const double xb = out[l];
       const double uz = a.zscale > 0 ? uc[l] : -uc[l];
-      const double zs = a.zscale > 0 ? zc[l] + s_zr[e][l * NP + t] : -(zc[l] + s_zr[e][l * NP + t]);
-      double xb = a.xb[n] - w;
-      if (PCG) xb = fma(ppb, a.apk[n], fma(pal, a.xconst[n], xb));
       a.xb[n] = xb;
       if (a.bb_op == 1) a.bb[n] = uc[l];
       else if (a.bb_op == 2) a.bb[n] += uc[l];
-      if (a.first) { a.Zm[n] = uz * vc_[l]; a.Zs[n] = zs; }
-      else { a.Zm[n] = fma(uz, vc_[l], a.Zm[n]); a.Zs[n] += zs; }
+      a.Zm[n] = a.first ? uz * vc_[l] : fma(uz, vc_[l], a.Zm[n]);
       if (PCG && a.has_next) part = fma(xb, a.p_next[n], part);
       if (SREV == SREV_CHEB && a.has_next) {
         const double dbv = a.db[n] + xb;

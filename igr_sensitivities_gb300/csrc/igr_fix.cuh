@@ -300,7 +300,7 @@ __device__ __forceinline__ double line_end(const BASIS& B, bool last, const doub
 // instructions in, 22 out, the products and sums 4 multiply-adds each).
 // ---------------------------------------------------------------------------
 
-// The fluxes of a line: k[i] (D x)[i] = P[i] 2^(e - 1082), and at the two end nodes as doubles. Lines outside the
+// The fluxes of a line: k[i] (D x)[i] = P[i] 2^(e - 1084), |P| < 2^62, and at the two end nodes as doubles. Lines outside the
 // integer path's range (see line_op) hold the doubles' bits in P (slow).
 template <int NP>
 struct FixFlux {
@@ -383,10 +383,10 @@ __device__ __forceinline__ void flux_line(const BASIS& B, const double* x, const
   unsigned any = 0;
 #pragma unroll
   for (int i = 0; i < NP; ++i) { const int h = (int)(f.P[i] >> 32); any |= h ^ (h >> 31); }
-  const int z = __clz(any) - 4;  // |P| < 2^60
+  const int z = __clz(any) - 2;  // to |P| < 2^62
 #pragma unroll
   for (int i = 0; i < NP; ++i) f.P[i] = (long long)((unsigned long long)f.P[i] << z);
-  if (m != 0) f.e -= z;
+  if (m != 0) f.e += 2 - z;
 }
 
 // The flux at one end of a line, with the bits of flux_line's t0 / tL; k is the coefficient there.
@@ -430,7 +430,7 @@ __device__ __forceinline__ bool div_line(const BASIS& B, const FixFlux<NP>& f, d
   fix::Limb S[NP];
 #pragma unroll
   for (int i = 0; i < NP; ++i) {
-    long long v = fix::sar(f.P[i], e - sd - f.e);
+    long long v = fix::sar(f.P[i], e - sd - f.e + 2);
     if (i == 0) v = fix::add<7>(v, u0, e - sd);
     if (i == NP - 1) v = fix::add<7>(v, uL, e - sd);
     S[i] = {(int)(v >> 32), (int)((unsigned)v >> 1)};
@@ -447,7 +447,7 @@ template <int NP, class BASIS>
 __device__ __forceinline__ void div_line_fp64(const BASIS& B, const FixFlux<NP>& f, double u0, double uL, double* acc) {
   double s[NP];
 #pragma unroll
-  for (int i = 0; i < NP; ++i) s[i] = f.slow ? __longlong_as_double(f.P[i]) : fix::to_double(f.P[i], f.e);
+  for (int i = 0; i < NP; ++i) s[i] = f.slow ? __longlong_as_double(f.P[i]) : fix::to_double(f.P[i], f.e - 2);
   s[0] += u0;
   s[NP - 1] += uL;
 #pragma unroll
@@ -509,6 +509,124 @@ __device__ __forceinline__ void column_sums(const BASIS& B, const FixFlux<NP>& f
   div_line_fp64<NP>(B, f, u0, uL, y);
 #pragma unroll
   for (int k = 0; k < NP; ++k) out[k] = sg > 0 ? acc[k] + y[k] : acc[k] - y[k];
+}
+
+// Derivatives of a line: (D v)[i] = G[i] 2^(e - 1084), |G| < 2^62 and shifted up to use these bits; e = 0: a line of zeros; slow: the
+// bits of doubles.
+template <int NP>
+struct FixDeriv { long long G[NP]; int e; bool slow; };
+
+template <int NP, class BASIS>
+__device__ __forceinline__ void deriv_line(const BASIS& B, const double* v, FixDeriv<NP>& d) {
+  const int m = fix::max_hi<NP>(v);
+  d.slow = fix::out_of_range<NP>(m, v);
+  d.e = 0;
+  if (d.slow) {
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+      double g = 0.0;
+#pragma unroll
+      for (int j = 0; j < NP; ++j) if (!fix::skip<NP>(i, j)) g = fma(B.D[i][j], v[j], g);
+      d.G[i] = __double_as_longlong(g);
+    }
+    return;
+  }
+  const int ex = max(m >> 20, fix::E_MIN);
+  fix::Limb X[NP];
+#pragma unroll
+  for (int i = 0; i < NP; ++i) X[i] = fix::limbs(v[i], ex);
+  unsigned any = 0;
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    d.G[i] = fix::line_sum<NP>(
+        X, [&](int j) { return fix::Limb{B.fD.h[i][j], B.fD.l[i][j]}; }, [&](int j) { return !fix::skip<NP>(i, j); }, 0);
+    const int h = (int)(d.G[i] >> 32);
+    any |= h ^ (h >> 31);
+  }
+  const int z = __clz(any) - 2;
+#pragma unroll
+  for (int i = 0; i < NP; ++i) d.G[i] = (long long)((unsigned long long)d.G[i] << z);
+  if (m != 0) d.e = ex + B.fD.s + 1 - z;
+}
+template <int NP>
+__device__ __forceinline__ double deriv_at(const FixDeriv<NP>& d, int i) {
+  return d.slow ? __longlong_as_double(d.G[i]) : fix::to_double(d.G[i], d.e - 2);
+}
+template <int NP>
+__device__ __forceinline__ double flux_at(const FixFlux<NP>& f, int i) {
+  return f.slow ? __longlong_as_double(f.P[i]) : fix::to_double(f.P[i], f.e - 2);
+}
+
+// The products flux_i (D v)_i, with z0 and zL added at the end nodes, in units of 2^60 / 2^(r.e - 1022) (r.e < 0: the
+// bits of doubles); need: the largest exponent of what the caller adds. The products go by the line's largest flux and
+// derivative and are not aligned to the operator's sums.
+template <int NP>
+__device__ __forceinline__ bool product_line(const FixFlux<NP>& f, const FixDeriv<NP>& d, double z0, double zL, int need,
+                                             bool all_zero, FixSums<NP>& r) {
+  const int mz = max(fix::abs_hi(z0), fix::abs_hi(zL)) >> 20;
+  const bool none = f.e == 0 || d.e == 0;
+  const int ep = none ? 0 : f.e + d.e - 1022;
+  int e = max(max(ep, mz), need);
+  if (f.slow || d.slow || e >= fix::E_MAX || (!none && ep < 64)) return false;
+  if (e < 128) {
+    if (!none || !fix::zero(z0) || !fix::zero(zL) || !all_zero) return false;
+    e = 128;
+  }
+  r.e = e;
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    const int ph = (int)(f.P[i] >> 32), pl = (int)((unsigned)f.P[i] >> 1);
+    const int gh = (int)(d.G[i] >> 32), gl = (int)((unsigned)d.G[i] >> 1);
+    const long long M = fix::mad(ph, gl, fix::mad(pl, gh, fix::HALF));
+    long long v = fix::sar(fix::mad((int)(M >> 32), 2, fix::mad(ph, gh, 0)), e - ep);
+    if (i == 0) v = fix::add<7>(v, z0, e);
+    if (i == NP - 1) v = fix::add<7>(v, zL, e);
+    r.G[i] = v;
+  }
+  return true;
+}
+template <int NP>
+__device__ __forceinline__ void row_products(const FixFlux<NP>& f, const FixDeriv<NP>& d, double z0, double zL,
+                                             FixSums<NP>& r) {
+  if (product_line<NP>(f, d, z0, zL, 0, true, r)) return;
+  r.e = -1;
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    double v = flux_at<NP>(f, i) * deriv_at<NP>(d, i);
+    if (i == 0) v += z0;
+    if (i == NP - 1) v += zL;
+    r.G[i] = __double_as_longlong(v);
+  }
+}
+// out[k] = acc[k] + sg (row part[k] + products[k]); R, er as row_products left them
+template <int NP>
+__device__ __forceinline__ void column_products(const FixFlux<NP>& f, const FixDeriv<NP>& d, double z0, double zL,
+                                                const long long* R, const int* er, const double* acc, int sg, double* out) {
+  int need = 0, el = er[0], eh = er[0];
+#pragma unroll
+  for (int k = 0; k < NP; ++k) {
+    need = max(need, fix::abs_hi(acc[k]));
+    el = el < er[k] ? el : er[k];
+    eh = max(eh, er[k]);
+  }
+  need = max(need >> 20, eh);
+  FixSums<NP> s;
+  if (el >= 0 && product_line<NP>(f, d, z0, zL, need, false, s)) {
+#pragma unroll
+    for (int k = 0; k < NP; ++k) {
+      const long long v = s.G[k] + fix::sar(R[k], s.e - er[k]);
+      out[k] = fix::to_double(fix::add<7>(sg > 0 ? v : -v, acc[k], s.e), s.e);
+    }
+    return;
+  }
+#pragma unroll
+  for (int k = 0; k < NP; ++k) {
+    double v = flux_at<NP>(f, k) * deriv_at<NP>(d, k);
+    if (k == 0) v += z0;
+    if (k == NP - 1) v += zL;
+    v += er[k] < 0 ? __longlong_as_double(R[k]) : fix::to_double(R[k], er[k]);
+    out[k] = sg > 0 ? acc[k] + v : acc[k] - v;
+  }
 }
 
 }  // namespace igrgpu

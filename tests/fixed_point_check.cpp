@@ -225,6 +225,72 @@ template <int NP> static int run() {
     bad += !ok;
     std::printf("NP%d sip kind%d %s %.3f %.3f\n", NP, kind, ok ? "ok" : "BAD", wf, ws);
   }
+  // products flux_i (D v)_i summed over a row part, end terms and what is there already; kinds as above
+  for (int kind = 0; kind <= 12; ++kind) {
+    double sum_i = 0, sum_f = 0;
+    bool ok = true;
+    for (int it = 0; it < 4000; ++it) {
+      double x[NP], v[NP], k[NP], acc[NP], out[NP], row[NP];
+      long long R[NP];
+      int er[NP];
+      const double d = kind >= 9 ? std::pow(100.0, 9 - kind) : 1;
+      const double c1 = 2 * uni() - 1, c2 = 2 * uni() - 1, c3 = 2 * uni() - 1;
+      for (int i = 0; i < NP; ++i) {
+        const double s = 2.0 * i / (NP - 1) - 1;
+        x[i] = kind >= 9 ? 1 + d * s * (c1 + s * (c2 + s * c3)) : value(kind);
+        v[i] = kind >= 9 ? 2 - d * s * (c3 + s * (c1 + s * c2)) : value(kind == 5 ? 0 : kind);
+        k[i] = (0.5 + uni()) * 1e-4;
+        const double w = kind >= 9 ? d * d * 1e-4 : (kind == 6 ? 0 : (kind == 5 ? 1e290 : (kind == 4 || kind == 7 ? 0 : 1e-4)));
+        acc[i] = w * (2 * uni() - 1);
+        row[i] = w * (2 * uni() - 1);
+      }
+      const double z0 = row[0] * 0.3, zL = row[0] * 0.2;
+      FixFlux<NP> f, zf;
+      FixDeriv<NP> dv, zd;
+      flux_line<NP>(B, x, k, f);
+      deriv_line<NP>(B, v, dv);
+      double zeros[NP] = {};
+      flux_line<NP>(B, zeros, k, zf);
+      deriv_line<NP>(B, zeros, zd);
+      for (int i = 0; i < NP; ++i) {
+        FixSums<NP> r;
+        row_products<NP>(zf, zd, row[i], 0.0, r);
+        R[i] = r.G[0];
+        er[i] = r.e;
+      }
+      const int sg = uni() < 0.5 ? 1 : -1;
+      column_products<NP>(f, dv, z0, zL, R, er, acc, sg, out);
+      if (kind == 8) continue;
+      long double top = 0, S[NP];
+      double c64[NP];
+      for (int i = 0; i < NP; ++i) {
+        long double gx = 0, gv = 0;
+        double hx = 0, hv = 0;
+        for (int j = 0; j < NP; ++j)
+          if (!fix::skip<NP>(i, j)) {
+            gx += (long double)B.D[i][j] * x[j]; gv += (long double)B.D[i][j] * v[j];
+            hx = std::fma(B.D[i][j], x[j], hx); hv = std::fma(B.D[i][j], v[j], hv);
+          }
+        S[i] = gx * k[i] * gv + (i == 0 ? z0 : 0.0) + (i == NP - 1 ? zL : 0.0) + row[i];
+        S[i] = acc[i] + sg * S[i];
+        double h = k[i] * hx * hv;
+        if (i == 0) h += z0;
+        if (i == NP - 1) h += zL;
+        c64[i] = acc[i] + sg * (h + row[i]);
+        top = fmaxl(top, fmaxl(fabsl((long double)acc[i]), fmaxl(fabsl((long double)row[i]), fabsl(gx * k[i] * gv))));
+      }
+      for (int i = 0; i < NP; ++i) {
+        if (top < 1e-300L) { ok &= kind == 4 || kind == 7 || out[i] == 0; continue; }
+        const long double ei = (out[i] - S[i]) / top, ef = (c64[i] - S[i]) / top;
+        sum_i += (double)(ei * ei);
+        sum_f += (double)(ef * ef);
+      }
+    }
+    const double ratio = sum_f > 0 && NP > 2 && kind != 4 && kind != 7 ? std::sqrt(sum_i / sum_f) : 0;
+    ok &= ratio <= 1;
+    bad += !ok;
+    std::printf("NP%d products kind%d %s %.3f\n", NP, kind, ok ? "ok" : "BAD", ratio);
+  }
   // infinities and NaN come out as not finite wherever the FP64 chain has them
   const double inf = std::numeric_limits<double>::infinity();
   for (double x : {inf, -inf, std::numeric_limits<double>::quiet_NaN()})
