@@ -550,8 +550,6 @@ struct HypArgs2D {
   int* status;
 };
 
-struct FaceState { double q[4], f[4], ws; };
-
 // Pointwise physics at one node (euler.jl:145-214): both directional fluxes
 // with P_bar = P + Sigma from one evaluation of the pressure.
 struct NodePhys {
@@ -561,185 +559,221 @@ struct NodePhys {
 __device__ __forceinline__ NodePhys node_phys(double g, double mx, double my, double E, double S, double ir) {
   NodePhys p;
   p.ux = mx * ir; p.uy = my * ir;
-  const double kin = fma(mx, mx, my * my) * (0.5 * ir);
-  p.P = (g - 1.0) * (E - kin);
+  const double m2r = fma(mx, mx, my * my) * ir;
+  p.P = (g - 1.0) * fma(-0.5, m2r, E);
   p.pb = p.P + S;
   const double epb = E + p.pb;
   p.fx[0] = fma(mx, p.ux, p.pb); p.fx[1] = my * p.ux; p.fx[2] = mx; p.fx[3] = epb * p.ux;
-  p.fy[0] = mx * p.uy; p.fy[1] = fma(my, p.uy, p.pb); p.fy[2] = my; p.fy[3] = epb * p.uy;
+  p.fy[0] = p.fx[1]; p.fy[1] = fma(my, p.uy, p.pb); p.fy[2] = my; p.fy[3] = epb * p.uy;
   return p;
 }
 // |u_n| + c, c = sqrt(gamma P / rho)
 __device__ __forceinline__ double wavespeed(double g, double un, double P, double ir) {
-  return fabs(un) + sqrt(g * P * ir);
+  return fabs(un) + square_root(g * P * ir);
 }
 
+// x[v] of an array in registers
+__device__ __forceinline__ double pick4(const double* x, int v) {
+  const double lo = (v & 1) ? x[1] : x[0], hi = (v & 1) ? x[3] : x[2];
+  return (v & 2) ? hi : lo;
+}
+
+// The LLF flux of one face less the own side's flux, doubled: f_partner - f_own + lambda (q_L - q_R)
+// (euler.jl:222-236), the form the DG lifting takes it in. dq = q_partner - q_own; lam has the sign that
+// makes lam dq = lambda (q_L - q_R).
+__device__ __forceinline__ double llf_jump(double fp, double fo, double lam, double dq) { return fma(lam, dq, fp - fo); }
+
+// What bounds it: FP64 issue. Volume terms, their scaling, the row parts and the stage combination's sum are integer work
+// (igr_fix.cuh); the stage coefficient is folded into the scale of the derivatives and face terms, so that
+// q_out = (c0 q^n + c1 q_s) + [c2 dt k] is one rounded sum and k itself is never formed. 8 x 128^2 P3: 427 us with FP64
+// contractions and IEEE square roots, 251 us now (FP64 pipe 79% busy); 64^2: 24.9 and 22.4. Shared memory holds each
+// quantity once (fy_0 = fx_1; the mass fluxes are the momenta), 29.5 KB for P3: 7 CTAs per SM where 45 KB gave 5.
 template <int NP>
 __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_hyp_rk(HypArgs2D a) {
   using TL = Tiling2D<NP>;
   constexpr int TE = TL::TE, NN = TL::NN, L = TL::L, TX = TL::TX, TY = TL::TY;
-  __shared__ double s_fy[4][TE][NN];    // y fluxes
-  __shared__ double s_k[4][TE][NN];     // x part of the RHS
-  __shared__ double s_q[4][TE][NN];     // state (y-face LLF states)
-  __shared__ double s_pw[TE][NN];       // pressure (y-face wave speeds)
-  __shared__ FaceState s_xf[TE][NP][2]; // x-face node data (left, right) per row
-  __shared__ FaceState s_yf[TE][NP][2]; // y-face node data (bottom, top) per column
+  __shared__ double s_q[4][TE][NN];       // state
+  __shared__ double s_fy[3][TE][NN];      // fy_0 = fx_1, fy_1, fy_3 (fy_2 is the y momentum)
+  __shared__ double s_pw[TE][NN];         // pressure (y-face wave speeds)
+  __shared__ long long s_k[4][TE][NN];    // x part of c2 dt k (fixed point), exponents s_ke
+  __shared__ int s_ke[4][TE][NP];
+  __shared__ double s_fx[TE][NP][2][2];   // fx_0, fx_3 at the x-face nodes (left, right)
+  __shared__ double s_wx[TE][NP][2], s_wy[TE][NP][2];  // wave speeds at x- and y-face nodes
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];
   const ElemView vr = elem_view<NP>(tl, I, 0), vc = elem_view<NP>(tl, I, 1);
   const BasisDev& B = a.B;
   const double g = I.gamma;
-  const double invJx = I.ijx, invJy = I.ijy;
+  const bool raw = a.k_out[0] != nullptr;  // compute_hyperbolic_rhs!: k itself
+  const double c2dt = raw ? 1.0 : a.c2 * I.dt;
+  const double sx = -c2dt * I.ijx, sy = -c2dt * I.ijy;
 
-  // ---- phase 1 (row of vr): fluxes, x volume term, x-face node data
+  // ---- phase 1 (row of vr): fluxes, x-face node data. The x fluxes wait in the thread's own row of s_k.
   if (vr.valid) {
     const int t = vr.t, e = vr.e;
-    double fx[4][NP];
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
       const long long n = vr.base + t * NP + i;
+      const int nd = t * NP + i;
       const double mx = a.q[0][n], my = a.q[1][n], r = a.q[2][n], E = a.q[3][n], S = a.S[n], ir = a.invr[n];
       const NodePhys ph = node_phys(g, mx, my, E, S, ir);
-      s_q[0][e][t * NP + i] = mx; s_q[1][e][t * NP + i] = my; s_q[2][e][t * NP + i] = r; s_q[3][e][t * NP + i] = E;
-      s_pw[e][t * NP + i] = ph.P;
+      s_q[0][e][nd] = mx; s_q[1][e][nd] = my; s_q[2][e][nd] = r; s_q[3][e][nd] = E;
+      s_pw[e][nd] = ph.P;
+      s_fy[0][e][nd] = ph.fy[0]; s_fy[1][e][nd] = ph.fy[1]; s_fy[2][e][nd] = ph.fy[3];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) { fx[c][i] = ph.fx[c]; s_fy[c][e][t * NP + i] = ph.fy[c]; }
+      for (int v = 0; v < 4; ++v) s_k[v][e][nd] = __double_as_longlong(ph.fx[v]);
       if (i == 0 || i == L) {
-        FaceState& fs = s_xf[e][t][i == 0 ? 0 : 1];
-        fs.q[0] = mx; fs.q[1] = my; fs.q[2] = r; fs.q[3] = E;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) fs.f[c] = ph.fx[c];
-        fs.ws = wavespeed(g, ph.ux, ph.P, ir);
-        if (a.ws_x) a.ws_x[n] = fs.ws;
+        const int s = i == 0 ? 0 : 1;
+        const double ws = wavespeed(g, ph.ux, ph.P, ir);
+        s_fx[e][t][s][0] = ph.fx[0]; s_fx[e][t][s][1] = ph.fx[3];
+        s_wx[e][t][s] = ws;
+        if (a.ws_x) a.ws_x[n] = ws;
       }
     }
-#pragma unroll
-    for (int c = 0; c < 4; ++c)
-#pragma unroll
-      for (int i = 0; i < NP; ++i) s_k[c][e][t * NP + i] = -invJx * dot_row<NP>(B, i, fx[c]);
   }
   __syncthreads();
-  // ---- phase 2 (column of vc): y-face node data
+  // ---- phase 2 (column of vc): y-face wave speeds
   if (vc.valid) {
     const int t = vc.t, e = vc.e;
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
-      const int l = s == 0 ? 0 : L;
-      const int nd = l * NP + t;
-      FaceState& fs = s_yf[e][t][s];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) { fs.q[c] = s_q[c][e][nd]; fs.f[c] = s_fy[c][e][nd]; }
+      const int nd = (s == 0 ? 0 : L) * NP + t;
       const double ir = a.invr[vc.base + nd];
-      fs.ws = wavespeed(g, fs.q[1] * ir, s_pw[e][nd], ir);
-      if (a.ws_y) a.ws_y[vc.base + nd] = fs.ws;
+      const double ws = wavespeed(g, s_q[1][e][nd] * ir, s_pw[e][nd], ir);
+      s_wy[e][t][s] = ws;
+      if (a.ws_y) a.ws_y[vc.base + nd] = ws;
     }
   }
-  __syncthreads();
-  // ---- phase 3 (row of vr): x faces (LLF, euler.jl:222-236), owner computes its side
+  // ---- (row of vr): x faces, owner computes its side
+  struct PF { double q[4], f0, f1, f3, ws; };  // f: the components that are not a momentum
   if (vr.valid) {
     const int t = vr.t, e = vr.e;
     auto fetch = [&](int s) {
       int it;
       const long long pb = neighbour<NP>(tl, I, vr.ex, vr.ey, s == 0 ? -1 : 1, 0, &it);
-      FaceState pf;
+      const int nd = t * NP + (s == 0 ? L : 0);
+      PF p;
       if (it >= 0) {
-        pf = s_xf[it][t][s == 0 ? 1 : 0];
-      } else {
-        const long long n = pb + t * NP + (s == 0 ? L : 0);
-        pf.q[0] = a.q[0][n]; pf.q[1] = a.q[1][n]; pf.q[2] = a.q[2][n]; pf.q[3] = a.q[3][n];
-        const double ir = a.invr[n];
-        const NodePhys ph = node_phys(g, pf.q[0], pf.q[1], pf.q[3], a.S[n], ir);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) pf.f[c] = ph.fx[c];
-        pf.ws = wavespeed(g, ph.ux, ph.P, ir);
+        for (int c = 0; c < 4; ++c) p.q[c] = s_q[c][it][nd];
+        const int ps = s == 0 ? 1 : 0;
+        p.f0 = s_fx[it][t][ps][0]; p.f1 = s_fy[0][it][nd]; p.f3 = s_fx[it][t][ps][1]; p.ws = s_wx[it][t][ps];
+      } else {
+        const long long n = pb + nd;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) p.q[c] = a.q[c][n];
+        const double ir = a.invr[n];
+        const NodePhys ph = node_phys(g, p.q[0], p.q[1], p.q[3], a.S[n], ir);
+        p.f0 = ph.fx[0]; p.f1 = ph.fx[1]; p.f3 = ph.fx[3];
+        p.ws = wavespeed(g, ph.ux, ph.P, ir);
       }
-      return pf;
+      return p;
     };
     const int sf = first_side(vr.ext, TX);
-    const FaceState pA = fetch(sf), pB = fetch(1 - sf);
+    const PF pA = fetch(sf), pB = fetch(1 - sf);
+    double add[2][4];
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
-      const FaceState& pf = (s == sf) ? pA : pB;
-      const FaceState& of = s_xf[e][t][s];
-      const FaceState& Ls = s == 0 ? pf : of;
-      const FaceState& Rs = s == 0 ? of : pf;
-      const double lam = max_nonneg(Rs.ws, Ls.ws);
-      const int io = s == 0 ? 0 : L;
-      const double cf = s == 0 ? invJx * B.iw0 : -invJx * B.iwL;
+      const PF& p = (s == sf) ? pA : pB;
+      const int nd = t * NP + (s == 0 ? 0 : L);
+      const double own = s_wx[e][t][s];
+      const double mag = max_nonneg(s == 0 ? own : p.ws, s == 0 ? p.ws : own);
+      const double lam = s == 0 ? mag : -mag;
+      const double cf = s == 0 ? -0.5 * B.iw0 * sx : 0.5 * B.iwL * sx;
+      const double dm = p.q[0] - s_q[0][e][nd];
+      add[s][0] = cf * llf_jump(p.f0, s_fx[e][t][s][0], lam, dm);
+      add[s][1] = cf * llf_jump(p.f1, s_fy[0][e][nd], lam, p.q[1] - s_q[1][e][nd]);
+      add[s][2] = cf * fma(lam, p.q[2] - s_q[2][e][nd], dm);  // the mass flux is the momentum
+      add[s][3] = cf * llf_jump(p.f3, s_fx[e][t][s][1], lam, p.q[3] - s_q[3][e][nd]);
+    }
+    // The field loops stay rolled: their bodies are a few hundred integer instructions, and four copies of them cost
+    // more in instruction fetch than they save.
+    const FixScale c = fix_scale(sx);
+#pragma unroll 1
+    for (int v = 0; v < 4; ++v) {
+      double f[NP];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const double fs = 0.5 * fma(lam, Ls.q[c] - Rs.q[c], Ls.f[c] + Rs.f[c]);
-        s_k[c][e][t * NP + io] = fma(cf, fs - of.f[c], s_k[c][e][t * NP + io]);
-      }
+      for (int i = 0; i < NP; ++i) f[i] = __longlong_as_double(s_k[v][e][t * NP + i]);
+      FixSums<NP> k;
+      row_scaled<NP, false>(B, c, f, k);
+      row_add_ends<NP>(k, pick4(add[0], v), pick4(add[1], v));
+#pragma unroll
+      for (int i = 0; i < NP; ++i) s_k[v][e][t * NP + i] = k.G[i];
+      s_ke[v][e][t] = k.e;
     }
   }
   __syncthreads();
   if (!vc.valid) return;
-  // ---- phase 4 (column of vc): y volume term, y faces, RK combination
+  // ---- phase 3 (column of vc): y faces, y volume term, RK combination
   const int t = vc.t, e = vc.e;
-  double kc[4][NP];
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    double fyc[NP];
-#pragma unroll
-    for (int l = 0; l < NP; ++l) fyc[l] = s_fy[c][e][l * NP + t];
-#pragma unroll
-    for (int l = 0; l < NP; ++l) kc[c][l] = fma(-invJy, dot_row<NP>(B, l, fyc), s_k[c][e][l * NP + t]);
-  }
   auto fetchy = [&](int s) {
     int it;
     const long long pb = neighbour<NP>(tl, I, vc.ex, vc.ey, 0, s == 0 ? -1 : 1, &it);
-    FaceState pf;
+    const int nd = (s == 0 ? L : 0) * NP + t;
+    PF p;
     if (it >= 0) {
-      pf = s_yf[it][t][s == 0 ? 1 : 0];
-    } else {
-      const long long n = pb + (s == 0 ? L : 0) * NP + t;
-      pf.q[0] = a.q[0][n]; pf.q[1] = a.q[1][n]; pf.q[2] = a.q[2][n]; pf.q[3] = a.q[3][n];
-      const double ir = a.invr[n];
-      const NodePhys ph = node_phys(g, pf.q[0], pf.q[1], pf.q[3], a.S[n], ir);
 #pragma unroll
-      for (int c = 0; c < 4; ++c) pf.f[c] = ph.fy[c];
-      pf.ws = wavespeed(g, ph.uy, ph.P, ir);
+      for (int c = 0; c < 4; ++c) p.q[c] = s_q[c][it][nd];
+      p.f0 = s_fy[0][it][nd]; p.f1 = s_fy[1][it][nd]; p.f3 = s_fy[2][it][nd]; p.ws = s_wy[it][t][s == 0 ? 1 : 0];
+    } else {
+      const long long n = pb + nd;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) p.q[c] = a.q[c][n];
+      const double ir = a.invr[n];
+      const NodePhys ph = node_phys(g, p.q[0], p.q[1], p.q[3], a.S[n], ir);
+      p.f0 = ph.fy[0]; p.f1 = ph.fy[1]; p.f3 = ph.fy[3];
+      p.ws = wavespeed(g, ph.uy, ph.P, ir);
     }
-    return pf;
+    return p;
   };
   const int sf = first_side(vc.eyt, TY);
-  const FaceState qA = fetchy(sf), qB = fetchy(1 - sf);
+  const PF qA = fetchy(sf), qB = fetchy(1 - sf);
+  double add[2][4], cf[2];
 #pragma unroll
   for (int s = 0; s < 2; ++s) {
-    const FaceState& pf = (s == sf) ? qA : qB;
-    const FaceState& of = s_yf[e][t][s];
-    const FaceState& Ls = s == 0 ? pf : of;
-    const FaceState& Rs = s == 0 ? of : pf;
-    const double lam = max_nonneg(Rs.ws, Ls.ws);
-    const int lo = s == 0 ? 0 : L;
-    const double cf = s == 0 ? invJy * B.iw0 : -invJy * B.iwL;
+    const PF& p = (s == sf) ? qA : qB;
+    const int nd = (s == 0 ? 0 : L) * NP + t;
+    const double own = s_wy[e][t][s];
+    const double mag = max_nonneg(s == 0 ? own : p.ws, s == 0 ? p.ws : own);
+    const double lam = s == 0 ? mag : -mag;
+    cf[s] = s == 0 ? -0.5 * B.iw0 * sy : 0.5 * B.iwL * sy;
+    const double dm = p.q[1] - s_q[1][e][nd];
+    add[s][0] = llf_jump(p.f0, s_fy[0][e][nd], lam, p.q[0] - s_q[0][e][nd]);
+    add[s][1] = llf_jump(p.f1, s_fy[1][e][nd], lam, dm);
+    add[s][2] = fma(lam, p.q[2] - s_q[2][e][nd], dm);
+    add[s][3] = llf_jump(p.f3, s_fy[2][e][nd], lam, p.q[3] - s_q[3][e][nd]);
+  }
+  const FixScale c = fix_scale(sy);
+  const bool with_qn = __double_as_longlong(a.c0) != 0;
+  unsigned bad = 0;
+#pragma unroll 1
+  for (int v = 0; v < 4; ++v) {
+    double f[NP], acc[NP], out[NP];
+    long long R[NP];
+    int er[NP];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const double fs = 0.5 * fma(lam, Ls.q[c] - Rs.q[c], Ls.f[c] + Rs.f[c]);
-      kc[c][lo] = fma(cf, fs - of.f[c], kc[c][lo]);
+    for (int l = 0; l < NP; ++l) {
+      const int nd = l * NP + t;
+      const long long n = vc.base + nd;
+      f[l] = v == 2 ? s_q[1][e][nd] : s_fy[v - (v >> 1)][e][nd];  // fy_0, fy_1, my, fy_3
+      R[l] = s_k[v][e][nd];
+      er[l] = s_ke[v][e][l];
+      const double qs = s_q[v][e][nd];
+      acc[l] = raw ? 0.0 : (with_qn ? fma(a.c0, a.qn[v][n], a.c1 * qs) : qs);  // without q^n: c1 = 1
+      if (l == 0) acc[l] = fma(cf[0], pick4(add[0], v), acc[l]);
+      if (l == L) acc[l] = fma(cf[1], pick4(add[1], v), acc[l]);
+    }
+    column_scaled<NP, false>(B, c, f, R, er, acc, out);
+#pragma unroll
+    for (int l = 0; l < NP; ++l) {
+      const long long n = vc.base + l * NP + t;
+      if (a.k_out[v]) a.k_out[v][n] = out[l];
+      if (a.qo[v]) a.qo[v][n] = out[l];
+      if (v == 2 && a.invro) a.invro[n] = reciprocal(out[l]);
+      bad |= v == 2 ? not_positive_finite(out[l]) : nonfinite_bits(out[l]);
     }
   }
-  const double c2dt = a.c2 * I.dt;
-  bool bad = false;
-#pragma unroll
-  for (int l = 0; l < NP; ++l) {
-    const long long n = vc.base + l * NP + t;
-    double qo[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      if (a.k_out[c]) a.k_out[c][n] = kc[c][l];
-      const double qs = s_q[c][e][l * NP + t];
-      double val = fma(c2dt, kc[c][l], a.c1 * qs);
-      if (a.c0 != 0.0) val = fma(a.c0, a.qn[c][n], val);
-      qo[c] = val;
-    }
-#pragma unroll
-    for (int c = 0; c < 4; ++c) if (a.qo[c]) a.qo[c][n] = qo[c];
-    if (a.invro) a.invro[n] = 1.0 / qo[2];
-    bad |= not_positive_finite(qo[2]) || nonfinite_bits(qo[0]) || nonfinite_bits(qo[1]) || nonfinite_bits(qo[3]);
-  }
-  if (bad) flag_nonfinite(a.status);
+  if (bad && a.status) flag_nonfinite(a.status);
 }
 
 }  // namespace igrgpu

@@ -629,4 +629,107 @@ __device__ __forceinline__ void column_products(const FixFlux<NP>& f, const FixD
   }
 }
 
+// ---------------------------------------------------------------------------
+// A scaled line derivative (or its transpose, T) kept as integers between the phases, and the sum that ends it:
+//   row:    r = c (D v) + (a0 at node 0, aL at node NP-1)
+//   column: out = acc + row parts + c (D v)
+// in units of 2^60 / 2^(e - 1022); r.e < 0: the bits of doubles (FP64 lines).
+// ---------------------------------------------------------------------------
+template <int NP, bool T, class BASIS>
+__device__ __forceinline__ bool scaled_line(const BASIS& B, const FixScale& c, const double* v, FixSums<NP>& r) {
+  const int m = fix::max_hi<NP>(v);
+  if (fix::out_of_range<NP>(m, v) || (unsigned)(c.e - 1022 + 256) > 512u) return false;
+  const int ex = max(m >> 20, fix::E_MIN), e = ex + B.fD.s + c.e - 1022;
+  if ((unsigned)(e - 64) >= (unsigned)(fix::E_MAX - 64)) return false;
+  fix::Limb X[NP];
+#pragma unroll
+  for (int k = 0; k < NP; ++k) X[k] = fix::limbs(v[k], ex);
+#pragma unroll
+  for (int i = 0; i < NP; ++i)
+    r.G[i] = fix::times(fix::line_sum<NP>(
+                            X, [&](int k) { return fix::Limb{T ? B.fD.h[k][i] : B.fD.h[i][k], T ? B.fD.l[k][i] : B.fD.l[i][k]}; },
+                            [&](int k) { return !fix::skip<NP>(i, k); }, 0), c.m);
+  r.e = m == 0 ? 0 : e;
+  return true;
+}
+template <int NP, bool T, class BASIS>
+__device__ __forceinline__ void scaled_line_fp64(const BASIS& B, const FixScale& c, const double* v, double* out) {
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    double s = 0.0;
+#pragma unroll
+    for (int k = 0; k < NP; ++k) if (!fix::skip<NP>(i, k)) s = fma(T ? B.D[k][i] : B.D[i][k], v[k], s);
+    out[i] = c.d * s;
+  }
+}
+template <int NP, bool T, class BASIS>
+__device__ __forceinline__ void row_scaled(const BASIS& B, const FixScale& c, const double* v, FixSums<NP>& r) {
+  if (scaled_line<NP, T>(B, c, v, r)) return;
+  double s[NP];
+  scaled_line_fp64<NP, T>(B, c, v, s);
+  r.e = -1;
+#pragma unroll
+  for (int i = 0; i < NP; ++i) r.G[i] = __double_as_longlong(s[i]);
+}
+// value i of such sums
+template <int NP>
+__device__ __forceinline__ double sums_at(const FixSums<NP>& r, int i) {
+  return r.e < 0 ? __longlong_as_double(r.G[i]) : fix::to_double(r.G[i], r.e);
+}
+template <int NP>
+__device__ __forceinline__ void row_add_ends(FixSums<NP>& r, double a0, double aL) {
+  const int ma = max(fix::abs_hi(a0), fix::abs_hi(aL)) >> 20;
+  const int e = max(r.e, ma);
+  if (r.e >= 0 && (e == 0 || e >= 128) && e < fix::E_MAX) {  // e = 0: zeros
+    const int sh = e - r.e;
+#pragma unroll
+    for (int i = 0; i < NP; ++i) r.G[i] = fix::sar(r.G[i], sh);
+    r.e = e;
+    if (e != 0) {
+      r.G[0] = fix::add<7>(r.G[0], a0, e);
+      r.G[NP - 1] = fix::add<7>(r.G[NP - 1], aL, e);
+      return;
+    }
+    if (fix::zero(a0) && fix::zero(aL)) return;
+    r.e = 64;  // subnormals: below
+  }
+  double s[NP];
+#pragma unroll
+  for (int i = 0; i < NP; ++i) s[i] = sums_at<NP>(r, i);
+  s[0] += a0;
+  s[NP - 1] += aL;
+  r.e = -1;
+#pragma unroll
+  for (int i = 0; i < NP; ++i) r.G[i] = __double_as_longlong(s[i]);
+}
+template <int NP, bool T, class BASIS>
+__device__ __forceinline__ void column_scaled(const BASIS& B, const FixScale& c, const double* v, const long long* R,
+                                              const int* er, const double* acc, double* out) {
+  int need = 0, el = er[0], eh = er[0];
+#pragma unroll
+  for (int k = 0; k < NP; ++k) {
+    need = max(need, fix::abs_hi(acc[k]));
+    el = el < er[k] ? el : er[k];
+    eh = max(eh, er[k]);
+  }
+  need = max(need >> 20, eh);
+  FixSums<NP> s;
+  if (el >= 0 && scaled_line<NP, T>(B, c, v, s)) {
+    const int e = max(need, s.e);
+    if (e >= 128 && e < fix::E_MAX) {
+#pragma unroll
+      for (int k = 0; k < NP; ++k) {
+        const long long w = fix::sar(s.G[k], e - s.e) + fix::sar(R[k], e - er[k]);
+        out[k] = fix::to_double(fix::add<7>(w, acc[k], e), e);
+      }
+      return;
+    }
+  }
+  double y[NP];
+  scaled_line_fp64<NP, T>(B, c, v, y);
+#pragma unroll
+  for (int k = 0; k < NP; ++k)
+    out[k] = acc[k] + (y[k] + (er[k] < 0 ? __longlong_as_double(R[k]) : (er[k] == 0 ? 0.0 : fix::to_double(R[k], er[k]))));
+}
+
 }  // namespace igrgpu

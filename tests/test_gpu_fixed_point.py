@@ -61,3 +61,26 @@ def test_nonfinite_operand_stays_in_its_neighbourhood(igr, oracle, p, value):
     assert np.count_nonzero(~np.isfinite(got)) > 0
     fine = ~bad
     assert np.linalg.norm(got[fine] - ref[fine]) <= RTOL_OP * np.linalg.norm(ref[fine])
+
+
+# the hyperbolic right-hand side is homogeneous of degree one in (state, Sigma), so powers of two scale it; a gas at rest
+# reaches the ends of the exponent range without squares of the momentum leaving it (1 / rho and the sound speed there
+# take the IEEE operations)
+@pytest.mark.parametrize("p", [1, 2, 3, 4])
+@pytest.mark.parametrize("power,moving", [(0, True), (-400, True), (400, True), (-890, False), (990, False), (-1000, False)])
+def test_hyperbolic_rhs_over_the_exponent_range(igr, oracle, p, power, moving):
+    basis = igr.DGBasis(p)
+    mesh = igr.CartesianMesh2D(5, 3, 1.0, 0.7, basis)
+    G = oracle.Grid2D(p, 5, 3, 1.0, 0.7)
+    rng = np.random.default_rng(200 + p)
+    sh = mesh.x.shape
+    rho = 1.0 + 0.4 * rng.random(sh)
+    mux, muy = [0.3 * rng.standard_normal(sh) if moving else np.zeros(sh) for _ in range(2)]
+    E = 2.0 + rng.random(sh) + 0.5 * (mux ** 2 + muy ** 2) / rho
+    S = 0.05 * rng.standard_normal(sh)
+    s = 2.0 ** power
+    out = [np.zeros(sh, order="F") for _ in range(4)]
+    igr.compute_hyperbolic_rhs_(*out, *[np.asfortranarray(a * s) for a in (mux, muy, rho, E, S)], basis, mesh, 1.4)
+    ref = oracle.hyperbolic_rhs_2d(G, 1.4, [flat(a) for a in (mux, muy, rho, E)], flat(S))
+    for a, b in zip(out, ref):
+        assert rel(a, flat(b) * s, s) <= RTOL_OP
