@@ -98,6 +98,7 @@ BasisDev make_basis_dev(int p, const double* xi, const double* w, const double* 
   for (int i = 0; i < B.np; ++i)
     for (int k = 0; k < B.np; ++k) B.W2[i][k] = B.w[i] * (B.D[i][k] * B.D[i][k]);
   B.fD = make_fix(B.D, B.np);
+  B.fW2 = make_fix(B.W2, B.np);
   // chebyshev_fixed!, elliptic.jl:373-378
   const double table[4] = {1.5, 2.0, 2.1, 2.2};
   const double lmax = table[std::min(p, 4) - 1], lmin = 1.0;
@@ -151,6 +152,7 @@ Plan2D make_plan2d(Ctx& c, const BasisDev& B, const std::vector<Inst2DDesc>& ins
     I.gamma = d.gamma; I.alpha = d.alpha; I.dt = d.dt;
     I.ijx = 1.0 / I.jx; I.ijy = 1.0 / I.jy; I.idx = 1.0 / I.dx; I.idy = 1.0 / I.dy;
     I.ialpha = d.alpha > 0 ? 1.0 / d.alpha : 0.0;
+    I.gsum = 1.0 / d.gamma + 1.0 / (d.gamma - 1.0);
     I.tile0 = (int)P.tiles.size();
     for (int ey0 = 0; ey0 < d.ney; ey0 += ty)
       for (int ex0 = 0; ex0 < d.nex; ex0 += tx) P.tiles.push_back(Tile2D{(int)i, ex0, ey0, 0});

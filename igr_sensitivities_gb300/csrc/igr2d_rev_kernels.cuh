@@ -59,28 +59,24 @@ __device__ __forceinline__ void node_phys_rev(double g, double mx, double my, do
   qb[2] -= kb * kin * ir;
 }
 
-// Reverse of |u_n| + sqrt(g P / rho) at one node with adjoint wb; c is the sound speed.
-__device__ __forceinline__ void wavespeed_rev(int dir, double g, double mx, double my, double E, double ir, double c,
+// Reverse of |u_n| + c, c = sqrt(g P / rho), at one node with adjoint wb. With Y = wb c / 2 and T = d/dP scaled to
+// the energy, T = (wb / 2c) g (g - 1) / rho:
+//   d/dE = T, d/dm = -T u (+ the sign of u_n / rho in the normal direction),
+//   d/drho = T |u|^2 / 2 - Y / rho - (that) u_n,  d/dgamma = Y (1/g + 1/(g - 1));   gs is that last factor.
+__device__ __forceinline__ void wavespeed_rev(int dir, double g, double gs, double mx, double my, double ir, double ws,
                                               double wb, double qb[4], double& gb) {
   const double ux = mx * ir, uy = my * ir;
-  const double kin = fma(mx, mx, my * my) * (0.5 * ir);
-  const double P = (g - 1.0) * (E - kin);
   const double un = dir == 0 ? ux : uy;
-  const double unb = signbit(un) ? -wb : wb;
-  qb[dir] += unb * ir;
-  qb[2] -= unb * un * ir;
-  // c = sqrt(X), X = g P / rho:  dX = wb / (2 c)
-  const double Xb = wb * 0.5 / c;
-  const double X = c * c;
-  gb = fma(Xb, P * ir, gb);
-  const double Pb = Xb * g * ir;
-  qb[2] -= Xb * X * ir;
-  gb = fma(Pb, E - kin, gb);
-  qb[3] = fma(Pb, g - 1.0, qb[3]);
-  const double kb = -Pb * (g - 1.0);
-  qb[0] = fma(kb, ux, qb[0]);
-  qb[1] = fma(kb, uy, qb[1]);
-  qb[2] -= kb * kin * ir;
+  const double c = ws - fabs(un);
+  const double h = 0.5 * wb, Y = h * c;
+  const double T = (h * reciprocal(c)) * ((g * (g - 1.0)) * ir);
+  const double t = (signbit(un) ? -wb : wb) * ir;
+  gb = fma(Y, gs, gb);
+  qb[0] = fma(-T, ux, qb[0]);
+  qb[1] = fma(-T, uy, qb[1]);
+  qb[dir] += t;
+  qb[2] = fma(0.5 * T, fma(ux, ux, uy * uy), fma(-Y, ir, fma(-t, un, qb[2])));
+  qb[3] += T;
 }
 
 enum { SREV_NONE = 0, SREV_CHEB = 1, SREV_JACOBI = 2, SREV_PCG = 3 };
@@ -115,14 +111,17 @@ struct HypRevArgs2D {
   double ca, cc, omega;              // Chebyshev a_n, c_n ; Jacobi omega
 };
 
+// What bounds it: FP64 issue. The transposed volume terms run on the integer pipes with the stage coefficient in their
+// scale; a face takes 7 FP64 instructions per component. 8 x 128^2 P3: 680 us with FP64 contractions, 442 us now; 64^2:
+// 40.8 and 37.5.
 template <int NP>
 __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_hyp_rev(HypRevArgs2D a) {
   using TL = Tiling2D<NP>;
-  constexpr int TE = TL::TE, NN = TL::NN, L = TL::L, TX = TL::TX, TY = TL::TY;
-  __shared__ double s_kb[4][TE][NN];      // kbar = c2 dt A
+  constexpr int TE = TL::TE, NN = TL::NN, L = TL::L;
+  __shared__ double s_A[4][TE][NN];       // adjoint of the stage output
   __shared__ double s_q[4][TE][NN];       // taped stage state
   __shared__ double s_fbx[4][TE][NN];     // adjoint of the x fluxes (row phase)
-  __shared__ double s_qbx[4][TE][NN];     // q adjoint from the x faces (row phase)
+  __shared__ double s_qbx[4][TE][NP][2];  // q adjoint from the x faces, at the row ends
   __shared__ double s_xw[TE][NP][2];      // x wave speed at x-face nodes
   __shared__ double s_yw[TE][NP][2];
   __shared__ double s_grow[TE][NP];       // row-phase d/dgamma partials
@@ -131,7 +130,6 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_hyp_rev(HypRevArgs2D a) {
   const ElemView vr = elem_view<NP>(tl, I, 0), vc = elem_view<NP>(tl, I, 1);
   const BasisDev& B = a.B;
   const double g = I.gamma;
-  const double invJx = I.ijx, invJy = I.ijy;
   const double c2dt = a.c2 * I.dt;
 
   // ---- phase 1: row data of vr into smem; face wave speeds
@@ -141,7 +139,7 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_hyp_rev(HypRevArgs2D a) {
     for (int i = 0; i < NP; ++i) {
       const long long n = vr.base + t * NP + i;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) { s_q[c][e][t * NP + i] = a.q[c][n]; s_kb[c][e][t * NP + i] = c2dt * a.A[c][n]; }
+      for (int c = 0; c < 4; ++c) { s_q[c][e][t * NP + i] = a.q[c][n]; s_A[c][e][t * NP + i] = a.A[c][n]; }
     }
     s_xw[e][t][0] = a.ws_x[vr.base + t * NP];
     s_xw[e][t][1] = a.ws_x[vr.base + t * NP + L];
@@ -151,127 +149,107 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_hyp_rev(HypRevArgs2D a) {
     s_yw[vc.e][vc.t][1] = a.ws_y[vc.base + L * NP + vc.t];
   }
   __syncthreads();
-  // Reverse of one face's LLF flux for the own side: kb/pkb are the RHS
-  // adjoints at the own and partner face nodes; returns the flux adjoint
-  // increment and accumulates the own-state adjoint.
-  auto face_rev = [&](int dir, int s, const double oq[4], const double okb[4], double ows, double pws, const double pq[4],
-                      const double pkb[4], double ir_own, double fb[4], double qbo[4], double& gb) {
-    const double invJ = dir == 0 ? invJx : invJy;
-    // correction coefficients: R side (node 0) +invJ/w0, L side (node L) -invJ/wL
-    const double cfo = s == 0 ? invJ * B.iw0 : -invJ * B.iwL;
-    const double cfp = s == 0 ? -invJ * B.iwL : invJ * B.iw0;
-    const double wsL = s == 0 ? pws : ows, wsR = s == 0 ? ows : pws;
-    const double lam = max_nonneg(wsR, wsL);
-    const bool own_wins = (s == 0) ? gt_nonneg(wsR, wsL) : !gt_nonneg(wsR, wsL);
-    double lamb = 0.0;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const double fsb = fma(cfo, okb[c], cfp * pkb[c]);
-      fb[c] = fma(-cfo, okb[c], fb[c]) + 0.5 * fsb;
-      const double dq = s == 0 ? pq[c] - oq[c] : oq[c] - pq[c];  // q_L - q_R
-      qbo[c] = fma((s == 0 ? -0.5 : 0.5) * lam, fsb, qbo[c]);
-      lamb = fma(0.5 * fsb, dq, lamb);
-    }
-    if (own_wins) {
-      const double un = (dir == 0 ? oq[0] : oq[1]) * ir_own;
-      wavespeed_rev(dir, g, oq[0], oq[1], oq[3], ir_own, ows - fabs(un), lamb, qbo, gb);
-    }
-  };
-  double gb = 0.0;
-  // ---- phase 2a (row of vr): x flux adjoint = transpose of the x volume term + x-face LLF reverse
-  if (vr.valid) {
-    const int t = vr.t, e = vr.e;
-    double kb[4][NP], fb[4][NP], qbo[4][NP];
-#pragma unroll
-    for (int c = 0; c < 4; ++c)
-#pragma unroll
-      for (int i = 0; i < NP; ++i) { kb[c][i] = s_kb[c][e][t * NP + i]; qbo[c][i] = 0.0; }
-#pragma unroll
-    for (int c = 0; c < 4; ++c)
-#pragma unroll
-      for (int k = 0; k < NP; ++k) fb[c][k] = -invJx * dot_col<NP>(B, k, kb[c], 0.0);
-    struct PF { double q[4], kb[4], ws; };
-    auto fetch = [&](int s) {
-      PF P;
-      int it;
-      const long long pb = neighbour<NP>(tl, I, vr.ex, vr.ey, s == 0 ? -1 : 1, 0, &it);
-      const int pi = s == 0 ? L : 0;
-      if (it >= 0) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) { P.q[c] = s_q[c][it][t * NP + pi]; P.kb[c] = s_kb[c][it][t * NP + pi]; }
-        P.ws = s_xw[it][t][s == 0 ? 1 : 0];
-      } else {
-        const long long pn = pb + t * NP + pi;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) { P.q[c] = a.q[c][pn]; P.kb[c] = c2dt * a.A[c][pn]; }
-        P.ws = a.ws_x[pn];
-      }
-      return P;
-    };
-    const int sf = first_side(vr.ext, TX);
-    const PF pA = fetch(sf), pB = fetch(1 - sf);
+
+  // One line (row: dir 0, column: dir 1) of all four components. Its flux adjoints are the transposed volume term of
+  // kbar = c2 dt A plus, at the end nodes, the LLF flux's reverse: with a = coefficient of the own correction times
+  // kbar / 2 and b the partner's, the own flux gets b - a, the own state +-lambda (a + b), and lambda (a + b) dq.
+  // put(v, fb, q0, qL) takes component v's flux adjoints and the own-state adjoints of the two faces. The components
+  // stay a rolled loop: its body is a few hundred integer instructions.
+  auto line = [&](int dir, const ElemView& w, double invJ, double (*s_w)[NP][2], const double* ws, auto&& put, double lamb[2],
+                  bool wins[2]) {
+    const int e = w.e, t = w.t;
+    const int st = dir == 0 ? 1 : NP, at = dir == 0 ? t * NP : t;  // node k of the line: at + k st
+    const double ci = c2dt * invJ;
+    const FixScale sc = fix_scale(-ci);
+    long long pn[2];
+    int it[2];
+    double lam[2], cfo[2], cfp[2];
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
-      const PF& P = (s == sf) ? pA : pB;
-      const int io = s == 0 ? 0 : L;
-      double oq[4], okb[4], f4[4], q4[4];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) { oq[c] = s_q[c][e][t * NP + io]; okb[c] = kb[c][io]; f4[c] = fb[c][io]; q4[c] = qbo[c][io]; }
-      face_rev(0, s, oq, okb, s_xw[e][t][s], P.ws, P.q, P.kb, a.invr[vr.base + t * NP + io], f4, q4, gb);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) { fb[c][io] = f4[c]; qbo[c][io] = q4[c]; }
+      const int d = s == 0 ? -1 : 1;
+      const long long pb = neighbour<NP>(tl, I, w.ex, w.ey, dir == 0 ? d : 0, dir == 0 ? 0 : d, &it[s]);
+      pn[s] = pb + at + (s == 0 ? L : 0) * st;
+      const double own = s_w[e][t][s], par = it[s] >= 0 ? s_w[it[s] >= 0 ? it[s] : 0][t][1 - s] : ws[pn[s]];
+      const double mag = s == 0 ? max_nonneg(own, par) : max_nonneg(par, own);  // max(ws_R, ws_L)
+      wins[s] = s == 0 ? gt_nonneg(own, par) : !gt_nonneg(par, own);
+      lam[s] = s == 0 ? -mag : mag;
+      // correction coefficients: R side (node 0) +invJ/w0, L side (node L) -invJ/wL
+      cfo[s] = s == 0 ? 0.5 * ci * B.iw0 : -0.5 * ci * B.iwL;
+      cfp[s] = s == 0 ? -0.5 * ci * B.iwL : 0.5 * ci * B.iw0;
+      lamb[s] = 0.0;
     }
+#pragma unroll 1
+    for (int v = 0; v < 4; ++v) {
+      double A[NP], acc[NP], fb[NP], qo[2];
 #pragma unroll
-    for (int c = 0; c < 4; ++c)
+      for (int k = 0; k < NP; ++k) A[k] = s_A[v][e][at + k * st];
 #pragma unroll
-      for (int i = 0; i < NP; ++i) { s_fbx[c][e][t * NP + i] = fb[c][i]; s_qbx[c][e][t * NP + i] = qbo[c][i]; }
+      for (int s = 0; s < 2; ++s) {
+        const int nd = at + (s == 0 ? L : 0) * st;
+        const double pA = it[s] >= 0 ? s_A[v][it[s] >= 0 ? it[s] : 0][nd] : a.A[v][pn[s]];
+        const double pq = it[s] >= 0 ? s_q[v][it[s] >= 0 ? it[s] : 0][nd] : a.q[v][pn[s]];
+        const double oq = s_q[v][e][at + (s == 0 ? 0 : L) * st];
+        const double x = cfo[s] * A[s == 0 ? 0 : L], y = cfp[s] * pA;
+        const double h = x + y;
+        acc[s == 0 ? 0 : L] = y - x;
+        qo[s] = lam[s] * h;
+        lamb[s] = fma(h, s == 0 ? pq - oq : oq - pq, lamb[s]);  // q_L - q_R
+      }
+      line_op<NP, true, true, true>(B.fD, B.D, &sc, A, acc, [](int k) { return k == 0 || k == L; }, fb);
+      put(v, fb, qo[0], qo[1]);
+    }
+  };
+  // reverse of the wave speed of face s where the own side sets lambda
+  auto speed = [&](int dir, const ElemView& w, int s, double ws, double lamb, double qb[4], double& gb) {
+    const int nd = dir == 0 ? w.t * NP + (s == 0 ? 0 : L) : (s == 0 ? 0 : L) * NP + w.t;
+    wavespeed_rev(dir, g, I.gsum, s_q[0][w.e][nd], s_q[1][w.e][nd], a.invr[w.base + nd], ws, lamb, qb, gb);
+  };
+  double gb = 0.0;
+  // ---- phase 2a (row of vr)
+  if (vr.valid) {
+    const int t = vr.t, e = vr.e;
+    double lamb[2];
+    bool wins[2];
+    line(0, vr, I.ijx, s_xw, a.ws_x,
+         [&](int v, const double* fb, double q0, double qL) {
+#pragma unroll
+           for (int i = 0; i < NP; ++i) s_fbx[v][e][t * NP + i] = fb[i];
+           s_qbx[v][e][t][0] = q0;
+           s_qbx[v][e][t][1] = qL;
+         },
+         lamb, wins);
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      if (!wins[s]) continue;
+      double qb[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) qb[c] = s_qbx[c][e][t][s];
+      speed(0, vr, s, s_xw[e][t][s], lamb[s], qb, gb);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) s_qbx[c][e][t][s] = qb[c];
+    }
     s_grow[e][t] = gb;
     gb = 0.0;
   }
-  // ---- phase 2b (column of vc): y flux adjoint + y-face LLF reverse (registers)
-  double fby[4][NP], qby[4][NP];
+  // ---- phase 2b (column of vc): the y flux and face-state adjoints stay in registers
+  double fby[4][NP], qby[2][4];
   if (vc.valid) {
-    const int t = vc.t, e = vc.e;
-    double kb[4][NP];
+    double lamb[2];
+    bool wins[2];
+    line(1, vc, I.ijy, s_yw, a.ws_y,
+         [&](int v, const double* fb, double q0, double qL) {
 #pragma unroll
-    for (int c = 0; c < 4; ++c)
+           for (int c = 0; c < 4; ++c) {  // fby[v] = fb with a register index
 #pragma unroll
-      for (int l = 0; l < NP; ++l) { kb[c][l] = s_kb[c][e][l * NP + t]; qby[c][l] = 0.0; }
+             for (int l = 0; l < NP; ++l) fby[c][l] = v == c ? fb[l] : fby[c][l];
+             qby[0][c] = v == c ? q0 : qby[0][c];
+             qby[1][c] = v == c ? qL : qby[1][c];
+           }
+         },
+         lamb, wins);
 #pragma unroll
-    for (int c = 0; c < 4; ++c)
-#pragma unroll
-      for (int k = 0; k < NP; ++k) fby[c][k] = -invJy * dot_col<NP>(B, k, kb[c], 0.0);
-    struct PF { double q[4], kb[4], ws; };
-    auto fetch = [&](int s) {
-      PF P;
-      int it;
-      const long long pb = neighbour<NP>(tl, I, vc.ex, vc.ey, 0, s == 0 ? -1 : 1, &it);
-      const int pl = s == 0 ? L : 0;
-      if (it >= 0) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) { P.q[c] = s_q[c][it][pl * NP + t]; P.kb[c] = s_kb[c][it][pl * NP + t]; }
-        P.ws = s_yw[it][t][s == 0 ? 1 : 0];
-      } else {
-        const long long pn = pb + pl * NP + t;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) { P.q[c] = a.q[c][pn]; P.kb[c] = c2dt * a.A[c][pn]; }
-        P.ws = a.ws_y[pn];
-      }
-      return P;
-    };
-    const int sf = first_side(vc.eyt, TY);
-    const PF pA = fetch(sf), pB = fetch(1 - sf);
-#pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      const PF& P = (s == sf) ? pA : pB;
-      const int lo = s == 0 ? 0 : L;
-      double oq[4], okb[4], f4[4], q4[4];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) { oq[c] = s_q[c][e][lo * NP + t]; okb[c] = kb[c][lo]; f4[c] = fby[c][lo]; q4[c] = qby[c][lo]; }
-      face_rev(1, s, oq, okb, s_yw[e][t][s], P.ws, P.q, P.kb, a.invr[vc.base + lo * NP + t], f4, q4, gb);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) { fby[c][lo] = f4[c]; qby[c][lo] = q4[c]; }
-    }
+    for (int s = 0; s < 2; ++s)
+      if (wins[s]) speed(1, vc, s, s_yw[vc.e][vc.t][s], lamb[s], qby[s], gb);
   }
   __syncthreads();
   if (!vc.valid) return;
@@ -284,7 +262,11 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_hyp_rev(HypRevArgs2D a) {
     const int nd = l * NP + t;
     double fbx[4], fbyl[4], qq[4];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) { fbx[c] = s_fbx[c][e][nd]; fbyl[c] = fby[c][l]; qq[c] = qby[c][l] + s_qbx[c][e][nd]; }
+    for (int c = 0; c < 4; ++c) {
+      fbx[c] = s_fbx[c][e][nd]; fbyl[c] = fby[c][l];
+      qq[c] = (t == 0 || t == L) ? s_qbx[c][e][l][t == 0 ? 0 : 1] : 0.0;
+      if (l == 0 || l == L) qq[c] += qby[l == 0 ? 0 : 1][c];
+    }
     double Sb = 0.0;
     node_phys_rev(g, s_q[0][e][nd], s_q[1][e][nd], s_q[3][e][nd], a.S[n], a.invr[n], fbx, fbyl, qq, Sb, gb);
 #pragma unroll

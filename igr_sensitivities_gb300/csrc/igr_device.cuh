@@ -27,7 +27,7 @@ struct BasisDev {
   double cheb_theta, cheb_delta, cheb_sigma;  // elliptic.jl:373-378
   double hw;                // -1 / (2 w_0): SIP face coefficient factor
   double iw0, iwL;          // 1 / w_0, 1 / w_L
-  FixMat fD;                // D as integers (igr_fix.cuh)
+  FixMat fD, fW2;           // D and W2 as integers (igr_fix.cuh)
 };
 
 // One problem instance of a batch (2D): mesh, physics parameters and where
@@ -39,6 +39,7 @@ struct Inst2D {
   double gamma, alpha, dt;
   // reciprocals precomputed on the host (an FP64 divide costs ~9 FMA slots)
   double ijx, ijy, idx, idy, ialpha;
+  double gsum;  // 1 / gamma + 1 / (gamma - 1)
   int tile0, ntiles;  // this instance's tiles in the tile list (contiguous)
 };
 
