@@ -149,30 +149,47 @@ struct SetupArgs2D {
   int always;  // compute the coefficients even when alpha <= 0 (operator application on its own)
 };
 
+// What bounds it: FP64 issue, at a third of the FP64 instructions of its FP64-contraction form: the velocity derivatives
+// and both diagonal contractions (with their scales, and for the column one with the sum of all other parts of diag(A))
+// are integer line operations, and the face constants are tabulated once per CTA. 8 x 128^2 P3: 259 us with FP64
+// contractions, 112 us now (95 FP64 instructions per warp of lines, pipe 77% busy); 64^2: 16.5 and 14.0.
 template <int NP>
 __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_setup(SetupArgs2D a) {
   using TL = Tiling2D<NP>;
   constexpr int TE = TL::TE, NN = TL::NN, L = TL::L;
   __shared__ double s_ux[TE][NN], s_uy[TE][NN], s_ir[TE][NN], s_uxx[TE][NN], s_uyx[TE][NN], s_mx[TE][NN];
-  __shared__ double s_c[3][NN];  // w_i w_j Jx Jy, alpha w_i w_j Jy/Jx, alpha w_i w_j Jx/Jy  [node j*NP+i]
+  // per node: w_i w_j Jx Jy, alpha w_i w_j Jy/Jx, alpha w_i w_j Jx/Jy, alpha times the first  [node j*NP+i]
+  __shared__ double s_c[4][NN];
+  // per face node of a side: alpha eta w J / d (penalty) and the self terms' -+alpha D_ee w J / J' (x: left, right; y: bottom, top)
+  __shared__ double s_p[2][NP], s_s[2][2][NP];
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];
   const ElemView vr = elem_view<NP>(tl, I, 0), vc = elem_view<NP>(tl, I, 1);
   const BasisDev& B = a.B;
   const double invJx = I.ijx, invJy = I.ijy;
   if (I.alpha <= 0.0 && !a.always) return;  // no elliptic solve for this instance (forward.jl:24-28)
-  if (threadIdx.x < NN) {
-    const int i = threadIdx.x % NP, j = threadIdx.x / NP;
+  for (int n = threadIdx.x; n < NN; n += blockDim.x) {
+    const int i = n % NP, j = n / NP;
     const double ww = B.w[i] * B.w[j];
-    s_c[0][threadIdx.x] = ww * I.jx * I.jy;
-    s_c[1][threadIdx.x] = I.alpha * ww * I.jy * invJx;
-    s_c[2][threadIdx.x] = I.alpha * ww * I.jx * invJy;
+    s_c[0][n] = ww * I.jx * I.jy;
+    s_c[1][n] = I.alpha * ww * I.jy * invJx;
+    s_c[2][n] = I.alpha * ww * I.jx * invJy;
+    s_c[3][n] = s_c[0][n] * I.alpha;
   }
+  if (threadIdx.x < 2 * NP) {
+    const int d = threadIdx.x / NP, k = threadIdx.x % NP;
+    const double wf = B.w[k] * (d == 0 ? I.jy : I.jx), aJ = I.alpha * (d == 0 ? invJx : invJy);
+    s_p[d][k] = I.alpha * (double)(NP * NP) * (d == 0 ? I.idx : I.idy) * wf;
+    s_s[d][0][k] = aJ * B.D[0][0] * wf;
+    s_s[d][1][k] = -aJ * B.D[L][L] * wf;
+  }
+  auto none = [](int) { return false; };
+  auto all = [](int) { return true; };
 
   // ---- row phase (row t of element vr): velocities, x-derivatives, x part of the stiffness diagonal
   if (vr.valid) {
     const int t = vr.t, e = vr.e;
-    double ux[NP], uy[NP], ir[NP];
+    double ux[NP], uy[NP], ir[NP], out[NP];
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
       const long long n = vr.base + t * NP + i;
@@ -184,32 +201,45 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_setup(SetupArgs2D a) {
         s_ux[e][t * NP + i] = ux[i]; s_uy[e][t * NP + i] = uy[i];
       }
     }
-    const double cxs = I.alpha * B.w[t] * I.jy * invJx;
+    if (a.b) {
+      const FixScale cx = fix_scale(invJx);
+      line_rows<NP>(B, cx, ux, out);
 #pragma unroll
-    for (int i = 0; i < NP; ++i) {
-      if (a.b) {
-        s_uxx[e][t * NP + i] = dot_row<NP>(B, i, ux) * invJx;
-        s_uyx[e][t * NP + i] = dot_row<NP>(B, i, uy) * invJx;
-      }
-      double m = B.W2[0][i] * ir[0];
+      for (int i = 0; i < NP; ++i) s_uxx[e][t * NP + i] = out[i];
+      line_rows<NP>(B, cx, uy, out);
 #pragma unroll
-      for (int k = 1; k < NP; ++k) m = fma(B.W2[k][i], ir[k], m);
-      s_mx[e][t * NP + i] = cxs * m;
+      for (int i = 0; i < NP; ++i) s_uyx[e][t * NP + i] = out[i];
     }
+    const FixScale cd = fix_scale(I.alpha * B.w[t] * I.jy * invJx);
+    line_op<NP, true, false, true>(B.fW2, B.W2, &cd, ir, nullptr, none, out);
+#pragma unroll
+    for (int i = 0; i < NP; ++i) s_mx[e][t * NP + i] = out[i];
   }
   __syncthreads();
   if (!vc.valid) return;
 
   // ---- column phase (column t of element vc): y-derivatives, source, diagonal, coefficients
   const int t = vc.t, e = vc.e;
-  double cux[NP], cuy[NP], cir[NP];
+  double cir[NP];
 #pragma unroll
-  for (int l = 0; l < NP; ++l) {
-    cir[l] = s_ir[e][l * NP + t];
-    if (a.b) { cux[l] = s_ux[e][l * NP + t]; cuy[l] = s_uy[e][l * NP + t]; }
+  for (int l = 0; l < NP; ++l) cir[l] = s_ir[e][l * NP + t];
+  if (a.b) {
+    double cux[NP], cuy[NP], uxy2[NP], uyy[NP];  // uxy2 = 2 d_y u_x
+#pragma unroll
+    for (int l = 0; l < NP; ++l) { cux[l] = s_ux[e][l * NP + t]; cuy[l] = s_uy[e][l * NP + t]; }
+    line_rows<NP>(B, fix_scale(2.0 * invJy), cux, uxy2);
+    line_rows<NP>(B, fix_scale(invJy), cuy, uyy);
+#pragma unroll
+    for (int l = 0; l < NP; ++l) {
+      const int nd = l * NP + t;
+      const double uxx = s_uxx[e][nd], uyx = s_uyx[e][nd];
+      const double s = uxx + uyy[l];
+      double R = fma(s, s, uxx * uxx);
+      R = fma(uxy2[l], uyx, R);
+      R = fma(uyy[l], uyy[l], R);
+      a.b[vc.base + nd] = s_c[3][nd] * R;
+    }
   }
-  const double cys = I.alpha * B.w[t] * I.jx * invJy;
-  const double eta = (double)(NP * NP);
   // partner 1/rho across the x faces of column t (only t == 0 or t == L) and the y faces (l == 0, l == L)
   double irx[NP];
   if (t == 0 || t == L) {
@@ -227,47 +257,38 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_setup(SetupArgs2D a) {
     const long long pt = neighbour<NP>(tl, I, vc.ex, vc.ey, 0, 1, &it);   // top partner: node (t, 0)
     iry[1] = it >= 0 ? s_ir[it][t] : a.invr[pt + t];
   }
+  double acc[NP], M[NP];
 #pragma unroll
   for (int l = 0; l < NP; ++l) {
     const long long n = vc.base + l * NP + t;
     const int nd = l * NP + t;
-    if (a.b) {
-      const double uxy = dot_row<NP>(B, l, cux) * invJy;
-      const double uyy = dot_row<NP>(B, l, cuy) * invJy;
-      const double uxx = s_uxx[e][l * NP + t], uyx = s_uyx[e][l * NP + t];
-      const double s = uxx + uyy;
-      double R = fma(s, s, uxx * uxx);
-      R = fma(2.0 * uxy, uyx, R);
-      R = fma(uyy, uyy, R);
-      a.b[n] = s_c[0][nd] * (I.alpha * R);
-    }
-    double my_ = B.W2[0][l] * cir[0];
-#pragma unroll
-    for (int k = 1; k < NP; ++k) my_ = fma(B.W2[k][l], cir[k], my_);
     const double mass = s_c[0][nd] * cir[l];
-    double M = fma(cys, my_, mass + s_mx[e][nd]);
+    double m = mass + s_mx[e][nd];
     double px = 0.0, py = 0.0;
     if (t == 0 || t == L) {
-      const double wf = B.w[l] * I.jy;
-      const double sig = eta * max_nonneg(t == L ? cir[l] : irx[l], t == L ? irx[l] : cir[l]) * I.idx;
-      px = I.alpha * sig * wf;
+      px = s_p[0][l] * max_nonneg(t == L ? cir[l] : irx[l], t == L ? irx[l] : cir[l]);
       // x-face self terms: right side of its left face (t == 0) / left side of its right face (t == L)
-      M += fma((t == L ? -I.alpha * invJx * B.D[L][L] : I.alpha * invJx * B.D[0][0]) * wf, cir[l], px);
+      m = fma(s_s[0][t == L ? 1 : 0][l], cir[l], m + px);
     }
     if (l == 0 || l == L) {
-      const double wf = B.w[t] * I.jx;
       const double ip = iry[l == 0 ? 0 : 1];
-      const double sig = eta * max_nonneg(l == L ? cir[l] : ip, l == L ? ip : cir[l]) * I.idy;
-      py = I.alpha * sig * wf;
-      M += fma((l == L ? -I.alpha * invJy * B.D[L][L] : I.alpha * invJy * B.D[0][0]) * wf, cir[l], py);
+      py = s_p[1][t] * max_nonneg(l == L ? cir[l] : ip, l == L ? ip : cir[l]);
+      m = fma(s_s[1][l == L ? 1 : 0][t], cir[l], m + py);
     }
+    acc[l] = m;
     a.cm[n] = mass;
     a.ckx[n] = s_c[1][nd] * cir[l];
     a.cky[n] = s_c[2][nd] * cir[l];
     a.cpx[n] = px;
     a.cpy[n] = py;
-    a.cinvM[n] = 1.0 / M;
-    if (a.cM) a.cM[n] = M;
+  }
+  const FixScale cd = fix_scale(I.alpha * B.w[t] * I.jx * invJy);
+  line_op<NP, true, false, true>(B.fW2, B.W2, &cd, cir, acc, all, M);
+#pragma unroll
+  for (int l = 0; l < NP; ++l) {
+    const long long n = vc.base + l * NP + t;
+    a.cinvM[n] = reciprocal(M[l]);
+    if (a.cM) a.cM[n] = M[l];
   }
 }
 
@@ -583,51 +604,59 @@ __device__ __forceinline__ double pick4(const double* x, int v) {
 // makes lam dq = lambda (q_L - q_R).
 __device__ __forceinline__ double llf_jump(double fp, double fo, double lam, double dq) { return fma(lam, dq, fp - fo); }
 
+// Flux data of one node: the transported quantities q, the flux components that are not one of them (fx_2 and fy_2 are
+// q_0 and q_1, fy_0 = fx_1), and what the y wave speed needs.
+struct FluxNode { double q[4], fx0, f1, fx3, fy1, fy3, aux; };
+
+template <int NP, bool AUX>
+struct StageSmem {
+  double q[4][Tiling2D<NP>::TE][Tiling2D<NP>::NN];
+  double fy[3][Tiling2D<NP>::TE][Tiling2D<NP>::NN];       // fy_0 = fx_1, fy_1, fy_3
+  double aux[AUX ? Tiling2D<NP>::TE : 1][Tiling2D<NP>::NN];
+  long long k[4][Tiling2D<NP>::TE][Tiling2D<NP>::NN];     // fx, then the x part of c2 dt k (fixed point, exponents ke)
+  int ke[4][Tiling2D<NP>::TE][NP];
+  double fx[Tiling2D<NP>::TE][NP][2][2];                  // fx_0, fx_3 at the x-face nodes (left, right)
+  double wx[Tiling2D<NP>::TE][NP][2], wy[Tiling2D<NP>::TE][NP][2];  // wave speeds at x- and y-face nodes
+};
+
+// DG volume and LLF face terms of one tile with the SSP-RK3 combination q_out = c0 q^n + c1 q_s + c2 dt k (raw: k itself)
+// for the physics PH (the Euler fluxes or their tangent):
+//   at(n)             the node's FluxNode
+//   speed_x(n, node)  wave speeds at own face nodes; speed_y(n, q_1, aux)
+//   partner(n, f)     the node across an out-of-tile face; its wave speed by partner_speed(dir, n, node)
+//   qn(v, n), put(v, n, value)
 // What bounds it: FP64 issue. Volume terms, their scaling, the row parts and the stage combination's sum are integer work
 // (igr_fix.cuh); the stage coefficient is folded into the scale of the derivatives and face terms, so that
-// q_out = (c0 q^n + c1 q_s) + [c2 dt k] is one rounded sum and k itself is never formed. 8 x 128^2 P3: 427 us with FP64
-// contractions and IEEE square roots, 251 us now (FP64 pipe 79% busy); 64^2: 24.9 and 22.4. Shared memory holds each
-// quantity once (fy_0 = fx_1; the mass fluxes are the momenta), 29.5 KB for P3: 7 CTAs per SM where 45 KB gave 5.
-template <int NP>
-__global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_hyp_rk(HypArgs2D a) {
+// q_out = (c0 q^n + c1 q_s) + [c2 dt k] is one rounded sum and k itself is never formed. Euler, 8 x 128^2 P3: 427 us with
+// FP64 contractions and IEEE square roots, 251 us now (FP64 pipe 79% busy); 64^2: 24.9 and 22.4. Shared memory holds each
+// quantity once, 29.5 KB for P3: 7 CTAs per SM where 45 KB gave 5.
+template <int NP, bool AUX, class PH>
+__device__ __forceinline__ void dg_stage(const PH& ph, const BasisDev& B, const Tile2D tl, const Inst2D& I, double c0, double c1,
+                                         double c2, bool raw, StageSmem<NP, AUX>& sm) {
   using TL = Tiling2D<NP>;
-  constexpr int TE = TL::TE, NN = TL::NN, L = TL::L, TX = TL::TX, TY = TL::TY;
-  __shared__ double s_q[4][TE][NN];       // state
-  __shared__ double s_fy[3][TE][NN];      // fy_0 = fx_1, fy_1, fy_3 (fy_2 is the y momentum)
-  __shared__ double s_pw[TE][NN];         // pressure (y-face wave speeds)
-  __shared__ long long s_k[4][TE][NN];    // x part of c2 dt k (fixed point), exponents s_ke
-  __shared__ int s_ke[4][TE][NP];
-  __shared__ double s_fx[TE][NP][2][2];   // fx_0, fx_3 at the x-face nodes (left, right)
-  __shared__ double s_wx[TE][NP][2], s_wy[TE][NP][2];  // wave speeds at x- and y-face nodes
-  const Tile2D tl = a.tiles[blockIdx.x];
-  const Inst2D I = a.inst[tl.inst];
+  constexpr int L = TL::L, TX = TL::TX, TY = TL::TY;
   const ElemView vr = elem_view<NP>(tl, I, 0), vc = elem_view<NP>(tl, I, 1);
-  const BasisDev& B = a.B;
-  const double g = I.gamma;
-  const bool raw = a.k_out[0] != nullptr;  // compute_hyperbolic_rhs!: k itself
-  const double c2dt = raw ? 1.0 : a.c2 * I.dt;
+  const double c2dt = raw ? 1.0 : c2 * I.dt;
   const double sx = -c2dt * I.ijx, sy = -c2dt * I.ijy;
 
-  // ---- phase 1 (row of vr): fluxes, x-face node data. The x fluxes wait in the thread's own row of s_k.
+  // ---- phase 1 (row of vr): fluxes, x-face node data. The x fluxes wait in the thread's own row of sm.k.
   if (vr.valid) {
     const int t = vr.t, e = vr.e;
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
       const long long n = vr.base + t * NP + i;
       const int nd = t * NP + i;
-      const double mx = a.q[0][n], my = a.q[1][n], r = a.q[2][n], E = a.q[3][n], S = a.S[n], ir = a.invr[n];
-      const NodePhys ph = node_phys(g, mx, my, E, S, ir);
-      s_q[0][e][nd] = mx; s_q[1][e][nd] = my; s_q[2][e][nd] = r; s_q[3][e][nd] = E;
-      s_pw[e][nd] = ph.P;
-      s_fy[0][e][nd] = ph.fy[0]; s_fy[1][e][nd] = ph.fy[1]; s_fy[2][e][nd] = ph.fy[3];
+      const FluxNode f = ph.at(n);
 #pragma unroll
-      for (int v = 0; v < 4; ++v) s_k[v][e][nd] = __double_as_longlong(ph.fx[v]);
+      for (int v = 0; v < 4; ++v) sm.q[v][e][nd] = f.q[v];
+      if (AUX) sm.aux[AUX ? e : 0][nd] = f.aux;
+      sm.fy[0][e][nd] = f.f1; sm.fy[1][e][nd] = f.fy1; sm.fy[2][e][nd] = f.fy3;
+      sm.k[0][e][nd] = __double_as_longlong(f.fx0); sm.k[1][e][nd] = __double_as_longlong(f.f1);
+      sm.k[2][e][nd] = __double_as_longlong(f.q[0]); sm.k[3][e][nd] = __double_as_longlong(f.fx3);
       if (i == 0 || i == L) {
         const int s = i == 0 ? 0 : 1;
-        const double ws = wavespeed(g, ph.ux, ph.P, ir);
-        s_fx[e][t][s][0] = ph.fx[0]; s_fx[e][t][s][1] = ph.fx[3];
-        s_wx[e][t][s] = ws;
-        if (a.ws_x) a.ws_x[n] = ws;
+        sm.fx[e][t][s][0] = f.fx0; sm.fx[e][t][s][1] = f.fx3;
+        sm.wx[e][t][s] = ph.speed_x(n, f);
       }
     }
   }
@@ -638,14 +667,11 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_hyp_rk(HypArgs2D a) {
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
       const int nd = (s == 0 ? 0 : L) * NP + t;
-      const double ir = a.invr[vc.base + nd];
-      const double ws = wavespeed(g, s_q[1][e][nd] * ir, s_pw[e][nd], ir);
-      s_wy[e][t][s] = ws;
-      if (a.ws_y) a.ws_y[vc.base + nd] = ws;
+      sm.wy[e][t][s] = ph.speed_y(vc.base + nd, sm.q[1][e][nd], AUX ? sm.aux[AUX ? e : 0][nd] : 0.0);
     }
   }
   // ---- (row of vr): x faces, owner computes its side
-  struct PF { double q[4], f0, f1, f3, ws; };  // f: the components that are not a momentum
+  struct PF { double q[4], f0, f1, f3, ws; };  // f: the components that are not a transported quantity
   if (vr.valid) {
     const int t = vr.t, e = vr.e;
     auto fetch = [&](int s) {
@@ -655,17 +681,15 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_hyp_rk(HypArgs2D a) {
       PF p;
       if (it >= 0) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) p.q[c] = s_q[c][it][nd];
+        for (int c = 0; c < 4; ++c) p.q[c] = sm.q[c][it][nd];
         const int ps = s == 0 ? 1 : 0;
-        p.f0 = s_fx[it][t][ps][0]; p.f1 = s_fy[0][it][nd]; p.f3 = s_fx[it][t][ps][1]; p.ws = s_wx[it][t][ps];
+        p.f0 = sm.fx[it][t][ps][0]; p.f1 = sm.fy[0][it][nd]; p.f3 = sm.fx[it][t][ps][1]; p.ws = sm.wx[it][t][ps];
       } else {
-        const long long n = pb + nd;
+        const FluxNode f = ph.at(pb + nd);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) p.q[c] = a.q[c][n];
-        const double ir = a.invr[n];
-        const NodePhys ph = node_phys(g, p.q[0], p.q[1], p.q[3], a.S[n], ir);
-        p.f0 = ph.fx[0]; p.f1 = ph.fx[1]; p.f3 = ph.fx[3];
-        p.ws = wavespeed(g, ph.ux, ph.P, ir);
+        for (int c = 0; c < 4; ++c) p.q[c] = f.q[c];
+        p.f0 = f.fx0; p.f1 = f.f1; p.f3 = f.fx3;
+        p.ws = ph.partner_speed(0, pb + nd, f);
       }
       return p;
     };
@@ -676,15 +700,15 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_hyp_rk(HypArgs2D a) {
     for (int s = 0; s < 2; ++s) {
       const PF& p = (s == sf) ? pA : pB;
       const int nd = t * NP + (s == 0 ? 0 : L);
-      const double own = s_wx[e][t][s];
+      const double own = sm.wx[e][t][s];
       const double mag = max_nonneg(s == 0 ? own : p.ws, s == 0 ? p.ws : own);
       const double lam = s == 0 ? mag : -mag;
       const double cf = s == 0 ? -0.5 * B.iw0 * sx : 0.5 * B.iwL * sx;
-      const double dm = p.q[0] - s_q[0][e][nd];
-      add[s][0] = cf * llf_jump(p.f0, s_fx[e][t][s][0], lam, dm);
-      add[s][1] = cf * llf_jump(p.f1, s_fy[0][e][nd], lam, p.q[1] - s_q[1][e][nd]);
-      add[s][2] = cf * fma(lam, p.q[2] - s_q[2][e][nd], dm);  // the mass flux is the momentum
-      add[s][3] = cf * llf_jump(p.f3, s_fx[e][t][s][1], lam, p.q[3] - s_q[3][e][nd]);
+      const double dm = p.q[0] - sm.q[0][e][nd];
+      add[s][0] = cf * llf_jump(p.f0, sm.fx[e][t][s][0], lam, dm);
+      add[s][1] = cf * llf_jump(p.f1, sm.fy[0][e][nd], lam, p.q[1] - sm.q[1][e][nd]);
+      add[s][2] = cf * fma(lam, p.q[2] - sm.q[2][e][nd], dm);  // fx_2 = q_0
+      add[s][3] = cf * llf_jump(p.f3, sm.fx[e][t][s][1], lam, p.q[3] - sm.q[3][e][nd]);
     }
     // The field loops stay rolled: their bodies are a few hundred integer instructions, and four copies of them cost
     // more in instruction fetch than they save.
@@ -693,13 +717,13 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_hyp_rk(HypArgs2D a) {
     for (int v = 0; v < 4; ++v) {
       double f[NP];
 #pragma unroll
-      for (int i = 0; i < NP; ++i) f[i] = __longlong_as_double(s_k[v][e][t * NP + i]);
+      for (int i = 0; i < NP; ++i) f[i] = __longlong_as_double(sm.k[v][e][t * NP + i]);
       FixSums<NP> k;
       row_scaled<NP, false>(B, c, f, k);
       row_add_ends<NP>(k, pick4(add[0], v), pick4(add[1], v));
 #pragma unroll
-      for (int i = 0; i < NP; ++i) s_k[v][e][t * NP + i] = k.G[i];
-      s_ke[v][e][t] = k.e;
+      for (int i = 0; i < NP; ++i) sm.k[v][e][t * NP + i] = k.G[i];
+      sm.ke[v][e][t] = k.e;
     }
   }
   __syncthreads();
@@ -713,16 +737,14 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_hyp_rk(HypArgs2D a) {
     PF p;
     if (it >= 0) {
 #pragma unroll
-      for (int c = 0; c < 4; ++c) p.q[c] = s_q[c][it][nd];
-      p.f0 = s_fy[0][it][nd]; p.f1 = s_fy[1][it][nd]; p.f3 = s_fy[2][it][nd]; p.ws = s_wy[it][t][s == 0 ? 1 : 0];
+      for (int c = 0; c < 4; ++c) p.q[c] = sm.q[c][it][nd];
+      p.f0 = sm.fy[0][it][nd]; p.f1 = sm.fy[1][it][nd]; p.f3 = sm.fy[2][it][nd]; p.ws = sm.wy[it][t][s == 0 ? 1 : 0];
     } else {
-      const long long n = pb + nd;
+      const FluxNode f = ph.at(pb + nd);
 #pragma unroll
-      for (int c = 0; c < 4; ++c) p.q[c] = a.q[c][n];
-      const double ir = a.invr[n];
-      const NodePhys ph = node_phys(g, p.q[0], p.q[1], p.q[3], a.S[n], ir);
-      p.f0 = ph.fy[0]; p.f1 = ph.fy[1]; p.f3 = ph.fy[3];
-      p.ws = wavespeed(g, ph.uy, ph.P, ir);
+      for (int c = 0; c < 4; ++c) p.q[c] = f.q[c];
+      p.f0 = f.f1; p.f1 = f.fy1; p.f3 = f.fy3;
+      p.ws = ph.partner_speed(1, pb + nd, f);
     }
     return p;
   };
@@ -733,19 +755,18 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_hyp_rk(HypArgs2D a) {
   for (int s = 0; s < 2; ++s) {
     const PF& p = (s == sf) ? qA : qB;
     const int nd = (s == 0 ? 0 : L) * NP + t;
-    const double own = s_wy[e][t][s];
+    const double own = sm.wy[e][t][s];
     const double mag = max_nonneg(s == 0 ? own : p.ws, s == 0 ? p.ws : own);
     const double lam = s == 0 ? mag : -mag;
     cf[s] = s == 0 ? -0.5 * B.iw0 * sy : 0.5 * B.iwL * sy;
-    const double dm = p.q[1] - s_q[1][e][nd];
-    add[s][0] = llf_jump(p.f0, s_fy[0][e][nd], lam, p.q[0] - s_q[0][e][nd]);
-    add[s][1] = llf_jump(p.f1, s_fy[1][e][nd], lam, dm);
-    add[s][2] = fma(lam, p.q[2] - s_q[2][e][nd], dm);
-    add[s][3] = llf_jump(p.f3, s_fy[2][e][nd], lam, p.q[3] - s_q[3][e][nd]);
+    const double dm = p.q[1] - sm.q[1][e][nd];
+    add[s][0] = llf_jump(p.f0, sm.fy[0][e][nd], lam, p.q[0] - sm.q[0][e][nd]);
+    add[s][1] = llf_jump(p.f1, sm.fy[1][e][nd], lam, dm);
+    add[s][2] = fma(lam, p.q[2] - sm.q[2][e][nd], dm);
+    add[s][3] = llf_jump(p.f3, sm.fy[2][e][nd], lam, p.q[3] - sm.q[3][e][nd]);
   }
   const FixScale c = fix_scale(sy);
-  const bool with_qn = __double_as_longlong(a.c0) != 0;
-  unsigned bad = 0;
+  const bool with_qn = __double_as_longlong(c0) != 0;
 #pragma unroll 1
   for (int v = 0; v < 4; ++v) {
     double f[NP], acc[NP], out[NP];
@@ -754,26 +775,63 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_hyp_rk(HypArgs2D a) {
 #pragma unroll
     for (int l = 0; l < NP; ++l) {
       const int nd = l * NP + t;
-      const long long n = vc.base + nd;
-      f[l] = v == 2 ? s_q[1][e][nd] : s_fy[v - (v >> 1)][e][nd];  // fy_0, fy_1, my, fy_3
-      R[l] = s_k[v][e][nd];
-      er[l] = s_ke[v][e][l];
-      const double qs = s_q[v][e][nd];
-      acc[l] = raw ? 0.0 : (with_qn ? fma(a.c0, a.qn[v][n], a.c1 * qs) : qs);  // without q^n: c1 = 1
+      f[l] = v == 2 ? sm.q[1][e][nd] : sm.fy[v - (v >> 1)][e][nd];  // fy_0, fy_1, q_1, fy_3
+      R[l] = sm.k[v][e][nd];
+      er[l] = sm.ke[v][e][l];
+      const double qs = sm.q[v][e][nd];
+      acc[l] = raw ? 0.0 : (with_qn ? fma(c0, ph.qn(v, vc.base + nd), c1 * qs) : qs);  // without q^n: c1 = 1
       if (l == 0) acc[l] = fma(cf[0], pick4(add[0], v), acc[l]);
       if (l == L) acc[l] = fma(cf[1], pick4(add[1], v), acc[l]);
     }
     column_scaled<NP, false>(B, c, f, R, er, acc, out);
 #pragma unroll
-    for (int l = 0; l < NP; ++l) {
-      const long long n = vc.base + l * NP + t;
-      if (a.k_out[v]) a.k_out[v][n] = out[l];
-      if (a.qo[v]) a.qo[v][n] = out[l];
-      if (v == 2 && a.invro) a.invro[n] = reciprocal(out[l]);
-      bad |= v == 2 ? not_positive_finite(out[l]) : nonfinite_bits(out[l]);
-    }
+    for (int l = 0; l < NP; ++l) ph.put(v, vc.base + l * NP + t, out[l]);
   }
-  if (bad && a.status) flag_nonfinite(a.status);
+}
+
+// The Euler fluxes (hyperbolic.jl) with the wave speeds computed here.
+struct EulerStage {
+  const HypArgs2D& a;
+  double g;
+  __device__ __forceinline__ FluxNode at(long long n) const {
+    FluxNode f;
+#pragma unroll
+    for (int v = 0; v < 4; ++v) f.q[v] = a.q[v][n];
+    const NodePhys p = node_phys(g, f.q[0], f.q[1], f.q[3], a.S[n], a.invr[n]);
+    f.fx0 = p.fx[0]; f.f1 = p.fx[1]; f.fx3 = p.fx[3]; f.fy1 = p.fy[1]; f.fy3 = p.fy[3];
+    f.aux = p.P;
+    return f;
+  }
+  __device__ __forceinline__ double partner_speed(int dir, long long n, const FluxNode& f) const {
+    const double ir = a.invr[n];
+    return wavespeed(g, f.q[dir] * ir, f.aux, ir);
+  }
+  __device__ __forceinline__ double speed_x(long long n, const FluxNode& f) const {
+    const double ws = partner_speed(0, n, f);
+    if (a.ws_x) a.ws_x[n] = ws;
+    return ws;
+  }
+  __device__ __forceinline__ double speed_y(long long n, double my, double P) const {
+    const double ir = a.invr[n];
+    const double ws = wavespeed(g, my * ir, P, ir);
+    if (a.ws_y) a.ws_y[n] = ws;
+    return ws;
+  }
+  __device__ __forceinline__ double qn(int v, long long n) const { return a.qn[v][n]; }
+  __device__ __forceinline__ void put(int v, long long n, double x) const {
+    if (a.k_out[v]) a.k_out[v][n] = x;
+    if (a.qo[v]) a.qo[v][n] = x;
+    if (v == 2 && a.invro) a.invro[n] = reciprocal(x);
+    if (a.status && (v == 2 ? not_positive_finite(x) : nonfinite_bits(x))) flag_nonfinite(a.status);
+  }
+};
+
+template <int NP>
+__global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_hyp_rk(HypArgs2D a) {
+  __shared__ StageSmem<NP, true> sm;
+  const Tile2D tl = a.tiles[blockIdx.x];
+  const Inst2D I = a.inst[tl.inst];
+  dg_stage<NP, true>(EulerStage{a, I.gamma}, a.B, tl, I, a.c0, a.c1, a.c2, a.k_out[0] != nullptr, sm);
 }
 
 }  // namespace igrgpu

@@ -554,14 +554,20 @@ struct SetupRevArgs2D {
   double *anode;
 };
 
+// What bounds it: FP64 issue. All derivatives, transposes and diagonal contractions are integer line operations, with
+// their scales and the terms they are added to; the x transposes have a row phase of their own. 8 x 128^2 P3: 409 us with
+// FP64 contractions, 198 us now; 64^2: 22.8 and 22.7 (five phases of latency).
 template <int NP>
 __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_setup_rev(SetupRevArgs2D a) {
   using TL = Tiling2D<NP>;
   constexpr int TE = TL::TE, NN = TL::NN, L = TL::L;
   __shared__ double s_ux[TE][NN], s_uy[TE][NN], s_Mb[TE][NN];
   __shared__ double s_uxx[TE][NN], s_uyx[TE][NN];       // x derivatives (row phase)
-  __shared__ double s_bxx[TE][NN], s_byx[TE][NN];       // adjoints of uxx, uyx (column phase)
+  __shared__ double s_bxx[TE][NN], s_byx[TE][NN];       // adjoints of uxx, uyx (columns), then their x transposes (rows)
   __shared__ double s_ir[TE][NN], s_ib[TE][NN];         // 1/rho; row-phase d/d(1/rho) from diag(A)
+  __shared__ double s_m0[NN];                           // w_i w_j Jx Jy
+  // per face node of a side: alpha eta w J / d (penalty) and the self terms' -+alpha D_ee w J / J' (x: left, right; y: bottom, top)
+  __shared__ double s_p[2][NP], s_s[2][2][NP];
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];
   const ElemView vr = elem_view<NP>(tl, I, 0), vc = elem_view<NP>(tl, I, 1);
@@ -569,12 +575,21 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_setup_rev(SetupRevArgs2D 
   const double invJx = I.ijx, invJy = I.ijy;
   const double alpha = I.alpha;
   if (alpha <= 0.0) return;
-  const double eta = (double)(NP * NP);
+  for (int n = threadIdx.x; n < NN; n += blockDim.x) s_m0[n] = B.w[n % NP] * B.w[n / NP] * I.jx * I.jy;
+  if (threadIdx.x < 2 * NP) {
+    const int d = threadIdx.x / NP, k = threadIdx.x % NP;
+    const double wf = B.w[k] * (d == 0 ? I.jy : I.jx), aJ = alpha * (d == 0 ? invJx : invJy);
+    s_p[d][k] = alpha * (double)(NP * NP) * (d == 0 ? I.idx : I.idy) * wf;
+    s_s[d][0][k] = aJ * B.D[0][0] * wf;
+    s_s[d][1][k] = -aJ * B.D[L][L] * wf;
+  }
+  auto none = [](int) { return false; };
+  auto all = [](int) { return true; };
+  const FixScale cx = fix_scale(invJx), cy = fix_scale(invJy);
 
   if (vr.valid) {
     const int t = vr.t, e = vr.e;
-    double ux[NP], uy[NP], Mbr[NP];
-    const double cxs = alpha * B.w[t] * I.jy * invJx;
+    double ux[NP], uy[NP], Mbr[NP], out[NP];
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
       const long long n = vr.base + t * NP + i;
@@ -583,65 +598,64 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_setup_rev(SetupRevArgs2D 
       ux[i] = a.mx[n] * ir; uy[i] = a.my[n] * ir; Mbr[i] = -(a.iMb[n] * im) * im;  // d/dM = -d/d(1/M) / M^2
       s_ux[e][t * NP + i] = ux[i]; s_uy[e][t * NP + i] = uy[i]; s_Mb[e][t * NP + i] = Mbr[i]; s_ir[e][t * NP + i] = ir;
     }
+    line_rows<NP>(B, cx, ux, out);
 #pragma unroll
-    for (int i = 0; i < NP; ++i) {
-      s_uxx[e][t * NP + i] = dot_row<NP>(B, i, ux) * invJx;
-      s_uyx[e][t * NP + i] = dot_row<NP>(B, i, uy) * invJx;
-      // x stiffness self-coupling of diag(A): d/d(1/rho[i,t]) = cxs * sum_k W2[i][k] Mb[k,t]
-      double s = B.W2[i][0] * Mbr[0];
+    for (int i = 0; i < NP; ++i) s_uxx[e][t * NP + i] = out[i];
+    line_rows<NP>(B, cx, uy, out);
 #pragma unroll
-      for (int k = 1; k < NP; ++k) s = fma(B.W2[i][k], Mbr[k], s);
-      s_ib[e][t * NP + i] = cxs * s;
-    }
+    for (int i = 0; i < NP; ++i) s_uyx[e][t * NP + i] = out[i];
+    // x stiffness self-coupling of diag(A): d/d(1/rho[i,t]) = cxs * sum_k W2[i][k] Mb[k,t]
+    const FixScale cd = fix_scale(alpha * B.w[t] * I.jy * invJx);
+    line_op<NP, false, false, true>(B.fW2, B.W2, &cd, Mbr, nullptr, none, out);
+#pragma unroll
+    for (int i = 0; i < NP; ++i) s_ib[e][t * NP + i] = out[i];
   }
   __syncthreads();
-  // ---- column of vc: y derivatives, source adjoint, y transposes, diag(A) y part and faces
-  double cux[NP], cuy[NP], cMb[NP], cir[NP];
-  double uxb[NP], uyb[NP], ib[NP];
+  // ---- column of vc: y derivatives, source adjoint, diag(A) y part and faces
+  double bxy[NP], byy[NP], ib[NP];
   if (vc.valid) {
     const int t = vc.t, e = vc.e;
+    {
+      double col[NP], uxy[NP], uyy[NP];
+#pragma unroll
+      for (int l = 0; l < NP; ++l) col[l] = s_ux[e][l * NP + t];
+      line_rows<NP>(B, cy, col, uxy);
+#pragma unroll
+      for (int l = 0; l < NP; ++l) col[l] = s_uy[e][l * NP + t];
+      line_rows<NP>(B, cy, col, uyy);
+#pragma unroll
+      for (int l = 0; l < NP; ++l) {
+        const int nd = l * NP + t;
+        const double uxx = s_uxx[e][nd], uyx = s_uyx[e][nd];
+        const double s = uxx + uyy[l];
+        const double Qb2 = a.bb[vc.base + nd] * (2.0 * alpha * s_m0[nd]);
+        s_bxx[e][nd] = Qb2 * (s + uxx);
+        s_byx[e][nd] = Qb2 * uxy[l];
+        bxy[l] = Qb2 * uyx;
+        byy[l] = Qb2 * (s + uyy[l]);
+      }
+    }
+    double Mb[NP], cir[NP], acc[NP];
 #pragma unroll
     for (int l = 0; l < NP; ++l) {
-      cux[l] = s_ux[e][l * NP + t]; cuy[l] = s_uy[e][l * NP + t]; cMb[l] = s_Mb[e][l * NP + t]; cir[l] = s_ir[e][l * NP + t];
+      Mb[l] = s_Mb[e][l * NP + t];
+      cir[l] = s_ir[e][l * NP + t];
+      acc[l] = fma(Mb[l], s_m0[l * NP + t], s_ib[e][l * NP + t]);
     }
-    const double cys = alpha * B.w[t] * I.jx * invJy;
-    double bxy[NP], byy[NP];
-#pragma unroll
-    for (int l = 0; l < NP; ++l) {
-      const long long n = vc.base + l * NP + t;
-      const double uxy = dot_row<NP>(B, l, cux) * invJy, uyy = dot_row<NP>(B, l, cuy) * invJy;
-      const double uxx = s_uxx[e][l * NP + t], uyx = s_uyx[e][l * NP + t];
-      const double s = uxx + uyy;
-      const double Qb2 = 2.0 * a.bb[n] * (B.w[t] * B.w[l] * I.jx * I.jy * alpha);
-      s_bxx[e][l * NP + t] = Qb2 * (s + uxx);
-      s_byx[e][l * NP + t] = Qb2 * uxy;
-      bxy[l] = Qb2 * uyx * invJy;
-      byy[l] = Qb2 * (s + uyy) * invJy;
-      // y stiffness self-coupling of diag(A)
-      double sm = B.W2[l][0] * cMb[0];
-#pragma unroll
-      for (int k = 1; k < NP; ++k) sm = fma(B.W2[l][k], cMb[k], sm);
-      ib[l] = cys * sm;
-    }
-    // y transposes of the source adjoint: ux[t,k] gets D[l][k] * bxy[l]
-#pragma unroll
-    for (int k = 0; k < NP; ++k) { uxb[k] = dot_col<NP>(B, k, bxy, 0.0); uyb[k] = dot_col<NP>(B, k, byy, 0.0); }
     // diag(A) face terms, x faces (t == 0: own R side; t == L: own L side)
     if (t == 0 || t == L) {
       int it;
       const long long pb = neighbour<NP>(tl, I, vc.ex, vc.ey, t == 0 ? -1 : 1, 0, &it);
       const int pi = t == 0 ? L : 0;
-      const double cself = (t == L ? -alpha * invJx * B.D[L][L] : alpha * invJx * B.D[0][0]);
 #pragma unroll
       for (int l = 0; l < NP; ++l) {
         const double pir = it >= 0 ? s_ir[it][l * NP + pi] : a.invr[pb + l * NP + pi];
         const long long pn = pb + l * NP + pi;
         const double pMb = it >= 0 ? s_Mb[it][l * NP + pi] : -(a.iMb[pn] * a.cinvM[pn]) * a.cinvM[pn];
-        const double wf = B.w[l] * I.jy;
-        ib[l] = fma(cMb[l] * cself, wf, ib[l]);
+        acc[l] = fma(Mb[l], s_s[0][t == L ? 1 : 0][l], acc[l]);
         const double iL = t == L ? cir[l] : pir, iR = t == L ? pir : cir[l];
         const bool own_wins = (t == L) ? !gt_nonneg(iR, iL) : gt_nonneg(iR, iL);
-        if (own_wins) ib[l] = fma((cMb[l] + pMb) * alpha * wf, eta * I.idx, ib[l]);
+        if (own_wins) acc[l] = fma(Mb[l] + pMb, s_p[0][l], acc[l]);
       }
     }
 #pragma unroll
@@ -653,46 +667,53 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_setup_rev(SetupRevArgs2D 
       const double pir = it >= 0 ? s_ir[it][pl * NP + t] : a.invr[pb + pl * NP + t];
       const long long pn = pb + pl * NP + t;
       const double pMb = it >= 0 ? s_Mb[it][pl * NP + t] : -(a.iMb[pn] * a.cinvM[pn]) * a.cinvM[pn];
-      const double wf = B.w[t] * I.jx;
-      ib[l] = fma(cMb[l] * (l == L ? -alpha * invJy * B.D[L][L] : alpha * invJy * B.D[0][0]), wf, ib[l]);
+      acc[l] = fma(Mb[l], s_s[1][s][t], acc[l]);
       const double iL = l == L ? cir[l] : pir, iR = l == L ? pir : cir[l];
       const bool own_wins = (l == L) ? !gt_nonneg(iR, iL) : gt_nonneg(iR, iL);
-      if (own_wins) ib[l] = fma((cMb[l] + pMb) * alpha * wf, eta * I.idy, ib[l]);
+      if (own_wins) acc[l] = fma(Mb[l] + pMb, s_p[1][t], acc[l]);
     }
+    // y stiffness self-coupling of diag(A), with the mass, x and face parts
+    const FixScale cd = fix_scale(alpha * B.w[t] * I.jx * invJy);
+    line_op<NP, false, false, true>(B.fW2, B.W2, &cd, Mb, acc, all, ib);
+  }
+  __syncthreads();
+  // ---- row of vr: x transposes of the source adjoint, in place: ux[t,l] gets sum_i D[i][t] * bxx[i,l] * invJx
+  if (vr.valid) {
+    const int t = vr.t, e = vr.e;
+    double v[NP], out[NP];
+#pragma unroll
+    for (int i = 0; i < NP; ++i) v[i] = s_bxx[e][t * NP + i];
+    line_cols<NP>(B, cx, v, out);
+#pragma unroll
+    for (int i = 0; i < NP; ++i) { s_bxx[e][t * NP + i] = out[i]; v[i] = s_byx[e][t * NP + i]; }
+    line_cols<NP>(B, cx, v, out);
+#pragma unroll
+    for (int i = 0; i < NP; ++i) s_byx[e][t * NP + i] = out[i];
   }
   __syncthreads();
   if (!vc.valid) return;
-  // ---- column of vc, final: x transposes of the source adjoint (need row data),
-  // mass part of diag(A), conversion to d/d rho and d/d alpha
+  // ---- column of vc, final: y transposes added to the x ones, conversion to d/d rho and d/d alpha
   const int t = vc.t, e = vc.e;
+  double acc[NP], uxb[NP], uyb[NP];
 #pragma unroll
-  for (int l = 0; l < NP; ++l) {
-    // ux[t,l] gets sum_i D[i][t] * bxx[i,l] * invJx (row l, x transpose at node t)
-    double sxv = 0.0, syv = 0.0;
+  for (int l = 0; l < NP; ++l) acc[l] = s_bxx[e][l * NP + t];
+  line_op<NP, true, true, true>(B.fD, B.D, &cy, bxy, acc, all, uxb);
 #pragma unroll
-    for (int i = 0; i < NP; ++i) {
-      sxv = fma(B.D[i][t], s_bxx[e][l * NP + i], sxv);
-      syv = fma(B.D[i][t], s_byx[e][l * NP + i], syv);
-    }
-    uxb[l] = fma(invJx, sxv, uxb[l]);
-    uyb[l] = fma(invJx, syv, uyb[l]);
-  }
+  for (int l = 0; l < NP; ++l) acc[l] = s_byx[e][l * NP + t];
+  line_op<NP, true, true, true>(B.fD, B.D, &cy, byy, acc, all, uyb);
 #pragma unroll
   for (int l = 0; l < NP; ++l) {
     const long long n = vc.base + l * NP + t;
-    const double ir = cir[l];
-    const double Mb = cMb[l];
+    const int nd = l * NP + t;
+    const double ir = s_ir[e][nd], Mb = s_Mb[e][nd];
     const double cmn = a.cm[n];
-    // d/d(1/rho) of diag(A): mass + row-phase x stiffness + column-phase y stiffness and faces
-    const double m0 = B.w[t] * B.w[l] * I.jx * I.jy;  // mass coefficient without 1/rho
-    const double ibt = fma(Mb, m0, s_ib[e][l * NP + t] + ib[l]);
     const double zs = a.Zs[n], zms = fma(cmn, a.Zm[n], zs);  // Zm + Zs, with Zm's mass coefficient
-    a.Qs[0][n] += uxb[l] * ir;
-    a.Qs[1][n] += uyb[l] * ir;
-    const double rb = -(fma(uxb[l], cux[l], uyb[l] * cuy[l]) * ir) - ir * fma(ibt, ir, zms);
-    a.Qs[2][n] += rb;
+    a.Qs[0][n] = fma(uxb[l], ir, a.Qs[0][n]);
+    a.Qs[1][n] = fma(uyb[l], ir, a.Qs[1][n]);
+    const double r = fma(uxb[l], s_ux[e][nd], fma(uyb[l], s_uy[e][nd], fma(ib[l], ir, zms)));
+    a.Qs[2][n] = fma(-ir, r, a.Qs[2][n]);
     // d/dalpha: Zs/alpha + Mb (M - mass)/alpha + bb b/alpha
-    a.anode[n] += fma(Mb, a.cM[n] - cmn, fma(a.bb[n], a.b[n], zs)) * I.ialpha;
+    a.anode[n] = fma(fma(Mb, a.cM[n] - cmn, fma(a.bb[n], a.b[n], zs)), I.ialpha, a.anode[n]);
   }
 }
 
