@@ -35,44 +35,60 @@ struct PdePrepArgs2D {
   double *ws_x, *ws_y;     // |u_x| + c, |u_y| + c
 };
 
+// What bounds it: FP64 issue (the source coefficients); the fourteen line derivatives are integer work in rolled loops.
 template <int NP>
 __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_pde_prep(PdePrepArgs2D a) {
   using TL = Tiling2D<NP>;
   constexpr int TE = TL::TE, NN = TL::NN;
-  // x-derivatives (physical) of mux, muy, rho, E, Sigma, u_x, u_y; 1/rho
-  __shared__ double s_dx[7][TE][NN];
+  // mux, muy, rho, E, Sigma, u_x, u_y: x-derivatives (physical); the fields, then their y-derivatives; 1/rho
+  __shared__ double s_dx[7][TE][NN], s_dy[7][TE][NN];
   __shared__ double s_ir[TE][NN];
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];
   const ElemView vr = elem_view<NP>(tl, I, 0), vc = elem_view<NP>(tl, I, 1);
   const BasisDev& B = a.B;
-  const double invJx = I.ijx, invJy = I.ijy;
+  const int nf = a.nl[0] ? 7 : 5;  // the velocity gradients serve the nonlocal source only
   if (vr.valid) {
     const int t = vr.t, e = vr.e;
-    double f[7][NP];
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
       const long long n = vr.base + t * NP + i;
-      const double r = a.q[2][n], ir = 1.0 / r;  // one FP64 divide per node, shared by both phases
-      s_ir[e][t * NP + i] = ir;
-      f[0][i] = a.q[0][n]; f[1][i] = a.q[1][n]; f[2][i] = r; f[3][i] = a.q[3][n]; f[4][i] = a.S[n];
-      f[5][i] = f[0][i] * ir; f[6][i] = f[1][i] * ir;
+      const int nd = t * NP + i;
+      const double mx = a.q[0][n], my = a.q[1][n], r = a.q[2][n], ir = reciprocal(r);
+      s_ir[e][nd] = ir;
+      s_dy[0][e][nd] = mx; s_dy[1][e][nd] = my; s_dy[2][e][nd] = r; s_dy[3][e][nd] = a.q[3][n]; s_dy[4][e][nd] = a.S[n];
+      s_dy[5][e][nd] = mx * ir; s_dy[6][e][nd] = my * ir;
     }
+    const FixScale sc = fix_scale(I.ijx);
+#pragma unroll 1
+    for (int v = 0; v < nf; ++v) {
+      double f[NP], d[NP];
 #pragma unroll
-    for (int v = 0; v < 7; ++v)
+      for (int i = 0; i < NP; ++i) f[i] = s_dy[v][e][t * NP + i];
+      line_rows<NP>(B, sc, f, d);
 #pragma unroll
-      for (int i = 0; i < NP; ++i) s_dx[v][e][t * NP + i] = dot_row<NP>(B, i, f[v]) * invJx;
+      for (int i = 0; i < NP; ++i) s_dx[v][e][t * NP + i] = d[i];
+    }
   }
   __syncthreads();
   if (!vc.valid) return;
   const int t = vc.t, e = vc.e;
-  double f[7][NP];
+  double f0[NP], f1[NP], f3[NP], f4[NP], u0[NP], u1[NP];
 #pragma unroll
   for (int l = 0; l < NP; ++l) {
-    const long long n = vc.base + l * NP + t;
-    const double ir = s_ir[e][l * NP + t];
-    f[0][l] = a.q[0][n]; f[1][l] = a.q[1][n]; f[2][l] = a.q[2][n]; f[3][l] = a.q[3][n]; f[4][l] = a.S[n];
-    f[5][l] = f[0][l] * ir; f[6][l] = f[1][l] * ir;
+    const int nd = l * NP + t;
+    f0[l] = s_dy[0][e][nd]; f1[l] = s_dy[1][e][nd]; f3[l] = s_dy[3][e][nd]; f4[l] = s_dy[4][e][nd];
+    u0[l] = s_dy[5][e][nd]; u1[l] = s_dy[6][e][nd];
+  }
+  const FixScale sc = fix_scale(I.ijy);
+#pragma unroll 1
+  for (int v = 0; v < nf; ++v) {  // in place: the column is the thread's own from here on
+    double f[NP], d[NP];
+#pragma unroll
+    for (int l = 0; l < NP; ++l) f[l] = s_dy[v][e][l * NP + t];
+    line_rows<NP>(B, sc, f, d);
+#pragma unroll
+    for (int l = 0; l < NP; ++l) s_dy[v][e][l * NP + t] = d[l];
   }
   const double g = I.gamma, gm = g - 1.0;
 #pragma unroll
@@ -80,12 +96,10 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_pde_prep(PdePrepArgs2D a)
     const long long n = vc.base + l * NP + t;
     const int nd = l * NP + t;
     const double mxx = s_dx[0][e][nd], myx = s_dx[1][e][nd], rx = s_dx[2][e][nd], Ex = s_dx[3][e][nd], Sx = s_dx[4][e][nd];
-    const double mxy = dot_row<NP>(B, l, f[0]) * invJy, myy = dot_row<NP>(B, l, f[1]) * invJy;
-    const double ry = dot_row<NP>(B, l, f[2]) * invJy, Ey = dot_row<NP>(B, l, f[3]) * invJy;
-    const double Sy = dot_row<NP>(B, l, f[4]) * invJy;
-    const double mx = f[0][l], my = f[1][l], en = f[3][l], Sg = f[4][l];
+    const double mxy = s_dy[0][e][nd], myy = s_dy[1][e][nd], ry = s_dy[2][e][nd], Ey = s_dy[3][e][nd], Sy = s_dy[4][e][nd];
+    const double mx = f0[l], my = f1[l], en = f3[l], Sg = f4[l];
     const double ir = s_ir[e][nd], ir2 = ir * ir, ir3 = ir2 * ir;
-    const double ux = f[5][l], uy = f[6][l];
+    const double ux = u0[l], uy = u1[l];
     // quotient-rule velocity gradients of the local source (adjoint_pde.jl:163-164)
     const double uxx = (mxx - ux * rx) * ir, uyy = (myy - uy * ry) * ir;
     const double m2 = fma(mx, mx, my * my);
@@ -118,13 +132,13 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_pde_prep(PdePrepArgs2D a)
     a.src[0][n] = c0; a.src[1][n] = c1; a.src[2][n] = c2; a.src[3][n] = c3; a.src[4][n] = c4;
     a.src[5][n] = c5; a.src[6][n] = c6; a.src[7][n] = c7; a.src[8][n] = c8; a.src[9][n] = c9;
     a.invr[n] = ir;
-    const double cs = sqrt(g * P * ir);
+    const double cs = square_root(g * P * ir);
     a.ws_x[n] = fabs(ux) + cs;
     a.ws_y[n] = fabs(uy) + cs;
     if (a.nl[0]) {
       // nodal-velocity gradients (adjoint_pde.jl:391-404)
       const double nxx = s_dx[5][e][nd], nyx = s_dx[6][e][nd];
-      const double nxy = dot_row<NP>(B, l, f[5]) * invJy, nyy = dot_row<NP>(B, l, f[6]) * invJy;
+      const double nxy = s_dy[5][e][nd], nyy = s_dy[6][e][nd];
       const double dv = nxx + nyy;
       double R = fma(dv, dv, nxx * nxx);
       R = fma(2.0 * nxy, nyx, R);
@@ -153,30 +167,37 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_pde_b(PdeBArgs2D a) {
   const BasisDev& B = a.B;
   if (vr.valid) {
     const int t = vr.t, e = vr.e;
-    double am[NP], aE[NP];
+    double am[NP], aE[NP], d[NP];
 #pragma unroll
     for (int i = 0; i < NP; ++i) { const long long n = vr.base + t * NP + i; am[i] = a.a[0][n]; aE[i] = a.a[3][n]; }
+    const FixScale sc = fix_scale(I.ijx);
+    line_rows<NP>(B, sc, am, d);
 #pragma unroll
-    for (int i = 0; i < NP; ++i) {
-      s_d[0][e][t * NP + i] = dot_row<NP>(B, i, am) * I.ijx;
-      s_d[1][e][t * NP + i] = dot_row<NP>(B, i, aE) * I.ijx;
-    }
+    for (int i = 0; i < NP; ++i) s_d[0][e][t * NP + i] = d[i];
+    line_rows<NP>(B, sc, aE, d);
+#pragma unroll
+    for (int i = 0; i < NP; ++i) s_d[1][e][t * NP + i] = d[i];
   }
   __syncthreads();
   if (!vc.valid) return;
   const int t = vc.t, e = vc.e;
-  double am[NP], aE[NP];
+  double am[NP], aE[NP], acc[NP], div[NP], aEy[NP];
 #pragma unroll
-  for (int l = 0; l < NP; ++l) { const long long n = vc.base + l * NP + t; am[l] = a.a[1][n]; aE[l] = a.a[3][n]; }
+  for (int l = 0; l < NP; ++l) {
+    const long long n = vc.base + l * NP + t;
+    am[l] = a.a[1][n]; aE[l] = a.a[3][n]; acc[l] = s_d[0][e][l * NP + t];
+  }
+  const FixScale sc = fix_scale(I.ijy);
+  line_rows_acc<NP>(B, sc, am, acc, div);  // d_x a_mux + d_y a_muy
+  line_rows<NP>(B, sc, aE, aEy);
   const double cw = I.alpha * B.w[t] * I.jx * I.jy;
 #pragma unroll
   for (int l = 0; l < NP; ++l) {
     const long long n = vc.base + l * NP + t;
     const int nd = l * NP + t;
-    const double amy_y = dot_row<NP>(B, l, am) * I.ijy, aE_y = dot_row<NP>(B, l, aE) * I.ijy;
     const double ir = a.invr[n];
     const double ux = a.mx[n] * ir, uy = a.my[n] * ir;
-    const double v = fma(aE_y, uy, fma(s_d[1][e][nd], ux, s_d[0][e][nd] + amy_y));
+    const double v = fma(aEy[l], uy, fma(s_d[1][e][nd], ux, div[l]));
     a.b[n] = v * (cw * B.w[l]);
   }
 }
@@ -221,17 +242,19 @@ __device__ __forceinline__ AdjFlux pde_adjoint_flux(double g, double mx, double 
   return F;
 }
 
-struct AdjFace { double a[4], f[4], ws; };
-
+// What bounds it: FP64 issue (adjoint fluxes, sources, faces). Volume terms and the nonlocal source's derivatives are
+// integer line operations; the faces take f_partner - f_own - lambda (a_L - a_R) (see llf_jump). 8 x 128^2 P3: 793 us with
+// FP64 contractions, 544 us now; k2_pde_prep and k2_pde_b together 285 and 165 us per launch.
 template <int NP>
 __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_pde_rk(PdeRkArgs2D a) {
   using TL = Tiling2D<NP>;
   constexpr int TE = TL::TE, NN = TL::NN, L = TL::L, TX = TL::TX, TY = TL::TY;
   __shared__ double s_fy[4][TE][NN];    // adjoint y fluxes
-  __shared__ double s_k[4][TE][NN];     // operator, x part
+  __shared__ double s_k[4][TE][NN];     // x fluxes, then the operator's x part
   __shared__ double s_a[4][TE][NN];     // adjoint stage input
-  __shared__ double s_w[3][TE][NN];     // x-derivative parts of W_x, W_y, div C
-  __shared__ AdjFace s_xf[TE][NP][2];   // x-face node data (left, right) per row
+  __shared__ double s_w[3][TE][NN];     // nonlocal source: x products, then the x-derivative parts of W_x, W_y, div C
+  __shared__ double s_fx[4][TE][NP][2]; // x fluxes at the row ends (left, right)
+  __shared__ double s_wx[TE][NP][2];    // wave speeds there
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];
   const ElemView vr = elem_view<NP>(tl, I, 0), vc = elem_view<NP>(tl, I, 1);
@@ -239,184 +262,194 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_pde_rk(PdeRkArgs2D a) {
   const double g = I.gamma;
   const double invJx = I.ijx, invJy = I.ijy;
   const bool nonlocal = a.Pi != nullptr;
+  auto ends = [](int k) { return k == 0 || k == L; };
+  auto flux = [&](long long n, const double av[4]) {
+    return pde_adjoint_flux(g, a.q[0][n], a.q[1][n], a.q[2][n], a.q[3][n], a.S[n], a.invr[n], av);
+  };
 
-  // ---- phase 1 (row of vr): adjoint fluxes, x volume term, x-face data, x parts of the nonlocal source
+  // ---- phase 1 (row of vr): adjoint fluxes, x-face data, products of the nonlocal source
   if (vr.valid) {
     const int t = vr.t, e = vr.e;
-    double fx[4][NP];
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
       const long long n = vr.base + t * NP + i;
+      const int nd = t * NP + i;
       const double av[4] = {a.a[0][n], a.a[1][n], a.a[2][n], a.a[3][n]};
-      const AdjFlux F = pde_adjoint_flux(g, a.q[0][n], a.q[1][n], a.q[2][n], a.q[3][n], a.S[n], a.invr[n], av);
+      const AdjFlux F = flux(n, av);
 #pragma unroll
-      for (int c = 0; c < 4; ++c) { fx[c][i] = F.fx[c]; s_fy[c][e][t * NP + i] = F.fy[c]; s_a[c][e][t * NP + i] = av[c]; }
-      if (i == 0 || i == L) {
-        AdjFace& fs = s_xf[e][t][i == 0 ? 0 : 1];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) { fs.a[c] = av[c]; fs.f[c] = F.fx[c]; }
-        fs.ws = a.ws_x[n];
+      for (int c = 0; c < 4; ++c) {
+        s_k[c][e][nd] = F.fx[c]; s_fy[c][e][nd] = F.fy[c]; s_a[c][e][nd] = av[c];
+        if (i == 0 || i == L) s_fx[c][e][t][i == 0 ? 0 : 1] = F.fx[c];
+      }
+      if (i == 0 || i == L) s_wx[e][t][i == 0 ? 0 : 1] = a.ws_x[n];
+      if (nonlocal) {
+        const double P = a.Pi[n], nxx = a.nl[0][n], nxy = a.nl[2][n], nyy = a.nl[3][n];
+        s_w[0][e][nd] = P * (nxx + nyy + nxx); s_w[1][e][nd] = P * nxy; s_w[2][e][nd] = P * a.nl[4][n];
       }
     }
-#pragma unroll
-    for (int c = 0; c < 4; ++c)
-#pragma unroll
-      for (int i = 0; i < NP; ++i) s_k[c][e][t * NP + i] = invJx * dot_row<NP>(B, i, fx[c]);
     if (nonlocal) {
-      double pd[NP], pxx[NP], pxy[NP], cx[NP];
+      const FixScale sc = fix_scale(invJx);
+#pragma unroll 1
+      for (int v = 0; v < 3; ++v) {
+        double f[NP], d[NP];
 #pragma unroll
-      for (int i = 0; i < NP; ++i) {
-        const long long n = vr.base + t * NP + i;
-        const double P = a.Pi[n], nxx = a.nl[0][n], nxy = a.nl[2][n], nyy = a.nl[3][n];
-        pd[i] = P * (nxx + nyy); pxx[i] = P * nxx; pxy[i] = P * nxy; cx[i] = P * a.nl[4][n];
-      }
+        for (int i = 0; i < NP; ++i) f[i] = s_w[v][e][t * NP + i];
+        line_rows<NP>(B, sc, f, d);
 #pragma unroll
-      for (int i = 0; i < NP; ++i) {
-        s_w[0][e][t * NP + i] = dot_row<NP>(B, i, pd) * invJx + dot_row<NP>(B, i, pxx) * invJx;
-        s_w[1][e][t * NP + i] = dot_row<NP>(B, i, pxy) * invJx;
-        s_w[2][e][t * NP + i] = dot_row<NP>(B, i, cx) * invJx;
+        for (int i = 0; i < NP; ++i) s_w[v][e][t * NP + i] = d[i];
       }
     }
   }
   __syncthreads();
-  // ---- phase 2 (row of vr): x faces; adjoint LLF (adjoint_pde.jl:89-128) with the
+  // ---- phase 2 (row of vr): x volume term and x faces; adjoint LLF (adjoint_pde.jl:89-128) with the
   // forward's face signs flipped (:275-289); the owner computes its side
   if (vr.valid) {
     const int t = vr.t, e = vr.e;
-    auto fetch = [&](int s) {
+    double pa[2][4], pf[2][4], lam[2];
+    const int sf = first_side(vr.ext, TX);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int s = h == 0 ? sf : 1 - sf;
       int it;
       const long long pb = neighbour<NP>(tl, I, vr.ex, vr.ey, s == 0 ? -1 : 1, 0, &it);
-      AdjFace pf;
+      const int nd = t * NP + (s == 0 ? L : 0);
+      double av[4], fv[4], ws;
       if (it >= 0) {
-        pf = s_xf[it][t][s == 0 ? 1 : 0];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) { av[c] = s_a[c][it][nd]; fv[c] = s_fx[c][it][t][1 - s]; }
+        ws = s_wx[it][t][1 - s];
       } else {
-        const long long n = pb + t * NP + (s == 0 ? L : 0);
+        const long long n = pb + nd;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) pf.a[c] = a.a[c][n];
-        const AdjFlux F = pde_adjoint_flux(g, a.q[0][n], a.q[1][n], a.q[2][n], a.q[3][n], a.S[n], a.invr[n], pf.a);
+        for (int c = 0; c < 4; ++c) av[c] = a.a[c][n];
+        const AdjFlux F = flux(n, av);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) pf.f[c] = F.fx[c];
-        pf.ws = a.ws_x[n];
+        for (int c = 0; c < 4; ++c) fv[c] = F.fx[c];
+        ws = a.ws_x[n];
       }
-      return pf;
-    };
-    const int sf = first_side(vr.ext, TX);
-    const AdjFace pA = fetch(sf), pB = fetch(1 - sf);
+      const double own = s_wx[e][t][s];
+      const double mag = s == 0 ? max_nonneg(own, ws) : max_nonneg(ws, own);
 #pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      const AdjFace& pf = (s == sf) ? pA : pB;
-      const AdjFace& of = s_xf[e][t][s];
-      const AdjFace& Ls = s == 0 ? pf : of;
-      const AdjFace& Rs = s == 0 ? of : pf;
-      const double lam = max_nonneg(Rs.ws, Ls.ws);
-      const int io = s == 0 ? 0 : L;
-      const double cf = s == 0 ? -invJx * B.iw0 : invJx * B.iwL;
+      for (int d = 0; d < 2; ++d) {  // register arrays by the run-time side
+        if (d != s) continue;
+        lam[d] = mag;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const double fs = 0.5 * fma(-lam, Ls.a[c] - Rs.a[c], Ls.f[c] + Rs.f[c]);
-        s_k[c][e][t * NP + io] = fma(cf, fs - of.f[c], s_k[c][e][t * NP + io]);
+        for (int c = 0; c < 4; ++c) { pa[d][c] = av[c]; pf[d][c] = fv[c]; }
       }
+    }
+    // fs - f_own = (f_partner - f_own - lambda (a_L - a_R)) / 2; a_L - a_R = +-(a_partner - a_own)
+    const double cf0 = -0.5 * invJx * B.iw0, cfL = 0.5 * invJx * B.iwL;
+    const FixScale sc = fix_scale(invJx);
+#pragma unroll 1
+    for (int c = 0; c < 4; ++c) {
+      double f[NP], acc[NP], k[NP];
+#pragma unroll
+      for (int i = 0; i < NP; ++i) f[i] = s_k[c][e][t * NP + i];
+      acc[0] = cf0 * llf_jump(pick4(pf[0], c), f[0], -lam[0], pick4(pa[0], c) - s_a[c][e][t * NP]);
+      acc[L] = cfL * llf_jump(pick4(pf[1], c), f[L], lam[1], pick4(pa[1], c) - s_a[c][e][t * NP + L]);
+      line_op<NP, false, true, true>(B.fD, B.D, &sc, f, acc, ends, k);
+#pragma unroll
+      for (int i = 0; i < NP; ++i) s_k[c][e][t * NP + i] = k[i];
     }
   }
   __syncthreads();
   if (!vc.valid) return;
   // ---- phase 3 (column of vc): y volume term, y faces, sources, RK combination
   const int t = vc.t, e = vc.e;
-  double kc[4][NP];
+  double pa[2][4], pf[2][4], lam[2];
+  {
+    const int sf = first_side(vc.eyt, TY);
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    double fyc[NP];
+    for (int h = 0; h < 2; ++h) {
+      const int s = h == 0 ? sf : 1 - sf;
+      int it;
+      const long long pb = neighbour<NP>(tl, I, vc.ex, vc.ey, 0, s == 0 ? -1 : 1, &it);
+      const int nd = (s == 0 ? L : 0) * NP + t;
+      double av[4], fv[4];
+      if (it >= 0) {
 #pragma unroll
-    for (int l = 0; l < NP; ++l) fyc[l] = s_fy[c][e][l * NP + t];
+        for (int c = 0; c < 4; ++c) { av[c] = s_a[c][it][nd]; fv[c] = s_fy[c][it][nd]; }
+      } else {
+        const long long n = pb + nd;
 #pragma unroll
-    for (int l = 0; l < NP; ++l) kc[c][l] = fma(invJy, dot_row<NP>(B, l, fyc), s_k[c][e][l * NP + t]);
-  }
-  auto own_y = [&](int s) {
-    const int nd = (s == 0 ? 0 : L) * NP + t;
-    AdjFace f;
+        for (int c = 0; c < 4; ++c) av[c] = a.a[c][n];
+        const AdjFlux F = flux(n, av);
 #pragma unroll
-    for (int c = 0; c < 4; ++c) { f.a[c] = s_a[c][e][nd]; f.f[c] = s_fy[c][e][nd]; }
-    f.ws = a.ws_y[vc.base + nd];
-    return f;
-  };
-  auto fetchy = [&](int s) {
-    int it;
-    const long long pb = neighbour<NP>(tl, I, vc.ex, vc.ey, 0, s == 0 ? -1 : 1, &it);
-    const int nd = (s == 0 ? L : 0) * NP + t;
-    AdjFace pf;
-    if (it >= 0) {
+        for (int c = 0; c < 4; ++c) fv[c] = F.fy[c];
+      }
+      const double ws = a.ws_y[pb + nd], own = a.ws_y[vc.base + (s == 0 ? 0 : L) * NP + t];
+      const double mag = s == 0 ? max_nonneg(own, ws) : max_nonneg(ws, own);
 #pragma unroll
-      for (int c = 0; c < 4; ++c) { pf.a[c] = s_a[c][it][nd]; pf.f[c] = s_fy[c][it][nd]; }
-    } else {
-      const long long n = pb + nd;
+      for (int d = 0; d < 2; ++d) {
+        if (d != s) continue;
+        lam[d] = mag;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) pf.a[c] = a.a[c][n];
-      const AdjFlux F = pde_adjoint_flux(g, a.q[0][n], a.q[1][n], a.q[2][n], a.q[3][n], a.S[n], a.invr[n], pf.a);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) pf.f[c] = F.fy[c];
-    }
-    pf.ws = a.ws_y[pb + nd];
-    return pf;
-  };
-  const int sf = first_side(vc.eyt, TY);
-  const AdjFace qA = fetchy(sf), qB = fetchy(1 - sf);
-#pragma unroll
-  for (int s = 0; s < 2; ++s) {
-    const AdjFace& pf = (s == sf) ? qA : qB;
-    const AdjFace of = own_y(s);
-    const AdjFace& Ls = s == 0 ? pf : of;
-    const AdjFace& Rs = s == 0 ? of : pf;
-    const double lam = max_nonneg(Rs.ws, Ls.ws);
-    const int lo = s == 0 ? 0 : L;
-    const double cf = s == 0 ? -invJy * B.iw0 : invJy * B.iwL;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const double fs = 0.5 * fma(-lam, Ls.a[c] - Rs.a[c], Ls.f[c] + Rs.f[c]);
-      kc[c][lo] = fma(cf, fs - of.f[c], kc[c][lo]);
+        for (int c = 0; c < 4; ++c) { pa[d][c] = av[c]; pf[d][c] = fv[c]; }
+      }
     }
   }
+  const FixScale sc = fix_scale(invJy);
   // nonlocal source, y parts (adjoint_pde.jl:420-466)
   double Wx[NP], Wy[NP], dC[NP];
   if (nonlocal) {
-    double pd[NP], pyx[NP], pyy[NP], cy[NP];
+    double f[3][NP], acc[NP];
 #pragma unroll
     for (int l = 0; l < NP; ++l) {
       const long long n = vc.base + l * NP + t;
-      const double P = a.Pi[n], nxx = a.nl[0][n], nyx = a.nl[1][n], nyy = a.nl[3][n];
-      pd[l] = P * (nxx + nyy); pyx[l] = P * nyx; pyy[l] = P * nyy; cy[l] = P * a.nl[5][n];
+      const double P = a.Pi[n], nyy = a.nl[3][n];
+      f[0][l] = P * a.nl[1][n]; f[1][l] = P * (a.nl[0][n] + nyy + nyy); f[2][l] = P * a.nl[5][n];
     }
 #pragma unroll
-    for (int l = 0; l < NP; ++l) {
-      const int nd = l * NP + t;
-      Wx[l] = s_w[0][e][nd] + dot_row<NP>(B, l, pyx) * invJy;
-      Wy[l] = (dot_row<NP>(B, l, pd) * invJy + s_w[1][e][nd]) + dot_row<NP>(B, l, pyy) * invJy;
-      dC[l] = s_w[2][e][nd] + dot_row<NP>(B, l, cy) * invJy;
-    }
+    for (int l = 0; l < NP; ++l) acc[l] = s_w[0][e][l * NP + t];
+    line_rows_acc<NP>(B, sc, f[0], acc, Wx);
+#pragma unroll
+    for (int l = 0; l < NP; ++l) acc[l] = s_w[1][e][l * NP + t];
+    line_rows_acc<NP>(B, sc, f[1], acc, Wy);
+#pragma unroll
+    for (int l = 0; l < NP; ++l) acc[l] = s_w[2][e][l * NP + t];
+    line_rows_acc<NP>(B, sc, f[2], acc, dC);
   }
-  const double c2dt = a.c2 * I.dt;
+  // the sources and the x part, summed with the y part
+  double kc[4][NP];
 #pragma unroll
   for (int l = 0; l < NP; ++l) {
     const long long n = vc.base + l * NP + t;
     const int nd = l * NP + t;
-    const double a0 = s_a[0][e][nd], a1 = s_a[1][e][nd], a2 = s_a[2][e][nd], a3 = s_a[3][e][nd];
+    const double a0 = s_a[0][e][nd], a1 = s_a[1][e][nd], a3 = s_a[3][e][nd];
     // minus the local source
-    kc[0][l] -= fma(a0, a.src[0][n], fma(a1, a.src[1][n], a3 * a.src[2][n]));
-    kc[1][l] -= fma(a0, a.src[3][n], fma(a1, a.src[4][n], a3 * a.src[5][n]));
-    kc[2][l] -= fma(a0, a.src[6][n], fma(a1, a.src[7][n], a3 * a.src[8][n]));
-    kc[3][l] -= a3 * a.src[9][n];
+    kc[0][l] = s_k[0][e][nd] - fma(a0, a.src[0][n], fma(a1, a.src[1][n], a3 * a.src[2][n]));
+    kc[1][l] = s_k[1][e][nd] - fma(a0, a.src[3][n], fma(a1, a.src[4][n], a3 * a.src[5][n]));
+    kc[2][l] = s_k[2][e][nd] - fma(a0, a.src[6][n], fma(a1, a.src[7][n], a3 * a.src[8][n]));
+    kc[3][l] = fma(-a3, a.src[9][n], s_k[3][e][nd]);
     if (nonlocal) {
-      const double ir = a.invr[n];
-      kc[0][l] += -2.0 * Wx[l] * ir;
-      kc[1][l] += -2.0 * Wy[l] * ir;
+      const double ir = a.invr[n], ir2 = -2.0 * ir;
+      kc[0][l] = fma(Wx[l], ir2, kc[0][l]);
+      kc[1][l] = fma(Wy[l], ir2, kc[1][l]);
       const double wm = fma(Wx[l], a.q[0][n], Wy[l] * a.q[1][n]);
-      kc[2][l] += fma(a.Pi[n], a.nl[6][n], dC[l]) * ir + 2.0 * wm * (ir * ir);
+      kc[2][l] = fma(fma(a.Pi[n], a.nl[6][n], dC[l]) - wm * ir2, ir, kc[2][l]);
     }
-    const double as[4] = {a0, a1, a2, a3};
+  }
+  const double cf0 = -0.5 * invJy * B.iw0, cfL = 0.5 * invJy * B.iwL;
+  const double c2dt = a.c2 * I.dt;
+  const bool with_an = __double_as_longlong(a.c0) != 0;
+#pragma unroll 1
+  for (int c = 0; c < 4; ++c) {
+    double f[NP], acc[NP], k[NP];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      if (a.k_out[c]) a.k_out[c][n] = kc[c][l];
-      double val = fma(c2dt, kc[c][l], a.c1 * as[c]);
-      if (a.c0 != 0.0) val = fma(a.c0, a.an[c][n], val);
+    for (int l = 0; l < NP; ++l) {
+      f[l] = s_fy[c][e][l * NP + t];
+      const double r[4] = {kc[0][l], kc[1][l], kc[2][l], kc[3][l]};
+      acc[l] = pick4(r, c);
+    }
+    acc[0] = fma(cf0, llf_jump(pick4(pf[0], c), f[0], -lam[0], pick4(pa[0], c) - s_a[c][e][t]), acc[0]);
+    acc[L] = fma(cfL, llf_jump(pick4(pf[1], c), f[L], lam[1], pick4(pa[1], c) - s_a[c][e][L * NP + t]), acc[L]);
+    line_rows_acc<NP>(B, sc, f, acc, k);
+#pragma unroll
+    for (int l = 0; l < NP; ++l) {
+      const long long n = vc.base + l * NP + t;
+      if (a.k_out[c]) a.k_out[c][n] = k[l];
+      double val = fma(c2dt, k[l], a.c1 * s_a[c][e][l * NP + t]);
+      if (with_an) val = fma(a.c0, a.an[c][n], val);
       if (a.ao[c]) a.ao[c][n] = val;
     }
   }

@@ -32,63 +32,75 @@ struct SensRhsArgs2D {
   double* b_out;
 };
 
+// What bounds it: FP64 issue; the twelve line derivatives are integer work in rolled loops over the fields. With
+// k2_sens_hyp_rk 393 us per launch on average with FP64 contractions, 199 us now (2 x 256^2 P3).
 template <int NP>
 __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_sens_rhs(SensRhsArgs2D a) {
   using TL = Tiling2D<NP>;
   constexpr int TE = TL::TE, NN = TL::NN;
   constexpr int NQ = 6;  // u_x, u_y, s_x, s_y, Sigma, sigma/rho
-  __shared__ double s_v[NQ][TE][NN];
-  __shared__ double s_dx[NQ][TE][NN];
+  __shared__ double s_v[NQ][TE][NN];   // the fields, then their y derivatives
+  __shared__ double s_dx[NQ][TE][NN];  // x derivatives
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];
   const ElemView vr = elem_view<NP>(tl, I, 0), vc = elem_view<NP>(tl, I, 1);
   const BasisDev& B = a.B;
   if (vr.valid) {
     const int t = vr.t, e = vr.e;
-    double v[NQ][NP];
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
       const long long n = vr.base + t * NP + i;
+      const int nd = t * NP + i;
       const double ir = a.invr[n];
       const double ux = a.q[0][n] * ir, uy = a.q[1][n] * ir, sr = a.s[2][n];
-      v[0][i] = ux; v[1][i] = uy;
-      v[2][i] = (a.s[0][n] - ux * sr) * ir;
-      v[3][i] = (a.s[1][n] - uy * sr) * ir;
-      v[4][i] = a.S[n];
-      v[5][i] = sr * ir;
-#pragma unroll
-      for (int c = 0; c < NQ; ++c) s_v[c][e][t * NP + i] = v[c][i];
+      s_v[0][e][nd] = ux; s_v[1][e][nd] = uy;
+      s_v[2][e][nd] = (a.s[0][n] - ux * sr) * ir;
+      s_v[3][e][nd] = (a.s[1][n] - uy * sr) * ir;
+      s_v[4][e][nd] = a.S[n];
+      s_v[5][e][nd] = sr * ir;
     }
+    const FixScale sc = fix_scale(I.ijx);
+#pragma unroll 1
+    for (int c = 0; c < NQ; ++c) {
+      double v[NP], d[NP];
 #pragma unroll
-    for (int c = 0; c < NQ; ++c)
+      for (int i = 0; i < NP; ++i) v[i] = s_v[c][e][t * NP + i];
+      line_rows<NP>(B, sc, v, d);
 #pragma unroll
-      for (int i = 0; i < NP; ++i) s_dx[c][e][t * NP + i] = I.ijx * dot_row<NP>(B, i, v[c]);
+      for (int i = 0; i < NP; ++i) s_dx[c][e][t * NP + i] = d[i];
+    }
   }
   __syncthreads();
   if (!vc.valid) return;
   const int t = vc.t, e = vc.e;
-  double dy[NQ][NP];
+  double so[NP];  // sigma / rho
 #pragma unroll
-  for (int c = 0; c < NQ; ++c) {
-    double col[NP];
+  for (int l = 0; l < NP; ++l) so[l] = s_v[5][e][l * NP + t];
+  const FixScale sc = fix_scale(I.ijy);
+#pragma unroll 1
+  for (int c = 0; c < NQ; ++c) {  // in place: the column is the thread's own from here on
+    double v[NP], d[NP];
 #pragma unroll
-    for (int l = 0; l < NP; ++l) col[l] = s_v[c][e][l * NP + t];
+    for (int l = 0; l < NP; ++l) v[l] = s_v[c][e][l * NP + t];
+    line_rows<NP>(B, sc, v, d);
 #pragma unroll
-    for (int l = 0; l < NP; ++l) dy[c][l] = I.ijy * dot_row<NP>(B, l, col);
+    for (int l = 0; l < NP; ++l) s_v[c][e][l * NP + t] = d[l];
   }
-  const double al = I.alpha;
+  const double wa = B.w[t] * (I.jx * I.jy) * I.alpha;
 #pragma unroll
   for (int l = 0; l < NP; ++l) {
     const int nd = l * NP + t;
     const long long n = vc.base + nd;
     const double uxx = s_dx[0][e][nd], uyx = s_dx[1][e][nd], sxx = s_dx[2][e][nd], syx = s_dx[3][e][nd];
     const double Sx = s_dx[4][e][nd], dxs = s_dx[5][e][nd];
-    const double uxy = dy[0][l], uyy = dy[1][l], sxy = dy[2][l], syy = dy[3][l], Sy = dy[4][l], dys = dy[5][l];
+    const double uxy = s_v[0][e][nd], uyy = s_v[1][e][nd], sxy = s_v[2][e][nd], syy = s_v[3][e][nd];
+    const double Sy = s_v[4][e][nd], dys = s_v[5][e][nd];
     const double divu = uxx + uyy, divs = sxx + syy;
-    const double Rp = al * (divu * divu + uxx * uxx + 2.0 * uxy * uyx + uyy * uyy);
-    const double Rs = al * (2.0 * divu * divs + 2.0 * (uxx * sxx + uxy * syx + uyx * sxy + uyy * syy));
-    const double bp = Rs + s_v[5][e][nd] * Rp - al * (dxs * Sx + dys * Sy) * a.invr[n];
-    a.b_out[n] = (B.w[t] * B.w[l]) * (I.jx * I.jy) * bp;
+    // Rp / alpha and Rs / (2 alpha)
+    const double Rp = fma(divu, divu, fma(uxx, uxx, fma(uyy, uyy, 2.0 * uxy * uyx)));
+    const double Rs = fma(divu, divs, fma(uxx, sxx, fma(uyy, syy, fma(uxy, syx, uyx * sxy))));
+    const double b = fma(so[l], Rp, fma(2.0, Rs, -(fma(dxs, Sx, dys * Sy) * a.invr[n])));
+    a.b_out[n] = (wa * B.w[l]) * b;
   }
 }
 
@@ -132,163 +144,38 @@ struct SensHypArgs2D {
   int* status;
 };
 
-struct SensFace { double s[4], f[4], ws; };
+// The tangent fluxes, lifted with the primal wave speeds.
+struct TangentStage {
+  const SensHypArgs2D& a;
+  double g;
+  __device__ __forceinline__ FluxNode at(long long n) const {
+    FluxNode f;
+#pragma unroll
+    for (int v = 0; v < 4; ++v) f.q[v] = a.s[v][n];
+    const SensNode p = sens_phys(g, a.s_gamma, a.q[0][n], a.q[1][n], a.q[2][n], a.q[3][n], a.S[n], a.invr[n], f.q[0], f.q[1],
+                                 f.q[2], f.q[3], a.vs[n]);
+    f.fx0 = p.fx[0]; f.f1 = p.fx[1]; f.fx3 = p.fx[3]; f.fy1 = p.fy[1]; f.fy3 = p.fy[3];
+    return f;
+  }
+  __device__ __forceinline__ double partner_speed(int dir, long long n, const FluxNode&) const {
+    return dir == 0 ? a.ws_x[n] : a.ws_y[n];
+  }
+  __device__ __forceinline__ double speed_x(long long n, const FluxNode&) const { return a.ws_x[n]; }
+  __device__ __forceinline__ double speed_y(long long n, double, double) const { return a.ws_y[n]; }
+  __device__ __forceinline__ double qn(int v, long long n) const { return a.sn[v][n]; }
+  __device__ __forceinline__ void put(int v, long long n, double x) const {
+    if (a.k_out[v]) a.k_out[v][n] = x;
+    if (a.so[v]) a.so[v][n] = x;
+    if (a.status && nonfinite_bits(x)) flag_nonfinite(a.status);
+  }
+};
 
 template <int NP>
 __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_sens_hyp_rk(SensHypArgs2D a) {
-  using TL = Tiling2D<NP>;
-  constexpr int TE = TL::TE, NN = TL::NN, L = TL::L, TX = TL::TX, TY = TL::TY;
-  __shared__ double s_fy[4][TE][NN];
-  __shared__ double s_k[4][TE][NN];
-  __shared__ double s_s[4][TE][NN];
-  __shared__ SensFace s_xf[TE][NP][2];
-  __shared__ SensFace s_yf[TE][NP][2];
+  __shared__ StageSmem<NP, false> sm;
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];
-  const ElemView vr = elem_view<NP>(tl, I, 0), vc = elem_view<NP>(tl, I, 1);
-  const BasisDev& B = a.B;
-  const double g = I.gamma, sg = a.s_gamma;
-  const double invJx = I.ijx, invJy = I.ijy;
-  auto node = [&](long long n) {
-    return sens_phys(g, sg, a.q[0][n], a.q[1][n], a.q[2][n], a.q[3][n], a.S[n], a.invr[n], a.s[0][n], a.s[1][n],
-                     a.s[2][n], a.s[3][n], a.vs[n]);
-  };
-
-  // ---- phase 1 (rows): tangent fluxes, x volume term, x-face node data
-  if (vr.valid) {
-    const int t = vr.t, e = vr.e;
-    double fx[4][NP];
-#pragma unroll
-    for (int i = 0; i < NP; ++i) {
-      const long long n = vr.base + t * NP + i;
-      const SensNode sp = node(n);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) { fx[c][i] = sp.fx[c]; s_fy[c][e][t * NP + i] = sp.fy[c]; s_s[c][e][t * NP + i] = a.s[c][n]; }
-      if (i == 0 || i == L) {
-        SensFace& fs = s_xf[e][t][i == 0 ? 0 : 1];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) { fs.s[c] = a.s[c][n]; fs.f[c] = sp.fx[c]; }
-        fs.ws = a.ws_x[n];
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < 4; ++c)
-#pragma unroll
-      for (int i = 0; i < NP; ++i) s_k[c][e][t * NP + i] = -invJx * dot_row<NP>(B, i, fx[c]);
-  }
-  __syncthreads();
-  // ---- phase 2 (columns): y-face node data
-  if (vc.valid) {
-    const int t = vc.t, e = vc.e;
-#pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      const int nd = (s == 0 ? 0 : L) * NP + t;
-      SensFace& fs = s_yf[e][t][s];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) { fs.s[c] = s_s[c][e][nd]; fs.f[c] = s_fy[c][e][nd]; }
-      fs.ws = a.ws_y[vc.base + nd];
-    }
-  }
-  __syncthreads();
-  // ---- phase 3 (rows): x faces
-  if (vr.valid) {
-    const int t = vr.t, e = vr.e;
-    auto fetch = [&](int s) {
-      int it;
-      const long long pb = neighbour<NP>(tl, I, vr.ex, vr.ey, s == 0 ? -1 : 1, 0, &it);
-      SensFace pf;
-      if (it >= 0) {
-        pf = s_xf[it][t][s == 0 ? 1 : 0];
-      } else {
-        const long long n = pb + t * NP + (s == 0 ? L : 0);
-        const SensNode sp = node(n);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) { pf.s[c] = a.s[c][n]; pf.f[c] = sp.fx[c]; }
-        pf.ws = a.ws_x[n];
-      }
-      return pf;
-    };
-    const int sf = first_side(vr.ext, TX);
-    const SensFace pA = fetch(sf), pB = fetch(1 - sf);
-#pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      const SensFace& pf = (s == sf) ? pA : pB;
-      const SensFace& of = s_xf[e][t][s];
-      const SensFace& Ls = s == 0 ? pf : of;
-      const SensFace& Rs = s == 0 ? of : pf;
-      const double lam = max_nonneg(Rs.ws, Ls.ws);
-      const int io = s == 0 ? 0 : L;
-      const double cf = s == 0 ? invJx * B.iw0 : -invJx * B.iwL;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const double fs = 0.5 * fma(lam, Ls.s[c] - Rs.s[c], Ls.f[c] + Rs.f[c]);
-        s_k[c][e][t * NP + io] = fma(cf, fs - of.f[c], s_k[c][e][t * NP + io]);
-      }
-    }
-  }
-  __syncthreads();
-  if (!vc.valid) return;
-  // ---- phase 4 (columns): y volume term, y faces, RK combination
-  const int t = vc.t, e = vc.e;
-  double kc[4][NP];
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    double fyc[NP];
-#pragma unroll
-    for (int l = 0; l < NP; ++l) fyc[l] = s_fy[c][e][l * NP + t];
-#pragma unroll
-    for (int l = 0; l < NP; ++l) kc[c][l] = fma(-invJy, dot_row<NP>(B, l, fyc), s_k[c][e][l * NP + t]);
-  }
-  auto fetchy = [&](int s) {
-    int it;
-    const long long pb = neighbour<NP>(tl, I, vc.ex, vc.ey, 0, s == 0 ? -1 : 1, &it);
-    SensFace pf;
-    if (it >= 0) {
-      pf = s_yf[it][t][s == 0 ? 1 : 0];
-    } else {
-      const long long n = pb + (s == 0 ? L : 0) * NP + t;
-      const SensNode sp = node(n);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) { pf.s[c] = a.s[c][n]; pf.f[c] = sp.fy[c]; }
-      pf.ws = a.ws_y[n];
-    }
-    return pf;
-  };
-  const int sf = first_side(vc.eyt, TY);
-  const SensFace qA = fetchy(sf), qB = fetchy(1 - sf);
-#pragma unroll
-  for (int s = 0; s < 2; ++s) {
-    const SensFace& pf = (s == sf) ? qA : qB;
-    const SensFace& of = s_yf[e][t][s];
-    const SensFace& Ls = s == 0 ? pf : of;
-    const SensFace& Rs = s == 0 ? of : pf;
-    const double lam = max_nonneg(Rs.ws, Ls.ws);
-    const int lo = s == 0 ? 0 : L;
-    const double cf = s == 0 ? invJy * B.iw0 : -invJy * B.iwL;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const double fs = 0.5 * fma(lam, Ls.s[c] - Rs.s[c], Ls.f[c] + Rs.f[c]);
-      kc[c][lo] = fma(cf, fs - of.f[c], kc[c][lo]);
-    }
-  }
-  const double c2dt = a.c2 * I.dt;
-  bool bad = false;
-#pragma unroll
-  for (int l = 0; l < NP; ++l) {
-    const long long n = vc.base + l * NP + t;
-    double so[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      if (a.k_out[c]) a.k_out[c][n] = kc[c][l];
-      double val = fma(c2dt, kc[c][l], a.c1 * s_s[c][e][l * NP + t]);
-      if (a.c0 != 0.0) val = fma(a.c0, a.sn[c][n], val);
-      so[c] = val;
-      bad |= nonfinite_bits(val);
-    }
-#pragma unroll
-    for (int c = 0; c < 4; ++c) if (a.so[c]) a.so[c][n] = so[c];
-  }
-  if (bad) flag_nonfinite(a.status);
+  dg_stage<NP, false>(TangentStage{a, I.gamma}, a.B, tl, I, a.c0, a.c1, a.c2, a.k_out[0] != nullptr, sm);
 }
 
 }  // namespace igrgpu
