@@ -82,9 +82,19 @@ long long forward1d_scratch_fields(const Inst1DDesc&, int) { return E1_FIELDS + 
 // over a cluster of up to 16 SMs (at least 16 elements per CTA); below T1
 // elements the cluster barrier costs more than it saves (measured on GB300:
 // N_e = 64 and 128 run 10-20% faster on one CTA), and batches that fill the
-// GPU use one CTA per instance. A context setting overrides the choice, and
-// autotuning replaces it with a measurement (cluster_size).
-static int cluster_heuristic(Ctx& c, const Plan1D& P) {
+// GPU use one CTA per instance. For everything between, the cluster size is
+// the one with the shortest estimate of a solver iteration, in rounds of one
+// warp of elements per SM sub-partition: the longest instance (its rounds per
+// CTA plus the barriers, 0.8 for a CTA's and 1.6 for a cluster's; half a round
+// where the iterate fits shared memory, d1_local_ok), the batch's CTAs over the
+// resident slots (two per SM; three for two SMs with clusters above 2, which a
+// GPC packs less densely) and the batch's warps over the sub-partitions.
+// Measured (two steps of the adjoint, ms, 1 / chosen): 256 instances of
+// 64..1024 elements, PCG 102: 94 / 73 (2 CTAs); 40 of 25..400, PCG 30: 11.7 /
+// 7.5 (4); 8 of 56..900, PCG 30: 23.2 / 7.5 (8); 150 of 12..200: one CTA, 7.7
+// (8.0 with 2). A context setting overrides the choice, and autotuning replaces
+// it with a measurement (cluster_size).
+static int cluster_heuristic(Ctx& c, const Plan1D& P, int solver) {
   int sms = 0;
   cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device), "attr");
   const long long ni = (long long)P.inst.size();
@@ -92,6 +102,25 @@ static int cluster_heuristic(Ctx& c, const Plan1D& P) {
   for (auto& I : P.inst) min_ne = std::min(min_ne, I.ne);
   int cs = 1;
   while (cs < 16 && min_ne >= T1 && ni * cs * 2 * 2 <= sms && min_ne / (cs * 2) >= 16) cs *= 2;
+  if (cs > 1) return cs;
+  const int lanes = P.np <= 2 ? 2 : (P.np <= 4 ? 4 : 8);  // per element in node form
+  auto estimate = [&](int k) {
+    double longest = 0.0, slots = 0.0, warps = 0.0;
+    for (auto& I : P.inst) {
+      const int per = (I.ne + k - 1) / k, w = (per + 31) / 32;
+      const bool local = solver != 0 && per * lanes <= T1 / 2;
+      const double t = (local ? 0.5 : (w + 3) / 4) + (k == 1 ? 0.8 : 1.6);
+      longest = std::max(longest, t);
+      slots += k * t;
+      warps += (double)k * w;
+    }
+    return std::max(longest, std::max(slots / ((k <= 2 ? 2.0 : 1.5) * sms), warps / (4.0 * sms) + (k == 1 ? 0.8 : 1.6)));
+  };
+  double best = estimate(1);
+  for (int k = 2; k <= 16 && min_ne >= k; k *= 2) {
+    const double t = estimate(k);
+    if (t < 0.92 * best) { cs = k; best = t; }
+  }
   return cs;
 }
 
@@ -120,7 +149,7 @@ static void launch_1d(Ctx& c, Args& a, int n_inst, F launch, const char* what) {
 // run, timed with CUDA events; results do not depend on the choice.
 static int cluster_size(Ctx& c, const Plan1D& P, const Solve2DOpts& o, const double* q) {
   if (c.cluster1d > 0) return c.cluster1d;
-  const int h = cluster_heuristic(c, P);
+  const int h = cluster_heuristic(c, P, o.solver);
   if (!c.tune.on || !q || P.inst.empty()) return h;
   int ne_min = 1 << 30, ne_max = 0;
   long long ne_sum = 0;
