@@ -106,11 +106,13 @@ __device__ __forceinline__ Limb limbs(double v, int e) {
   const int sg = (__double2hiint(v) >> 31) | 1;
   return {(int)(t >> 32) * sg, (int)((unsigned)t >> 1) * sg};
 }
-// a + v, v in units of 2^(53 + PRE) / 2^(e - 1022), truncated
+// a + v, v in units of 2^(53 + PRE) / 2^(e - 1022), rounded to nearest: addends come back in the next solver iteration
+// or are summed over the mesh, where a truncation's bias would add up.
 template <int PRE>
 __device__ __forceinline__ long long add(long long a, double v, int e) {
   const long long s = __double2hiint(v) >> 31;
-  return a + ((long long)magnitude<PRE>(v, e) ^ s) - s;
+  const long long t = (long long)((magnitude<PRE + 1>(v, e) + 1) >> 1);
+  return a + (t ^ s) - s;
 }
 
 // G 2^(e - 1082) rounded to nearest, |G| < 2^62
@@ -317,10 +319,12 @@ __device__ __forceinline__ Limb mantissa(double v) {
   const int sg = ((int)hi >> 31) | 1;
   return {(int)__funnelshift_l(lo, (hi & 0xfffffu) | 0x100000u, 10) * sg, (int)((lo << 9) & 0x7fffffffu) * sg};
 }
+// A dropped product of two low words of one sign is a quarter unit on average; M carries it.
+constexpr long long LOW = 1LL << 29;
 // G c / 2^64 for |G| < 2^62 and c of 63 bits
 __device__ __forceinline__ long long times(long long G, Limb c) {
   const int gh = (int)(G >> 32), gl = (int)((unsigned)G >> 1);
-  const long long M = mad(gl, c.h, mad(gh, c.l, HALF));
+  const long long M = mad(gl, c.h, mad(gh, c.l, HALF + (c.h < 0 ? -LOW : LOW)));
   return mad((int)(M >> 32), 2, mad(gh, c.h, 0));
 }
 __device__ __forceinline__ long long sar(long long a, unsigned s) {
@@ -577,7 +581,7 @@ __device__ __forceinline__ bool product_line(const FixFlux<NP>& f, const FixDeri
   for (int i = 0; i < NP; ++i) {
     const int ph = (int)(f.P[i] >> 32), pl = (int)((unsigned)f.P[i] >> 1);
     const int gh = (int)(d.G[i] >> 32), gl = (int)((unsigned)d.G[i] >> 1);
-    const long long M = fix::mad(ph, gl, fix::mad(pl, gh, fix::HALF));
+    const long long M = fix::mad(ph, gl, fix::mad(pl, gh, fix::HALF + fix::LOW));
     long long v = fix::sar(fix::mad((int)(M >> 32), 2, fix::mad(ph, gh, 0)), e - ep);
     if (i == 0) v = fix::add<7>(v, z0, e);
     if (i == NP - 1) v = fix::add<7>(v, zL, e);
