@@ -30,6 +30,7 @@ struct Tiling2D {
   // keeps the rows 16-byte aligned (128-bit accesses, also without conflicts). 5 does it for P1; 9 and 25 are odd.
   static constexpr int SN = NP == 4 ? 18 : (NP == 2 ? 5 : NN);
   static constexpr int NT = TE * NP;       // threads per CTA (one per line)
+  static constexpr int NH = (NT + 31) / 32 * 32;  // threads of each half where rows and columns run side by side
   static constexpr int L = NP - 1;
 };
 
@@ -46,28 +47,33 @@ struct ElemView {
 // phase's faces and warp 1 the 8 interior ones, so the out-of-tile partner
 // work of a phase runs in one warp, with every lane on the same path.
 template <int NP>
-__device__ __forceinline__ ElemView elem_view(const Tile2D& tl, const Inst2D& I, int phase) {
+__device__ __forceinline__ ElemView elem_view(const Tile2D& tl, const Inst2D& I, int phase, int tid) {
   constexpr int TX = Tiling2D<NP>::TX, TY = Tiling2D<NP>::TY;
   ElemView v;
   if (NP == 4 && TX == 4 && TY == 4) {
-    const int w = threadIdx.x >> 5, k = (threadIdx.x >> 2) & 7;
-    v.t = threadIdx.x & 3;
+    const int w = tid >> 5, k = (tid >> 2) & 7;
+    v.t = tid & 3;
     const int across = (w == 0) ? ((k & 4) ? 3 : 0) : ((k & 4) ? 2 : 1);
     const int along = k & 3;
     v.ext = phase == 0 ? across : along;
     v.eyt = phase == 0 ? along : across;
   } else {
-    const int e = threadIdx.x / NP;
-    v.t = threadIdx.x % NP;
+    const int e = tid / NP;
+    v.t = tid % NP;
     v.ext = e % TX;
     v.eyt = e / TX;
   }
   v.e = v.ext + TX * v.eyt;
   v.ex = tl.ex0 + v.ext;
   v.ey = tl.ey0 + v.eyt;
-  v.valid = (v.ex < I.nex) && (v.ey < I.ney);
+  v.valid = tid < Tiling2D<NP>::NT && v.ex < I.nex && v.ey < I.ney;
   v.base = I.off + (long long)NP * NP * ((long long)v.ex + (long long)I.nex * v.ey);
   return v;
+}
+
+template <int NP>
+__device__ __forceinline__ ElemView elem_view(const Tile2D& tl, const Inst2D& I, int phase) {
+  return elem_view<NP>(tl, I, phase, threadIdx.x);
 }
 
 // Neighbour element (dx, dy in {-1,0,1}) with periodic wrap; returns its base
@@ -329,32 +335,26 @@ struct ApplyArgs2D {
 // Partner data across one face: its value and its flux k (D x) at the face node.
 struct Partner1 { double x, t; };
 
-// Shared memory of one tile's operator application: the tile's x, the x-phase
-// sums (fixed point, with each row's exponent) and the end-node fluxes of
-// every line; f: the fields a solver epilogue's last phase reads, copied while
-// the first phases run (NF = 5: cky, cm, b, cinvM, d; 0: read from global memory
-// there, for the PCG epilogues, whose persistent form has no room for them).
-__host__ __device__ constexpr int apply_fields(int epi) { return epi == EPI_CHEB || epi == EPI_JACOBI ? 5 : 0; }
-template <int NP, int NF>
+// Shared memory of one tile's PCG operator application: the tile's x, the
+// x-phase sums (fixed point, with each row's exponent) and the end-node fluxes
+// of every line.
+template <int NP>
 struct ApplySmem {
-  alignas(16) double f[NF ? NF : 1][NF ? Tiling2D<NP>::TE : 1][Tiling2D<NP>::SN];
   alignas(16) double x[Tiling2D<NP>::TE][Tiling2D<NP>::SN];
   alignas(16) long long yx[Tiling2D<NP>::TE][Tiling2D<NP>::SN];
   int ex[Tiling2D<NP>::TE][NP];
   double txf[Tiling2D<NP>::TE][NP][2], tyf[Tiling2D<NP>::TE][NP][2];
 };
 
-// y = A x on tile tl (of instance I) with the EPI epilogue, by the CTA's
-// Tiling2D<NP>::NT threads (all of which call it; it synchronises the CTA
-// twice). Returns this thread's PCG inner-product partial (EPI_PCG0 / EPI_PCG;
-// 0 otherwise). k2_apply runs it on tile blockIdx.x; the persistent PCG kernel
-// on every tile of its CTA.
+// y = A x on tile tl (of instance I) with a PCG epilogue (EPI_PCG0 / EPI_PCG), by
+// the CTA's Tiling2D<NP>::NT threads (all of which call it; it synchronises the
+// CTA twice). Returns this thread's inner-product partial. k2_apply_pcg runs it
+// on tile blockIdx.x; the persistent PCG kernel on every tile of its CTA, whose
+// eight resident CTAs per SM leave no room for the halves of k2_apply.
 template <int NP, int EPI>
-__device__ __forceinline__ double apply_tile(const ApplyArgs2D& a, const Tile2D tl, const Inst2D& I,
-                                             ApplySmem<NP, apply_fields(EPI)>& sm) {
+__device__ __forceinline__ double apply_tile(const ApplyArgs2D& a, const Tile2D tl, const Inst2D& I, ApplySmem<NP>& sm) {
   using TL = Tiling2D<NP>;
   constexpr int L = TL::L, TX = TL::TX, TY = TL::TY;
-  constexpr bool PCG = EPI == EPI_PCG0 || EPI == EPI_PCG;
   auto& s_x = sm.x;
   auto& s_yx = sm.yx;
   auto& s_ex = sm.ex;
@@ -370,21 +370,6 @@ __device__ __forceinline__ double apply_tile(const ApplyArgs2D& a, const Tile2D 
     if (form_p) return fma(beta, a.pcg_p[n], a.pcg_r[n] * a.cinvM[n]);
     return a.x[n];
   };
-
-  constexpr int NF = apply_fields(EPI);
-  if (NF && vr.valid) {
-    const double* src[5] = {a.cky, a.cm, a.b, a.cinvM, a.d_in};
-#pragma unroll
-    for (int f = 0; f < NF; ++f) {
-      if (src[f]) {
-#pragma unroll
-        for (int i = 0; i < NP; ++i) copy_async8(&sm.f[f][vr.e][vr.t * NP + i], src[f] + vr.base + vr.t * NP + i);
-      }
-      if (f == 0) copy_async_commit();
-    }
-  }
-  copy_async_commit();
-  auto field = [&](int f, const double* g, int e, long long base, int nd) { return NF ? sm.f[NF ? f : 0][NF ? e : 0][nd] : g[base + nd]; };
 
   // ---- xi-phase part 1: row fluxes
   double xr[NP], kx0, kxL;
@@ -408,7 +393,6 @@ __device__ __forceinline__ double apply_tile(const ApplyArgs2D& a, const Tile2D 
       for (int i = 0; i < NP; ++i) a.tape_x[vr.base + t * NP + i] = xr[i];
     }
   }
-  if (NF) copy_async_wait<1>();
   __syncthreads();
   double xc[NP], ky0, kyL;
   FixFlux<NP> fc;
@@ -416,7 +400,7 @@ __device__ __forceinline__ double apply_tile(const ApplyArgs2D& a, const Tile2D 
     const int t = vc.t, e = vc.e;
     double k[NP];
 #pragma unroll
-    for (int l = 0; l < NP; ++l) { xc[l] = s_x[e][l * NP + t]; k[l] = field(0, a.cky, e, vc.base, l * NP + t); }
+    for (int l = 0; l < NP; ++l) { xc[l] = s_x[e][l * NP + t]; k[l] = a.cky[vc.base + l * NP + t]; }
     flux_line<NP>(B, xc, k, fc);
     s_tyf[e][t][0] = fc.t0; s_tyf[e][t][1] = fc.tL;
     ky0 = k[0]; kyL = k[L];
@@ -455,9 +439,7 @@ __device__ __forceinline__ double apply_tile(const ApplyArgs2D& a, const Tile2D 
     for (int k = 0; k < NP; ++k) s_yx[e][t * NP + k] = sums.G[k];
     s_ex[e][t] = sums.e;
   }
-  if (NF) copy_async_wait<0>();
   __syncthreads();
-  if (!PCG && !vc.valid) return 0.0;
   double part = 0.0;  // PCG inner-product partial of this thread
 
   // ---- eta-phase: y faces of the column, y-stiffness transpose, mass, epilogue
@@ -487,15 +469,15 @@ __device__ __forceinline__ double apply_tile(const ApplyArgs2D& a, const Tile2D 
     const double Fb = fma(a.cpy[vc.base + t], jb, hw * (qb.t + fc.t0));
     const double jt = xc[L] - qt.x;
     const double Ft = fma(a.cpy[vc.base + L * NP + t], jt, hw * (fc.tL + qt.t));
-    // the residual epilogues form b - A x at once: b - cm x enters the last sum, the rest with a minus sign
-    constexpr bool RES = EPI == EPI_CHEB || EPI == EPI_JACOBI || EPI == EPI_PCG0;
+    // EPI_PCG0 forms b - A x at once: b - cm x enters the last sum, the rest with a minus sign
+    constexpr bool RES = EPI == EPI_PCG0;
     double acc[NP], yy[NP];
     long long R[NP];
     int er[NP];
 #pragma unroll
     for (int l = 0; l < NP; ++l) {
-      const double cm = field(1, a.cm, e, vc.base, l * NP + t);
-      acc[l] = RES ? fma(-cm, xc[l], field(2, a.b, e, vc.base, l * NP + t)) : cm * xc[l];
+      const long long n = vc.base + l * NP + t;
+      acc[l] = RES ? fma(-a.cm[n], xc[l], a.b[n]) : a.cm[n] * xc[l];
       R[l] = s_yx[e][l * NP + t];
       er[l] = s_ex[e][l];
     }
@@ -503,53 +485,146 @@ __device__ __forceinline__ double apply_tile(const ApplyArgs2D& a, const Tile2D 
 #pragma unroll
     for (int l = 0; l < NP; ++l) {
       const long long n = vc.base + l * NP + t;
-      const double y = yy[l];  // A x, or b - A x (RES)
-      if (EPI == EPI_RESID) { a.y_out[n] = y; continue; }
       if (EPI == EPI_PCG) {
-        a.ap_out[n] = y;
-        part = fma(xc[l], y, part);
-        continue;
-      }
-      if (EPI == EPI_PCG0) {
-        const double r0 = y;
-        const double z0 = r0 * a.cinvM[n];
+        a.ap_out[n] = yy[l];
+        part = fma(xc[l], yy[l], part);
+      } else {
+        const double r0 = yy[l], z0 = r0 * a.cinvM[n];
         a.r_out[n] = r0;
         a.p_out[n] = z0;
         part = fma(r0, z0, part);
-        continue;
-      }
-      const double r = y;
-      if (a.tape_r) a.tape_r[n] = r;
-      if (EPI == EPI_CHEB) {
-        const double z = r * field(3, a.cinvM, e, vc.base, l * NP + t);
-        const double d = a.d_in ? fma(a.ca, field(4, a.d_in, e, vc.base, l * NP + t), a.cc * z) : a.cc * z;
-        a.d_out[n] = d;
-        a.x_out[n] = xc[l] + d;
-      } else {  // EPI_JACOBI: x + omega (b - A x) / M   (elliptic.jl:358)
-        a.x_out[n] = fma(a.omega * r, field(3, a.cinvM, e, vc.base, l * NP + t), xc[l]);
       }
     }
   }
   return part;
 }
 
-// What bounds it: per warp of 32 lines 50 FP64 instructions (106 with FP64 contractions), 1018 on the integer ALU and 482
-// integer multiply-adds; at 2.1 M nodes (P3, Chebyshev) the FP64 pipe is 60% busy, the ALU 38%, DRAM 32%, and the rest is
-// latency under 18 warps per SM. 127 us with FP64 contractions, 79 us now; the last phase's fields are copied to shared
-// memory while the first phases run, which shows on small meshes (64 x 64: 12.3 against 11.3 us) and costs nothing here.
 template <int NP, int EPI>
-__global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_apply(ApplyArgs2D a) {
+__global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_apply_pcg(ApplyArgs2D a) {
   using TL = Tiling2D<NP>;
-  constexpr bool PCG = EPI == EPI_PCG0 || EPI == EPI_PCG;
   constexpr int P2 = pow2_at_least(TL::NT);
-  __shared__ ApplySmem<NP, apply_fields(EPI)> sm;
-  __shared__ double s_red[PCG ? P2 : 1];
+  __shared__ ApplySmem<NP> sm;
+  __shared__ double s_red[P2];
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];
   const double part = apply_tile<NP, EPI>(a, tl, I, sm);
-  if (PCG) {
-    const double tot = block_sum<P2>(part, s_red);
-    inst_sum_last_block(a.isum, tl.inst, I.ntiles, tot, a.partials, blockIdx.x, I.tile0, I.ntiles);
+  const double tot = block_sum<P2>(part, s_red);
+  inst_sum_last_block(a.isum, tl.inst, I.ntiles, tot, a.partials, blockIdx.x, I.tile0, I.ntiles);
+}
+
+// y = A x with the Jacobi / Chebyshev / plain epilogue. Rows and columns run side by side, one half of the CTA each: the
+// two directions are independent up to their sums, so a line's chain of loads, integer sums and FP64 faces is all that a
+// warp runs before the CTA meets, and the epilogue is pointwise over all threads with coalesced accesses.
+// What bounds it: FP64 issue (68% busy), the integer ALU (59%) and L2 latency, with 32 warps per SM. 8 x 128^2 P3,
+// Chebyshev: 127 us with FP64 contractions; 79 us with integer ones and one thread per pair of lines (18 warps); 69 us in
+// halves; 65 us with the pointwise loads ahead of its stores. 64^2: 12.3, 11.3, 10.2, 9.9.
+template <int NP, int EPI>
+__global__ void __launch_bounds__(2 * Tiling2D<NP>::NH) k2_apply(ApplyArgs2D a) {
+  using TL = Tiling2D<NP>;
+  constexpr int TE = TL::TE, NN = TL::NN, SN = TL::SN, L = TL::L, TX = TL::TX, TY = TL::TY, NH = TL::NH;
+  __shared__ __align__(16) double s_x[TE][SN];
+  __shared__ __align__(16) long long s_y[2][TE][SN];  // sums of the rows and of the columns (fixed point)
+  __shared__ int s_e[2][TE][NP];                      // their exponents
+  __shared__ double s_t[2][TE][NP][2];                // end-node fluxes of every line
+  const Tile2D tl = a.tiles[blockIdx.x];
+  const Inst2D I = a.inst[tl.inst];
+  const BasisDev& B = a.B;
+  const double hw = B.hw;
+  const int dir = threadIdx.x >= NH;  // 0: rows and x faces, 1: columns and y faces
+  const ElemView w = elem_view<NP>(tl, I, dir, threadIdx.x - dir * NH);
+  const int e = w.e, t = w.t;
+  const int st = dir == 0 ? 1 : NP, at = dir == 0 ? t * NP : t;  // node k of the line: at + k st
+  const double* ck = dir == 0 ? a.ckx : a.cky;
+  double x0 = 0.0, xL = 0.0, k0 = 0.0, kL = 0.0;
+  FixFlux<NP> f;
+  if (w.valid) {
+    double x[NP], k[NP];
+#pragma unroll
+    for (int i = 0; i < NP; ++i) { x[i] = a.x[w.base + at + i * st]; k[i] = ck[w.base + at + i * st]; }
+    if (dir == 0) {
+#pragma unroll
+      for (int i = 0; i < NP; ++i) s_x[e][at + i] = x[i];
+    }
+    flux_line<NP>(B, x, k, f);
+    s_t[dir][e][t][0] = f.t0; s_t[dir][e][t][1] = f.tL;
+    x0 = x[0]; xL = x[L]; k0 = k[0]; kL = k[L];
+  }
+  __syncthreads();
+  if (w.valid) {
+    const double* cp = dir == 0 ? a.cpx : a.cpy;
+    auto fetch = [&](int s) {
+      Partner1 P;
+      int it;
+      const int d = s == 0 ? -1 : 1;
+      const long long pb = neighbour<NP>(tl, I, w.ex, w.ey, dir == 0 ? d : 0, dir == 0 ? 0 : d, &it);
+      const int pn = at + (s == 0 ? L : 0) * st;  // partner face node
+      if (it >= 0) {
+        P.x = s_x[it][pn];
+        P.t = s_t[dir][it][t][1 - s];
+      } else {
+        double p[NP];
+#pragma unroll
+        for (int k = 0; k < NP; ++k) p[k] = a.x[pb + at + k * st];
+        P.x = s == 0 ? p[L] : p[0];
+        P.t = flux_end<NP>(B, s == 0, p, ck[pb + pn]);
+      }
+      return P;
+    };
+    const int sf = dir == 0 ? first_side(w.ext, TX) : first_side(w.eyt, TY);
+    const Partner1 pA = fetch(sf), pB = fetch(1 - sf);
+    const Partner1 pl = sf == 0 ? pA : pB, pr = sf == 0 ? pB : pA;
+    // left face: own node 0 is the R side; right face: own node L is the L side
+    const double jl = pl.x - x0, jr = xL - pr.x;
+    const double Fl = fma(cp[w.base + at], jl, hw * (pl.t + f.t0));
+    const double Fr = fma(cp[w.base + at + L * st], jr, hw * (f.tL + pr.t));
+    FixSums<NP> sums;
+    row_sums<NP>(B, f, hw * k0 * jl, hw * kL * jr, -Fl, Fr, sums);
+#pragma unroll
+    for (int k = 0; k < NP; ++k) s_y[dir][e][at + k * st] = sums.G[k];
+    s_e[dir][e][t] = sums.e;
+  }
+  // ---- pointwise: mass term, sums, epilogue. Everything is loaded before anything is stored (the compiler has to assume
+  // that a store changes what a later load reads), and before the barrier.
+  constexpr int NQ = (TE * NN + 2 * NH - 1) / (2 * NH);
+  long long node[NQ];
+  double cm[NQ], b[NQ], im[NQ], din[NQ];
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) {
+    const int m = threadIdx.x + q * 2 * NH;
+    const int el = m / NN, nd = m % NN, ex = tl.ex0 + el % TX, ey = tl.ey0 + el / TX;
+    const bool live = m < TE * NN && ex < I.nex && ey < I.ney;
+    const long long n = I.off + (long long)NN * (ex + (long long)I.nex * ey) + nd;
+    node[q] = live ? n : -1;
+    if (!live) continue;
+    cm[q] = a.cm[n];
+    if (EPI != EPI_RESID) {
+      b[q] = a.b[n];
+      im[q] = a.cinvM[n];
+      din[q] = EPI == EPI_CHEB && a.d_in ? a.d_in[n] : 0.0;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) {
+    const long long n = node[q];
+    if (n < 0) continue;
+    const int m = threadIdx.x + q * 2 * NH;
+    const int el = m / NN, nd = m % NN;
+    const double x = s_x[el][nd];
+    const double acc = EPI == EPI_RESID ? cm[q] * x : fma(-cm[q], x, b[q]);
+    const double y = node_total<59>(s_y[0][el][nd], s_e[0][el][nd / NP], s_y[1][el][nd], s_e[1][el][nd % NP], acc,
+                                    EPI == EPI_RESID ? 1 : -1);  // A x, or b - A x
+    if (EPI == EPI_RESID) { a.y_out[n] = y; continue; }
+    if (a.tape_x) a.tape_x[n] = x;
+    if (a.tape_r) a.tape_r[n] = y;
+    if (EPI == EPI_CHEB) {
+      const double z = y * im[q];
+      const double d = a.d_in ? fma(a.ca, din[q], a.cc * z) : a.cc * z;
+      a.d_out[n] = d;
+      a.x_out[n] = x + d;
+    } else {  // EPI_JACOBI: x + omega (b - A x) / M   (elliptic.jl:358)
+      a.x_out[n] = fma(a.omega * y, im[q], x);
+    }
   }
 }
 

@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT, 8) k2_pcg_persist(PcgPersist
   constexpr int cnt = TL::TE * NP * NP;  // nodes of a tile
   static_assert(cnt <= UV, "one tree slot per node");
   static_assert(TL::NT >= PCG_BCAST, "one thread per published copy");
-  __shared__ ApplySmem<NP, 0> sm;
+  __shared__ ApplySmem<NP> sm;
   __shared__ double s_red[UV > P2 ? UV : P2];
   __shared__ double s_val, s_beta[PCG_PERSIST_MAX_INST], s_stage[persist_max_inst_tiles<NP>()];
   __shared__ int s_ok;

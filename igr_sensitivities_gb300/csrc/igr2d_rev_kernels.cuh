@@ -327,25 +327,23 @@ struct ApplyRevArgs2D {
 // Partner data across one face for the reverse apply: values of u and x_k, the flux of u at the face node and 1/rho.
 struct Partner2 { double u, v, t, ir; };
 
-// What bounds it: FP64 issue and latency, about evenly. The line contractions, fluxes, coefficient products and sums run
-// on the integer pipes (igr_fix.cuh); 8 x 128^2 P3, Chebyshev: 226 us with FP64 contractions, 138 us now. Eight CTAs per
-// SM for P3 (128 registers): 156 us with the 146 the compiler takes unbounded (7 CTAs), 135 us with nine, which costs
-// a single 64 x 64 instance 7% (17.9 against 16.7 us per launch, 18.9 before).
+// Rows and columns run side by side, one half of the CTA each, and the outputs are pointwise over all threads (see
+// k2_apply). What bounds it: FP64 issue (67% busy) and the integer ALU (54%). 8 x 128^2 P3, Chebyshev: 226 us with FP64
+// contractions; 140 us with integer ones and one thread per pair of lines; in halves, with the pointwise loads ahead of
+// its stores, 114 us at seven CTAs per SM (72 registers; 137 us at the 80 the compiler takes). 64^2: 18.9, 17.4, 12.4.
 template <int NP, int SREV>
-__global__ void __launch_bounds__(Tiling2D<NP>::NT, NP == 4 ? 8 : 1) k2_apply_rev(ApplyRevArgs2D a) {
+__global__ void __launch_bounds__(2 * Tiling2D<NP>::NH, NP == 4 ? 7 : 1) k2_apply_rev(ApplyRevArgs2D a) {
   using TL = Tiling2D<NP>;
-  constexpr int TE = TL::TE, SN = TL::SN, L = TL::L, TX = TL::TX, TY = TL::TY;
+  constexpr int TE = TL::TE, NN = TL::NN, SN = TL::SN, L = TL::L, TX = TL::TX, TY = TL::TY, NH = TL::NH;
   constexpr bool PCG = SREV == SREV_PCG;
-  constexpr int P2 = pow2_at_least(TL::NT);
+  constexpr int P2 = pow2_at_least(2 * NH);
   __shared__ __align__(16) double s_u[TE][SN], s_v[TE][SN];
-  __shared__ __align__(16) long long s_yx[TE][SN], s_zr[TE][SN];  // row sums and products (fixed point)
-  __shared__ int s_ey[TE][NP], s_ez[TE][NP];                      // their exponents
-  __shared__ double s_tx[TE][NP][2], s_ty[TE][NP][2];             // end-node fluxes of u
-  __shared__ __align__(16) double s_f[3][TE][SN];                 // cky, cm, xb, copied while the row phase runs
+  __shared__ __align__(16) long long s_y[2][TE][SN], s_z[2][TE][SN];  // sums and products of rows and columns (fixed point)
+  __shared__ int s_ey[2][TE][NP], s_ez[2][TE][NP];                    // their exponents
+  __shared__ double s_t[2][TE][NP][2];                                // end-node fluxes of u
   __shared__ double s_red[PCG ? P2 : 1];
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];
-  const ElemView vr = elem_view<NP>(tl, I, 0), vc = elem_view<NP>(tl, I, 1);
   const BasisDev& B = a.B;
   const double hw = B.hw;
   double pal = 0.0, ppb = 0.0;  // PCG: alpha_it and the adjoint of pAp_it
@@ -358,180 +356,141 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT, NP == 4 ? 8 : 1) k2_apply_re
     if (PCG) return fma(pal, a.u[n], -ppb * xkv);
     return a.u[n];
   };
-  if (vr.valid) {
-    const double* src[3] = {a.cky, a.cm, a.xb};
-#pragma unroll
-    for (int f = 0; f < 3; ++f) {
-#pragma unroll
-      for (int i = 0; i < NP; ++i) copy_async8(&s_f[f][vr.e][vr.t * NP + i], src[f] + vr.base + vr.t * NP + i);
-      if (f == 0) copy_async_commit();
-    }
-  }
-  copy_async_commit();
-
-  // the ends of a row or column: values of u and x_k, the stiffness coefficient of u's jump terms
-  double ur0 = 0.0, urL = 0.0, vr0 = 0.0, vrL = 0.0, kx0 = 0.0, kxL = 0.0;
-  FixFlux<NP> fr;
-  FixDeriv<NP> dr;
-  if (vr.valid) {
-    const int t = vr.t, e = vr.e;
+  const int dir = threadIdx.x >= NH;  // 0: rows and x faces, 1: columns and y faces
+  const ElemView w = elem_view<NP>(tl, I, dir, threadIdx.x - dir * NH);
+  const int e = w.e, t = w.t;
+  const int st = dir == 0 ? 1 : NP, at = dir == 0 ? t * NP : t;  // node k of the line: at + k st
+  const double* ck = dir == 0 ? a.ckx : a.cky;
+  // the ends of the line: u, x_k and the stiffness coefficient
+  double u0 = 0.0, uL = 0.0, v0 = 0.0, vL = 0.0, k0 = 0.0, kL = 0.0;
+  FixFlux<NP> f;
+  FixDeriv<NP> d;
+  if (w.valid) {
     double u[NP], v[NP], k[NP];
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
-      const long long n = vr.base + t * NP + i;
-      v[i] = a.xk[n]; u[i] = ldu(n, v[i]); k[i] = a.ckx[n];
-      s_u[e][t * NP + i] = u[i]; s_v[e][t * NP + i] = v[i];
+      const long long n = w.base + at + i * st;
+      v[i] = a.xk[n]; u[i] = ldu(n, v[i]); k[i] = ck[n];
     }
-    flux_line<NP>(B, u, k, fr);
-    deriv_line<NP>(B, v, dr);
-    s_tx[e][t][0] = fr.t0; s_tx[e][t][1] = fr.tL;
-    ur0 = u[0]; urL = u[L]; vr0 = v[0]; vrL = v[L]; kx0 = k[0]; kxL = k[L];
-  }
-  copy_async_wait<1>();
-  __syncthreads();
-  double uc[NP], vc_[NP], ky0 = 0.0, kyL = 0.0;
-  FixFlux<NP> fc;
-  FixDeriv<NP> dc;
-  if (vc.valid) {
-    const int t = vc.t, e = vc.e;
-    double k[NP];
+    if (dir == 0) {
 #pragma unroll
-    for (int l = 0; l < NP; ++l) { uc[l] = s_u[e][l * NP + t]; vc_[l] = s_v[e][l * NP + t]; k[l] = s_f[0][e][l * NP + t]; }
-    flux_line<NP>(B, uc, k, fc);
-    deriv_line<NP>(B, vc_, dc);
-    s_ty[e][t][0] = fc.t0; s_ty[e][t][1] = fc.tL;
-    ky0 = k[0]; kyL = k[L];
+      for (int i = 0; i < NP; ++i) { s_u[e][at + i] = u[i]; s_v[e][at + i] = v[i]; }
+    }
+    flux_line<NP>(B, u, k, f);
+    deriv_line<NP>(B, v, d);
+    s_t[dir][e][t][0] = f.t0; s_t[dir][e][t][1] = f.tL;
+    u0 = u[0]; uL = u[L]; v0 = v[0]; vL = v[L]; k0 = k[0]; kL = k[L];
   }
-  // One face of a line: own end values (uo, vo, stiffness k, flux t0, derivative of x_k gv, 1/rho io, penalty p), the
-  // partner P; s = +1 when the own node is the left side, else -1 (jumps are left minus right). F: the flux terms
-  // (consistency + penalty, as added to the left side), us: the symmetry term hw k [u], z: the coefficient adjoint's
-  // face terms hw k ([u] gv + gu [x_k]) and, where the own 1/rho sets the penalty, p [u] [x_k].
-  auto face = [&](int s, double uo, double vo, double k, double t0, double gv, double io, double p, const Partner2& P,
-                  double& F, double& us, double& z) {
-    const double ju = s > 0 ? uo - P.u : P.u - uo, jv = s > 0 ? vo - P.v : P.v - vo;
-    const double pj = p * ju;
-    F = fma(hw, s > 0 ? t0 + P.t : P.t + t0, pj);
-    us = hw * k * ju;
-    const bool wins = s > 0 ? !gt_nonneg(P.ir, io) : gt_nonneg(io, P.ir);  // the right side wins only when strictly larger
-    z = fma(gv, us, jv * fma(hw, t0, wins ? pj : 0.0));
-  };
-  if (vr.valid) {
-    // ---- row of vr: x faces
-    const int t = vr.t, e = vr.e;
+  __syncthreads();
+  if (w.valid) {
+    const double* cp = dir == 0 ? a.cpx : a.cpy;
     auto fetch = [&](int s) {
       Partner2 P;
       int it;
-      const long long pb = neighbour<NP>(tl, I, vr.ex, vr.ey, s == 0 ? -1 : 1, 0, &it);
-      const int pi = s == 0 ? L : 0;
-      P.ir = a.invr[pb + t * NP + pi];
+      const int dd = s == 0 ? -1 : 1;
+      const long long pb = neighbour<NP>(tl, I, w.ex, w.ey, dir == 0 ? dd : 0, dir == 0 ? 0 : dd, &it);
+      const int pn = at + (s == 0 ? L : 0) * st;  // partner face node
+      P.ir = a.invr[pb + pn];
       if (it >= 0) {
-        P.u = s_u[it][t * NP + pi]; P.v = s_v[it][t * NP + pi];
-        P.t = s_tx[it][t][s == 0 ? 1 : 0];
+        P.u = s_u[it][pn]; P.v = s_v[it][pn];
+        P.t = s_t[dir][it][t][1 - s];
       } else {
-        double pr[NP];
-        P.v = a.xk[pb + t * NP + pi];
+        double p[NP];
+        P.v = a.xk[pb + pn];
 #pragma unroll
-        for (int k = 0; k < NP; ++k) pr[k] = ldu(pb + t * NP + k, PCG ? a.xk[pb + t * NP + k] : 0.0);
-        P.u = s == 0 ? pr[L] : pr[0];
-        P.t = flux_end<NP>(B, s == 0, pr, a.ckx[pb + t * NP + pi]);
+        for (int k = 0; k < NP; ++k) p[k] = ldu(pb + at + k * st, PCG ? a.xk[pb + at + k * st] : 0.0);
+        P.u = s == 0 ? p[L] : p[0];
+        P.t = flux_end<NP>(B, s == 0, p, ck[pb + pn]);
       }
       return P;
     };
-    const int sf = first_side(vr.ext, TX);
+    // One face: own end values (uo, vo, stiffness k, flux t0, derivative of x_k gv, 1/rho io, penalty p), the partner P;
+    // s = +1 when the own node is the left side, else -1 (jumps are left minus right). F: the flux terms (consistency +
+    // penalty, as added to the left side), us: the symmetry term hw k [u], z: the coefficient adjoint's face terms
+    // hw k ([u] gv + gu [x_k]) and, where the own 1/rho sets the penalty, p [u] [x_k].
+    auto face = [&](int s, double uo, double vo, double k, double t0, double gv, double io, double p, const Partner2& P,
+                    double& F, double& us, double& z) {
+      const double ju = s > 0 ? uo - P.u : P.u - uo, jv = s > 0 ? vo - P.v : P.v - vo;
+      const double pj = p * ju;
+      F = fma(hw, s > 0 ? t0 + P.t : P.t + t0, pj);
+      us = hw * k * ju;
+      const bool wins = s > 0 ? !gt_nonneg(P.ir, io) : gt_nonneg(io, P.ir);  // the right side wins only when strictly larger
+      z = fma(gv, us, jv * fma(hw, t0, wins ? pj : 0.0));
+    };
+    const int sf = dir == 0 ? first_side(w.ext, TX) : first_side(w.eyt, TY);
     const Partner2 pA = fetch(sf), pB = fetch(1 - sf);
-    const Partner2 pl = sf == 0 ? pA : pB, prt = sf == 0 ? pB : pA;
+    const Partner2 pl = sf == 0 ? pA : pB, pr = sf == 0 ? pB : pA;
     double Fl, Fr, us0, usL, z0, zL;
-    const long long n0 = vr.base + t * NP;
-    face(-1, ur0, vr0, kx0, fr.t0, deriv_at<NP>(dr, 0), a.invr[n0], a.cpx[n0], pl, Fl, us0, z0);
-    face(1, urL, vrL, kxL, fr.tL, deriv_at<NP>(dr, L), a.invr[n0 + L], a.cpx[n0 + L], prt, Fr, usL, zL);
+    const long long n0 = w.base + at, nL = w.base + at + L * st;
+    face(-1, u0, v0, k0, f.t0, deriv_at<NP>(d, 0), a.invr[n0], cp[n0], pl, Fl, us0, z0);
+    face(1, uL, vL, kL, f.tL, deriv_at<NP>(d, L), a.invr[nL], cp[nL], pr, Fr, usL, zL);
     FixSums<NP> sums;
-    row_products<NP>(fr, dr, z0, zL, sums);
+    row_products<NP>(f, d, z0, zL, sums);
 #pragma unroll
-    for (int k = 0; k < NP; ++k) s_zr[e][t * NP + k] = sums.G[k];
-    s_ez[e][t] = sums.e;
-    row_sums<NP>(B, fr, us0, usL, -Fl, Fr, sums);
+    for (int k = 0; k < NP; ++k) s_z[dir][e][at + k * st] = sums.G[k];
+    s_ez[dir][e][t] = sums.e;
+    row_sums<NP>(B, f, us0, usL, -Fl, Fr, sums);
 #pragma unroll
-    for (int k = 0; k < NP; ++k) s_yx[e][t * NP + k] = sums.G[k];
-    s_ey[e][t] = sums.e;
+    for (int k = 0; k < NP; ++k) s_y[dir][e][at + k * st] = sums.G[k];
+    s_ey[dir][e][t] = sums.e;
   }
-  copy_async_wait<0>();
+  // ---- pointwise: sums, coefficient adjoints, solver epilogue. Everything is loaded before anything is stored (the
+  // compiler has to assume that a store changes what a later load reads), and before the barrier.
+  constexpr bool EPI = SREV == SREV_CHEB || SREV == SREV_JACOBI;
+  constexpr int NQ = (TE * NN + 2 * NH - 1) / (2 * NH);
+  long long node[NQ];
+  double acc[NQ], zs[NQ], zm[NQ], bb[NQ], cM[NQ], db[NQ], im[NQ], rp[NQ], iMb[NQ];
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) {
+    const int m = threadIdx.x + q * 2 * NH;
+    const int el = m / NN, nd = m % NN, ex = tl.ex0 + el % TX, ey = tl.ey0 + el / TX;
+    const bool live = m < TE * NN && ex < I.nex && ey < I.ney;
+    const long long n = I.off + (long long)NN * (ex + (long long)I.nex * ey) + nd;
+    node[q] = live ? n : -1;
+    if (!live) continue;
+    // xb - cm u (and, for PCG, + alpha_it xconst + pApb apk)
+    acc[q] = a.xb[n];
+    cM[q] = a.cm[n];
+    if (PCG) acc[q] = fma(ppb, a.apk[n], fma(pal, a.xconst[n], acc[q]));
+    zs[q] = a.first ? 0.0 : a.Zs[n];
+    zm[q] = a.first ? 0.0 : a.Zm[n];
+    bb[q] = a.bb_op == 2 ? a.bb[n] : 0.0;
+    if (PCG && a.has_next) rp[q] = a.p_next[n];
+    if (EPI && a.has_next) {
+      im[q] = a.cinvM[n];
+      rp[q] = a.r_prev[n];
+      iMb[q] = a.iMb[n];
+      db[q] = SREV == SREV_CHEB ? a.db[n] : 0.0;
+    }
+  }
   __syncthreads();
-  if (!PCG && !vc.valid) return;
-  double part = 0.0;  // PCG: betab partial of this thread
-  // ---- column of vc: y faces, transposes, outputs
-  if (vc.valid) {
-    const int t = vc.t, e = vc.e;
-    auto fetchy = [&](int s) {
-      Partner2 P;
-      int it;
-      const long long pb = neighbour<NP>(tl, I, vc.ex, vc.ey, 0, s == 0 ? -1 : 1, &it);
-      const int pl = s == 0 ? L : 0;
-      P.ir = a.invr[pb + pl * NP + t];
-      if (it >= 0) {
-        P.u = s_u[it][pl * NP + t]; P.v = s_v[it][pl * NP + t];
-        P.t = s_ty[it][t][s == 0 ? 1 : 0];
-      } else {
-        double pc[NP];
-        P.v = a.xk[pb + pl * NP + t];
+  const int zsg = a.zscale > 0 ? 1 : -1;  // -1 (r = b - A x) or +1 (A p): applied through operand signs, not a multiply
+  double part = 0.0;                      // PCG: betab partial of this thread
 #pragma unroll
-        for (int k = 0; k < NP; ++k) pc[k] = ldu(pb + k * NP + t, PCG ? a.xk[pb + k * NP + t] : 0.0);
-        P.u = s == 0 ? pc[L] : pc[0];
-        P.t = flux_end<NP>(B, s == 0, pc, a.cky[pb + pl * NP + t]);
-      }
-      return P;
-    };
-    const int sf = first_side(vc.eyt, TY);
-    const Partner2 qA = fetchy(sf), qB = fetchy(1 - sf);
-    const Partner2 qb = sf == 0 ? qA : qB, qt = sf == 0 ? qB : qA;
-    double Fb, Ft, us0, usL, z0, zL;
-    const long long n0 = vc.base + t, nL = vc.base + L * NP + t;
-    face(-1, uc[0], vc_[0], ky0, fc.t0, deriv_at<NP>(dc, 0), a.invr[n0], a.cpy[n0], qb, Fb, us0, z0);
-    face(1, uc[L], vc_[L], kyL, fc.tL, deriv_at<NP>(dc, L), a.invr[nL], a.cpy[nL], qt, Ft, usL, zL);
-    // zscale is -1 (r = b - A x) or +1 (A p): applied through operand signs, not a multiply
-    const int zsg = a.zscale > 0 ? 1 : -1;
-    double acc[NP], out[NP];
-    long long R[NP];
-    int er[NP];
-#pragma unroll
-    for (int l = 0; l < NP; ++l) {
-      R[l] = s_zr[e][l * NP + t];
-      er[l] = s_ez[e][l];
-      acc[l] = a.first ? 0.0 : a.Zs[vc.base + l * NP + t];
-    }
-    column_products<NP>(fc, dc, z0, zL, R, er, acc, zsg, out);
-#pragma unroll
-    for (int l = 0; l < NP; ++l) a.Zs[vc.base + l * NP + t] = out[l];
-    // xb - A u (and, for PCG, + alpha_it xconst + pApb apk) in one sum
-#pragma unroll
-    for (int l = 0; l < NP; ++l) {
-      const long long n = vc.base + l * NP + t;
-      R[l] = s_yx[e][l * NP + t];
-      er[l] = s_ey[e][l];
-      acc[l] = fma(-s_f[1][e][l * NP + t], uc[l], s_f[2][e][l * NP + t]);
-      if (PCG) acc[l] = fma(ppb, a.apk[n], fma(pal, a.xconst[n], acc[l]));
-    }
-    column_sums<NP>(B, fc, us0, usL, -Fb, Ft, R, er, acc, -1, out);
-#pragma unroll
-    for (int l = 0; l < NP; ++l) {
-      const long long n = vc.base + l * NP + t;
-      const double xb = out[l];
-      const double uz = a.zscale > 0 ? uc[l] : -uc[l];
-      a.xb[n] = xb;
-      if (a.bb_op == 1) a.bb[n] = uc[l];
-      else if (a.bb_op == 2) a.bb[n] += uc[l];
-      a.Zm[n] = a.first ? uz * vc_[l] : fma(uz, vc_[l], a.Zm[n]);
-      if (PCG && a.has_next) part = fma(xb, a.p_next[n], part);
-      if (SREV == SREV_CHEB && a.has_next) {
-        const double dbv = a.db[n] + xb;
-        const double zb = a.cc * dbv;
-        a.u_out[n] = a.cinvM[n] * zb;
-        a.iMb[n] = fma(zb, a.r_prev[n], a.iMb[n]);
-        a.db[n] = a.ca * dbv;
-      } else if (SREV == SREV_JACOBI && a.has_next) {
-        const double tb = a.omega * xb;
-        a.u_out[n] = tb * a.cinvM[n];
-        a.iMb[n] = fma(tb, a.r_prev[n], a.iMb[n]);
-      }
+  for (int q = 0; q < NQ; ++q) {
+    const long long n = node[q];
+    if (n < 0) continue;
+    const int m = threadIdx.x + q * 2 * NH;
+    const int el = m / NN, nd = m % NN, j = nd / NP, i = nd % NP;
+    const double u = s_u[el][nd], v = s_v[el][nd], uz = zsg > 0 ? u : -u;
+    const double xb = node_total<59>(s_y[0][el][nd], s_ey[0][el][j], s_y[1][el][nd], s_ey[1][el][i],
+                                     fma(-cM[q], u, acc[q]), -1);
+    a.xb[n] = xb;
+    a.Zs[n] = node_total<60>(s_z[0][el][nd], s_ez[0][el][j], s_z[1][el][nd], s_ez[1][el][i], zs[q], zsg);
+    a.Zm[n] = a.first ? uz * v : fma(uz, v, zm[q]);
+    if (a.bb_op == 1) a.bb[n] = u;
+    else if (a.bb_op == 2) a.bb[n] = bb[q] + u;
+    if (PCG && a.has_next) part = fma(xb, rp[q], part);
+    if (SREV == SREV_CHEB && a.has_next) {
+      const double dbv = db[q] + xb;
+      const double zb = a.cc * dbv;
+      a.u_out[n] = im[q] * zb;
+      a.iMb[n] = fma(zb, rp[q], iMb[q]);
+      a.db[n] = a.ca * dbv;
+    } else if (SREV == SREV_JACOBI && a.has_next) {
+      const double tb = a.omega * xb;
+      a.u_out[n] = tb * im[q];
+      a.iMb[n] = fma(tb, rp[q], iMb[q]);
     }
   }
   if (PCG && a.has_next) {

@@ -602,35 +602,18 @@ __device__ __forceinline__ void row_products(const FixFlux<NP>& f, const FixDeri
     r.G[i] = __double_as_longlong(v);
   }
 }
-// out[k] = acc[k] + sg (row part[k] + products[k]); R, er as row_products left them
-template <int NP>
-__device__ __forceinline__ void column_products(const FixFlux<NP>& f, const FixDeriv<NP>& d, double z0, double zL,
-                                                const long long* R, const int* er, const double* acc, int sg, double* out) {
-  int need = 0, el = er[0], eh = er[0];
-#pragma unroll
-  for (int k = 0; k < NP; ++k) {
-    need = max(need, fix::abs_hi(acc[k]));
-    el = el < er[k] ? el : er[k];
-    eh = max(eh, er[k]);
+// acc + sg (row + column) at one node, rounded once: r and c are sums of a row and a column in units of
+// 2^U / 2^(e - 1022) (e < 0: the bits of doubles).
+template <int U>
+__device__ __forceinline__ double node_total(long long r, int er, long long c, int ec, double acc, int sg) {
+  const int e = max(max(er, ec), fix::abs_hi(acc) >> 20);
+  if (er >= 0 && ec >= 0 && e >= 128 && e < fix::E_MAX) {
+    const long long v = fix::sar(r, e - er) + fix::sar(c, e - ec);
+    return fix::to_double(fix::add<U - 53>(sg > 0 ? v : -v, acc, e), e + 60 - U);
   }
-  need = max(need >> 20, eh);
-  FixSums<NP> s;
-  if (el >= 0 && product_line<NP>(f, d, z0, zL, need, false, s)) {
-#pragma unroll
-    for (int k = 0; k < NP; ++k) {
-      const long long v = s.G[k] + fix::sar(R[k], s.e - er[k]);
-      out[k] = fix::to_double(fix::add<7>(sg > 0 ? v : -v, acc[k], s.e), s.e);
-    }
-    return;
-  }
-#pragma unroll
-  for (int k = 0; k < NP; ++k) {
-    double v = flux_at<NP>(f, k) * deriv_at<NP>(d, k);
-    if (k == 0) v += z0;
-    if (k == NP - 1) v += zL;
-    v += er[k] < 0 ? __longlong_as_double(R[k]) : fix::to_double(R[k], er[k]);
-    out[k] = sg > 0 ? acc[k] + v : acc[k] - v;
-  }
+  const double x = er < 0 ? __longlong_as_double(r) : (er < 64 ? 0.0 : fix::to_double(r, er + 60 - U));
+  const double y = ec < 0 ? __longlong_as_double(c) : (ec < 64 ? 0.0 : fix::to_double(c, ec + 60 - U));
+  return sg > 0 ? acc + (x + y) : acc - (x + y);
 }
 
 // ---------------------------------------------------------------------------

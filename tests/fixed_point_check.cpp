@@ -259,7 +259,9 @@ template <int NP> static int run() {
         er[i] = r.e;
       }
       const int sg = uni() < 0.5 ? 1 : -1;
-      column_products<NP>(f, dv, z0, zL, R, er, acc, sg, out);
+      FixSums<NP> col;
+      row_products<NP>(f, dv, z0, zL, col);
+      for (int i = 0; i < NP; ++i) out[i] = node_total<60>(R[i], er[i], col.G[i], col.e, acc[i], sg);
       if (kind == 8) continue;
       long double top = 0, S[NP];
       double c64[NP];
