@@ -108,6 +108,10 @@ BasisDev make_basis_dev(int p, const double* xi, const double* w, const double* 
   B.hw = -0.5 / B.w[0];
   B.iw0 = 1.0 / B.w[0];
   B.iwL = 1.0 / B.w[B.np - 1];
+  std::memcpy(B.Dr, B.D, sizeof(B.D));
+  B.Dr[0][0] += 0.5 * B.iw0;
+  B.Dr[B.np - 1][B.np - 1] -= 0.5 * B.iwL;
+  B.fDr = make_fix(B.Dr, B.np);
   return B;
 }
 

@@ -27,7 +27,7 @@ template <int NP> void launch_k2_hyp_rk(const HypArgs2D& a, int nb, cudaStream_t
   k2_hyp_rk<NP><<<nb, Tiling2D<NP>::NT, 0, s>>>(a);
 }
 template <int NP> void launch_k2_hyp_rev(const HypRevArgs2D& a, int nb, cudaStream_t s) {
-  k2_hyp_rev<NP><<<nb, Tiling2D<NP>::NT, 0, s>>>(a);
+  k2_hyp_rev<NP><<<nb, 2 * Tiling2D<NP>::NH, 0, s>>>(a);
 }
 template <int NP> void launch_k2_apply_rev(int srev, const ApplyRevArgs2D& a, int nb, cudaStream_t s) {
   constexpr int NT2 = 2 * Tiling2D<NP>::NH;

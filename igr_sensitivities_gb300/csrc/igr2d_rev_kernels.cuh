@@ -29,54 +29,50 @@ namespace igrgpu {
 
 // Reverse of node_phys for both flux directions at one node: fbx, fby are
 // the adjoints of the x and y flux components; accumulates into qb[4]
-// (mx, my, rho, E), Sb and gb.
+// (mx, my, rho, E) and sets Sb and gb. With u = m / rho, H = (E + P + Sigma) /
+// rho, e3 = fbx_3 u_x + fby_3 u_y, pb = fbx_0 + fby_1 + e3 (d/dP_bar) and
+// k = -(g-1) pb - T, where T is what the node's wave speeds add to d/dE
+// (wavespeed_rev), the flux components and the kinetic part of the pressure
+// collect to
+//   d/dmx  = u_x (2 fbx_0 + k) + u_y (fbx_1 + fby_0) + fbx_2 + fbx_3 H
+//   d/dmy  = u_y (2 fby_1 + k) + u_x (fbx_1 + fby_0) + fby_2 + fby_3 H
+//   d/drho = -[u_x^2 (2 fbx_0 + k) / 2 + u_y^2 (2 fby_1 + k) / 2 + u_x u_y (fbx_1 + fby_0) + e3 H]
+//   d/dE   = e3 - k.
 __device__ __forceinline__ void node_phys_rev(double g, double mx, double my, double E, double S, double ir,
-                                              const double fbx[4], const double fby[4], double qb[4], double& Sb,
+                                              const double fbx[4], const double fby[4], double T, double qb[4], double& Sb,
                                               double& gb) {
   const double ux = mx * ir, uy = my * ir;
-  const double kin = fma(mx, mx, my * my) * (0.5 * ir);
   const double gm1 = g - 1.0;
-  const double P = gm1 * (E - kin), pb = P + S, epb = E + pb;
-  // fx = (mx ux + pb, my ux, mx, (E+pb) ux), fy = (mx uy, my uy + pb, my, (E+pb) uy)
-  const double uxb = fma(fbx[0], mx, fma(fbx[1], my, fbx[3] * epb));
-  const double uyb = fma(fby[0], mx, fma(fby[1], my, fby[3] * epb));
-  const double e3 = fma(fbx[3], ux, fby[3] * uy);   // d/dE through E + pb, and part of d/d pb
-  const double pbb = fbx[0] + fby[1] + e3;
-  qb[0] += fma(fbx[0], ux, fma(fby[0], uy, fbx[2]));
-  qb[1] += fma(fby[1], uy, fma(fbx[1], ux, fby[2]));
-  qb[3] += e3;
-  Sb += pbb;
-  // u = m / rho
-  qb[0] += uxb * ir;
-  qb[1] += uyb * ir;
-  qb[2] -= fma(uxb, ux, uyb * uy) * ir;
-  // P = (g-1)(E - kin), kin = |m|^2 / (2 rho)
-  gb = fma(pbb, E - kin, gb);
-  qb[3] = fma(pbb, gm1, qb[3]);
-  const double kb = -pbb * gm1;
-  qb[0] = fma(kb, ux, qb[0]);
-  qb[1] = fma(kb, uy, qb[1]);
-  qb[2] -= kb * kin * ir;
+  const double Ek = fma(-0.5, fma(mx, ux, my * uy), E);
+  const double H = fma(gm1, Ek, E + S) * ir;
+  const double e3 = fma(fbx[3], ux, fby[3] * uy);
+  const double pb = fbx[0] + fby[1] + e3;
+  const double k = fma(-gm1, pb, -T);
+  const double c = fbx[1] + fby[0];
+  const double p = ux * fma(2.0, fbx[0], k), q = uy * fma(2.0, fby[1], k), r = c * uy;
+  qb[0] = fma(fbx[3], H, qb[0]) + fbx[2] + (p + r);
+  qb[1] = fma(c, ux, fma(fby[3], H, qb[1])) + fby[2] + q;
+  qb[2] = fma(-ux, fma(0.5, p, r), fma(-uy, 0.5 * q, fma(-e3, H, qb[2])));
+  qb[3] += e3 - k;
+  Sb = pb;
+  gb = pb * Ek;
 }
 
-// Reverse of |u_n| + c, c = sqrt(g P / rho), at one node with adjoint wb. With Y = wb c / 2 and T = d/dP scaled to
-// the energy, T = (wb / 2c) g (g - 1) / rho:
-//   d/dE = T, d/dm = -T u (+ the sign of u_n / rho in the normal direction),
-//   d/drho = T |u|^2 / 2 - Y / rho - (that) u_n,  d/dgamma = Y (1/g + 1/(g - 1));   gs is that last factor.
-__device__ __forceinline__ void wavespeed_rev(int dir, double g, double gs, double mx, double my, double ir, double ws,
-                                              double wb, double qb[4], double& gb) {
-  const double ux = mx * ir, uy = my * ir;
-  const double un = dir == 0 ? ux : uy;
+// Reverse of |u_n| + c, c = sqrt(g P / rho), at one node with adjoint wb. With
+// Y = wb c / 2 it adds the sign of u_n / rho times wb to the normal momentum,
+// -Y / rho - (that) u_n to rho, Y (1/g + 1/(g - 1)) (gs is that factor) to
+// d/dgamma, and returns T = (wb / 2c) g (g - 1) / rho, its d/dE: the rest,
+// -T u to the momenta and T |u|^2 / 2 to rho, joins node_phys_rev.
+__device__ __forceinline__ double wavespeed_rev(double g, double gs, double mn, double ir, double ws, double wb, double& qn,
+                                                double& qr, double& gb) {
+  const double un = mn * ir;
   const double c = ws - fabs(un);
   const double h = 0.5 * wb, Y = h * c;
-  const double T = (h * reciprocal(c)) * ((g * (g - 1.0)) * ir);
   const double t = (signbit(un) ? -wb : wb) * ir;
   gb = fma(Y, gs, gb);
-  qb[0] = fma(-T, ux, qb[0]);
-  qb[1] = fma(-T, uy, qb[1]);
-  qb[dir] += t;
-  qb[2] = fma(0.5 * T, fma(ux, ux, uy * uy), fma(-Y, ir, fma(-t, un, qb[2])));
-  qb[3] += T;
+  qn += t;
+  qr = fma(-Y, ir, fma(-t, un, qr));
+  return (h * reciprocal(c)) * ((g * (g - 1.0)) * ir);
 }
 
 enum { SREV_NONE = 0, SREV_CHEB = 1, SREV_JACOBI = 2, SREV_PCG = 3 };
@@ -111,65 +107,70 @@ struct HypRevArgs2D {
   double ca, cc, omega;              // Chebyshev a_n, c_n ; Jacobi omega
 };
 
-// What bounds it: FP64 issue. The transposed volume terms run on the integer pipes with the stage coefficient in their
-// scale; a face takes 7 FP64 instructions per component. 8 x 128^2 P3: 680 us with FP64 contractions, 442 us now; 64^2:
-// 40.8 and 37.5.
+// Rows and columns run side by side, one half of the CTA each; the node work (flux reverse, combination) is spread over
+// all threads. What bounds it: FP64 issue. The transposed volume terms run on the integer pipes with the stage
+// coefficient and the own side of the face corrections in their matrix; a face takes 5 FP64 instructions per component.
+// 8 x 128^2 P3: 680 us with FP64 contractions; 442 with integer ones; 390 with the shorter faces and node reverse (191
+// FP64 instructions per warp of half the lines, pipe 84% busy). 64^2: 40.8, 37.8, and 23.6 in halves.
 template <int NP>
-__global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_hyp_rev(HypRevArgs2D a) {
+__global__ void __launch_bounds__(2 * Tiling2D<NP>::NH) k2_hyp_rev(HypRevArgs2D a) {
   using TL = Tiling2D<NP>;
-  constexpr int TE = TL::TE, NN = TL::NN, L = TL::L;
-  __shared__ double s_A[4][TE][NN];       // adjoint of the stage output
-  __shared__ double s_q[4][TE][NN];       // taped stage state
-  __shared__ double s_fbx[4][TE][NN];     // adjoint of the x fluxes (row phase)
-  __shared__ double s_qbx[4][TE][NP][2];  // q adjoint from the x faces, at the row ends
-  __shared__ double s_xw[TE][NP][2];      // x wave speed at x-face nodes
-  __shared__ double s_yw[TE][NP][2];
-  __shared__ double s_grow[TE][NP];       // row-phase d/dgamma partials
+  constexpr int TE = TL::TE, NN = TL::NN, L = TL::L, TX = TL::TX, NH = TL::NH;
+  constexpr int NQ = (TE * NN + 2 * NH - 1) / (2 * NH);  // nodes per thread
+  __shared__ double s_A[4][TE][NN];         // adjoint of the stage output; [0] last holds the nodes' d/dgamma
+  __shared__ double s_q[4][TE][NN];         // taped stage state
+  __shared__ double s_fb[2][4][TE][NN];     // adjoints of the x and y fluxes
+  __shared__ double s_qb[2][4][TE][NP][2];  // state adjoints from the faces, at the line ends
+  __shared__ double s_w[2][TE][NP][2];      // wave speeds at the line ends
+  __shared__ double s_T[2][TE][NP][2];      // what their wave speeds add to d/dE (wavespeed_rev)
+  __shared__ double s_g[2][TE][NP];         // the lines' d/dgamma
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];
-  const ElemView vr = elem_view<NP>(tl, I, 0), vc = elem_view<NP>(tl, I, 1);
   const BasisDev& B = a.B;
   const double g = I.gamma;
   const double c2dt = a.c2 * I.dt;
+  const int dir = threadIdx.x >= NH;  // 0: rows and x faces, 1: columns and y faces
+  const ElemView w = elem_view<NP>(tl, I, dir, threadIdx.x - dir * NH);
+  const int e = w.e, t = w.t;
+  const int st = dir == 0 ? 1 : NP, at = dir == 0 ? t * NP : t;  // node k of the line: at + k st
+  const double* ws = dir == 0 ? a.ws_x : a.ws_y;
 
-  // ---- phase 1: row data of vr into smem; face wave speeds
-  if (vr.valid) {
-    const int t = vr.t, e = vr.e;
+  // ---- node data into shared memory
+  long long node[NQ];
 #pragma unroll
-    for (int i = 0; i < NP; ++i) {
-      const long long n = vr.base + t * NP + i;
+  for (int q = 0; q < NQ; ++q) {
+    const int m = threadIdx.x + q * 2 * NH;
+    const int el = m / NN, nd = m % NN, ex = tl.ex0 + el % TX, ey = tl.ey0 + el / TX;
+    const bool live = m < TE * NN && ex < I.nex && ey < I.ney;
+    const long long n = I.off + (long long)NN * (ex + (long long)I.nex * ey) + nd;
+    node[q] = live ? n : -1;
+    if (!live) continue;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) { s_q[c][e][t * NP + i] = a.q[c][n]; s_A[c][e][t * NP + i] = a.A[c][n]; }
-    }
-    s_xw[e][t][0] = a.ws_x[vr.base + t * NP];
-    s_xw[e][t][1] = a.ws_x[vr.base + t * NP + L];
+    for (int c = 0; c < 4; ++c) { s_q[c][el][nd] = a.q[c][n]; s_A[c][el][nd] = a.A[c][n]; }
   }
-  if (vc.valid) {
-    s_yw[vc.e][vc.t][0] = a.ws_y[vc.base + vc.t];
-    s_yw[vc.e][vc.t][1] = a.ws_y[vc.base + L * NP + vc.t];
+  if (w.valid) {
+    s_w[dir][e][t][0] = ws[w.base + at];
+    s_w[dir][e][t][1] = ws[w.base + at + L * st];
   }
   __syncthreads();
 
-  // One line (row: dir 0, column: dir 1) of all four components. Its flux adjoints are the transposed volume term of
-  // kbar = c2 dt A plus, at the end nodes, the LLF flux's reverse: with a = coefficient of the own correction times
-  // kbar / 2 and b the partner's, the own flux gets b - a, the own state +-lambda (a + b), and lambda (a + b) dq.
-  // put(v, fb, q0, qL) takes component v's flux adjoints and the own-state adjoints of the two faces. The components
-  // stay a rolled loop: its body is a few hundred integer instructions.
-  auto line = [&](int dir, const ElemView& w, double invJ, double (*s_w)[NP][2], const double* ws, auto&& put, double lamb[2],
-                  bool wins[2]) {
-    const int e = w.e, t = w.t;
-    const int st = dir == 0 ? 1 : NP, at = dir == 0 ? t * NP : t;  // node k of the line: at + k st
-    const double ci = c2dt * invJ;
+  // ---- one line of all four components. Its flux adjoints are the transposed volume term of kbar = c2 dt A plus, at the
+  // end nodes, the LLF flux's reverse: with x = coefficient of the own correction times kbar / 2 and y the partner's, the
+  // own flux gets y - x (-x sits in the matrix, fDr), the own state +-lambda (x + y), and lambda (x + y) dq. The
+  // components stay a rolled loop: its body is a few hundred integer instructions.
+  if (w.valid) {
+    const double ci = c2dt * (dir == 0 ? I.ijx : I.ijy);
     const FixScale sc = fix_scale(-ci);
     long long pn[2];
     int it[2];
-    double lam[2], cfo[2], cfp[2];
+    double lam[2], cfo[2], cfp[2], lamb[2];
+    bool wins[2];
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
       const int d = s == 0 ? -1 : 1;
       const long long pb = neighbour<NP>(tl, I, w.ex, w.ey, dir == 0 ? d : 0, dir == 0 ? 0 : d, &it[s]);
       pn[s] = pb + at + (s == 0 ? L : 0) * st;
-      const double own = s_w[e][t][s], par = it[s] >= 0 ? s_w[it[s] >= 0 ? it[s] : 0][t][1 - s] : ws[pn[s]];
+      const double own = s_w[dir][e][t][s], par = it[s] >= 0 ? s_w[dir][it[s] >= 0 ? it[s] : 0][t][1 - s] : ws[pn[s]];
       const double mag = s == 0 ? max_nonneg(own, par) : max_nonneg(par, own);  // max(ws_R, ws_L)
       wins[s] = s == 0 ? gt_nonneg(own, par) : !gt_nonneg(par, own);
       lam[s] = s == 0 ? -mag : mag;
@@ -180,7 +181,7 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_hyp_rev(HypRevArgs2D a) {
     }
 #pragma unroll 1
     for (int v = 0; v < 4; ++v) {
-      double A[NP], acc[NP], fb[NP], qo[2];
+      double A[NP], acc[NP], fb[NP];
 #pragma unroll
       for (int k = 0; k < NP; ++k) A[k] = s_A[v][e][at + k * st];
 #pragma unroll
@@ -189,110 +190,99 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_hyp_rev(HypRevArgs2D a) {
         const double pA = it[s] >= 0 ? s_A[v][it[s] >= 0 ? it[s] : 0][nd] : a.A[v][pn[s]];
         const double pq = it[s] >= 0 ? s_q[v][it[s] >= 0 ? it[s] : 0][nd] : a.q[v][pn[s]];
         const double oq = s_q[v][e][at + (s == 0 ? 0 : L) * st];
-        const double x = cfo[s] * A[s == 0 ? 0 : L], y = cfp[s] * pA;
-        const double h = x + y;
-        acc[s == 0 ? 0 : L] = y - x;
-        qo[s] = lam[s] * h;
+        const double y = cfp[s] * pA, h = fma(cfo[s], A[s == 0 ? 0 : L], y);
+        acc[s == 0 ? 0 : L] = y;
+        s_qb[dir][v][e][t][s] = lam[s] * h;
         lamb[s] = fma(h, s == 0 ? pq - oq : oq - pq, lamb[s]);  // q_L - q_R
       }
-      line_op<NP, true, true, true>(B.fD, B.D, &sc, A, acc, [](int k) { return k == 0 || k == L; }, fb);
-      put(v, fb, qo[0], qo[1]);
-    }
-  };
-  // reverse of the wave speed of face s where the own side sets lambda
-  auto speed = [&](int dir, const ElemView& w, int s, double ws, double lamb, double qb[4], double& gb) {
-    const int nd = dir == 0 ? w.t * NP + (s == 0 ? 0 : L) : (s == 0 ? 0 : L) * NP + w.t;
-    wavespeed_rev(dir, g, I.gsum, s_q[0][w.e][nd], s_q[1][w.e][nd], a.invr[w.base + nd], ws, lamb, qb, gb);
-  };
-  double gb = 0.0;
-  // ---- phase 2a (row of vr)
-  if (vr.valid) {
-    const int t = vr.t, e = vr.e;
-    double lamb[2];
-    bool wins[2];
-    line(0, vr, I.ijx, s_xw, a.ws_x,
-         [&](int v, const double* fb, double q0, double qL) {
+      line_op<NP, true, true, true>(B.fDr, B.Dr, &sc, A, acc, [](int k) { return k == 0 || k == L; }, fb);
 #pragma unroll
-           for (int i = 0; i < NP; ++i) s_fbx[v][e][t * NP + i] = fb[i];
-           s_qbx[v][e][t][0] = q0;
-           s_qbx[v][e][t][1] = qL;
-         },
-         lamb, wins);
+      for (int k = 0; k < NP; ++k) s_fb[dir][v][e][at + k * st] = fb[k];
+    }
+    // reverse of the wave speed where the own side sets lambda
+    double gb = 0.0;
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
-      if (!wins[s]) continue;
-      double qb[4];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) qb[c] = s_qbx[c][e][t][s];
-      speed(0, vr, s, s_xw[e][t][s], lamb[s], qb, gb);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) s_qbx[c][e][t][s] = qb[c];
+      double T = 0.0;
+      if (wins[s]) {
+        const int nd = at + (s == 0 ? 0 : L) * st;
+        double qn = s_qb[dir][dir][e][t][s], qr = s_qb[dir][2][e][t][s];
+        T = wavespeed_rev(g, I.gsum, s_q[dir][e][nd], a.invr[w.base + nd], s_w[dir][e][t][s], lamb[s], qn, qr, gb);
+        s_qb[dir][dir][e][t][s] = qn;
+        s_qb[dir][2][e][t][s] = qr;
+      }
+      s_T[dir][e][t][s] = T;
     }
-    s_grow[e][t] = gb;
-    gb = 0.0;
+    s_g[dir][e][t] = gb;
   }
-  // ---- phase 2b (column of vc): the y flux and face-state adjoints stay in registers
-  double fby[4][NP], qby[2][4];
-  if (vc.valid) {
-    double lamb[2];
-    bool wins[2];
-    line(1, vc, I.ijy, s_yw, a.ws_y,
-         [&](int v, const double* fb, double q0, double qL) {
+  // ---- nodes: merged flux reverse, combination, outputs. What they read is loaded before the barrier and before anything
+  // is stored.
+  double S[NQ], ir[NQ], Sb[NQ], Qn[NQ][4], Qs[NQ][4], im[NQ], rl[NQ];
 #pragma unroll
-           for (int c = 0; c < 4; ++c) {  // fby[v] = fb with a register index
+  for (int q = 0; q < NQ; ++q) {
+    const long long n = node[q];
+    if (n < 0) continue;
+    S[q] = a.S[n];
+    ir[q] = a.invr[n];
+    Sb[q] = a.Sb_add ? a.Sb[n] : 0.0;
 #pragma unroll
-             for (int l = 0; l < NP; ++l) fby[c][l] = v == c ? fb[l] : fby[c][l];
-             qby[0][c] = v == c ? q0 : qby[0][c];
-             qby[1][c] = v == c ? qL : qby[1][c];
-           }
-         },
-         lamb, wins);
-#pragma unroll
-    for (int s = 0; s < 2; ++s)
-      if (wins[s]) speed(1, vc, s, s_yw[vc.e][vc.t][s], lamb[s], qby[s], gb);
+    for (int c = 0; c < 4; ++c) {
+      Qn[q][c] = a.qn_mode == 2 ? a.Qn[c][n] : 0.0;
+      Qs[q][c] = a.qs_add ? a.Qs[c][n] : 0.0;
+    }
+    if (a.srev != SREV_NONE) {
+      im[q] = a.cinvM[n];
+      rl[q] = a.r_last[n];
+    }
   }
   __syncthreads();
-  if (!vc.valid) return;
-  // ---- phase 3 (column of vc): merged flux reverse per node, combination, outputs
-  const int t = vc.t, e = vc.e;
-  gb += s_grow[e][t];
 #pragma unroll
-  for (int l = 0; l < NP; ++l) {
-    const long long n = vc.base + l * NP + t;
-    const int nd = l * NP + t;
-    double fbx[4], fbyl[4], qq[4];
+  for (int q = 0; q < NQ; ++q) {
+    const long long n = node[q];
+    if (n < 0) continue;
+    const int m = threadIdx.x + q * 2 * NH;
+    const int el = m / NN, nd = m % NN, j = nd / NP, i = nd % NP;
+    double fbx[4], fby[4], qq[4], A[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      fbx[c] = s_fbx[c][e][nd]; fbyl[c] = fby[c][l];
-      qq[c] = (t == 0 || t == L) ? s_qbx[c][e][l][t == 0 ? 0 : 1] : 0.0;
-      if (l == 0 || l == L) qq[c] += qby[l == 0 ? 0 : 1][c];
+      fbx[c] = s_fb[0][c][el][nd]; fby[c] = s_fb[1][c][el][nd]; A[c] = s_A[c][el][nd];
+      qq[c] = (i == 0 || i == L) ? s_qb[0][c][el][j][i == 0 ? 0 : 1] : 0.0;
+      if (j == 0 || j == L) qq[c] += s_qb[1][c][el][i][j == 0 ? 0 : 1];
     }
-    double Sb = 0.0;
-    node_phys_rev(g, s_q[0][e][nd], s_q[1][e][nd], s_q[3][e][nd], a.S[n], a.invr[n], fbx, fbyl, qq, Sb, gb);
+    double T = (i == 0 || i == L) ? s_T[0][el][j][i == 0 ? 0 : 1] : 0.0;
+    if (j == 0 || j == L) T += s_T[1][el][i][j == 0 ? 0 : 1];
+    double sb, gb;
+    node_phys_rev(g, s_q[0][el][nd], s_q[1][el][nd], s_q[3][el][nd], S[q], ir[q], fbx, fby, T, qq, sb, gb);
+    s_A[0][el][nd] = gb;  // read by this thread alone so far
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      const double Av = a.A[c][n];
-      if (a.qn_mode == 1) a.Qn[c][n] = a.c0 * Av;
-      else if (a.qn_mode == 2) a.Qn[c][n] = fma(a.c0, Av, a.Qn[c][n]);
-      const double val = fma(a.c1, Av, qq[c]);
-      a.Qs[c][n] = a.qs_add ? a.Qs[c][n] + val : val;
+      if (a.qn_mode == 1) a.Qn[c][n] = a.c0 * A[c];
+      else if (a.qn_mode == 2) a.Qn[c][n] = fma(a.c0, A[c], Qn[q][c]);
+      const double val = fma(a.c1, A[c], qq[c]);
+      a.Qs[c][n] = a.qs_add ? Qs[q][c] + val : val;
     }
-    const double Sbt = a.Sb_add ? a.Sb[n] + Sb : Sb;
+    const double Sbt = a.Sb_add ? Sb[q] + sb : sb;
     a.Sb[n] = Sbt;
     if (a.srev == SREV_CHEB) {
       // x_n = x_{n-1} + d_n ; d_n = a_n d_{n-1} + c_n z_n ; z_n = (1/M) r_{n-1}
       const double zb = a.cc * Sbt;
-      a.u_out[n] = a.cinvM[n] * zb;
-      a.iMb[n] = zb * a.r_last[n];
+      a.u_out[n] = im[q] * zb;
+      a.iMb[n] = zb * rl[q];
       a.db[n] = a.ca * Sbt;
     } else if (a.srev == SREV_JACOBI) {
       // x_n = x_{n-1} + (omega r_{n-1}) (1/M)
       const double tb = a.omega * Sbt;
-      a.u_out[n] = tb * a.cinvM[n];
-      a.iMb[n] = tb * a.r_last[n];
+      a.u_out[n] = tb * im[q];
+      a.iMb[n] = tb * rl[q];
     }
   }
-  a.gnode[vc.base + t] += gb;
+  __syncthreads();
+  if (dir == 1 && w.valid) {
+    double gb = s_g[0][e][t] + s_g[1][e][t];
+#pragma unroll
+    for (int l = 0; l < NP; ++l) gb += s_A[0][e][l * NP + t];
+    a.gnode[w.base + t] += gb;
+  }
 }
 
 // ---------------------------------------------------------------------------

@@ -28,6 +28,8 @@ struct BasisDev {
   double hw;                // -1 / (2 w_0): SIP face coefficient factor
   double iw0, iwL;          // 1 / w_0, 1 / w_L
   FixMat fD, fW2;           // D and W2 as integers (igr_fix.cuh)
+  double Dr[MAXNP][MAXNP];  // D + diag(1/(2 w_0), 0, .., -1/(2 w_L)): with the own side's share of the face corrections
+  FixMat fDr;
 };
 
 // One problem instance of a batch (2D): mesh, physics parameters and where
