@@ -686,181 +686,167 @@ struct FluxNode { double q[4], fx0, f1, fx3, fy1, fy3, aux; };
 template <int NP, bool AUX>
 struct StageSmem {
   double q[4][Tiling2D<NP>::TE][Tiling2D<NP>::NN];
-  double fy[3][Tiling2D<NP>::TE][Tiling2D<NP>::NN];       // fy_0 = fx_1, fy_1, fy_3
+  double f[5][Tiling2D<NP>::TE][Tiling2D<NP>::NN];            // fx_0, fx_1 = fy_0, fx_3, fy_1, fy_3
   double aux[AUX ? Tiling2D<NP>::TE : 1][Tiling2D<NP>::NN];
-  long long k[4][Tiling2D<NP>::TE][Tiling2D<NP>::NN];     // fx, then the x part of c2 dt k (fixed point, exponents ke)
-  int ke[4][Tiling2D<NP>::TE][NP];
-  double fx[Tiling2D<NP>::TE][NP][2][2];                  // fx_0, fx_3 at the x-face nodes (left, right)
-  double wx[Tiling2D<NP>::TE][NP][2], wy[Tiling2D<NP>::TE][NP][2];  // wave speeds at x- and y-face nodes
+  long long k[2][4][Tiling2D<NP>::TE][Tiling2D<NP>::NN];      // row and column parts of c2 dt k (fixed point)
+  int ke[2][4][Tiling2D<NP>::TE][NP];                         // their exponents
+  double w[2][Tiling2D<NP>::TE][NP][2];                       // wave speeds at the line ends
 };
 
 // DG volume and LLF face terms of one tile with the SSP-RK3 combination q_out = c0 q^n + c1 q_s + c2 dt k (raw: k itself)
 // for the physics PH (the Euler fluxes or their tangent):
-//   at(n)             the node's FluxNode
-//   speed_x(n, node)  wave speeds at own face nodes; speed_y(n, q_1, aux)
-//   partner(n, f)     the node across an out-of-tile face; its wave speed by partner_speed(dir, n, node)
+//   at(n)                 the node's FluxNode
+//   speed(dir, n, q, aux, own)  wave speed at a face node, q the quantity that is the mass flux; own: of this tile
 //   qn(v, n), put(v, n, value)
-// What bounds it: FP64 issue. Volume terms, their scaling, the row parts and the stage combination's sum are integer work
-// (igr_fix.cuh); the stage coefficient is folded into the scale of the derivatives and face terms, so that
-// q_out = (c0 q^n + c1 q_s) + [c2 dt k] is one rounded sum and k itself is never formed. Euler, 8 x 128^2 P3: 427 us with
-// FP64 contractions and IEEE square roots, 251 us now (FP64 pipe 79% busy); 64^2: 24.9 and 22.4. Shared memory holds each
-// quantity once, 29.5 KB for P3: 7 CTAs per SM where 45 KB gave 5.
+// Node work is spread over all 2 NH threads of the CTA; line work runs with rows and columns side by side, one half each.
+// What bounds it: FP64 issue. Volume terms, their scaling, the row and column parts and the stage combination's sum are
+// integer work (igr_fix.cuh); the stage coefficient is folded into the scale of the derivatives and face terms, so that
+// q_out = c0 q^n + c1 q_s + [c2 dt k] is one rounded sum and k itself is never formed. Euler, 8 x 128^2 P3: 427 us with
+// FP64 contractions and IEEE square roots, 248 us now (FP64 pipe 80% busy; 252 with the state weights in FP64); 64^2: 24.9,
+// 22.4 with one thread per pair of lines, 18.6 in halves.
 template <int NP, bool AUX, class PH>
 __device__ __forceinline__ void dg_stage(const PH& ph, const BasisDev& B, const Tile2D tl, const Inst2D& I, double c0, double c1,
                                          double c2, bool raw, StageSmem<NP, AUX>& sm) {
   using TL = Tiling2D<NP>;
-  constexpr int L = TL::L, TX = TL::TX, TY = TL::TY;
-  const ElemView vr = elem_view<NP>(tl, I, 0), vc = elem_view<NP>(tl, I, 1);
+  constexpr int TE = TL::TE, NN = TL::NN, L = TL::L, TX = TL::TX, TY = TL::TY, NH = TL::NH;
+  constexpr int NQ = (TE * NN + 2 * NH - 1) / (2 * NH);  // nodes per thread
+  const int dir = threadIdx.x >= NH;  // 0: rows and x faces, 1: columns and y faces
+  const ElemView w = elem_view<NP>(tl, I, dir, threadIdx.x - dir * NH);
+  const int e = w.e, t = w.t;
+  const int st = dir == 0 ? 1 : NP, at = dir == 0 ? t * NP : t;  // node k of the line: at + k st
   const double c2dt = raw ? 1.0 : c2 * I.dt;
-  const double sx = -c2dt * I.ijx, sy = -c2dt * I.ijy;
+  const double sl = -c2dt * (dir == 0 ? I.ijx : I.ijy);
 
-  // ---- phase 1 (row of vr): fluxes, x-face node data. The x fluxes wait in the thread's own row of sm.k.
-  if (vr.valid) {
-    const int t = vr.t, e = vr.e;
+  // ---- nodes: fluxes
+  long long node[NQ];
 #pragma unroll
-    for (int i = 0; i < NP; ++i) {
-      const long long n = vr.base + t * NP + i;
-      const int nd = t * NP + i;
-      const FluxNode f = ph.at(n);
+  for (int q = 0; q < NQ; ++q) {
+    const int m = threadIdx.x + q * 2 * NH;
+    const int el = m / NN, nd = m % NN, ex = tl.ex0 + el % TX, ey = tl.ey0 + el / TX;
+    const bool live = m < TE * NN && ex < I.nex && ey < I.ney;
+    const long long n = I.off + (long long)NN * (ex + (long long)I.nex * ey) + nd;
+    node[q] = live ? n : -1;
+    if (!live) continue;
+    const FluxNode f = ph.at(n);
 #pragma unroll
-      for (int v = 0; v < 4; ++v) sm.q[v][e][nd] = f.q[v];
-      if (AUX) sm.aux[AUX ? e : 0][nd] = f.aux;
-      sm.fy[0][e][nd] = f.f1; sm.fy[1][e][nd] = f.fy1; sm.fy[2][e][nd] = f.fy3;
-      sm.k[0][e][nd] = __double_as_longlong(f.fx0); sm.k[1][e][nd] = __double_as_longlong(f.f1);
-      sm.k[2][e][nd] = __double_as_longlong(f.q[0]); sm.k[3][e][nd] = __double_as_longlong(f.fx3);
-      if (i == 0 || i == L) {
-        const int s = i == 0 ? 0 : 1;
-        sm.fx[e][t][s][0] = f.fx0; sm.fx[e][t][s][1] = f.fx3;
-        sm.wx[e][t][s] = ph.speed_x(n, f);
-      }
-    }
+    for (int v = 0; v < 4; ++v) sm.q[v][el][nd] = f.q[v];
+    sm.f[0][el][nd] = f.fx0; sm.f[1][el][nd] = f.f1; sm.f[2][el][nd] = f.fx3;
+    sm.f[3][el][nd] = f.fy1; sm.f[4][el][nd] = f.fy3;
+    if (AUX) sm.aux[AUX ? el : 0][nd] = f.aux;
   }
   __syncthreads();
-  // ---- phase 2 (column of vc): y-face wave speeds
-  if (vc.valid) {
-    const int t = vc.t, e = vc.e;
+  // The line's flux of component v: the mass flux is the quantity q[dir] itself.
+  auto flux = [&](int v, int el, int nd) {
+    if (v == 2) return sm.q[dir][el][nd];
+    return sm.f[dir == 0 ? v - (v >> 1) : (v == 0 ? 1 : (v == 1 ? 3 : 4))][el][nd];
+  };
+  // ---- lines: wave speeds at the ends, volume term. The field loops stay rolled: their bodies are a few hundred integer
+  // instructions, and four copies of them cost more in instruction fetch than they save.
+  if (w.valid) {
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
-      const int nd = (s == 0 ? 0 : L) * NP + t;
-      sm.wy[e][t][s] = ph.speed_y(vc.base + nd, sm.q[1][e][nd], AUX ? sm.aux[AUX ? e : 0][nd] : 0.0);
+      const int nd = at + (s == 0 ? 0 : L) * st;
+      sm.w[dir][e][t][s] = ph.speed(dir, w.base + nd, sm.q[dir][e][nd], AUX ? sm.aux[AUX ? e : 0][nd] : 0.0, true);
     }
-  }
-  // ---- (row of vr): x faces, owner computes its side
-  struct PF { double q[4], f0, f1, f3, ws; };  // f: the components that are not a transported quantity
-  if (vr.valid) {
-    const int t = vr.t, e = vr.e;
-    auto fetch = [&](int s) {
-      int it;
-      const long long pb = neighbour<NP>(tl, I, vr.ex, vr.ey, s == 0 ? -1 : 1, 0, &it);
-      const int nd = t * NP + (s == 0 ? L : 0);
-      PF p;
-      if (it >= 0) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) p.q[c] = sm.q[c][it][nd];
-        const int ps = s == 0 ? 1 : 0;
-        p.f0 = sm.fx[it][t][ps][0]; p.f1 = sm.fy[0][it][nd]; p.f3 = sm.fx[it][t][ps][1]; p.ws = sm.wx[it][t][ps];
-      } else {
-        const FluxNode f = ph.at(pb + nd);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) p.q[c] = f.q[c];
-        p.f0 = f.fx0; p.f1 = f.f1; p.f3 = f.fx3;
-        p.ws = ph.partner_speed(0, pb + nd, f);
-      }
-      return p;
-    };
-    const int sf = first_side(vr.ext, TX);
-    const PF pA = fetch(sf), pB = fetch(1 - sf);
-    double add[2][4];
-#pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      const PF& p = (s == sf) ? pA : pB;
-      const int nd = t * NP + (s == 0 ? 0 : L);
-      const double own = sm.wx[e][t][s];
-      const double mag = max_nonneg(s == 0 ? own : p.ws, s == 0 ? p.ws : own);
-      const double lam = s == 0 ? mag : -mag;
-      const double cf = s == 0 ? -0.5 * B.iw0 * sx : 0.5 * B.iwL * sx;
-      const double dm = p.q[0] - sm.q[0][e][nd];
-      add[s][0] = cf * llf_jump(p.f0, sm.fx[e][t][s][0], lam, dm);
-      add[s][1] = cf * llf_jump(p.f1, sm.fy[0][e][nd], lam, p.q[1] - sm.q[1][e][nd]);
-      add[s][2] = cf * fma(lam, p.q[2] - sm.q[2][e][nd], dm);  // fx_2 = q_0
-      add[s][3] = cf * llf_jump(p.f3, sm.fx[e][t][s][1], lam, p.q[3] - sm.q[3][e][nd]);
-    }
-    // The field loops stay rolled: their bodies are a few hundred integer instructions, and four copies of them cost
-    // more in instruction fetch than they save.
-    const FixScale c = fix_scale(sx);
+    const FixScale c = fix_scale(sl);
 #pragma unroll 1
     for (int v = 0; v < 4; ++v) {
       double f[NP];
 #pragma unroll
-      for (int i = 0; i < NP; ++i) f[i] = __longlong_as_double(sm.k[v][e][t * NP + i]);
-      FixSums<NP> k;
-      row_scaled<NP, false>(B, c, f, k);
-      row_add_ends<NP>(k, pick4(add[0], v), pick4(add[1], v));
+      for (int k = 0; k < NP; ++k) f[k] = flux(v, e, at + k * st);
+      FixSums<NP> r;
+      row_scaled<NP, false>(B, c, f, r);
 #pragma unroll
-      for (int i = 0; i < NP; ++i) sm.k[v][e][t * NP + i] = k.G[i];
-      sm.ke[v][e][t] = k.e;
+      for (int k = 0; k < NP; ++k) sm.k[dir][v][e][at + k * st] = r.G[k];
+      sm.ke[dir][v][e][t] = r.e;
     }
   }
   __syncthreads();
-  if (!vc.valid) return;
-  // ---- phase 3 (column of vc): y faces, y volume term, RK combination
-  const int t = vc.t, e = vc.e;
-  auto fetchy = [&](int s) {
-    int it;
-    const long long pb = neighbour<NP>(tl, I, vc.ex, vc.ey, 0, s == 0 ? -1 : 1, &it);
-    const int nd = (s == 0 ? L : 0) * NP + t;
-    PF p;
-    if (it >= 0) {
+  // ---- lines: faces, owner computes its side
+  if (w.valid) {
+    double pq[2][4], pf[2][3], lam[2];  // the partners' quantities, fluxes (0, 1, 3) and the signed lambda
+    const int sf = dir == 0 ? first_side(w.ext, TX) : first_side(w.eyt, TY);
 #pragma unroll
-      for (int c = 0; c < 4; ++c) p.q[c] = sm.q[c][it][nd];
-      p.f0 = sm.fy[0][it][nd]; p.f1 = sm.fy[1][it][nd]; p.f3 = sm.fy[2][it][nd]; p.ws = sm.wy[it][t][s == 0 ? 1 : 0];
-    } else {
-      const FluxNode f = ph.at(pb + nd);
+    for (int h = 0; h < 2; ++h) {
+      const int s = h == 0 ? sf : 1 - sf, d = s == 0 ? -1 : 1;
+      int it;
+      const long long pb = neighbour<NP>(tl, I, w.ex, w.ey, dir == 0 ? d : 0, dir == 0 ? 0 : d, &it);
+      const int nd = at + (s == 0 ? L : 0) * st;
+      double q[4], f[3], ws;
+      if (it >= 0) {
 #pragma unroll
-      for (int c = 0; c < 4; ++c) p.q[c] = f.q[c];
-      p.f0 = f.f1; p.f1 = f.fy1; p.f3 = f.fy3;
-      p.ws = ph.partner_speed(1, pb + nd, f);
+        for (int v = 0; v < 4; ++v) q[v] = sm.q[v][it][nd];
+        f[0] = flux(0, it, nd); f[1] = flux(1, it, nd); f[2] = flux(3, it, nd);
+        ws = sm.w[dir][it][t][1 - s];
+      } else {
+        const FluxNode p = ph.at(pb + nd);
+#pragma unroll
+        for (int v = 0; v < 4; ++v) q[v] = p.q[v];
+        f[0] = dir == 0 ? p.fx0 : p.f1; f[1] = dir == 0 ? p.f1 : p.fy1; f[2] = dir == 0 ? p.fx3 : p.fy3;
+        ws = ph.speed(dir, pb + nd, p.q[dir], p.aux, false);
+      }
+      const double own = sm.w[dir][e][t][s];
+      const double mag = max_nonneg(s == 0 ? own : ws, s == 0 ? ws : own);
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {  // register arrays by the run-time side
+        if (r != s) continue;
+        lam[r] = r == 0 ? mag : -mag;
+#pragma unroll
+        for (int v = 0; v < 4; ++v) pq[r][v] = q[v];
+#pragma unroll
+        for (int v = 0; v < 3; ++v) pf[r][v] = f[v];
+      }
     }
-    return p;
-  };
-  const int sf = first_side(vc.eyt, TY);
-  const PF qA = fetchy(sf), qB = fetchy(1 - sf);
-  double add[2][4], cf[2];
+    double add[2][4];
 #pragma unroll
-  for (int s = 0; s < 2; ++s) {
-    const PF& p = (s == sf) ? qA : qB;
-    const int nd = (s == 0 ? 0 : L) * NP + t;
-    const double own = sm.wy[e][t][s];
-    const double mag = max_nonneg(s == 0 ? own : p.ws, s == 0 ? p.ws : own);
-    const double lam = s == 0 ? mag : -mag;
-    cf[s] = s == 0 ? -0.5 * B.iw0 * sy : 0.5 * B.iwL * sy;
-    const double dm = p.q[1] - sm.q[1][e][nd];
-    add[s][0] = llf_jump(p.f0, sm.fy[0][e][nd], lam, p.q[0] - sm.q[0][e][nd]);
-    add[s][1] = llf_jump(p.f1, sm.fy[1][e][nd], lam, dm);
-    add[s][2] = fma(lam, p.q[2] - sm.q[2][e][nd], dm);
-    add[s][3] = llf_jump(p.f3, sm.fy[2][e][nd], lam, p.q[3] - sm.q[3][e][nd]);
-  }
-  const FixScale c = fix_scale(sy);
-  const bool with_qn = __double_as_longlong(c0) != 0;
+    for (int s = 0; s < 2; ++s) {
+      const int nd = at + (s == 0 ? 0 : L) * st;
+      const double cf = s == 0 ? -0.5 * B.iw0 * sl : 0.5 * B.iwL * sl;
+      double dq[4];
+#pragma unroll
+      for (int v = 0; v < 4; ++v) dq[v] = pq[s][v] - sm.q[v][e][nd];
+      add[s][0] = cf * llf_jump(pf[s][0], flux(0, e, nd), lam[s], dq[0]);
+      add[s][1] = cf * llf_jump(pf[s][1], flux(1, e, nd), lam[s], dq[1]);
+      add[s][2] = cf * fma(lam[s], dq[2], dir == 0 ? dq[0] : dq[1]);  // the mass flux is q[dir]
+      add[s][3] = cf * llf_jump(pf[s][2], flux(3, e, nd), lam[s], dq[3]);
+    }
 #pragma unroll 1
-  for (int v = 0; v < 4; ++v) {
-    double f[NP], acc[NP], out[NP];
-    long long R[NP];
-    int er[NP];
+    for (int v = 0; v < 4; ++v) {
+      FixSums<NP> r;
 #pragma unroll
-    for (int l = 0; l < NP; ++l) {
-      const int nd = l * NP + t;
-      f[l] = v == 2 ? sm.q[1][e][nd] : sm.fy[v - (v >> 1)][e][nd];  // fy_0, fy_1, q_1, fy_3
-      R[l] = sm.k[v][e][nd];
-      er[l] = sm.ke[v][e][l];
-      const double qs = sm.q[v][e][nd];
-      acc[l] = raw ? 0.0 : (with_qn ? fma(c0, ph.qn(v, vc.base + nd), c1 * qs) : qs);  // without q^n: c1 = 1
-      if (l == 0) acc[l] = fma(cf[0], pick4(add[0], v), acc[l]);
-      if (l == L) acc[l] = fma(cf[1], pick4(add[1], v), acc[l]);
+      for (int k = 0; k < NP; ++k) r.G[k] = sm.k[dir][v][e][at + k * st];
+      r.e = sm.ke[dir][v][e][t];
+      row_add_ends<NP>(r, pick4(add[0], v), pick4(add[1], v));
+#pragma unroll
+      for (int k = 0; k < NP; ++k) sm.k[dir][v][e][at + k * st] = r.G[k];
+      sm.ke[dir][v][e][t] = r.e;
     }
-    column_scaled<NP, false>(B, c, f, R, er, acc, out);
+  }
+  // ---- nodes: RK combination; q^n is loaded before the barrier and before anything is stored
+  const bool with_qn = !raw && __double_as_longlong(c0) != 0;
+  const FixScale w0 = fix_scale(c0), w1 = fix_scale(c1);
+  double qn[NQ][4];
 #pragma unroll
-    for (int l = 0; l < NP; ++l) ph.put(v, vc.base + l * NP + t, out[l]);
+  for (int q = 0; q < NQ; ++q) {
+    if (node[q] < 0) continue;
+#pragma unroll
+    for (int v = 0; v < 4; ++v) qn[q][v] = with_qn ? ph.qn(v, node[q]) : 0.0;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) {
+    const long long n = node[q];
+    if (n < 0) continue;
+    const int m = threadIdx.x + q * 2 * NH;
+    const int el = m / NN, nd = m % NN, j = nd / NP, i = nd % NP;
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const double qs = sm.q[v][el][nd];
+      const long long r = sm.k[0][v][el][nd], c = sm.k[1][v][el][nd];
+      const int er = sm.ke[0][v][el][j], ec = sm.ke[1][v][el][i];
+      ph.put(v, n, with_qn ? node_blend(r, er, c, ec, qs, w1, qn[q][v], w0)
+                           : node_total<60>(r, er, c, ec, raw ? 0.0 : qs, 1));  // without q^n: c1 = 1
+    }
   }
 }
 
@@ -877,19 +863,11 @@ struct EulerStage {
     f.aux = p.P;
     return f;
   }
-  __device__ __forceinline__ double partner_speed(int dir, long long n, const FluxNode& f) const {
+  __device__ __forceinline__ double speed(int dir, long long n, double m, double P, bool own) const {
     const double ir = a.invr[n];
-    return wavespeed(g, f.q[dir] * ir, f.aux, ir);
-  }
-  __device__ __forceinline__ double speed_x(long long n, const FluxNode& f) const {
-    const double ws = partner_speed(0, n, f);
-    if (a.ws_x) a.ws_x[n] = ws;
-    return ws;
-  }
-  __device__ __forceinline__ double speed_y(long long n, double my, double P) const {
-    const double ir = a.invr[n];
-    const double ws = wavespeed(g, my * ir, P, ir);
-    if (a.ws_y) a.ws_y[n] = ws;
+    const double ws = wavespeed(g, m * ir, P, ir);
+    double* out = dir == 0 ? a.ws_x : a.ws_y;
+    if (own && out) out[n] = ws;
     return ws;
   }
   __device__ __forceinline__ double qn(int v, long long n) const { return a.qn[v][n]; }
@@ -902,7 +880,7 @@ struct EulerStage {
 };
 
 template <int NP>
-__global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_hyp_rk(HypArgs2D a) {
+__global__ void __launch_bounds__(2 * Tiling2D<NP>::NH) k2_hyp_rk(HypArgs2D a) {
   __shared__ StageSmem<NP, true> sm;
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];

@@ -24,7 +24,7 @@ template <int NP> void launch_k2_apply(int epi, const ApplyArgs2D& a, int nb, cu
   else k2_apply<NP, EPI_RESID><<<nb, NT2, 0, s>>>(a);
 }
 template <int NP> void launch_k2_hyp_rk(const HypArgs2D& a, int nb, cudaStream_t s) {
-  k2_hyp_rk<NP><<<nb, Tiling2D<NP>::NT, 0, s>>>(a);
+  k2_hyp_rk<NP><<<nb, 2 * Tiling2D<NP>::NH, 0, s>>>(a);
 }
 template <int NP> void launch_k2_hyp_rev(const HypRevArgs2D& a, int nb, cudaStream_t s) {
   k2_hyp_rev<NP><<<nb, 2 * Tiling2D<NP>::NH, 0, s>>>(a);
@@ -44,7 +44,7 @@ template <int NP> void launch_k2_sens_rhs(const SensRhsArgs2D& a, int nb, cudaSt
   k2_sens_rhs<NP><<<nb, Tiling2D<NP>::NT, 0, s>>>(a);
 }
 template <int NP> void launch_k2_sens_hyp_rk(const SensHypArgs2D& a, int nb, cudaStream_t s) {
-  k2_sens_hyp_rk<NP><<<nb, Tiling2D<NP>::NT, 0, s>>>(a);
+  k2_sens_hyp_rk<NP><<<nb, 2 * Tiling2D<NP>::NH, 0, s>>>(a);
 }
 
 template <int NP> void launch_k2_pde_prep(const PdePrepArgs2D& a, int nb, cudaStream_t s) {

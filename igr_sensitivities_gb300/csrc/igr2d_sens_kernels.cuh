@@ -127,8 +127,8 @@ __device__ __forceinline__ SensNode sens_phys(double g, double sg, double mx, do
   const double Pt = Phi + vs;
   const double etp = et + Pt, eps = E + P + S;
   const double f1 = fma(zx, uy, mx * suy);
-  o.fx[0] = fma(zx, ux, mx * sux) + Pt; o.fx[1] = f1; o.fx[2] = zx; o.fx[3] = fma(etp, ux, eps * sux);
-  o.fy[0] = f1; o.fy[1] = fma(zy, uy, my * suy) + Pt; o.fy[2] = zy; o.fy[3] = fma(etp, uy, eps * suy);
+  o.fx[0] = fma(zx, ux, fma(mx, sux, Pt)); o.fx[1] = f1; o.fx[2] = zx; o.fx[3] = fma(etp, ux, eps * sux);
+  o.fy[0] = f1; o.fy[1] = fma(zy, uy, fma(my, suy, Pt)); o.fy[2] = zy; o.fy[3] = fma(etp, uy, eps * suy);
   return o;
 }
 
@@ -157,11 +157,9 @@ struct TangentStage {
     f.fx0 = p.fx[0]; f.f1 = p.fx[1]; f.fx3 = p.fx[3]; f.fy1 = p.fy[1]; f.fy3 = p.fy[3];
     return f;
   }
-  __device__ __forceinline__ double partner_speed(int dir, long long n, const FluxNode&) const {
+  __device__ __forceinline__ double speed(int dir, long long n, double, double, bool) const {
     return dir == 0 ? a.ws_x[n] : a.ws_y[n];
   }
-  __device__ __forceinline__ double speed_x(long long n, const FluxNode&) const { return a.ws_x[n]; }
-  __device__ __forceinline__ double speed_y(long long n, double, double) const { return a.ws_y[n]; }
   __device__ __forceinline__ double qn(int v, long long n) const { return a.sn[v][n]; }
   __device__ __forceinline__ void put(int v, long long n, double x) const {
     if (a.k_out[v]) a.k_out[v][n] = x;
@@ -171,7 +169,7 @@ struct TangentStage {
 };
 
 template <int NP>
-__global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_sens_hyp_rk(SensHypArgs2D a) {
+__global__ void __launch_bounds__(2 * Tiling2D<NP>::NH) k2_sens_hyp_rk(SensHypArgs2D a) {
   __shared__ StageSmem<NP, false> sm;
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];

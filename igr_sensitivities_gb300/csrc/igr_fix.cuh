@@ -616,6 +616,25 @@ __device__ __forceinline__ double node_total(long long r, int er, long long c, i
   return sg > 0 ? acc + (x + y) : acc - (x + y);
 }
 
+// c v in units of 2^62 / 2^(e - 1022), e = exponent of v + that of c - 1022 (v normal, c.e of FixScale)
+__device__ __forceinline__ long long weighted(double v, const FixScale& c) {
+  const fix::Limb x = fix::mantissa(v);
+  const long long M = fix::mad(x.h, c.m.l, fix::mad(x.l, c.m.h, fix::HALF));
+  return fix::mad((int)(M >> 32), 2, fix::mad(x.h, c.m.h, 0));
+}
+// a qa + b qb + row + column at one node (units of 2^60; see node_total), rounded once; 0 < a, b <= 1
+__device__ __forceinline__ double node_blend(long long r, int er, long long c, int ec, double qa, const FixScale& a, double qb,
+                                             const FixScale& b) {
+  const int xa = fix::abs_hi(qa) >> 20, xb = fix::abs_hi(qb) >> 20;
+  const int e = max(max(er, ec), max(xa, xb));
+  if (er >= 0 && ec >= 0 && e >= 128 && e < fix::E_MAX) {
+    long long v = fix::sar(r, e - er) + fix::sar(c, e - ec);
+    v += fix::sar(weighted(qa, a), min(e - (xa + a.e - 1022) + 2, 63)) + fix::sar(weighted(qb, b), min(e - (xb + b.e - 1022) + 2, 63));
+    return fix::to_double(v, e);
+  }
+  return node_total<60>(r, er, c, ec, fma(b.d, qb, a.d * qa), 1);
+}
+
 // ---------------------------------------------------------------------------
 // A scaled line derivative (or its transpose, T) kept as integers between the phases, and the sum that ends it:
 //   row:    r = c (D v) + (a0 at node 0, aL at node NP-1)

@@ -22,6 +22,7 @@ static double __longlong_as_double(long long b) { double v; std::memcpy(&v, &b, 
 static unsigned __funnelshift_l(unsigned lo, unsigned hi, unsigned s) { return (unsigned)((((uint64_t)hi << 32) | lo) << s >> 32); }
 static int __clz(unsigned m) { return m ? __builtin_clz(m) : 32; }
 static int max(int a, int b) { return a > b ? a : b; }
+static int min(int a, int b) { return a < b ? a : b; }
 #include "../igr_sensitivities_gb300/csrc/igr_fix.cuh"
 using namespace igrgpu;
 
@@ -292,6 +293,35 @@ template <int NP> static int run() {
     ok &= ratio <= 1;
     bad += !ok;
     std::printf("NP%d products kind%d %s %.3f\n", NP, kind, ok ? "ok" : "BAD", ratio);
+  }
+  // a qa + b qb + row + column at a node, against long double and against the FP64 form of the weights
+  {
+    double sum_i = 0, sum_f = 0;
+    bool ok = true;
+    for (int it = 0; it < 20000; ++it) {
+      const double ws[3][2] = {{0.25, 0.75}, {2.0 / 3, 1.0 / 3}, {1.0, 0.5}};
+      const FixScale a = fix_scale(ws[it % 3][0]), b = fix_scale(ws[it % 3][1]);
+      double qa = 1 + 0.3 * (2 * uni() - 1), qb = qa * (1 + 1e-2 * uni());
+      if (it % 5 == 1) qa = 0.0;
+      if (it % 5 == 2) qb = -qb;
+      if (it % 5 == 3) { qa *= 1e-9; qb *= 1e-9; }
+      double x[NP], y[NP], k[NP], zero[NP] = {};
+      for (int i = 0; i < NP; ++i) { x[i] = 1e-3 * (2 * uni() - 1); y[i] = 1e-3 * (2 * uni() - 1); k[i] = 1; }
+      FixSums<NP> r, c;
+      const FixScale one = fix_scale(1.0);
+      row_scaled<NP, false>(B, one, x, r);
+      row_scaled<NP, false>(B, one, y, c);
+      long double R = 0, C = 0;
+      for (int j = 0; j < NP; ++j) { R += (long double)B.D[0][j] * x[j]; C += (long double)B.D[0][j] * y[j]; }
+      const double got = node_blend(r.G[0], r.e, c.G[0], c.e, qa, a, qb, b);
+      const long double want = (long double)a.d * qa + (long double)b.d * qb + R + C;
+      const double f64 = std::fma(b.d, qb, a.d * qa) + ((double)R + (double)C);
+      sum_i += (double)((got - want) * (got - want));
+      sum_f += (double)((f64 - want) * (f64 - want));
+    }
+    if (NP > 2) ok = sum_i <= sum_f;
+    bad += !ok;
+    std::printf("NP%d blend 0 %s %.3f\n", NP, ok ? "ok" : "BAD", std::sqrt(sum_i / sum_f));
   }
   // infinities and NaN come out as not finite wherever the FP64 chain has them
   const double inf = std::numeric_limits<double>::infinity();
