@@ -335,218 +335,87 @@ struct ApplyArgs2D {
 // Partner data across one face: its value and its flux k (D x) at the face node.
 struct Partner1 { double x, t; };
 
-// Shared memory of one tile's PCG operator application: the tile's x, the
-// x-phase sums (fixed point, with each row's exponent) and the end-node fluxes
-// of every line.
+// Shared memory of one tile's operator application: x, the sums of the rows and
+// of the columns (fixed point, with each line's exponent) and the end-node
+// fluxes of every line.
 template <int NP>
 struct ApplySmem {
   alignas(16) double x[Tiling2D<NP>::TE][Tiling2D<NP>::SN];
-  alignas(16) long long yx[Tiling2D<NP>::TE][Tiling2D<NP>::SN];
-  int ex[Tiling2D<NP>::TE][NP];
-  double txf[Tiling2D<NP>::TE][NP][2], tyf[Tiling2D<NP>::TE][NP][2];
+  alignas(16) long long y[2][Tiling2D<NP>::TE][Tiling2D<NP>::SN];
+  int e[2][Tiling2D<NP>::TE][NP];
+  double t[2][Tiling2D<NP>::TE][NP][2];
 };
 
-// y = A x on tile tl (of instance I) with a PCG epilogue (EPI_PCG0 / EPI_PCG), by
-// the CTA's Tiling2D<NP>::NT threads (all of which call it; it synchronises the
-// CTA twice). Returns this thread's inner-product partial. k2_apply_pcg runs it
-// on tile blockIdx.x; the persistent PCG kernel on every tile of its CTA, whose
-// eight resident CTAs per SM leave no room for the halves of k2_apply.
+// y = A x on tile tl (of instance I) with the EPI epilogue, by the CTA's
+// 2 NH threads (all of which call it; it synchronises the CTA). Returns this
+// thread's PCG inner-product partial (EPI_PCG0 / EPI_PCG; 0 otherwise).
+// k2_apply runs it on tile blockIdx.x; the persistent PCG kernel on the CTA's tile.
+// Rows and columns run side by side, one half of the CTA each: the two directions are independent up to their sums, so a
+// line's chain of loads, integer sums and FP64 faces is all that a warp runs before the CTA meets, and the epilogue is
+// pointwise over all threads with coalesced accesses. PCG's direction update p_k = M^-1 r_k + beta p_{k-1} is pointwise
+// too and is formed once per node, in front of the lines.
+// What bounds it: FP64 issue (68% busy), the integer ALU (59%) and L2 latency, with 32 warps per SM. 8 x 128^2 P3,
+// Chebyshev: 127 us with FP64 contractions; 79 us with integer ones and one thread per pair of lines (18 warps); 69 us in
+// halves; 65 us with the pointwise loads ahead of its stores. 64^2: 12.3, 11.3, 10.2, 9.9.
 template <int NP, int EPI>
 __device__ __forceinline__ double apply_tile(const ApplyArgs2D& a, const Tile2D tl, const Inst2D& I, ApplySmem<NP>& sm) {
   using TL = Tiling2D<NP>;
-  constexpr int L = TL::L, TX = TL::TX, TY = TL::TY;
-  auto& s_x = sm.x;
-  auto& s_yx = sm.yx;
-  auto& s_ex = sm.ex;
-  auto& s_txf = sm.txf;
-  auto& s_tyf = sm.tyf;
-  const ElemView vr = elem_view<NP>(tl, I, 0), vc = elem_view<NP>(tl, I, 1);
+  constexpr int TE = TL::TE, NN = TL::NN, L = TL::L, TX = TL::TX, TY = TL::TY, NH = TL::NH;
+  constexpr int NQ = (TE * NN + 2 * NH - 1) / (2 * NH);  // nodes per thread
+  constexpr bool PCG = EPI == EPI_PCG0 || EPI == EPI_PCG;
+  // b - cm x enters the last sum and the rest with a minus sign where the epilogue wants the residual
+  constexpr bool RES = EPI == EPI_CHEB || EPI == EPI_JACOBI || EPI == EPI_PCG0;
   const BasisDev& B = a.B;
   const double hw = B.hw;
-  // PCG direction update fused into the loads (p_k is pointwise in r_k, p_{k-1})
   const bool form_p = EPI == EPI_PCG && a.pcg_p != nullptr;
   const double beta = form_p ? a.pcg_beta[tl.inst] : 0.0;
   auto ldx = [&](long long n) -> double {
     if (form_p) return fma(beta, a.pcg_p[n], a.pcg_r[n] * a.cinvM[n]);
     return a.x[n];
   };
-
-  // ---- xi-phase part 1: row fluxes
-  double xr[NP], kx0, kxL;
-  FixFlux<NP> fr;
-  if (vr.valid) {
-    const int t = vr.t, e = vr.e;
-    double k[NP];
-#pragma unroll
-    for (int i = 0; i < NP; ++i) { xr[i] = ldx(vr.base + t * NP + i); s_x[e][t * NP + i] = xr[i]; }
-#pragma unroll
-    for (int i = 0; i < NP; ++i) k[i] = a.ckx[vr.base + t * NP + i];
-    if (form_p) {
-#pragma unroll
-      for (int i = 0; i < NP; ++i) a.p_out[vr.base + t * NP + i] = xr[i];
-    }
-    flux_line<NP>(B, xr, k, fr);
-    s_txf[e][t][0] = fr.t0; s_txf[e][t][1] = fr.tL;
-    kx0 = k[0]; kxL = k[L];
-    if (a.tape_x) {
-#pragma unroll
-      for (int i = 0; i < NP; ++i) a.tape_x[vr.base + t * NP + i] = xr[i];
-    }
-  }
-  __syncthreads();
-  double xc[NP], ky0, kyL;
-  FixFlux<NP> fc;
-  if (vc.valid) {
-    const int t = vc.t, e = vc.e;
-    double k[NP];
-#pragma unroll
-    for (int l = 0; l < NP; ++l) { xc[l] = s_x[e][l * NP + t]; k[l] = a.cky[vc.base + l * NP + t]; }
-    flux_line<NP>(B, xc, k, fc);
-    s_tyf[e][t][0] = fc.t0; s_tyf[e][t][1] = fc.tL;
-    ky0 = k[0]; kyL = k[L];
-  }
-  if (vr.valid) {
-    // ---- xi-phase part 2: x faces of the row and the x-stiffness transpose
-    const int t = vr.t, e = vr.e;
-    auto fetch = [&](int s) {
-      Partner1 P;
-      int it;
-      const long long pb = neighbour<NP>(tl, I, vr.ex, vr.ey, s == 0 ? -1 : 1, 0, &it);
-      const int pi = s == 0 ? L : 0;  // partner face node index along x
-      if (it >= 0) {
-        P.x = s_x[it][t * NP + pi];
-        P.t = s_txf[it][t][s == 0 ? 1 : 0];
-      } else {
-        double pr[NP];
-#pragma unroll
-        for (int k = 0; k < NP; ++k) pr[k] = ldx(pb + t * NP + k);
-        P.x = s == 0 ? pr[L] : pr[0];
-        P.t = flux_end<NP>(B, s == 0, pr, a.ckx[pb + t * NP + pi]);
-      }
-      return P;
-    };
-    const int sf = first_side(vr.ext, TX);
-    const Partner1 pA = fetch(sf), pB = fetch(1 - sf);
-    const Partner1 pl = sf == 0 ? pA : pB, prt = sf == 0 ? pB : pA;
-    // left face: own node (0,t) is the R side; right face: own node (L,t) is the L side
-    const double jl = pl.x - xr[0];
-    const double Fl = fma(a.cpx[vr.base + t * NP], jl, hw * (pl.t + fr.t0));
-    const double jr = xr[L] - prt.x;
-    const double Fr = fma(a.cpx[vr.base + t * NP + L], jr, hw * (fr.tL + prt.t));
-    FixSums<NP> sums;
-    row_sums<NP>(B, fr, hw * kx0 * jl, hw * kxL * jr, -Fl, Fr, sums);
-#pragma unroll
-    for (int k = 0; k < NP; ++k) s_yx[e][t * NP + k] = sums.G[k];
-    s_ex[e][t] = sums.e;
-  }
-  __syncthreads();
-  double part = 0.0;  // PCG inner-product partial of this thread
-
-  // ---- eta-phase: y faces of the column, y-stiffness transpose, mass, epilogue
-  if (vc.valid) {
-    const int t = vc.t, e = vc.e;
-    auto fetchy = [&](int s) {
-      Partner1 P;
-      int it;
-      const long long pb = neighbour<NP>(tl, I, vc.ex, vc.ey, 0, s == 0 ? -1 : 1, &it);
-      const int pl = s == 0 ? L : 0;
-      if (it >= 0) {
-        P.x = s_x[it][pl * NP + t];
-        P.t = s_tyf[it][t][s == 0 ? 1 : 0];
-      } else {
-        double pc[NP];
-#pragma unroll
-        for (int k = 0; k < NP; ++k) pc[k] = ldx(pb + k * NP + t);
-        P.x = s == 0 ? pc[L] : pc[0];
-        P.t = flux_end<NP>(B, s == 0, pc, a.cky[pb + pl * NP + t]);
-      }
-      return P;
-    };
-    const int sf = first_side(vc.eyt, TY);
-    const Partner1 qA = fetchy(sf), qB = fetchy(1 - sf);
-    const Partner1 qb = sf == 0 ? qA : qB, qt = sf == 0 ? qB : qA;
-    const double jb = qb.x - xc[0];
-    const double Fb = fma(a.cpy[vc.base + t], jb, hw * (qb.t + fc.t0));
-    const double jt = xc[L] - qt.x;
-    const double Ft = fma(a.cpy[vc.base + L * NP + t], jt, hw * (fc.tL + qt.t));
-    // EPI_PCG0 forms b - A x at once: b - cm x enters the last sum, the rest with a minus sign
-    constexpr bool RES = EPI == EPI_PCG0;
-    double acc[NP], yy[NP];
-    long long R[NP];
-    int er[NP];
-#pragma unroll
-    for (int l = 0; l < NP; ++l) {
-      const long long n = vc.base + l * NP + t;
-      acc[l] = RES ? fma(-a.cm[n], xc[l], a.b[n]) : a.cm[n] * xc[l];
-      R[l] = s_yx[e][l * NP + t];
-      er[l] = s_ex[e][l];
-    }
-    column_sums<NP>(B, fc, hw * ky0 * jb, hw * kyL * jt, -Fb, Ft, R, er, acc, RES ? -1 : 1, yy);
-#pragma unroll
-    for (int l = 0; l < NP; ++l) {
-      const long long n = vc.base + l * NP + t;
-      if (EPI == EPI_PCG) {
-        a.ap_out[n] = yy[l];
-        part = fma(xc[l], yy[l], part);
-      } else {
-        const double r0 = yy[l], z0 = r0 * a.cinvM[n];
-        a.r_out[n] = r0;
-        a.p_out[n] = z0;
-        part = fma(r0, z0, part);
-      }
-    }
-  }
-  return part;
-}
-
-template <int NP, int EPI>
-__global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_apply_pcg(ApplyArgs2D a) {
-  using TL = Tiling2D<NP>;
-  constexpr int P2 = pow2_at_least(TL::NT);
-  __shared__ ApplySmem<NP> sm;
-  __shared__ double s_red[P2];
-  const Tile2D tl = a.tiles[blockIdx.x];
-  const Inst2D I = a.inst[tl.inst];
-  const double part = apply_tile<NP, EPI>(a, tl, I, sm);
-  const double tot = block_sum<P2>(part, s_red);
-  inst_sum_last_block(a.isum, tl.inst, I.ntiles, tot, a.partials, blockIdx.x, I.tile0, I.ntiles);
-}
-
-// y = A x with the Jacobi / Chebyshev / plain epilogue. Rows and columns run side by side, one half of the CTA each: the
-// two directions are independent up to their sums, so a line's chain of loads, integer sums and FP64 faces is all that a
-// warp runs before the CTA meets, and the epilogue is pointwise over all threads with coalesced accesses.
-// What bounds it: FP64 issue (68% busy), the integer ALU (59%) and L2 latency, with 32 warps per SM. 8 x 128^2 P3,
-// Chebyshev: 127 us with FP64 contractions; 79 us with integer ones and one thread per pair of lines (18 warps); 69 us in
-// halves; 65 us with the pointwise loads ahead of its stores. 64^2: 12.3, 11.3, 10.2, 9.9.
-template <int NP, int EPI>
-__global__ void __launch_bounds__(2 * Tiling2D<NP>::NH) k2_apply(ApplyArgs2D a) {
-  using TL = Tiling2D<NP>;
-  constexpr int TE = TL::TE, NN = TL::NN, SN = TL::SN, L = TL::L, TX = TL::TX, TY = TL::TY, NH = TL::NH;
-  __shared__ __align__(16) double s_x[TE][SN];
-  __shared__ __align__(16) long long s_y[2][TE][SN];  // sums of the rows and of the columns (fixed point)
-  __shared__ int s_e[2][TE][NP];                      // their exponents
-  __shared__ double s_t[2][TE][NP][2];                // end-node fluxes of every line
-  const Tile2D tl = a.tiles[blockIdx.x];
-  const Inst2D I = a.inst[tl.inst];
-  const BasisDev& B = a.B;
-  const double hw = B.hw;
+  // the thread's nodes: node(q) or -1; m = el NN + nd
+  auto node = [&](int m) -> long long {
+    const int el = m / NN, nd = m % NN, ex = tl.ex0 + el % TX, ey = tl.ey0 + el / TX;
+    return m < TE * NN && ex < I.nex && ey < I.ney ? I.off + (long long)NN * (ex + (long long)I.nex * ey) + nd : -1;
+  };
   const int dir = threadIdx.x >= NH;  // 0: rows and x faces, 1: columns and y faces
   const ElemView w = elem_view<NP>(tl, I, dir, threadIdx.x - dir * NH);
   const int e = w.e, t = w.t;
   const int st = dir == 0 ? 1 : NP, at = dir == 0 ? t * NP : t;  // node k of the line: at + k st
   const double* ck = dir == 0 ? a.ckx : a.cky;
+  if (PCG) {
+    double x[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+      const long long n = node(threadIdx.x + q * 2 * NH);
+      if (n >= 0) x[q] = ldx(n);
+    }
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+      const int m = threadIdx.x + q * 2 * NH;
+      const long long n = node(m);
+      if (n < 0) continue;
+      sm.x[m / NN][m % NN] = x[q];
+      if (form_p) a.p_out[n] = x[q];
+      if (a.tape_x) a.tape_x[n] = x[q];
+    }
+    __syncthreads();
+  }
   double x0 = 0.0, xL = 0.0, k0 = 0.0, kL = 0.0;
   FixFlux<NP> f;
   if (w.valid) {
     double x[NP], k[NP];
 #pragma unroll
-    for (int i = 0; i < NP; ++i) { x[i] = a.x[w.base + at + i * st]; k[i] = ck[w.base + at + i * st]; }
-    if (dir == 0) {
+    for (int i = 0; i < NP; ++i) {
+      x[i] = PCG ? sm.x[e][at + i * st] : a.x[w.base + at + i * st];
+      k[i] = ck[w.base + at + i * st];
+    }
+    if (!PCG && dir == 0) {
 #pragma unroll
-      for (int i = 0; i < NP; ++i) s_x[e][at + i] = x[i];
+      for (int i = 0; i < NP; ++i) sm.x[e][at + i] = x[i];
     }
     flux_line<NP>(B, x, k, f);
-    s_t[dir][e][t][0] = f.t0; s_t[dir][e][t][1] = f.tL;
+    sm.t[dir][e][t][0] = f.t0; sm.t[dir][e][t][1] = f.tL;
     x0 = x[0]; xL = x[L]; k0 = k[0]; kL = k[L];
   }
   __syncthreads();
@@ -559,12 +428,12 @@ __global__ void __launch_bounds__(2 * Tiling2D<NP>::NH) k2_apply(ApplyArgs2D a) 
       const long long pb = neighbour<NP>(tl, I, w.ex, w.ey, dir == 0 ? d : 0, dir == 0 ? 0 : d, &it);
       const int pn = at + (s == 0 ? L : 0) * st;  // partner face node
       if (it >= 0) {
-        P.x = s_x[it][pn];
-        P.t = s_t[dir][it][t][1 - s];
+        P.x = sm.x[it][pn];
+        P.t = sm.t[dir][it][t][1 - s];
       } else {
         double p[NP];
 #pragma unroll
-        for (int k = 0; k < NP; ++k) p[k] = a.x[pb + at + k * st];
+        for (int k = 0; k < NP; ++k) p[k] = ldx(pb + at + k * st);
         P.x = s == 0 ? p[L] : p[0];
         P.t = flux_end<NP>(B, s == 0, p, ck[pb + pn]);
       }
@@ -580,51 +449,73 @@ __global__ void __launch_bounds__(2 * Tiling2D<NP>::NH) k2_apply(ApplyArgs2D a) 
     FixSums<NP> sums;
     row_sums<NP>(B, f, hw * k0 * jl, hw * kL * jr, -Fl, Fr, sums);
 #pragma unroll
-    for (int k = 0; k < NP; ++k) s_y[dir][e][at + k * st] = sums.G[k];
-    s_e[dir][e][t] = sums.e;
+    for (int k = 0; k < NP; ++k) sm.y[dir][e][at + k * st] = sums.G[k];
+    sm.e[dir][e][t] = sums.e;
   }
   // ---- pointwise: mass term, sums, epilogue. Everything is loaded before anything is stored (the compiler has to assume
   // that a store changes what a later load reads), and before the barrier.
-  constexpr int NQ = (TE * NN + 2 * NH - 1) / (2 * NH);
-  long long node[NQ];
   double cm[NQ], b[NQ], im[NQ], din[NQ];
 #pragma unroll
   for (int q = 0; q < NQ; ++q) {
-    const int m = threadIdx.x + q * 2 * NH;
-    const int el = m / NN, nd = m % NN, ex = tl.ex0 + el % TX, ey = tl.ey0 + el / TX;
-    const bool live = m < TE * NN && ex < I.nex && ey < I.ney;
-    const long long n = I.off + (long long)NN * (ex + (long long)I.nex * ey) + nd;
-    node[q] = live ? n : -1;
-    if (!live) continue;
+    const long long n = node(threadIdx.x + q * 2 * NH);
+    if (n < 0) continue;
     cm[q] = a.cm[n];
-    if (EPI != EPI_RESID) {
+    if (RES) {
       b[q] = a.b[n];
       im[q] = a.cinvM[n];
       din[q] = EPI == EPI_CHEB && a.d_in ? a.d_in[n] : 0.0;
     }
   }
   __syncthreads();
+  double part = 0.0;  // PCG inner-product partial of this thread
 #pragma unroll
   for (int q = 0; q < NQ; ++q) {
-    const long long n = node[q];
-    if (n < 0) continue;
     const int m = threadIdx.x + q * 2 * NH;
+    const long long n = node(m);
+    if (n < 0) continue;
     const int el = m / NN, nd = m % NN;
-    const double x = s_x[el][nd];
-    const double acc = EPI == EPI_RESID ? cm[q] * x : fma(-cm[q], x, b[q]);
-    const double y = node_total<59>(s_y[0][el][nd], s_e[0][el][nd / NP], s_y[1][el][nd], s_e[1][el][nd % NP], acc,
-                                    EPI == EPI_RESID ? 1 : -1);  // A x, or b - A x
-    if (EPI == EPI_RESID) { a.y_out[n] = y; continue; }
-    if (a.tape_x) a.tape_x[n] = x;
-    if (a.tape_r) a.tape_r[n] = y;
+    const double x = sm.x[el][nd];
+    const double acc = RES ? fma(-cm[q], x, b[q]) : cm[q] * x;
+    const double y = node_total<59>(sm.y[0][el][nd], sm.e[0][el][nd / NP], sm.y[1][el][nd], sm.e[1][el][nd % NP], acc,
+                                    RES ? -1 : 1);  // A x, or b - A x (RES)
+    if (EPI == EPI_RESID) a.y_out[n] = y;
+    if (EPI == EPI_PCG) {
+      a.ap_out[n] = y;
+      part = fma(x, y, part);
+    }
+    if (EPI == EPI_PCG0) {
+      const double z0 = y * im[q];
+      a.r_out[n] = y;
+      a.p_out[n] = z0;
+      part = fma(y, z0, part);
+    }
+    if (EPI == EPI_CHEB || EPI == EPI_JACOBI) {
+      if (a.tape_x) a.tape_x[n] = x;
+      if (a.tape_r) a.tape_r[n] = y;
+    }
     if (EPI == EPI_CHEB) {
       const double z = y * im[q];
       const double d = a.d_in ? fma(a.ca, din[q], a.cc * z) : a.cc * z;
       a.d_out[n] = d;
       a.x_out[n] = x + d;
-    } else {  // EPI_JACOBI: x + omega (b - A x) / M   (elliptic.jl:358)
-      a.x_out[n] = fma(a.omega * y, im[q], x);
     }
+    if (EPI == EPI_JACOBI) a.x_out[n] = fma(a.omega * y, im[q], x);  // x + omega (b - A x) / M   (elliptic.jl:358)
+  }
+  return part;
+}
+
+template <int NP, int EPI>
+__global__ void __launch_bounds__(2 * Tiling2D<NP>::NH) k2_apply(ApplyArgs2D a) {
+  constexpr bool PCG = EPI == EPI_PCG0 || EPI == EPI_PCG;
+  constexpr int P2 = pow2_at_least(2 * Tiling2D<NP>::NH);
+  __shared__ ApplySmem<NP> sm;
+  __shared__ double s_red[PCG ? P2 : 1];
+  const Tile2D tl = a.tiles[blockIdx.x];
+  const Inst2D I = a.inst[tl.inst];
+  const double part = apply_tile<NP, EPI>(a, tl, I, sm);
+  if (PCG) {
+    const double tot = block_sum<P2>(part, s_red);
+    inst_sum_last_block(a.isum, tl.inst, I.ntiles, tot, a.partials, blockIdx.x, I.tile0, I.ntiles);
   }
 }
 

@@ -16,11 +16,11 @@ template <int NP> void launch_k2_setup(const SetupArgs2D& a, int nb, cudaStream_
   k2_setup<NP><<<nb, Tiling2D<NP>::NT, 0, s>>>(a);
 }
 template <int NP> void launch_k2_apply(int epi, const ApplyArgs2D& a, int nb, cudaStream_t s) {
-  constexpr int NT = Tiling2D<NP>::NT, NT2 = 2 * Tiling2D<NP>::NH;
+  constexpr int NT2 = 2 * Tiling2D<NP>::NH;
   if (epi == EPI_CHEB) k2_apply<NP, EPI_CHEB><<<nb, NT2, 0, s>>>(a);
   else if (epi == EPI_JACOBI) k2_apply<NP, EPI_JACOBI><<<nb, NT2, 0, s>>>(a);
-  else if (epi == EPI_PCG0) k2_apply_pcg<NP, EPI_PCG0><<<nb, NT, 0, s>>>(a);
-  else if (epi == EPI_PCG) k2_apply_pcg<NP, EPI_PCG><<<nb, NT, 0, s>>>(a);
+  else if (epi == EPI_PCG0) k2_apply<NP, EPI_PCG0><<<nb, NT2, 0, s>>>(a);
+  else if (epi == EPI_PCG) k2_apply<NP, EPI_PCG><<<nb, NT2, 0, s>>>(a);
   else k2_apply<NP, EPI_RESID><<<nb, NT2, 0, s>>>(a);
 }
 template <int NP> void launch_k2_hyp_rk(const HypArgs2D& a, int nb, cudaStream_t s) {
@@ -59,13 +59,13 @@ template <int NP> void launch_k2_pde_rk(const PdeRkArgs2D& a, int nb, cudaStream
 
 template <int NP> int pcg_persist_blocks_per_sm() {
   int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k2_pcg_persist<NP>, Tiling2D<NP>::NT, 0) != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k2_pcg_persist<NP>, persist_threads<NP>(), 0) != cudaSuccess) return 0;
   return n;
 }
 template <int NP> cudaError_t launch_k2_pcg_persist(const PcgPersistArgs& a, int grid, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid, 1, 1);
-  cfg.blockDim = dim3(Tiling2D<NP>::NT, 1, 1);
+  cfg.blockDim = dim3(persist_threads<NP>(), 1, 1);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = s;
   cudaLaunchAttribute at[1];

@@ -50,14 +50,19 @@ constexpr int PCG_COUNTED_TILES = 256;               // instances up to this man
 constexpr int PCG_BCAST = 32;                        // copies of a published scalar
 constexpr int PCG_CNT_STRIDE = 32;                   // words between arrival counters (one 128-byte line each)
 
+// Threads per CTA: the operator's.
+template <int NP>
+__host__ __device__ constexpr int persist_threads() { return 2 * Tiling2D<NP>::NH; }
+
 // Partial slots each writer thread polls, and so the tiles an instance may
 // have (slots per thread x threads per CTA, about 1280).
 template <int NP>
 __host__ __device__ constexpr int persist_slots_per_thread() {
-  return (1280 + Tiling2D<NP>::NT - 1) / Tiling2D<NP>::NT < 32 ? (1280 + Tiling2D<NP>::NT - 1) / Tiling2D<NP>::NT : 32;
+  const int n = (1280 + persist_threads<NP>() - 1) / persist_threads<NP>();
+  return n < 32 ? n : 32;
 }
 template <int NP>
-__host__ __device__ constexpr int persist_max_inst_tiles() { return persist_slots_per_thread<NP>() * Tiling2D<NP>::NT; }
+__host__ __device__ constexpr int persist_max_inst_tiles() { return persist_slots_per_thread<NP>() * persist_threads<NP>(); }
 
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
@@ -133,7 +138,7 @@ template <int NP>
 __device__ __forceinline__ double gathered_sum(const double* slots, int count, double* stage, int* status,
                                                double* s_sum, int* s_ok) {
   constexpr int SPT = persist_slots_per_thread<NP>();
-  constexpr int NT = Tiling2D<NP>::NT;
+  constexpr int NT = persist_threads<NP>();
   constexpr int CH = 16;  // loads in flight per thread (registers)
   const int tid = threadIdx.x;
   __syncthreads();
@@ -200,13 +205,13 @@ __device__ __forceinline__ double wait_published(const double* slot, int* status
 }
 
 template <int NP>
-__global__ void __launch_bounds__(Tiling2D<NP>::NT, 8) k2_pcg_persist(PcgPersistArgs a) {
+__global__ void __launch_bounds__(persist_threads<NP>(), 8) k2_pcg_persist(PcgPersistArgs a) {
   using TL = Tiling2D<NP>;
-  constexpr int P2 = pow2_at_least(TL::NT);
+  constexpr int P2 = pow2_at_least(persist_threads<NP>());
   constexpr int UV = PCG_THREADS;        // slots of a tile's update tree
   constexpr int cnt = TL::TE * NP * NP;  // nodes of a tile
   static_assert(cnt <= UV, "one tree slot per node");
-  static_assert(TL::NT >= PCG_BCAST, "one thread per published copy");
+  static_assert(persist_threads<NP>() >= PCG_BCAST, "one thread per published copy");
   __shared__ ApplySmem<NP> sm;
   __shared__ double s_red[UV > P2 ? UV : P2];
   __shared__ double s_val, s_beta[PCG_PERSIST_MAX_INST], s_stage[persist_max_inst_tiles<NP>()];
