@@ -170,6 +170,7 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_setup(SetupArgs2D a) {
   __shared__ double s_p[2][NP], s_s[2][2][NP];
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];
+  chained_start();
   const ElemView vr = elem_view<NP>(tl, I, 0), vc = elem_view<NP>(tl, I, 1);
   const BasisDev& B = a.B;
   const double invJx = I.ijx, invJy = I.ijy;
@@ -512,6 +513,7 @@ __global__ void __launch_bounds__(2 * Tiling2D<NP>::NH) k2_apply(ApplyArgs2D a) 
   __shared__ double s_red[PCG ? P2 : 1];
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];
+  chained_start();
   const double part = apply_tile<NP, EPI>(a, tl, I, sm);
   if (PCG) {
     const double tot = block_sum<P2>(part, s_red);
@@ -775,6 +777,7 @@ __global__ void __launch_bounds__(2 * Tiling2D<NP>::NH) k2_hyp_rk(HypArgs2D a) {
   __shared__ StageSmem<NP, true> sm;
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];
+  chained_start();
   dg_stage<NP, true>(EulerStage{a, I.gamma}, a.B, tl, I, a.c0, a.c1, a.c2, a.k_out[0] != nullptr, sm);
 }
 

@@ -13,48 +13,48 @@ template <int NP> int threads2d() { return Tiling2D<NP>::NT; }
 template <int NP> void tile_shape2d(int* tx, int* ty) { *tx = Tiling2D<NP>::TX; *ty = Tiling2D<NP>::TY; }
 
 template <int NP> void launch_k2_setup(const SetupArgs2D& a, int nb, cudaStream_t s) {
-  k2_setup<NP><<<nb, Tiling2D<NP>::NT, 0, s>>>(a);
+  launch_chained(k2_setup<NP>, nb, Tiling2D<NP>::NT, s, a);
 }
 template <int NP> void launch_k2_apply(int epi, const ApplyArgs2D& a, int nb, cudaStream_t s) {
   constexpr int NT2 = 2 * Tiling2D<NP>::NH;
-  if (epi == EPI_CHEB) k2_apply<NP, EPI_CHEB><<<nb, NT2, 0, s>>>(a);
-  else if (epi == EPI_JACOBI) k2_apply<NP, EPI_JACOBI><<<nb, NT2, 0, s>>>(a);
-  else if (epi == EPI_PCG0) k2_apply<NP, EPI_PCG0><<<nb, NT2, 0, s>>>(a);
-  else if (epi == EPI_PCG) k2_apply<NP, EPI_PCG><<<nb, NT2, 0, s>>>(a);
-  else k2_apply<NP, EPI_RESID><<<nb, NT2, 0, s>>>(a);
+  if (epi == EPI_CHEB) launch_chained(k2_apply<NP, EPI_CHEB>, nb, NT2, s, a);
+  else if (epi == EPI_JACOBI) launch_chained(k2_apply<NP, EPI_JACOBI>, nb, NT2, s, a);
+  else if (epi == EPI_PCG0) launch_chained(k2_apply<NP, EPI_PCG0>, nb, NT2, s, a);
+  else if (epi == EPI_PCG) launch_chained(k2_apply<NP, EPI_PCG>, nb, NT2, s, a);
+  else launch_chained(k2_apply<NP, EPI_RESID>, nb, NT2, s, a);
 }
 template <int NP> void launch_k2_hyp_rk(const HypArgs2D& a, int nb, cudaStream_t s) {
-  k2_hyp_rk<NP><<<nb, 2 * Tiling2D<NP>::NH, 0, s>>>(a);
+  launch_chained(k2_hyp_rk<NP>, nb, 2 * Tiling2D<NP>::NH, s, a);
 }
 template <int NP> void launch_k2_hyp_rev(const HypRevArgs2D& a, int nb, cudaStream_t s) {
-  k2_hyp_rev<NP><<<nb, 2 * Tiling2D<NP>::NH, 0, s>>>(a);
+  launch_chained(k2_hyp_rev<NP>, nb, 2 * Tiling2D<NP>::NH, s, a);
 }
 template <int NP> void launch_k2_apply_rev(int srev, const ApplyRevArgs2D& a, int nb, cudaStream_t s) {
   constexpr int NT2 = 2 * Tiling2D<NP>::NH;
-  if (srev == SREV_CHEB) k2_apply_rev<NP, SREV_CHEB><<<nb, NT2, 0, s>>>(a);
-  else if (srev == SREV_JACOBI) k2_apply_rev<NP, SREV_JACOBI><<<nb, NT2, 0, s>>>(a);
-  else if (srev == SREV_PCG) k2_apply_rev<NP, SREV_PCG><<<nb, NT2, 0, s>>>(a);
-  else k2_apply_rev<NP, SREV_NONE><<<nb, NT2, 0, s>>>(a);
+  if (srev == SREV_CHEB) launch_chained(k2_apply_rev<NP, SREV_CHEB>, nb, NT2, s, a);
+  else if (srev == SREV_JACOBI) launch_chained(k2_apply_rev<NP, SREV_JACOBI>, nb, NT2, s, a);
+  else if (srev == SREV_PCG) launch_chained(k2_apply_rev<NP, SREV_PCG>, nb, NT2, s, a);
+  else launch_chained(k2_apply_rev<NP, SREV_NONE>, nb, NT2, s, a);
 }
 template <int NP> void launch_k2_setup_rev(const SetupRevArgs2D& a, int nb, cudaStream_t s) {
-  k2_setup_rev<NP><<<nb, Tiling2D<NP>::NT, 0, s>>>(a);
+  launch_chained(k2_setup_rev<NP>, nb, Tiling2D<NP>::NT, s, a);
 }
 
 template <int NP> void launch_k2_sens_rhs(const SensRhsArgs2D& a, int nb, cudaStream_t s) {
-  k2_sens_rhs<NP><<<nb, Tiling2D<NP>::NT, 0, s>>>(a);
+  launch_chained(k2_sens_rhs<NP>, nb, Tiling2D<NP>::NT, s, a);
 }
 template <int NP> void launch_k2_sens_hyp_rk(const SensHypArgs2D& a, int nb, cudaStream_t s) {
-  k2_sens_hyp_rk<NP><<<nb, 2 * Tiling2D<NP>::NH, 0, s>>>(a);
+  launch_chained(k2_sens_hyp_rk<NP>, nb, 2 * Tiling2D<NP>::NH, s, a);
 }
 
 template <int NP> void launch_k2_pde_prep(const PdePrepArgs2D& a, int nb, cudaStream_t s) {
-  k2_pde_prep<NP><<<nb, Tiling2D<NP>::NT, 0, s>>>(a);
+  launch_chained(k2_pde_prep<NP>, nb, Tiling2D<NP>::NT, s, a);
 }
 template <int NP> void launch_k2_pde_b(const PdeBArgs2D& a, int nb, cudaStream_t s) {
-  k2_pde_b<NP><<<nb, Tiling2D<NP>::NT, 0, s>>>(a);
+  launch_chained(k2_pde_b<NP>, nb, Tiling2D<NP>::NT, s, a);
 }
 template <int NP> void launch_k2_pde_rk(const PdeRkArgs2D& a, int nb, cudaStream_t s) {
-  k2_pde_rk<NP><<<nb, Tiling2D<NP>::NT, 0, s>>>(a);
+  launch_chained(k2_pde_rk<NP>, nb, Tiling2D<NP>::NT, s, a);
 }
 
 template <int NP> int pcg_persist_blocks_per_sm() {

@@ -120,12 +120,13 @@ __global__ void __launch_bounds__(PCG_THREADS) k2_pcg_update(PcgUpdateArgs a) {
   __shared__ double s_red[G][P2];
   const TileGroup g = a.groups[blockIdx.x];
   const Inst2D I = a.inst[g.inst];
-  const double al = a.al[g.inst];
   const int idx = threadIdx.x;
   long long n[G];
   bool ok[G];
 #pragma unroll
   for (int j = 0; j < G; ++j) ok[j] = idx < cnt && j < g.count && tile_node<NP>(a.tiles[g.first + j], I, idx, &n[j]);
+  chained_start();
+  const double al = a.al[g.inst];
   double p[G], ap[G], x[G], r[G], im[G];
 #pragma unroll
   for (int j = 0; j < G; ++j)
@@ -192,6 +193,7 @@ __global__ void __launch_bounds__(PCG_THREADS) k2_pcg_rev_update(PcgRevArgs a) {
   __shared__ double s_red[P2];
   const TileGroup g = a.groups[blockIdx.x];
   const Inst2D I = a.inst[g.inst];
+  chained_start();
   const double beta = a.beta[g.inst], rzb1 = a.first ? 0.0 : a.rzb1[g.inst];
   constexpr int cnt = Tiling2D<NP>::TE * NP * NP;
   double part = 0.0;
@@ -227,11 +229,11 @@ __global__ void __launch_bounds__(PCG_THREADS) k2_pcg_rev_update(PcgRevArgs a) {
 
 template <int NP>
 void launch_k2_pcg_update(const PcgUpdateArgs& a, int nblocks, cudaStream_t s) {
-  k2_pcg_update<NP><<<nblocks, PCG_THREADS, 0, s>>>(a);
+  launch_chained(k2_pcg_update<NP>, nblocks, PCG_THREADS, s, a);
 }
 template <int NP>
 void launch_k2_pcg_rev_update(const PcgRevArgs& a, int nblocks, cudaStream_t s) {
-  k2_pcg_rev_update<NP><<<nblocks, PCG_THREADS, 0, s>>>(a);
+  launch_chained(k2_pcg_rev_update<NP>, nblocks, PCG_THREADS, s, a);
 }
 
 // Per-instance sums in a separate launch (InstSum with cnt null): one
@@ -242,6 +244,7 @@ static __global__ void __launch_bounds__(64) k2_inst_sum(const Inst2D* inst, con
   __shared__ double s_acc[64];
   const int i = blockIdx.x;
   const Inst2D I = inst[i];
+  chained_start();
   const double* p = partials + I.tile0;
   const int count = grouped ? inst_groups(I) : I.ntiles;
   double acc = 0.0;
@@ -270,6 +273,7 @@ template <int NP>
 __global__ void __launch_bounds__(PCG_THREADS) k2_pcg_rev_final(PcgRevFinalArgs a) {
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];
+  chained_start();
   const double rzb0 = a.RZB[tl.inst];
   constexpr int cnt = Tiling2D<NP>::TE * NP * NP;
   for (int idx = threadIdx.x; idx < cnt; idx += blockDim.x) {
@@ -284,7 +288,7 @@ __global__ void __launch_bounds__(PCG_THREADS) k2_pcg_rev_final(PcgRevFinalArgs 
 
 template <int NP>
 void launch_k2_pcg_rev_final(const PcgRevFinalArgs& a, int nblocks, cudaStream_t s) {
-  k2_pcg_rev_final<NP><<<nblocks, PCG_THREADS, 0, s>>>(a);
+  launch_chained(k2_pcg_rev_final<NP>, nblocks, PCG_THREADS, s, a);
 }
 
 }  // namespace igrgpu

@@ -45,6 +45,7 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_pde_prep(PdePrepArgs2D a)
   __shared__ double s_ir[TE][NN];
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];
+  chained_start();
   const ElemView vr = elem_view<NP>(tl, I, 0), vc = elem_view<NP>(tl, I, 1);
   const BasisDev& B = a.B;
   const int nf = a.nl[0] ? 7 : 5;  // the velocity gradients serve the nonlocal source only
@@ -163,6 +164,7 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_pde_b(PdeBArgs2D a) {
   __shared__ double s_d[2][TE][NN];  // d_x a_mux, d_x a_E
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];
+  chained_start();
   const ElemView vr = elem_view<NP>(tl, I, 0), vc = elem_view<NP>(tl, I, 1);
   const BasisDev& B = a.B;
   if (vr.valid) {
@@ -257,6 +259,7 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_pde_rk(PdeRkArgs2D a) {
   __shared__ double s_wx[TE][NP][2];    // wave speeds there
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];
+  chained_start();
   const ElemView vr = elem_view<NP>(tl, I, 0), vc = elem_view<NP>(tl, I, 1);
   const BasisDev& B = a.B;
   const double g = I.gamma;

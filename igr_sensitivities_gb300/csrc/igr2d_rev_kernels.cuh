@@ -126,6 +126,7 @@ __global__ void __launch_bounds__(2 * Tiling2D<NP>::NH) k2_hyp_rev(HypRevArgs2D 
   __shared__ double s_g[2][TE][NP];         // the lines' d/dgamma
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];
+  chained_start();
   const BasisDev& B = a.B;
   const double g = I.gamma;
   const double c2dt = a.c2 * I.dt;
@@ -334,6 +335,7 @@ __global__ void __launch_bounds__(2 * Tiling2D<NP>::NH, NP == 4 ? 7 : 1) k2_appl
   __shared__ double s_red[PCG ? P2 : 1];
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];
+  chained_start();
   const BasisDev& B = a.B;
   const double hw = B.hw;
   double pal = 0.0, ppb = 0.0;  // PCG: alpha_it and the adjoint of pAp_it
@@ -519,6 +521,7 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_setup_rev(SetupRevArgs2D 
   __shared__ double s_p[2][NP], s_s[2][2][NP];
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];
+  chained_start();
   const ElemView vr = elem_view<NP>(tl, I, 0), vc = elem_view<NP>(tl, I, 1);
   const BasisDev& B = a.B;
   const double invJx = I.ijx, invJy = I.ijy;

@@ -43,6 +43,7 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_sens_rhs(SensRhsArgs2D a)
   __shared__ double s_dx[NQ][TE][NN];  // x derivatives
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];
+  chained_start();
   const ElemView vr = elem_view<NP>(tl, I, 0), vc = elem_view<NP>(tl, I, 1);
   const BasisDev& B = a.B;
   if (vr.valid) {
@@ -173,6 +174,7 @@ __global__ void __launch_bounds__(2 * Tiling2D<NP>::NH) k2_sens_hyp_rk(SensHypAr
   __shared__ StageSmem<NP, false> sm;
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];
+  chained_start();
   dg_stage<NP, false>(TangentStage{a, I.gamma}, a.B, tl, I, a.c0, a.c1, a.c2, a.k_out[0] != nullptr, sm);
 }
 

@@ -343,4 +343,32 @@ __host__ __device__ constexpr int pow2_at_least(int n) {
          (n <= 128 ? 128 : (n <= 256 ? 256 : (n <= 512 ? 512 : 1024)))))))));
 }
 
+// Launches of a step follow one another on one stream, most of them as short
+// as the gap between two. launch_chained lets the next kernel's CTAs come up
+// while this one's last CTAs run: they load their tile and instance, which only
+// the plan's upload writes, and hold in chained_start until the kernels before
+// are complete and their writes visible. The order of the two instructions
+// matters: a kernel releases its successor only when its own predecessor is
+// complete, so at most two kernels of the chain are in flight, and every CTA of a
+// chained kernel comes here before it returns. Nothing but the plan's
+// descriptors may be read, and nothing written, ahead of it.
+__device__ __forceinline__ void chained_start() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <class... P, class... A>
+void launch_chained(void (*kernel)(P...), int blocks, int threads, cudaStream_t s, const A&... args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)blocks, 1, 1);
+  cfg.blockDim = dim3((unsigned)threads, 1, 1);
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 }  // namespace igrgpu
