@@ -68,11 +68,13 @@ template <int NP> cudaError_t launch_k2_pcg_persist(const PcgPersistArgs& a, int
   cfg.blockDim = dim3(persist_threads<NP>(), 1, 1);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeCooperative;
   at[0].val.cooperative = 1;
+  at[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+  at[1].val.sharedMemCarveout = SMALL_GRID_CARVEOUT;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = grid <= SMALL_GRID ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, k2_pcg_persist<NP>, a);
 }
 

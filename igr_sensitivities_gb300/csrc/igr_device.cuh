@@ -357,17 +357,27 @@ __device__ __forceinline__ void chained_start() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// The driver sizes an SM's shared memory for each launch by what its grid needs, and an SM empties before its split
+// between L1 and shared memory changes. With under three tiles per SM these needs differ from kernel to kernel, so all kernels
+// of a step then ask for the same split, 100 KB (three to eleven CTAs of the solver's kernels, two of k2_hyp_rev);
+// above that they all ask for nearly everything by themselves and a larger L1 is worth more. P3 gradients, ms, driver's
+// split / 100 KB / all shared: 64^2 (256 tiles) 4.68 / 3.94 / 4.03, 40^2 3.12 / 3.04 / 3.07, 76^2 5.57 / 5.34 / 5.31; 8 x 128^2
+// (8192 tiles) 43.1 / 47.8 / 43.5.
+constexpr int SMALL_GRID = 3 * 152;
+constexpr unsigned SMALL_GRID_CARVEOUT = 44;  // percent of 228 KB
 template <class... P, class... A>
 void launch_chained(void (*kernel)(P...), int blocks, int threads, cudaStream_t s, const A&... args) {
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+  at[1].val.sharedMemCarveout = SMALL_GRID_CARVEOUT;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)blocks, 1, 1);
   cfg.blockDim = dim3((unsigned)threads, 1, 1);
   cfg.stream = s;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = blocks <= SMALL_GRID ? 2 : 1;
   cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
