@@ -156,14 +156,18 @@ struct SetupArgs2D {
 };
 
 // What bounds it: FP64 issue, at a third of the FP64 instructions of its FP64-contraction form: the velocity derivatives
-// and both diagonal contractions (with their scales, and for the column one with the sum of all other parts of diag(A))
-// are integer line operations, and the face constants are tabulated once per CTA. 8 x 128^2 P3: 259 us with FP64
-// contractions, 112 us now (95 FP64 instructions per warp of lines, pipe 77% busy); 64^2: 16.5 and 14.0.
+// and both diagonal contractions (with their scales and the face terms) are integer line operations, and the face
+// constants are tabulated once per CTA. Rows and columns run side by side like the operator's, between two pointwise
+// passes. 8 x 128^2 P3: 259 us with FP64 contractions, 113 us with integer ones, 103 us in halves; 64^2: 16.5, 13.9, 12.4.
 template <int NP>
-__global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_setup(SetupArgs2D a) {
+__global__ void __launch_bounds__(2 * Tiling2D<NP>::NH) k2_setup(SetupArgs2D a) {
   using TL = Tiling2D<NP>;
-  constexpr int TE = TL::TE, NN = TL::NN, L = TL::L;
-  __shared__ double s_ux[TE][NN], s_uy[TE][NN], s_ir[TE][NN], s_uxx[TE][NN], s_uyx[TE][NN], s_mx[TE][NN];
+  constexpr int TE = TL::TE, NN = TL::NN, SN = TL::SN, L = TL::L, TX = TL::TX, TY = TL::TY, NH = TL::NH;
+  constexpr int NQ = (TE * NN + 2 * NH - 1) / (2 * NH);  // nodes per thread
+  __shared__ __align__(16) double s_ir[TE][SN], s_ux[TE][SN], s_uy[TE][SN];
+  // per direction: derivatives of the velocities (columns: twice that of u_x), the line's share of diag(A), face penalties
+  __shared__ __align__(16) double s_dx[2][TE][SN], s_dy[2][TE][SN], s_m[2][TE][SN];
+  __shared__ double s_f[2][TE][NP][2];
   // per node: w_i w_j Jx Jy, alpha w_i w_j Jy/Jx, alpha w_i w_j Jx/Jy, alpha times the first  [node j*NP+i]
   __shared__ double s_c[4][NN];
   // per face node of a side: alpha eta w J / d (penalty) and the self terms' -+alpha D_ee w J / J' (x: left, right; y: bottom, top)
@@ -171,131 +175,113 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_setup(SetupArgs2D a) {
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];
   chained_start();
-  const ElemView vr = elem_view<NP>(tl, I, 0), vc = elem_view<NP>(tl, I, 1);
   const BasisDev& B = a.B;
   const double invJx = I.ijx, invJy = I.ijy;
   if (I.alpha <= 0.0 && !a.always) return;  // no elliptic solve for this instance (forward.jl:24-28)
-  for (int n = threadIdx.x; n < NN; n += blockDim.x) {
-    const int i = n % NP, j = n / NP;
-    const double ww = B.w[i] * B.w[j];
-    s_c[0][n] = ww * I.jx * I.jy;
-    s_c[1][n] = I.alpha * ww * I.jy * invJx;
-    s_c[2][n] = I.alpha * ww * I.jx * invJy;
-    s_c[3][n] = s_c[0][n] * I.alpha;
-  }
-  if (threadIdx.x < 2 * NP) {
-    const int d = threadIdx.x / NP, k = threadIdx.x % NP;
-    const double wf = B.w[k] * (d == 0 ? I.jy : I.jx), aJ = I.alpha * (d == 0 ? invJx : invJy);
-    s_p[d][k] = I.alpha * (double)(NP * NP) * (d == 0 ? I.idx : I.idy) * wf;
-    s_s[d][0][k] = aJ * B.D[0][0] * wf;
-    s_s[d][1][k] = -aJ * B.D[L][L] * wf;
-  }
-  auto none = [](int) { return false; };
-  auto all = [](int) { return true; };
-
-  // ---- row phase (row t of element vr): velocities, x-derivatives, x part of the stiffness diagonal
-  if (vr.valid) {
-    const int t = vr.t, e = vr.e;
-    double ux[NP], uy[NP], ir[NP], out[NP];
+  // the thread's nodes: node(m) or -1; m = el NN + nd
+  auto node = [&](int m) -> long long {
+    const int el = m / NN, nd = m % NN, ex = tl.ex0 + el % TX, ey = tl.ey0 + el / TX;
+    return m < TE * NN && ex < I.nex && ey < I.ney ? I.off + (long long)NN * (ex + (long long)I.nex * ey) + nd : -1;
+  };
+  // ---- pointwise: velocities and 1/rho
+  {
+    double ir[NQ], ux[NQ], uy[NQ];
 #pragma unroll
-    for (int i = 0; i < NP; ++i) {
-      const long long n = vr.base + t * NP + i;
-      ir[i] = a.invr[n];
-      s_ir[e][t * NP + i] = ir[i];
-      if (a.b) {
-        ux[i] = a.mx[n] * ir[i];
-        uy[i] = a.my[n] * ir[i];
-        s_ux[e][t * NP + i] = ux[i]; s_uy[e][t * NP + i] = uy[i];
-      }
+    for (int q = 0; q < NQ; ++q) {
+      const long long n = node(threadIdx.x + q * 2 * NH);
+      if (n < 0) continue;
+      ir[q] = a.invr[n];
+      if (a.b) { ux[q] = a.mx[n]; uy[q] = a.my[n]; }
     }
-    if (a.b) {
-      const FixScale cx = fix_scale(invJx);
-      line_rows<NP>(B, cx, ux, out);
-#pragma unroll
-      for (int i = 0; i < NP; ++i) s_uxx[e][t * NP + i] = out[i];
-      line_rows<NP>(B, cx, uy, out);
-#pragma unroll
-      for (int i = 0; i < NP; ++i) s_uyx[e][t * NP + i] = out[i];
+    for (int n = threadIdx.x; n < NN; n += blockDim.x) {
+      const int i = n % NP, j = n / NP;
+      const double ww = B.w[i] * B.w[j];
+      s_c[0][n] = ww * I.jx * I.jy;
+      s_c[1][n] = I.alpha * ww * I.jy * invJx;
+      s_c[2][n] = I.alpha * ww * I.jx * invJy;
+      s_c[3][n] = s_c[0][n] * I.alpha;
     }
-    const FixScale cd = fix_scale(I.alpha * B.w[t] * I.jy * invJx);
-    line_op<NP, true, false, true>(B.fW2, B.W2, &cd, ir, nullptr, none, out);
+    if (threadIdx.x < 2 * NP) {
+      const int d = threadIdx.x / NP, k = threadIdx.x % NP;
+      const double wf = B.w[k] * (d == 0 ? I.jy : I.jx), aJ = I.alpha * (d == 0 ? invJx : invJy);
+      s_p[d][k] = I.alpha * (double)(NP * NP) * (d == 0 ? I.idx : I.idy) * wf;
+      s_s[d][0][k] = aJ * B.D[0][0] * wf;
+      s_s[d][1][k] = -aJ * B.D[L][L] * wf;
+    }
 #pragma unroll
-    for (int i = 0; i < NP; ++i) s_mx[e][t * NP + i] = out[i];
+    for (int q = 0; q < NQ; ++q) {
+      const int m = threadIdx.x + q * 2 * NH;
+      if (node(m) < 0) continue;
+      const int el = m / NN, nd = m % NN;
+      s_ir[el][nd] = ir[q];
+      if (a.b) { s_ux[el][nd] = ux[q] * ir[q]; s_uy[el][nd] = uy[q] * ir[q]; }
+    }
   }
   __syncthreads();
-  if (!vc.valid) return;
-
-  // ---- column phase (column t of element vc): y-derivatives, source, diagonal, coefficients
-  const int t = vc.t, e = vc.e;
-  double cir[NP];
+  // ---- lines: derivatives, stiffness diagonal with the face terms
+  const int dir = threadIdx.x >= NH;  // 0: rows and x faces, 1: columns and y faces
+  const ElemView w = elem_view<NP>(tl, I, dir, threadIdx.x - dir * NH);
+  if (w.valid) {
+    const int e = w.e, t = w.t;
+    const int st = dir == 0 ? 1 : NP, at = dir == 0 ? t * NP : t;  // node k of the line: at + k st
+    auto partner = [&](int s) {  // 1/rho across the line's face s
+      int it;
+      const int d = s == 0 ? -1 : 1, pn = at + (s == 0 ? L : 0) * st;
+      const long long pb = neighbour<NP>(tl, I, w.ex, w.ey, dir == 0 ? d : 0, dir == 0 ? 0 : d, &it);
+      return it >= 0 ? s_ir[it][pn] : a.invr[pb + pn];
+    };
+    const int sf = dir == 0 ? first_side(w.ext, TX) : first_side(w.eyt, TY);
+    const double pA = partner(sf), pB = partner(1 - sf);
+    double v[NP], out[NP];
+    if (a.b) {
+      const FixScale c1 = fix_scale(dir == 0 ? invJx : invJy);
 #pragma unroll
-  for (int l = 0; l < NP; ++l) cir[l] = s_ir[e][l * NP + t];
-  if (a.b) {
-    double cux[NP], cuy[NP], uxy2[NP], uyy[NP];  // uxy2 = 2 d_y u_x
+      for (int k = 0; k < NP; ++k) v[k] = s_ux[e][at + k * st];
+      line_rows<NP>(B, fix_scale(dir == 0 ? invJx : 2.0 * invJy), v, out);
 #pragma unroll
-    for (int l = 0; l < NP; ++l) { cux[l] = s_ux[e][l * NP + t]; cuy[l] = s_uy[e][l * NP + t]; }
-    line_rows<NP>(B, fix_scale(2.0 * invJy), cux, uxy2);
-    line_rows<NP>(B, fix_scale(invJy), cuy, uyy);
+      for (int k = 0; k < NP; ++k) { s_dx[dir][e][at + k * st] = out[k]; v[k] = s_uy[e][at + k * st]; }
+      line_rows<NP>(B, c1, v, out);
 #pragma unroll
-    for (int l = 0; l < NP; ++l) {
-      const int nd = l * NP + t;
-      const double uxx = s_uxx[e][nd], uyx = s_uyx[e][nd];
-      const double s = uxx + uyy[l];
+      for (int k = 0; k < NP; ++k) s_dy[dir][e][at + k * st] = out[k];
+    }
+    double acc[NP];
+#pragma unroll
+    for (int k = 0; k < NP; ++k) v[k] = s_ir[e][at + k * st];
+    // right side of the face at node 0, left side of the one at node L
+    const double f0 = s_p[dir][t] * max_nonneg(sf == 0 ? pA : pB, v[0]), fL = s_p[dir][t] * max_nonneg(v[L], sf == 0 ? pB : pA);
+    s_f[dir][e][t][0] = f0; s_f[dir][e][t][1] = fL;
+    acc[0] = fma(s_s[dir][0][t], v[0], f0);
+    acc[L] = fma(s_s[dir][1][t], v[L], fL);
+    const FixScale cd = fix_scale(I.alpha * B.w[t] * (dir == 0 ? I.jy * invJx : I.jx * invJy));
+    line_op<NP, true, false, true>(B.fW2, B.W2, &cd, v, acc, [](int k) { return k == 0 || k == L; }, out);
+#pragma unroll
+    for (int k = 0; k < NP; ++k) s_m[dir][e][at + k * st] = out[k];
+  }
+  __syncthreads();
+  // ---- pointwise: source, diagonal, coefficients
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) {
+    const int m = threadIdx.x + q * 2 * NH;
+    const long long n = node(m);
+    if (n < 0) continue;
+    const int el = m / NN, nd = m % NN, i = nd % NP, j = nd / NP;
+    if (a.b) {
+      const double uxx = s_dx[0][el][nd], uyx = s_dy[0][el][nd], uxy2 = s_dx[1][el][nd], uyy = s_dy[1][el][nd];
+      const double s = uxx + uyy;
       double R = fma(s, s, uxx * uxx);
-      R = fma(uxy2[l], uyx, R);
-      R = fma(uyy[l], uyy[l], R);
-      a.b[vc.base + nd] = s_c[3][nd] * R;
+      R = fma(uxy2, uyx, R);
+      R = fma(uyy, uyy, R);
+      a.b[n] = s_c[3][nd] * R;
     }
-  }
-  // partner 1/rho across the x faces of column t (only t == 0 or t == L) and the y faces (l == 0, l == L)
-  double irx[NP];
-  if (t == 0 || t == L) {
-    int it;
-    const long long pb = neighbour<NP>(tl, I, vc.ex, vc.ey, t == 0 ? -1 : 1, 0, &it);
-    const int pi = t == 0 ? L : 0;
-#pragma unroll
-    for (int l = 0; l < NP; ++l) irx[l] = it >= 0 ? s_ir[it][l * NP + pi] : a.invr[pb + l * NP + pi];
-  }
-  double iry[2];
-  {
-    int it;
-    const long long pb = neighbour<NP>(tl, I, vc.ex, vc.ey, 0, -1, &it);  // bottom partner: node (t, L)
-    iry[0] = it >= 0 ? s_ir[it][L * NP + t] : a.invr[pb + L * NP + t];
-    const long long pt = neighbour<NP>(tl, I, vc.ex, vc.ey, 0, 1, &it);   // top partner: node (t, 0)
-    iry[1] = it >= 0 ? s_ir[it][t] : a.invr[pt + t];
-  }
-  double acc[NP], M[NP];
-#pragma unroll
-  for (int l = 0; l < NP; ++l) {
-    const long long n = vc.base + l * NP + t;
-    const int nd = l * NP + t;
-    const double mass = s_c[0][nd] * cir[l];
-    double m = mass + s_mx[e][nd];
-    double px = 0.0, py = 0.0;
-    if (t == 0 || t == L) {
-      px = s_p[0][l] * max_nonneg(t == L ? cir[l] : irx[l], t == L ? irx[l] : cir[l]);
-      // x-face self terms: right side of its left face (t == 0) / left side of its right face (t == L)
-      m = fma(s_s[0][t == L ? 1 : 0][l], cir[l], m + px);
-    }
-    if (l == 0 || l == L) {
-      const double ip = iry[l == 0 ? 0 : 1];
-      py = s_p[1][t] * max_nonneg(l == L ? cir[l] : ip, l == L ? ip : cir[l]);
-      m = fma(s_s[1][l == L ? 1 : 0][t], cir[l], m + py);
-    }
-    acc[l] = m;
+    const double ir = s_ir[el][nd], mass = s_c[0][nd] * ir;
+    const double M = mass + (s_m[0][el][nd] + s_m[1][el][nd]);
     a.cm[n] = mass;
-    a.ckx[n] = s_c[1][nd] * cir[l];
-    a.cky[n] = s_c[2][nd] * cir[l];
-    a.cpx[n] = px;
-    a.cpy[n] = py;
-  }
-  const FixScale cd = fix_scale(I.alpha * B.w[t] * I.jx * invJy);
-  line_op<NP, true, false, true>(B.fW2, B.W2, &cd, cir, acc, all, M);
-#pragma unroll
-  for (int l = 0; l < NP; ++l) {
-    const long long n = vc.base + l * NP + t;
-    a.cinvM[n] = reciprocal(M[l]);
-    if (a.cM) a.cM[n] = M[l];
+    a.ckx[n] = s_c[1][nd] * ir;
+    a.cky[n] = s_c[2][nd] * ir;
+    a.cpx[n] = i == 0 || i == L ? s_f[0][el][j][i == L] : 0.0;
+    a.cpy[n] = j == 0 || j == L ? s_f[1][el][i][j == L] : 0.0;
+    a.cinvM[n] = reciprocal(M);
+    if (a.cM) a.cM[n] = M;
   }
 }
 

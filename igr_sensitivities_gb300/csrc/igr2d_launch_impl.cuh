@@ -13,7 +13,7 @@ template <int NP> int threads2d() { return Tiling2D<NP>::NT; }
 template <int NP> void tile_shape2d(int* tx, int* ty) { *tx = Tiling2D<NP>::TX; *ty = Tiling2D<NP>::TY; }
 
 template <int NP> void launch_k2_setup(const SetupArgs2D& a, int nb, cudaStream_t s) {
-  launch_chained(k2_setup<NP>, nb, Tiling2D<NP>::NT, s, a);
+  launch_chained(k2_setup<NP>, nb, 2 * Tiling2D<NP>::NH, s, a);
 }
 template <int NP> void launch_k2_apply(int epi, const ApplyArgs2D& a, int nb, cudaStream_t s) {
   constexpr int NT2 = 2 * Tiling2D<NP>::NH;
@@ -37,7 +37,7 @@ template <int NP> void launch_k2_apply_rev(int srev, const ApplyRevArgs2D& a, in
   else launch_chained(k2_apply_rev<NP, SREV_NONE>, nb, NT2, s, a);
 }
 template <int NP> void launch_k2_setup_rev(const SetupRevArgs2D& a, int nb, cudaStream_t s) {
-  launch_chained(k2_setup_rev<NP>, nb, Tiling2D<NP>::NT, s, a);
+  launch_chained(k2_setup_rev<NP>, nb, 2 * Tiling2D<NP>::NH, s, a);
 }
 
 template <int NP> void launch_k2_sens_rhs(const SensRhsArgs2D& a, int nb, cudaStream_t s) {

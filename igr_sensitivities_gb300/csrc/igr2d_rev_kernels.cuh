@@ -505,167 +505,166 @@ struct SetupRevArgs2D {
   double *anode;
 };
 
-// What bounds it: FP64 issue. All derivatives, transposes and diagonal contractions are integer line operations, with
-// their scales and the terms they are added to; the x transposes have a row phase of their own. 8 x 128^2 P3: 409 us with
-// FP64 contractions, 198 us now; 64^2: 22.8 and 22.7 (five phases of latency).
+// What bounds it: FP64 issue. All derivatives, transposes and diagonal contractions are integer line operations; the two
+// transposes of a node meet as integers. Rows and columns run side by side, between pointwise passes whose loads
+// come before any store. 8 x 128^2 P3: 409 us with FP64 contractions, 196 us with integer ones, 158 us in halves; 64^2: 22.8,
+// 22.7, 14.9.
 template <int NP>
-__global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_setup_rev(SetupRevArgs2D a) {
+__global__ void __launch_bounds__(2 * Tiling2D<NP>::NH) k2_setup_rev(SetupRevArgs2D a) {
   using TL = Tiling2D<NP>;
-  constexpr int TE = TL::TE, NN = TL::NN, L = TL::L;
-  __shared__ double s_ux[TE][NN], s_uy[TE][NN], s_Mb[TE][NN];
-  __shared__ double s_uxx[TE][NN], s_uyx[TE][NN];       // x derivatives (row phase)
-  __shared__ double s_bxx[TE][NN], s_byx[TE][NN];       // adjoints of uxx, uyx (columns), then their x transposes (rows)
-  __shared__ double s_ir[TE][NN], s_ib[TE][NN];         // 1/rho; row-phase d/d(1/rho) from diag(A)
-  __shared__ double s_m0[NN];                           // w_i w_j Jx Jy
+  constexpr int TE = TL::TE, NN = TL::NN, SN = TL::SN, L = TL::L, TX = TL::TX, TY = TL::TY, NH = TL::NH;
+  constexpr int NQ = (TE * NN + 2 * NH - 1) / (2 * NH);  // nodes per thread
+  __shared__ __align__(16) double s_ux[TE][SN], s_uy[TE][SN], s_ir[TE][SN], s_Mb[TE][SN];
+  // per direction: derivatives of the velocities, then the adjoints of these, then (integers) their transposes
+  __shared__ __align__(16) long long s_dx[2][TE][SN], s_dy[2][TE][SN];
+  __shared__ int s_ex[2][TE][NP], s_ey[2][TE][NP];
+  __shared__ __align__(16) double s_ib[2][TE][SN];  // d/d(1/rho) from the line's share of diag(A)
+  __shared__ double s_m0[NN];                       // w_i w_j Jx Jy
   // per face node of a side: alpha eta w J / d (penalty) and the self terms' -+alpha D_ee w J / J' (x: left, right; y: bottom, top)
   __shared__ double s_p[2][NP], s_s[2][2][NP];
   const Tile2D tl = a.tiles[blockIdx.x];
   const Inst2D I = a.inst[tl.inst];
   chained_start();
-  const ElemView vr = elem_view<NP>(tl, I, 0), vc = elem_view<NP>(tl, I, 1);
   const BasisDev& B = a.B;
   const double invJx = I.ijx, invJy = I.ijy;
   const double alpha = I.alpha;
   if (alpha <= 0.0) return;
-  for (int n = threadIdx.x; n < NN; n += blockDim.x) s_m0[n] = B.w[n % NP] * B.w[n / NP] * I.jx * I.jy;
-  if (threadIdx.x < 2 * NP) {
-    const int d = threadIdx.x / NP, k = threadIdx.x % NP;
-    const double wf = B.w[k] * (d == 0 ? I.jy : I.jx), aJ = alpha * (d == 0 ? invJx : invJy);
-    s_p[d][k] = alpha * (double)(NP * NP) * (d == 0 ? I.idx : I.idy) * wf;
-    s_s[d][0][k] = aJ * B.D[0][0] * wf;
-    s_s[d][1][k] = -aJ * B.D[L][L] * wf;
-  }
-  auto none = [](int) { return false; };
-  auto all = [](int) { return true; };
-  const FixScale cx = fix_scale(invJx), cy = fix_scale(invJy);
-
-  if (vr.valid) {
-    const int t = vr.t, e = vr.e;
-    double ux[NP], uy[NP], Mbr[NP], out[NP];
+  // the thread's nodes: node(m) or -1; m = el NN + nd
+  auto node = [&](int m) -> long long {
+    const int el = m / NN, nd = m % NN, ex = tl.ex0 + el % TX, ey = tl.ey0 + el / TX;
+    return m < TE * NN && ex < I.nex && ey < I.ney ? I.off + (long long)NN * (ex + (long long)I.nex * ey) + nd : -1;
+  };
+  auto mbar = [&](double iMb, double im) { return -(iMb * im) * im; };  // d/dM = -d/d(1/M) / M^2
+  // ---- pointwise: velocities, 1/rho, adjoint of diag(A)
+  double bb[NQ];
+  {
+    double ir[NQ], mx[NQ], my[NQ], im[NQ], imb[NQ];
 #pragma unroll
-    for (int i = 0; i < NP; ++i) {
-      const long long n = vr.base + t * NP + i;
-      const double ir = a.invr[n];
-      const double im = a.cinvM[n];
-      ux[i] = a.mx[n] * ir; uy[i] = a.my[n] * ir; Mbr[i] = -(a.iMb[n] * im) * im;  // d/dM = -d/d(1/M) / M^2
-      s_ux[e][t * NP + i] = ux[i]; s_uy[e][t * NP + i] = uy[i]; s_Mb[e][t * NP + i] = Mbr[i]; s_ir[e][t * NP + i] = ir;
+    for (int q = 0; q < NQ; ++q) {
+      const long long n = node(threadIdx.x + q * 2 * NH);
+      if (n < 0) continue;
+      ir[q] = a.invr[n]; mx[q] = a.mx[n]; my[q] = a.my[n]; im[q] = a.cinvM[n]; imb[q] = a.iMb[n];
+      bb[q] = a.bb[n];
     }
-    line_rows<NP>(B, cx, ux, out);
-#pragma unroll
-    for (int i = 0; i < NP; ++i) s_uxx[e][t * NP + i] = out[i];
-    line_rows<NP>(B, cx, uy, out);
-#pragma unroll
-    for (int i = 0; i < NP; ++i) s_uyx[e][t * NP + i] = out[i];
-    // x stiffness self-coupling of diag(A): d/d(1/rho[i,t]) = cxs * sum_k W2[i][k] Mb[k,t]
-    const FixScale cd = fix_scale(alpha * B.w[t] * I.jy * invJx);
-    line_op<NP, false, false, true>(B.fW2, B.W2, &cd, Mbr, nullptr, none, out);
-#pragma unroll
-    for (int i = 0; i < NP; ++i) s_ib[e][t * NP + i] = out[i];
-  }
-  __syncthreads();
-  // ---- column of vc: y derivatives, source adjoint, diag(A) y part and faces
-  double bxy[NP], byy[NP], ib[NP];
-  if (vc.valid) {
-    const int t = vc.t, e = vc.e;
-    {
-      double col[NP], uxy[NP], uyy[NP];
-#pragma unroll
-      for (int l = 0; l < NP; ++l) col[l] = s_ux[e][l * NP + t];
-      line_rows<NP>(B, cy, col, uxy);
-#pragma unroll
-      for (int l = 0; l < NP; ++l) col[l] = s_uy[e][l * NP + t];
-      line_rows<NP>(B, cy, col, uyy);
-#pragma unroll
-      for (int l = 0; l < NP; ++l) {
-        const int nd = l * NP + t;
-        const double uxx = s_uxx[e][nd], uyx = s_uyx[e][nd];
-        const double s = uxx + uyy[l];
-        const double Qb2 = a.bb[vc.base + nd] * (2.0 * alpha * s_m0[nd]);
-        s_bxx[e][nd] = Qb2 * (s + uxx);
-        s_byx[e][nd] = Qb2 * uxy[l];
-        bxy[l] = Qb2 * uyx;
-        byy[l] = Qb2 * (s + uyy[l]);
-      }
-    }
-    double Mb[NP], cir[NP], acc[NP];
-#pragma unroll
-    for (int l = 0; l < NP; ++l) {
-      Mb[l] = s_Mb[e][l * NP + t];
-      cir[l] = s_ir[e][l * NP + t];
-      acc[l] = fma(Mb[l], s_m0[l * NP + t], s_ib[e][l * NP + t]);
-    }
-    // diag(A) face terms, x faces (t == 0: own R side; t == L: own L side)
-    if (t == 0 || t == L) {
-      int it;
-      const long long pb = neighbour<NP>(tl, I, vc.ex, vc.ey, t == 0 ? -1 : 1, 0, &it);
-      const int pi = t == 0 ? L : 0;
-#pragma unroll
-      for (int l = 0; l < NP; ++l) {
-        const double pir = it >= 0 ? s_ir[it][l * NP + pi] : a.invr[pb + l * NP + pi];
-        const long long pn = pb + l * NP + pi;
-        const double pMb = it >= 0 ? s_Mb[it][l * NP + pi] : -(a.iMb[pn] * a.cinvM[pn]) * a.cinvM[pn];
-        acc[l] = fma(Mb[l], s_s[0][t == L ? 1 : 0][l], acc[l]);
-        const double iL = t == L ? cir[l] : pir, iR = t == L ? pir : cir[l];
-        const bool own_wins = (t == L) ? !gt_nonneg(iR, iL) : gt_nonneg(iR, iL);
-        if (own_wins) acc[l] = fma(Mb[l] + pMb, s_p[0][l], acc[l]);
-      }
+    for (int n = threadIdx.x; n < NN; n += blockDim.x) s_m0[n] = B.w[n % NP] * B.w[n / NP] * I.jx * I.jy;
+    if (threadIdx.x < 2 * NP) {
+      const int d = threadIdx.x / NP, k = threadIdx.x % NP;
+      const double wf = B.w[k] * (d == 0 ? I.jy : I.jx), aJ = alpha * (d == 0 ? invJx : invJy);
+      s_p[d][k] = alpha * (double)(NP * NP) * (d == 0 ? I.idx : I.idy) * wf;
+      s_s[d][0][k] = aJ * B.D[0][0] * wf;
+      s_s[d][1][k] = -aJ * B.D[L][L] * wf;
     }
 #pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      const int l = s == 0 ? 0 : L;
-      int it;
-      const long long pb = neighbour<NP>(tl, I, vc.ex, vc.ey, 0, s == 0 ? -1 : 1, &it);
-      const int pl = s == 0 ? L : 0;
-      const double pir = it >= 0 ? s_ir[it][pl * NP + t] : a.invr[pb + pl * NP + t];
-      const long long pn = pb + pl * NP + t;
-      const double pMb = it >= 0 ? s_Mb[it][pl * NP + t] : -(a.iMb[pn] * a.cinvM[pn]) * a.cinvM[pn];
-      acc[l] = fma(Mb[l], s_s[1][s][t], acc[l]);
-      const double iL = l == L ? cir[l] : pir, iR = l == L ? pir : cir[l];
-      const bool own_wins = (l == L) ? !gt_nonneg(iR, iL) : gt_nonneg(iR, iL);
-      if (own_wins) acc[l] = fma(Mb[l] + pMb, s_p[1][t], acc[l]);
+    for (int q = 0; q < NQ; ++q) {
+      const int m = threadIdx.x + q * 2 * NH;
+      if (node(m) < 0) continue;
+      const int el = m / NN, nd = m % NN;
+      s_ir[el][nd] = ir[q];
+      s_ux[el][nd] = mx[q] * ir[q]; s_uy[el][nd] = my[q] * ir[q];
+      s_Mb[el][nd] = mbar(imb[q], im[q]);
     }
-    // y stiffness self-coupling of diag(A), with the mass, x and face parts
-    const FixScale cd = fix_scale(alpha * B.w[t] * I.jx * invJy);
-    line_op<NP, false, false, true>(B.fW2, B.W2, &cd, Mb, acc, all, ib);
   }
   __syncthreads();
-  // ---- row of vr: x transposes of the source adjoint, in place: ux[t,l] gets sum_i D[i][t] * bxx[i,l] * invJx
-  if (vr.valid) {
-    const int t = vr.t, e = vr.e;
+  // ---- lines: derivatives, diag(A)'s stiffness and faces
+  const int dir = threadIdx.x >= NH;  // 0: rows and x faces, 1: columns and y faces
+  const ElemView w = elem_view<NP>(tl, I, dir, threadIdx.x - dir * NH);
+  const int e = w.e, t = w.t;
+  const int st = dir == 0 ? 1 : NP, at = dir == 0 ? t * NP : t;  // node k of the line: at + k st
+  const FixScale c = fix_scale(dir == 0 ? invJx : invJy);
+  if (w.valid) {
+    struct Partner { double ir, Mb; };
+    auto partner = [&](int s) {
+      Partner P;
+      int it;
+      const int d = s == 0 ? -1 : 1, pn = at + (s == 0 ? L : 0) * st;
+      const long long pb = neighbour<NP>(tl, I, w.ex, w.ey, dir == 0 ? d : 0, dir == 0 ? 0 : d, &it);
+      if (it >= 0) { P.ir = s_ir[it][pn]; P.Mb = s_Mb[it][pn]; }
+      else { P.ir = a.invr[pb + pn]; P.Mb = mbar(a.iMb[pb + pn], a.cinvM[pb + pn]); }
+      return P;
+    };
+    const int sf = dir == 0 ? first_side(w.ext, TX) : first_side(w.eyt, TY);
+    const Partner pA = partner(sf), pB = partner(1 - sf);
     double v[NP], out[NP];
 #pragma unroll
-    for (int i = 0; i < NP; ++i) v[i] = s_bxx[e][t * NP + i];
-    line_cols<NP>(B, cx, v, out);
+    for (int k = 0; k < NP; ++k) v[k] = s_ux[e][at + k * st];
+    line_rows<NP>(B, c, v, out);
 #pragma unroll
-    for (int i = 0; i < NP; ++i) { s_bxx[e][t * NP + i] = out[i]; v[i] = s_byx[e][t * NP + i]; }
-    line_cols<NP>(B, cx, v, out);
+    for (int k = 0; k < NP; ++k) { s_dx[dir][e][at + k * st] = __double_as_longlong(out[k]); v[k] = s_uy[e][at + k * st]; }
+    line_rows<NP>(B, c, v, out);
 #pragma unroll
-    for (int i = 0; i < NP; ++i) s_byx[e][t * NP + i] = out[i];
+    for (int k = 0; k < NP; ++k) { s_dy[dir][e][at + k * st] = __double_as_longlong(out[k]); v[k] = s_Mb[e][at + k * st]; }
+    const Partner p0 = sf == 0 ? pA : pB, pL = sf == 0 ? pB : pA;
+    double acc[NP];
+    acc[0] = v[0] * s_s[dir][0][t];
+    if (gt_nonneg(s_ir[e][at], p0.ir)) acc[0] = fma(v[0] + p0.Mb, s_p[dir][t], acc[0]);
+    acc[L] = v[L] * s_s[dir][1][t];
+    if (!gt_nonneg(pL.ir, s_ir[e][at + L * st])) acc[L] = fma(v[L] + pL.Mb, s_p[dir][t], acc[L]);
+    // stiffness self-coupling of diag(A): d/d(1/rho_i) = c sum_k W2[i][k] Mb_k
+    const FixScale cd = fix_scale(alpha * B.w[t] * (dir == 0 ? I.jy * invJx : I.jx * invJy));
+    line_op<NP, false, false, true>(B.fW2, B.W2, &cd, v, acc, [](int k) { return k == 0 || k == L; }, out);
+#pragma unroll
+    for (int k = 0; k < NP; ++k) s_ib[dir][e][at + k * st] = out[k];
   }
   __syncthreads();
-  if (!vc.valid) return;
-  // ---- column of vc, final: y transposes added to the x ones, conversion to d/d rho and d/d alpha
-  const int t = vc.t, e = vc.e;
-  double acc[NP], uxb[NP], uyb[NP];
+  // ---- pointwise, in place: adjoints of the derivatives
 #pragma unroll
-  for (int l = 0; l < NP; ++l) acc[l] = s_bxx[e][l * NP + t];
-  line_op<NP, true, true, true>(B.fD, B.D, &cy, bxy, acc, all, uxb);
+  for (int q = 0; q < NQ; ++q) {
+    const int m = threadIdx.x + q * 2 * NH;
+    if (node(m) < 0) continue;
+    const int el = m / NN, nd = m % NN;
+    const double uxx = __longlong_as_double(s_dx[0][el][nd]), uyx = __longlong_as_double(s_dy[0][el][nd]);
+    const double uxy = __longlong_as_double(s_dx[1][el][nd]), uyy = __longlong_as_double(s_dy[1][el][nd]);
+    const double s = uxx + uyy;
+    const double Qb2 = bb[q] * (2.0 * alpha * s_m0[nd]);
+    s_dx[0][el][nd] = __double_as_longlong(Qb2 * (s + uxx));
+    s_dy[0][el][nd] = __double_as_longlong(Qb2 * uxy);
+    s_dx[1][el][nd] = __double_as_longlong(Qb2 * uyx);
+    s_dy[1][el][nd] = __double_as_longlong(Qb2 * (s + uyy));
+  }
+  __syncthreads();
+  // ---- lines, in place: transposes
+  if (w.valid) {
+    double v[NP];
+    FixSums<NP> r;
 #pragma unroll
-  for (int l = 0; l < NP; ++l) acc[l] = s_byx[e][l * NP + t];
-  line_op<NP, true, true, true>(B.fD, B.D, &cy, byy, acc, all, uyb);
+    for (int k = 0; k < NP; ++k) v[k] = __longlong_as_double(s_dx[dir][e][at + k * st]);
+    row_scaled<NP, true>(B, c, v, r);
 #pragma unroll
-  for (int l = 0; l < NP; ++l) {
-    const long long n = vc.base + l * NP + t;
-    const int nd = l * NP + t;
-    const double ir = s_ir[e][nd], Mb = s_Mb[e][nd];
-    const double cmn = a.cm[n];
-    const double zs = a.Zs[n], zms = fma(cmn, a.Zm[n], zs);  // Zm + Zs, with Zm's mass coefficient
-    a.Qs[0][n] = fma(uxb[l], ir, a.Qs[0][n]);
-    a.Qs[1][n] = fma(uyb[l], ir, a.Qs[1][n]);
-    const double r = fma(uxb[l], s_ux[e][nd], fma(uyb[l], s_uy[e][nd], fma(ib[l], ir, zms)));
-    a.Qs[2][n] = fma(-ir, r, a.Qs[2][n]);
+    for (int k = 0; k < NP; ++k) { s_dx[dir][e][at + k * st] = r.G[k]; v[k] = __longlong_as_double(s_dy[dir][e][at + k * st]); }
+    s_ex[dir][e][t] = r.e;
+    row_scaled<NP, true>(B, c, v, r);
+#pragma unroll
+    for (int k = 0; k < NP; ++k) s_dy[dir][e][at + k * st] = r.G[k];
+    s_ey[dir][e][t] = r.e;
+  }
+  // ---- pointwise: transposes of both directions, conversion to d/d rho and d/d alpha
+  double b[NQ], cm[NQ], cM[NQ], Zm[NQ], Zs[NQ], Q[NQ][3], an[NQ];
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) {
+    const long long n = node(threadIdx.x + q * 2 * NH);
+    if (n < 0) continue;
+    b[q] = a.b[n]; cm[q] = a.cm[n]; cM[q] = a.cM[n]; Zm[q] = a.Zm[n]; Zs[q] = a.Zs[n]; an[q] = a.anode[n];
+#pragma unroll
+    for (int v = 0; v < 3; ++v) Q[q][v] = a.Qs[v][n];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) {
+    const int m = threadIdx.x + q * 2 * NH;
+    const long long n = node(m);
+    if (n < 0) continue;
+    const int el = m / NN, nd = m % NN, i = nd % NP, j = nd / NP;
+    const double uxb = node_total<60>(s_dx[0][el][nd], s_ex[0][el][j], s_dx[1][el][nd], s_ex[1][el][i], 0.0, 1);
+    const double uyb = node_total<60>(s_dy[0][el][nd], s_ey[0][el][j], s_dy[1][el][nd], s_ey[1][el][i], 0.0, 1);
+    const double ir = s_ir[el][nd], Mb = s_Mb[el][nd];
+    const double ib = fma(Mb, s_m0[nd], s_ib[0][el][nd] + s_ib[1][el][nd]);
+    const double zms = fma(cm[q], Zm[q], Zs[q]);  // Zm + Zs, with Zm's mass coefficient
+    const double r = fma(uxb, s_ux[el][nd], fma(uyb, s_uy[el][nd], fma(ib, ir, zms)));
+    a.Qs[0][n] = fma(uxb, ir, Q[q][0]);
+    a.Qs[1][n] = fma(uyb, ir, Q[q][1]);
+    a.Qs[2][n] = fma(-ir, r, Q[q][2]);
     // d/dalpha: Zs/alpha + Mb (M - mass)/alpha + bb b/alpha
-    a.anode[n] = fma(fma(Mb, a.cM[n] - cmn, fma(a.bb[n], a.b[n], zs)), I.ialpha, a.anode[n]);
+    a.anode[n] = fma(fma(Mb, cM[q] - cm[q], fma(bb[q], b[q], Zs[q])), I.ialpha, an[q]);
   }
 }
 

@@ -53,9 +53,10 @@ inline FixMat make_fix(const double A[FIX_MAXNP][FIX_MAXNP], int np) {
     most = std::fmax(most, std::fmax(r, c));
   }
   while (F.s < 64 && 0.7 * std::ldexp(1.0, F.s) < most) ++F.s;
+  const double unit = std::ldexp(1.0, 63 - F.s);
   for (int i = 0; i < np; ++i)
     for (int k = 0; k < np; ++k) {
-      const long long f = std::llrint(std::ldexp(A[i][k], 63 - F.s));
+      const long long f = std::llrint(A[i][k] * unit);
       const long long h = (f + (1LL << 31)) >> 32;
       F.h[i][k] = (int)h;
       F.l[i][k] = (int)((f - h * (1LL << 32)) / 2);
