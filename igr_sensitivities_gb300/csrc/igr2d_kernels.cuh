@@ -1,19 +1,21 @@
 // 2D IGR-Euler forward kernels (sm_103a, FP64 CUDA cores).
 //
-// Thread mapping: a CTA owns a TX x TY tile of elements of one instance and
-// runs one thread per element *line*. In the xi-phase a thread owns one row
-// (nodes (0..NP-1, t)) of an element and handles that row's x faces; in the
-// eta-phase it owns one column and the y faces. The 1D contractions with the
-// LGL differentiation matrix then run in registers, unrolled per line, so the
-// structurally zero interior diagonal of D is skipped for every lane alike.
+// Thread mapping: a CTA owns a TX x TY tile of elements of one instance. The
+// line work (1D contractions with the LGL differentiation matrix and the faces
+// across the line's ends) takes one thread per element *line*; in most kernels
+// rows and columns run side by side, one half of 2 NH threads each, between
+// pointwise passes over all threads (coalesced, loads before stores). The
+// remaining ones (tangent right-hand side, adjoint PDE) run a row phase and then
+// a column phase on NT threads.
 //
 // GB300 issues about 1.2 TFLOP/s of FP64 against 6.6 TB/s of HBM (about
-// 5.6 B per FP64 flop), so these kernels are FP64-issue bound and trade
-// memory for FP64 instructions: per-stage operator coefficients are computed
+// 5.6 B per FP64 flop), so these kernels are bound by FP64 issue and trade
+// memory and integer instructions for FP64 ones: the line contractions are
+// integer sums (igr_fix.cuh), per-stage operator coefficients are computed
 // once and re-read by every solver iteration, reciprocals of mesh constants
 // come precomputed from the host, the SIP face terms are folded into the
 // stiffness transpose, and out-of-tile (halo) work is packed into one warp
-// per phase (see elem_view) so that it is paid once per tile, converged.
+// per direction (see elem_view) so that it is paid once per tile, converged.
 #pragma once
 #include "igr_device.cuh"
 

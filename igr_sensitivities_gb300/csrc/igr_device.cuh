@@ -84,16 +84,6 @@ __device__ __forceinline__ void flag_nonfinite(int* status) {
   if (status) atomicOr(status, DEV_NONFINITE);
 }
 
-// Asynchronous copies of 8 bytes from global to shared memory (no register and
-// no scoreboard holds them; completion is waited for by group).
-__device__ __forceinline__ void copy_async8(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int PENDING>
-__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
-
 // Comparisons on bit patterns. GB300 issues a double compare (DSETP), fmax and
 // isfinite through the FP64 unit at ~94 cycles per warp instruction per SM
 // sub-partition (measured with a micro-probe; a DFMA takes ~64), while the

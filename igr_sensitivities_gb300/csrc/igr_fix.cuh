@@ -264,38 +264,6 @@ __device__ __forceinline__ void line_rows_acc(const BASIS& B, const FixScale& c,
                                               double* out) {
   line_op<NP, false, true, true>(B.fD, B.D, &c, v, acc, [](int) { return true; }, out);
 }
-// out[k] = c sum_i D[i][k] v[i]
-template <int NP, class BASIS>
-__device__ __forceinline__ void line_cols(const BASIS& B, const FixScale& c, const double* v, double* out) {
-  line_op<NP, true, true, true>(B.fD, B.D, &c, v, nullptr, [](int) { return false; }, out);
-}
-// out[k] = acc[k] (where has(k)) + sum_i D[i][k] v[i]
-template <int NP, class BASIS, class HAS>
-__device__ __forceinline__ void line_cols_acc(const BASIS& B, const double* v, const double* acc, HAS has, double* out) {
-  line_op<NP, true, true, false>(B.fD, B.D, nullptr, v, acc, has, out);
-}
-
-// sum_k D[last ? NP-1 : 0][k] v[k]: the bits of line_rows at that end node
-template <int NP, class BASIS>
-__device__ __forceinline__ double line_end(const BASIS& B, bool last, const double* v) {
-  const FixMat& F = B.fD;
-  const int m = fix::max_hi<NP>(v);
-  if (fix::out_of_range<NP>(m, v)) {
-    double s = 0.0;
-#pragma unroll
-    for (int k = 0; k < NP; ++k) s = fma(last ? B.D[NP - 1][k] : B.D[0][k], v[k], s);
-    return s;
-  }
-  const int e = max(m >> 20, fix::E_MIN);
-  fix::Limb x[NP];
-#pragma unroll
-  for (int k = 0; k < NP; ++k) x[k] = fix::limbs(v[k], e);
-  const long long G = fix::line_sum<NP>(
-      x, [&](int k) { return fix::Limb{last ? F.h[NP - 1][k] : F.h[0][k], last ? F.l[NP - 1][k] : F.l[0][k]}; },
-      [](int) { return true; }, 0);
-  return fix::to_double(G, e + F.s - 1);
-}
-
 // ---------------------------------------------------------------------------
 // A line of the SIP operator without leaving the integers: fluxes k (D x) and
 // their transposed contraction, so that neither the derivatives nor the fluxes
@@ -480,42 +448,6 @@ __device__ __forceinline__ void row_sums(const BASIS& B, const FixFlux<NP>& f, d
   for (int k = 0; k < NP; ++k) r.G[k] = __double_as_longlong(acc[k]);
 }
 
-// out[k] = acc[k] + sg (row part[k] + D^T(f + u)[k] + (a0 at node 0, aL at node NP-1)), sg = +-1, rounded once: the
-// column's share of the operator, the rows' sums R (units of exponent er, e < 0: doubles) and the caller's terms.
-template <int NP, class BASIS>
-__device__ __forceinline__ void column_sums(const BASIS& B, const FixFlux<NP>& f, double u0, double uL, double a0, double aL,
-                                            const long long* R, const int* er, const double* acc, int sg, double* out) {
-  int need = max(fix::abs_hi(a0), fix::abs_hi(aL)), el = er[0], eh = er[0];
-#pragma unroll
-  for (int k = 0; k < NP; ++k) {
-    need = max(need, fix::abs_hi(acc[k]));
-    el = el < er[k] ? el : er[k];
-    eh = max(eh, er[k]);
-  }
-  need = max(need >> 20, eh);
-  FixSums<NP> s;
-  if (el >= 0 && div_line<NP>(B, f, u0, uL, need, false, s)) {
-#pragma unroll
-    for (int k = 0; k < NP; ++k) {
-      long long v = s.G[k] + fix::sar(R[k], s.e - er[k]);
-      if (k == 0) v = fix::add<6>(v, a0, s.e);
-      if (k == NP - 1) v = fix::add<6>(v, aL, s.e);
-      out[k] = fix::to_double(fix::add<6>(sg > 0 ? v : -v, acc[k], s.e), s.e + 1);
-    }
-    return;
-  }
-  double y[NP];
-#pragma unroll
-  for (int k = 0; k < NP; ++k) {
-    y[k] = er[k] < 0 ? __longlong_as_double(R[k]) : fix::to_double(R[k], er[k] + 1);
-    if (k == 0) y[k] += a0;
-    if (k == NP - 1) y[k] += aL;
-  }
-  div_line_fp64<NP>(B, f, u0, uL, y);
-#pragma unroll
-  for (int k = 0; k < NP; ++k) out[k] = sg > 0 ? acc[k] + y[k] : acc[k] - y[k];
-}
-
 // Derivatives of a line: (D v)[i] = G[i] 2^(e - 1084), |G| < 2^62 and shifted up to use these bits; e = 0: a line of zeros; slow: the
 // bits of doubles.
 template <int NP>
@@ -637,10 +569,8 @@ __device__ __forceinline__ double node_blend(long long r, int er, long long c, i
 }
 
 // ---------------------------------------------------------------------------
-// A scaled line derivative (or its transpose, T) kept as integers between the phases, and the sum that ends it:
-//   row:    r = c (D v) + (a0 at node 0, aL at node NP-1)
-//   column: out = acc + row parts + c (D v)
-// in units of 2^60 / 2^(e - 1022); r.e < 0: the bits of doubles (FP64 lines).
+// A scaled line derivative (or its transpose, T) kept as integers, c (D v), with row_add_ends' terms at its end nodes,
+// in units of 2^60 / 2^(e - 1022); r.e < 0: the bits of doubles (FP64 lines). node_total and node_blend end the sums.
 // ---------------------------------------------------------------------------
 template <int NP, bool T, class BASIS>
 __device__ __forceinline__ bool scaled_line(const BASIS& B, const FixScale& c, const double* v, FixSums<NP>& r) {
@@ -709,34 +639,4 @@ __device__ __forceinline__ void row_add_ends(FixSums<NP>& r, double a0, double a
 #pragma unroll
   for (int i = 0; i < NP; ++i) r.G[i] = __double_as_longlong(s[i]);
 }
-template <int NP, bool T, class BASIS>
-__device__ __forceinline__ void column_scaled(const BASIS& B, const FixScale& c, const double* v, const long long* R,
-                                              const int* er, const double* acc, double* out) {
-  int need = 0, el = er[0], eh = er[0];
-#pragma unroll
-  for (int k = 0; k < NP; ++k) {
-    need = max(need, fix::abs_hi(acc[k]));
-    el = el < er[k] ? el : er[k];
-    eh = max(eh, er[k]);
-  }
-  need = max(need >> 20, eh);
-  FixSums<NP> s;
-  if (el >= 0 && scaled_line<NP, T>(B, c, v, s)) {
-    const int e = max(need, s.e);
-    if (e >= 128 && e < fix::E_MAX) {
-#pragma unroll
-      for (int k = 0; k < NP; ++k) {
-        const long long w = fix::sar(s.G[k], e - s.e) + fix::sar(R[k], e - er[k]);
-        out[k] = fix::to_double(fix::add<7>(w, acc[k], e), e);
-      }
-      return;
-    }
-  }
-  double y[NP];
-  scaled_line_fp64<NP, T>(B, c, v, y);
-#pragma unroll
-  for (int k = 0; k < NP; ++k)
-    out[k] = acc[k] + (y[k] + (er[k] < 0 ? __longlong_as_double(R[k]) : (er[k] == 0 ? 0.0 : fix::to_double(R[k], er[k]))));
-}
-
 }  // namespace igrgpu

@@ -67,7 +67,7 @@ template <int NP> static int run() {
   const Basis B = make(NP);
   int bad = 0;
   // T: transposed; S: scaled; acc: 0 none, 1 the end nodes, 2 all
-  auto check = [&](const char* name, bool T, bool S, int acc, bool end) {
+  auto check = [&](const char* name, bool T, bool S, int acc) {
     for (int kind = 0; kind <= 8; ++kind) {
       double worst = 0;
       bool ok = true;
@@ -79,24 +79,17 @@ template <int NP> static int run() {
         const double c = S ? (uni() < 0.5 ? -1 : 1) * std::ldexp(1 + uni(), (int)(24 * uni()) - 8) : 1.0;
         const FixScale f = fix_scale(c);
         auto has = [&](int k) { return acc == 2 || (acc == 1 && (k == 0 || k == NP - 1)); };
-        auto ends = [](int k) { return k == 0 || k == NP - 1; };
-        if (end) { out[0] = line_end<NP>(B, false, v); out[NP - 1] = line_end<NP>(B, true, v); }
-        else if (!T && !S) line_rows<NP>(B, v, out);
+        if (!T && !S) line_rows<NP>(B, v, out);
         else if (!T && S && !acc) line_rows<NP>(B, f, v, out);
         else if (!T && S) line_rows_acc<NP>(B, f, v, ac, out);
-        else if (T && S) line_cols<NP>(B, f, v, out);
-        else if (acc == 1) line_cols_acc<NP>(B, v, ac, ends, out);
-        else line_cols_acc<NP>(B, v, ac, [](int) { return true; }, out);
-        double rows[NP];
-        if (end) line_rows<NP>(B, v, rows);
+        else if (S) line_op<NP, true, true, true>(B.fD, B.D, &f, v, ac, has, out);
+        else line_op<NP, true, true, false>(B.fD, B.D, nullptr, v, ac, has, out);
         // the largest the sum's exponent can be, by the line and by the accumulands
         long double top = 0;
         for (int k = 0; k < NP; ++k) top = fmaxl(top, fabsl((long double)v[k]));
         top *= std::ldexp(fabs(c), B.fD.s);
         for (int k = 0; k < NP; ++k) if (has(k)) top = fmaxl(top, fabsl((long double)ac[k]));
         for (int i = 0; i < NP; ++i) {
-          if (end && i != 0 && i != NP - 1) continue;
-          if (end && std::memcmp(&out[i], &rows[i], 8)) ok = false;  // the halo's bits are the owner's
           long double s = 0;
           for (int k = 0; k < NP; ++k)
             if (!fix::skip<NP>(i, k)) s += (long double)(T ? B.D[k][i] : B.D[i][k]) * v[k];
@@ -123,13 +116,12 @@ template <int NP> static int run() {
       std::printf("NP%d %s kind%d %s %.3f\n", NP, name, kind, ok ? "ok" : "BAD", worst);
     }
   };
-  check("rows", false, false, 0, false);
-  check("rows_scaled", false, true, 0, false);
-  check("rows_scaled_acc", false, true, 2, false);
-  check("cols_scaled", true, true, 0, false);
-  check("cols_acc_ends", true, false, 1, false);
-  check("cols_acc", true, false, 2, false);
-  check("end", false, false, 0, true);
+  check("rows", false, false, 0);
+  check("rows_scaled", false, true, 0);
+  check("rows_scaled_acc", false, true, 2);
+  check("cols_scaled", true, true, 0);
+  check("cols_acc_ends", true, false, 1);
+  check("cols_acc", true, false, 2);
   // fluxes k (D x) and column sums acc +- (R + D^T (flux + u) + a)
   // kinds 9..12: smooth lines 1 + d (polynomial) of ever smaller variation, with the mass and row terms of such a field
   for (int kind = 0; kind <= 12; ++kind) {
@@ -188,7 +180,9 @@ template <int NP> static int run() {
         er[i] = r.e;
       }
       const int sg = uni() < 0.5 ? 1 : -1;
-      column_sums<NP>(B, f, u0, uL, a0, aL, R, er, acc, sg, out);
+      FixSums<NP> col;
+      row_sums<NP>(B, f, u0, uL, a0, aL, col);
+      for (int i = 0; i < NP; ++i) out[i] = node_total<59>(R[i], er[i], col.G[i], col.e, acc[i], sg);
       // the same in FP64, in the order of a chain of multiply-adds
       double c64[NP], s64[NP];
       for (int i = 0; i < NP; ++i) {
@@ -333,10 +327,10 @@ template <int NP> static int run() {
       bool ok = true;
       line_rows<NP>(B, v, out);
       for (int i = 0; i < NP; ++i) ok &= std::isfinite(out[i]) == fix::skip<NP>(i, at);
-      line_cols_acc<NP>(B, v, ac, [](int) { return true; }, out);
+      line_op<NP, true, true, false>(B.fD, B.D, nullptr, v, ac, [](int) { return true; }, out);
       for (int i = 0; i < NP; ++i) ok &= std::isfinite(out[i]) == fix::skip<NP>(i, at);
       v[at] = 0.25; ac[at] = x;
-      line_cols_acc<NP>(B, v, ac, [](int) { return true; }, out);
+      line_op<NP, true, true, false>(B.fD, B.D, nullptr, v, ac, [](int) { return true; }, out);
       for (int i = 0; i < NP; ++i) ok &= std::isfinite(out[i]) == (i != at);
       bad += !ok;
       std::printf("NP%d nonfinite%d %s 0\n", NP, at, ok ? "ok" : "BAD");
