@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(2 * Tiling2D<NP>::NH) k2_setup(SetupArgs2D a) 
     a.cky[n] = s_c[2][nd] * ir;
     a.cpx[n] = i == 0 || i == L ? s_f[0][el][j][i == L] : 0.0;
     a.cpy[n] = j == 0 || j == L ? s_f[1][el][i][j == L] : 0.0;
-    a.cinvM[n] = reciprocal(M);
+    a.cinvM[n] = 1.0 / M;
     if (a.cM) a.cM[n] = M;
   }
 }
@@ -546,7 +546,7 @@ __device__ __forceinline__ NodePhys node_phys(double g, double mx, double my, do
 }
 // |u_n| + c, c = sqrt(gamma P / rho)
 __device__ __forceinline__ double wavespeed(double g, double un, double P, double ir) {
-  return fabs(un) + square_root(g * P * ir);
+  return fabs(un) + sqrt(g * P * ir);
 }
 
 // x[v] of an array in registers
@@ -755,7 +755,7 @@ struct EulerStage {
   __device__ __forceinline__ void put(int v, long long n, double x) const {
     if (a.k_out[v]) a.k_out[v][n] = x;
     if (a.qo[v]) a.qo[v][n] = x;
-    if (v == 2 && a.invro) a.invro[n] = reciprocal(x);
+    if (v == 2 && a.invro) a.invro[n] = 1.0 / x;
     if (a.status && (v == 2 ? not_positive_finite(x) : nonfinite_bits(x))) flag_nonfinite(a.status);
   }
 };

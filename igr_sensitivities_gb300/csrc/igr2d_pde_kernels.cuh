@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_pde_prep(PdePrepArgs2D a)
     for (int i = 0; i < NP; ++i) {
       const long long n = vr.base + t * NP + i;
       const int nd = t * NP + i;
-      const double mx = a.q[0][n], my = a.q[1][n], r = a.q[2][n], ir = reciprocal(r);
+      const double mx = a.q[0][n], my = a.q[1][n], r = a.q[2][n], ir = 1.0 / r;
       s_ir[e][nd] = ir;
       s_dy[0][e][nd] = mx; s_dy[1][e][nd] = my; s_dy[2][e][nd] = r; s_dy[3][e][nd] = a.q[3][n]; s_dy[4][e][nd] = a.S[n];
       s_dy[5][e][nd] = mx * ir; s_dy[6][e][nd] = my * ir;
@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_pde_prep(PdePrepArgs2D a)
     a.src[0][n] = c0; a.src[1][n] = c1; a.src[2][n] = c2; a.src[3][n] = c3; a.src[4][n] = c4;
     a.src[5][n] = c5; a.src[6][n] = c6; a.src[7][n] = c7; a.src[8][n] = c8; a.src[9][n] = c9;
     a.invr[n] = ir;
-    const double cs = square_root(g * P * ir);
+    const double cs = sqrt(g * P * ir);
     a.ws_x[n] = fabs(ux) + cs;
     a.ws_y[n] = fabs(uy) + cs;
     if (a.nl[0]) {

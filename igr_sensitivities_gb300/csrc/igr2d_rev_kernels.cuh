@@ -72,7 +72,7 @@ __device__ __forceinline__ double wavespeed_rev(double g, double gs, double mn, 
   gb = fma(Y, gs, gb);
   qn += t;
   qr = fma(-Y, ir, fma(-t, un, qr));
-  return (h * reciprocal(c)) * ((g * (g - 1.0)) * ir);
+  return (h / c) * ((g * (g - 1.0)) * ir);
 }
 
 enum { SREV_NONE = 0, SREV_CHEB = 1, SREV_JACOBI = 2, SREV_PCG = 3 };

@@ -103,47 +103,6 @@ __device__ __forceinline__ bool not_positive_finite(double x) {
   return __double_as_longlong(x) <= 0 || nonfinite_bits(x);
 }
 
-// Reciprocal and square root of positive normal doubles from the 24-bit
-// approximations of the FP32 units: one iteration of third order for 1/x
-// (y (1 + e + e^2), e = 1 - x y), one Newton step and one residual correction
-// for sqrt. 3 and 5 FP64 instructions against 5.5 and 10 of 1.0 / x and
-// sqrt(x); within 0.51 ulp of the exact value (the residual terms are below
-// 2^-66). Everything else (zero, negative, subnormal, infinite, NaN and the
-// ends of the exponent range) takes the IEEE operation.
-__device__ __forceinline__ float mantissa_to_float(int hi, int lo) {  // of a double in [1, 4)
-  return __int_as_float((int)(__funnelshift_l((unsigned)lo, (unsigned)hi, 3) - (896u << 23)));
-}
-__device__ __forceinline__ double widen(float f) {  // positive, normal
-  const unsigned b = __float_as_uint(f);
-  return __hiloint2double((int)((b >> 3) + (896u << 20)), (int)(b << 29));
-}
-__device__ __forceinline__ double reciprocal(double x) {
-  const int hi = __double2hiint(x), lo = __double2loint(x);
-  if ((unsigned)(hi - (64 << 20)) >= (unsigned)(1919 << 20)) return 1.0 / x;
-  const int ex = (hi & 0x7ff00000) - 0x3ff00000;
-  const double m = __hiloint2double(hi - ex, lo);  // [1, 2)
-  float f;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(f) : "f"(mantissa_to_float(hi - ex, lo)));
-  const double y = widen(f);
-  const double e = fma(-m, y, 1.0);
-  const double r = fma(y, fma(e, e, e), y);
-  return __hiloint2double(__double2hiint(r) - ex, __double2loint(r));
-}
-__device__ __forceinline__ double square_root(double x) {
-  const int hi = __double2hiint(x), lo = __double2loint(x);
-  if ((unsigned)(hi - (64 << 20)) >= (unsigned)(1919 << 20)) return sqrt(x);
-  const int ex = ((hi & 0x7ff00000) - 0x3ff00000) & ~0x1fffff;  // an even power of two
-  const double m = __hiloint2double(hi - ex, lo);               // [1, 4)
-  float f;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(f) : "f"(mantissa_to_float(hi - ex, lo)));
-  const double y = widen(f);
-  const double h = __hiloint2double(__double2hiint(y) - (1 << 20), __double2loint(y));  // y / 2
-  double g = m * y;
-  g = fma(g, fma(-g, h, 0.5), g);
-  g = fma(fma(-g, g, m), h, g);
-  return __hiloint2double(__double2hiint(g) + (ex >> 1), __double2loint(g));
-}
-
 // The last levels of a pairwise tree whose 32 (or fewer) remaining values sit
 // in the lanes of one warp: lane v adds lane v + w for w = W/2 .. 1, the pairs
 // (and so the bits) of the shared-memory tree; lane 0 ends with the sum.
