@@ -67,6 +67,7 @@ inline FixMat make_fix(const double A[FIX_MAXNP][FIX_MAXNP], int np) {
 namespace fix {
 
 constexpr int E_MIN = 128, E_MAX = 2030;  // biased exponents the integer path takes
+constexpr int E_FLUX = 96;                // and the least of a flux
 
 // One instruction each on the GPU; the C forms serve host builds of this header (the unit test).
 __device__ __forceinline__ long long mad(int a, int b, long long c) {
@@ -313,17 +314,19 @@ __device__ __forceinline__ bool plain_coef(int k_hi) { return (unsigned)(k_hi - 
 template <int NP, class BASIS>
 __device__ __forceinline__ void flux_line(const BASIS& B, const double* x, const double* k, FixFlux<NP>& f) {
   const int m = fix::max_hi<NP>(x);
-  int ke[NP], km = 0;
+  int ke[NP], km = 0, kn = 0x7fffffff;
   bool ok = true;
 #pragma unroll
   for (int i = 0; i < NP; ++i) {
     ke[i] = fix::abs_hi(k[i]);
     ok &= fix::plain_coef(ke[i]);
     km = max(km, ke[i]);
+    kn = min(kn, ke[i]);
   }
   const int ex = max(m >> 20, fix::E_MIN);
   const int eg = ex + B.fD.s - 1022;  // P_i before alignment has exponent eg + ke_i
-  f.slow = fix::out_of_range<NP>(m, x) || !ok || (unsigned)(eg + (km >> 20) - 64) >= (unsigned)(fix::E_MAX - 64);
+  // Every P_i, and the line's after its shift by up to 30 below, stays where to_double's exponent cannot pass below zero.
+  f.slow = fix::out_of_range<NP>(m, x) || !ok || eg + (kn >> 20) < fix::E_FLUX || eg + (km >> 20) >= fix::E_MAX;
   if (f.slow) {
     f.e = 0;
 #pragma unroll
@@ -367,7 +370,7 @@ template <int NP, class BASIS>
 __device__ __forceinline__ double flux_end(const BASIS& B, bool last, const double* x, double k) {
   const int m = fix::max_hi<NP>(x), ke = fix::abs_hi(k);
   const int ex = max(m >> 20, fix::E_MIN), e = ex + B.fD.s - 1022 + (ke >> 20);
-  if (fix::out_of_range<NP>(m, x) || !fix::plain_coef(ke) || (unsigned)(e - 64) >= (unsigned)(fix::E_MAX - 64)) {
+  if (fix::out_of_range<NP>(m, x) || !fix::plain_coef(ke) || (unsigned)(e - fix::E_FLUX) >= (unsigned)(fix::E_MAX - fix::E_FLUX)) {
     double s = 0.0;
 #pragma unroll
     for (int j = 0; j < NP; ++j) s = fma(last ? B.D[NP - 1][j] : B.D[0][j], x[j], s);
