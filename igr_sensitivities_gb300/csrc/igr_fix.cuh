@@ -10,21 +10,28 @@
 // per SM). P4 lines: 1673 against 547.
 //
 // Representation: the values of one line share the exponent e of their largest
-// member and become integers |X| < 2^62, split as X = h 2^32 + 2 l with |h| <
-// 2^30 and |l| < 2^31; the matrix is scaled by a power of two so that no row or
-// column has an absolute sum above 0.7, and stored the same way with a balanced
-// l (|l| <= 2^30). A product then takes three 32 x 32 -> 64 bit multiply-adds
-// (h h, h l, l h), whose sums over at most five terms stay below 2^63:
+// member and become integers |X| < 2^62, split as X = h 2^32 + 2 l with |h| <=
+// 2^30 and a balanced l (|l| <= 2^30); the matrix is scaled by a power of two so
+// that no row or column has an absolute sum above 0.7, and stored the same way.
+// A product then takes three 32 x 32 -> 64 bit multiply-adds (h h, h l, l h),
+// whose sums over at most five terms stay below 2^63:
 //   H = sum h_D h_X,  M = sum (h_D l_X + l_D h_X),  G = H + M / 2^31.
 // The low x low products and the truncation of the line's values are a few units
-// of 2^-61 of the line's scale, and one rounding to nearest ends the sum: against
-// 128-bit sums the results are off by 3.3e-17 rms of |D||x| where the FP64 chain
-// is off by 4.5e-17. A whole SIP line (flux, transposed contraction, mass and
-// face terms) has 0.2 to 0.7 times the chain's rms error (tests/test_fixed_point.py).
+// of 2^-61 of the line's scale, and one rounding to nearest ends the sum: over
+// random lines the results are off by 3.6e-17 rms of |D||x| where the FP64 chain
+// is off by 4.8e-17. A whole SIP line (flux, transposed contraction, mass and
+// face terms) has 0.2 to 0.85 times the chain's rms error (tests/test_fixed_point.py).
+// No step has a mean error (ties and inexact shifts go to the odd neighbour, low
+// words are balanced): a mean of half a unit, invisible in any field, made
+// dJ/dalpha, a sum over the mesh, the stages and the iterations with a cancellation
+// of 1e3 to 1e6, 2 to 60 times less exact than the FP64 chain's
+// (tests/test_gpu_long_double.py). The cycles above were measured before that; it
+// costs 8% of k2_apply and k2_apply_rev.
 //
 // Lines that hold infinities, NaN or values beyond 2^1007, and lines of nothing
 // but subnormal-range values (below 2^-894), take the FP64 chain, as before. A
-// line of zeros gives zeros.
+// line of zeros gives zeros, a negated line the negated result to the bit (but for a
+// tie of 32 low bits).
 #pragma once
 #include <cmath>
 
@@ -89,46 +96,69 @@ __device__ __forceinline__ unsigned long long shr(unsigned long long a, unsigned
   return s > 63 ? 0 : a >> s;
 #endif
 }
+// 1 where a / 2^s is inexact, else 0; lo is a's low word, which stands for all that a shift beyond 32 bits drops
+__device__ __forceinline__ unsigned inexact(unsigned lo, unsigned s) {
+#ifdef __CUDA_ARCH__
+  unsigned mask;
+  asm("bmsk.clamp.b32 %0, 0, %1;" : "=r"(mask) : "r"(s));  // the low s bits
+  return min(lo & mask, 1u);
+#else
+  return s != 0 && lo << (s > 32 ? 0 : 32 - s) != 0;
+#endif
+}
 __device__ __forceinline__ int abs_hi(double v) { return __double2hiint(v) & 0x7fffffff; }
 
-// |v| 2^(53 + PRE) / 2^(e - 1022), truncated; e is a biased exponent >= v's
-template <int PRE>
+// |v| 2^(53 + PRE) / 2^(e - 1022), truncated or (ODD) to the odd neighbour; e is a biased exponent >= v's
+template <int PRE, bool ODD = false>
 __device__ __forceinline__ unsigned long long magnitude(double v, int e) {
   const unsigned hi = __double2hiint(v), lo = __double2loint(v);
   const unsigned m = (hi & 0xfffffu) | 0x100000u;
   const unsigned long long t = ((unsigned long long)__funnelshift_l(lo, m, PRE) << 32) | (lo << PRE);
-  return shr(t, e - ((hi & 0x7fffffffu) >> 20));
+  const unsigned s = e - ((hi & 0x7fffffffu) >> 20);
+  return shr(t, s) | (ODD ? inexact((unsigned)t, s) : 0);
 }
 
+// A product drops l l of its two factors. One of them always has a balanced l (|l| <= 2^30, no mean): a mean would add up over the
+// nodes and iterations behind a sum such as dJ/dalpha. The last bit of an odd t goes to the odd neighbour, like sar's (even():
+// t is even, or a magnitude whose last bits are zero but for values far below the line's largest).
 struct Limb { int h, l; };
-// v 2^(53 + PRE) / 2^(e - 1022) as h 2^32 + 2 l
-template <int PRE = 9>
+__device__ __forceinline__ Limb even(long long t) { return {(int)((t + (1LL << 31)) >> 32), (int)(unsigned)t >> 1}; }
+__device__ __forceinline__ Limb balanced(long long t) {
+  const Limb x = even(t);
+  return {x.h, x.l | ((int)(unsigned)t & 1)};
+}
+// v 2^62 / 2^(e - 1022) as h 2^32 + 2 l, l balanced
 __device__ __forceinline__ Limb limbs(double v, int e) {
-  const unsigned long long t = magnitude<PRE>(v, e);
+  const Limb t = even((long long)magnitude<9>(v, e));
+  const int sg = (__double2hiint(v) >> 31) | 1;
+  return {t.h * sg, t.l * sg};
+}
+// v 2^63 / 2^(e - 1022) as h 2^32 + 2 l, l of v's sign
+__device__ __forceinline__ Limb factor(double v, int e) {
+  const unsigned long long t = magnitude<10>(v, e);
   const int sg = (__double2hiint(v) >> 31) | 1;
   return {(int)(t >> 32) * sg, (int)((unsigned)t >> 1) * sg};
 }
-// a + v, v in units of 2^(53 + PRE) / 2^(e - 1022), rounded to nearest: addends come back in the next solver iteration
-// or are summed over the mesh, where a truncation's bias would add up.
+// a + v, v in units of 2^(53 + PRE) / 2^(e - 1022), an inexact v to the odd neighbour (see sar)
 template <int PRE>
 __device__ __forceinline__ long long add(long long a, double v, int e) {
   const long long s = __double2hiint(v) >> 31;
-  const long long t = (long long)((magnitude<PRE + 1>(v, e) + 1) >> 1);
-  return a + (t ^ s) - s;
+  return a + ((long long)magnitude<PRE, true>(v, e) ^ s) - s;
 }
 
-// G 2^(e - 1082) rounded to nearest, |G| < 2^62
+// G 2^(e - 1082) rounded to nearest, ties to even, |G| < 2^62
 __device__ __forceinline__ double to_double(long long G, int e) {
-  const int gh = (int)(G >> 32), sg = gh >> 31;
-  const unsigned mh = gh ^ sg, ml = (unsigned)G ^ sg;
+  const long long sg = G >> 63;
+  const unsigned long long a = (unsigned long long)((G ^ sg) - sg);
+  const unsigned mh = (unsigned)(a >> 32);
   const bool z = mh == 0;
-  const unsigned m = z ? ml : mh;
+  const unsigned m = z ? (unsigned)a : mh;
   int lz = __clz(m);
   lz = z ? lz + 32 : lz;
-  unsigned long long t = (((unsigned long long)mh << 32) | ml) << (lz - 1);  // leading bit 62
-  t += 0x200;
+  unsigned long long t = a << (lz - 1);  // leading bit 62
+  t += 0x1ff + ((unsigned)(t >> 10) & 1);
   unsigned hi = (unsigned)(t >> 42) + (unsigned)((e + 3 - lz) << 20);  // the implicit bit adds one to the exponent
-  hi |= gh & 0x80000000;
+  hi |= (unsigned)(sg & 0x80000000);
   return __hiloint2double(m ? hi : 0, (unsigned)(t >> 10));
 }
 
@@ -164,7 +194,9 @@ constexpr long long HALF = 1LL << 31;  // M / 2^31 is added as 2 (M >> 32): roun
 // One sum of a line: coefficient (h, l)[k] by index function cf(k) -> Limb, over the terms keep(k) lets through
 template <int NP, class CF, class KEEP>
 __device__ __forceinline__ long long line_sum(const Limb* x, CF cf, KEEP keep, long long acc) {
-  long long H = acc, M = HALF;
+  // P2's matrix has few bits: one in 32 of its M is a tie. The line's first value says which way these go, by its last bit
+  // and its sign (so that the negated line gives the negated sum).
+  long long H = acc, M = NP == 3 ? HALF - 1 + ((x[0].h ^ (x[0].h >> 31)) & 1) : HALF;
 #pragma unroll
   for (int k = 0; k < NP; ++k) {
     if (!keep(k)) continue;
@@ -174,6 +206,13 @@ __device__ __forceinline__ long long line_sum(const Limb* x, CF cf, KEEP keep, l
     M = mad(c.l, x[k].h, M);
   }
   return mad((int)(M >> 32), 2, H);
+}
+
+// acc + G c / 2^64 for |G| < 2^62 and c of 63 bits
+__device__ __forceinline__ long long times(long long G, Limb c, long long acc = 0) {
+  const Limb g = balanced(G);
+  const long long M = mad(g.l, c.h, mad(g.h, c.l, HALF));
+  return mad((int)(M >> 32), 2, mad(g.h, c.h, acc));
 }
 
 }  // namespace fix
@@ -188,7 +227,7 @@ __device__ __forceinline__ FixScale fix_scale(double d) {
   FixScale s;
   s.d = d;
   s.e = fix::abs_hi(d) >> 20;
-  s.m = fix::limbs<10>(d, s.e);
+  s.m = fix::factor(d, s.e);
   return s;
 }
 
@@ -240,11 +279,7 @@ __device__ __forceinline__ void line_op(const FixMat& F, const MAT& A, const Fix
     long long G = fix::line_sum<NP>(
         x, [&](int k) { return fix::Limb{T ? F.h[k][i] : F.h[i][k], T ? F.l[k][i] : F.l[i][k]}; },
         [&](int k) { return !(SKIP && fix::skip<NP>(i, k)); }, SCALED ? 0 : A0);
-    if (SCALED) {
-      const int gh = (int)(G >> 32), gl = (int)((unsigned)G >> 1);
-      const long long M = fix::mad(gl, c->m.h, fix::mad(gh, c->m.l, fix::HALF));
-      G = fix::mad((int)(M >> 32), 2, fix::mad(gh, c->m.h, A0));
-    }
+    if (SCALED) G = fix::times(G, c->m, A0);
     out[i] = fix::to_double(G, e + up - (SCALED ? 0 : 1));
   }
 }
@@ -289,22 +324,16 @@ __device__ __forceinline__ Limb mantissa(double v) {
   const int sg = ((int)hi >> 31) | 1;
   return {(int)__funnelshift_l(lo, (hi & 0xfffffu) | 0x100000u, 10) * sg, (int)((lo << 9) & 0x7fffffffu) * sg};
 }
-// A dropped product of two low words of one sign is a quarter unit on average; M carries it.
-constexpr long long LOW = 1LL << 29;
-// G c / 2^64 for |G| < 2^62 and c of 63 bits
-__device__ __forceinline__ long long times(long long G, Limb c) {
-  const int gh = (int)(G >> 32), gl = (int)((unsigned)G >> 1);
-  const long long M = mad(gl, c.h, mad(gh, c.l, HALF + (c.h < 0 ? -LOW : LOW)));
-  return mad((int)(M >> 32), 2, mad(gh, c.h, 0));
-}
+// a / 2^s, an inexact result rounded to its odd neighbour: as a floor it would be low by half a unit on average, which adds up
+// over the nodes and iterations behind a sum such as dJ/dalpha (2 to 60 times the FP64 chain's error there).
 __device__ __forceinline__ long long sar(long long a, unsigned s) {
 #ifdef __CUDA_ARCH__
   long long r;
   asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"(a), "r"(s));
-  return r;
 #else
-  return a >> (s > 63 ? 63 : s);
+  const long long r = a >> (s > 63 ? 63 : s);
 #endif
+  return r | inexact((unsigned)a, s);
 }
 __device__ __forceinline__ bool zero(double v) { return (((unsigned)abs_hi(v)) | (unsigned)__double2loint(v)) == 0; }
 // k is a coefficient the integer path takes: nonzero, finite, of moderate exponent
@@ -349,9 +378,12 @@ __device__ __forceinline__ void flux_line(const BASIS& B, const double* x, const
   for (int i = 0; i < NP; ++i) {
     const long long G = fix::line_sum<NP>(
         X, [&](int j) { return fix::Limb{B.fD.h[i][j], B.fD.l[i][j]}; }, [&](int j) { return !fix::skip<NP>(i, j); }, 0);
+    if (i > 0 && i < NP - 1) {  // k in units of the line's largest: 63 bits, exact down to 2^-10 of it
+      f.P[i] = fix::times(G, fix::factor(k[i], km >> 20));
+      continue;
+    }
     const long long P = fix::times(G, fix::mantissa(k[i]));
-    if (i == 0) f.t0 = fix::to_double(P, eg + (ke[i] >> 20));
-    if (i == NP - 1) f.tL = fix::to_double(P, eg + (ke[i] >> 20));
+    (i == 0 ? f.t0 : f.tL) = fix::to_double(P, eg + (ke[i] >> 20));
     f.P[i] = fix::sar(P, (km >> 20) - (ke[i] >> 20));
   }
   // A smooth line's fluxes are far below what its values allow: shifted up to use their bits, so that the units of the
@@ -406,10 +438,10 @@ __device__ __forceinline__ bool div_line(const BASIS& B, const FixFlux<NP>& f, d
   fix::Limb S[NP];
 #pragma unroll
   for (int i = 0; i < NP; ++i) {
-    long long v = fix::sar(f.P[i], e - sd - f.e + 2);
-    if (i == 0) v = fix::add<7>(v, u0, e - sd);
-    if (i == NP - 1) v = fix::add<7>(v, uL, e - sd);
-    S[i] = {(int)(v >> 32), (int)((unsigned)v >> 1)};
+    long long v = fix::sar(f.P[i], e - sd - f.e + 3);
+    if (i == 0) v = fix::add<6>(v, u0, e - sd);
+    if (i == NP - 1) v = fix::add<6>(v, uL, e - sd);
+    S[i] = fix::even(2 * v);
   }
 #pragma unroll
   for (int k = 0; k < NP; ++k)
@@ -515,10 +547,9 @@ __device__ __forceinline__ bool product_line(const FixFlux<NP>& f, const FixDeri
   r.e = e;
 #pragma unroll
   for (int i = 0; i < NP; ++i) {
-    const int ph = (int)(f.P[i] >> 32), pl = (int)((unsigned)f.P[i] >> 1);
-    const int gh = (int)(d.G[i] >> 32), gl = (int)((unsigned)d.G[i] >> 1);
-    const long long M = fix::mad(ph, gl, fix::mad(pl, gh, fix::HALF + fix::LOW));
-    long long v = fix::sar(fix::mad((int)(M >> 32), 2, fix::mad(ph, gh, 0)), e - ep);
+    const fix::Limb p = fix::balanced(f.P[i]), g = fix::balanced(d.G[i]);
+    const long long M = fix::mad(p.h, g.l, fix::mad(p.l, g.h, fix::HALF));
+    long long v = fix::sar(fix::mad((int)(M >> 32), 2, fix::mad(p.h, g.h, 0)), e - ep);
     if (i == 0) v = fix::add<7>(v, z0, e);
     if (i == NP - 1) v = fix::add<7>(v, zL, e);
     r.G[i] = v;
@@ -555,7 +586,8 @@ __device__ __forceinline__ double node_total(long long r, int er, long long c, i
 // c v in units of 2^62 / 2^(e - 1022), e = exponent of v + that of c - 1022 (v normal, c.e of FixScale)
 __device__ __forceinline__ long long weighted(double v, const FixScale& c) {
   const fix::Limb x = fix::mantissa(v);
-  const long long M = fix::mad(x.h, c.m.l, fix::mad(x.l, c.m.h, fix::HALF));
+  // plus the mean of the dropped product of the low words, both of their factor's sign
+  const long long M = fix::mad(x.h, c.m.l, fix::mad(x.l, c.m.h, fix::HALF + (x.h < 0 ? -(c.m.l >> 1) : c.m.l >> 1)));
   return fix::mad((int)(M >> 32), 2, fix::mad(x.h, c.m.h, 0));
 }
 // a qa + b qb + row + column at one node (units of 2^60; see node_total), rounded once; 0 < a, b <= 1
@@ -565,7 +597,7 @@ __device__ __forceinline__ double node_blend(long long r, int er, long long c, i
   const int e = max(max(er, ec), max(xa, xb));
   if (er >= 0 && ec >= 0 && e >= 128 && e < fix::E_MAX) {
     long long v = fix::sar(r, e - er) + fix::sar(c, e - ec);
-    v += fix::sar(weighted(qa, a), min(e - (xa + a.e - 1022) + 2, 63)) + fix::sar(weighted(qb, b), min(e - (xb + b.e - 1022) + 2, 63));
+    v += fix::sar(weighted(qa, a), e - (xa + a.e - 1022) + 2) + fix::sar(weighted(qb, b), e - (xb + b.e - 1022) + 2);
     return fix::to_double(v, e);
   }
   return node_total<60>(r, er, c, ec, fma(b.d, qb, a.d * qa), 1);

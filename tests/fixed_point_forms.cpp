@@ -3,6 +3,7 @@
 #define main fixed_point_main
 #include "fixed_point_check.cpp"
 #undef main
+#include <type_traits>
 
 static int report(const char* name, int np, bool ok, double worst) {
   std::printf("%s NP%d %s %.3g\n", name, np, ok ? "ok" : "BAD", worst);
@@ -48,8 +49,131 @@ template <int NP> static int flux_range() {
   return report("flux_range", NP, worst <= 1, worst);
 }
 
+// The matrices of the kernels' forms: D, D with the own side's share of the face corrections, W2 = w D^2 elementwise.
+struct Full { double D[FIX_MAXNP][FIX_MAXNP], Dr[FIX_MAXNP][FIX_MAXNP], W2[FIX_MAXNP][FIX_MAXNP]; FixMat fD, fDr, fW2; };
+static Full full(int np) {
+  const Basis B = make(np);
+  const double w[6][5] = {{0}, {0}, {1, 1}, {1. / 3, 4. / 3, 1. / 3}, {1. / 6, 5. / 6, 5. / 6, 1. / 6}, {.1, 49. / 90, 32. / 45, 49. / 90, .1}};
+  Full F = {};
+  std::memcpy(F.D, B.D, sizeof(F.D));
+  std::memcpy(F.Dr, B.D, sizeof(F.D));
+  F.Dr[0][0] += 0.5 / w[np][0];
+  F.Dr[np - 1][np - 1] -= 0.5 / w[np][np - 1];
+  for (int i = 0; i < np; ++i) for (int k = 0; k < np; ++k) F.W2[i][k] = w[np][i] * (B.D[i][k] * B.D[i][k]);
+  F.fD = make_fix(F.D, np); F.fDr = make_fix(F.Dr, np); F.fW2 = make_fix(F.W2, np);
+  return F;
+}
+
+// No result is high or low on average: the mean error over random lines stays within five standard errors of zero.
+template <int NP> static int mean() {
+  if (NP == 2) return 0;
+  const Full B = full(NP);
+  int bad = 0;
+  const int n = 200000;
+  const char* forms[] = {"conversion", "scaled", "deriv", "flux", "operator", "products", "stage"};
+  for (int kind = 0; kind < 3; ++kind) {  // both signs; positive; a slope with noise, v against x
+    long double s1[7] = {}, s2[7] = {};
+    for (int it = 0; it < n; ++it) {
+      double x[NP], v[NP], k[NP], out[NP];
+      for (int i = 0; i < NP; ++i) {
+        const double s = 2.0 * i / (NP - 1) - 1, u = uni();
+        x[i] = kind == 0 ? 2 * u - 1 : (kind == 1 ? 1 + u : 1 + 0.3 * s + 1e-3 * u);
+        v[i] = kind == 0 ? 2 * uni() - 1 : (kind == 1 ? 1 + uni() : -0.7 * x[i] + 1e-3 * uni());
+        k[i] = 1e-4 * (1 + 0.3 * uni());
+      }
+      const int at = it % NP, other = (at + 1) % NP;
+      auto contract = [&](bool T, int i, const long double* a) {
+        long double r = 0;
+        for (int j = 0; j < NP; ++j) if (!fix::skip<NP>(i, j)) r += (long double)(T ? B.D[j][i] : B.D[i][j]) * a[j];
+        return r;
+      };
+      long double X[NP], V[NP], P[NP];
+      for (int i = 0; i < NP; ++i) { X[i] = x[i]; V[i] = v[i]; }
+      for (int i = 0; i < NP; ++i) P[i] = contract(false, i, X) * k[i];
+      const FixScale c = fix_scale(3.7 + uni());
+      FixFlux<NP> f;
+      FixDeriv<NP> d;
+      FixSums<NP> y, z, q;
+      line_op<NP, true, true, true>(B.fD, B.D, &c, v, nullptr, [](int) { return false; }, out);
+      flux_line<NP>(B, x, k, f);
+      deriv_line<NP>(B, v, d);
+      row_sums<NP>(B, f, 0.0, 0.0, 0.0, 0.0, y);
+      row_products<NP>(f, d, 0.0, 0.0, z);
+      row_scaled<NP, false>(B, c, v, q);
+      const double m = 1e-5 * (1 + uni()) * x[at], zs = 1e-4 * (2 * uni() - 1), qa = 100 + uni(), qb = 100 + uni();
+      const FixScale wa = fix_scale(0.25), wb = fix_scale(0.75);
+      const long long G = (long long)rs >> (2 + it % 9);
+      const long double e[7] = {
+          fix::to_double(G, 1082) - (long double)G,
+          out[at] - contract(true, at, V) * c.d,
+          deriv_at<NP>(d, at) - contract(false, at, V),
+          flux_at<NP>(f, at) - P[at],
+          node_total<59>(y.G[at], y.e, y.G[other], y.e, m, 1) - (contract(true, at, P) + contract(true, other, P) + m),
+          node_total<60>(z.G[at], z.e, z.G[other], z.e, zs, -1) - (zs - P[at] * contract(false, at, V) - P[other] * contract(false, other, V)),
+          node_blend(q.G[at], q.e, q.G[other], q.e, qa, wa, qb, wb) -
+              (0.25L * qa + 0.75L * qb + c.d * (contract(false, at, V) + contract(false, other, V)))};
+      for (int j = 0; j < 7; ++j) { s1[j] += e[j]; s2[j] += e[j] * e[j]; }
+    }
+    for (int j = 0; j < 7; ++j) {
+      const double sigma = s2[j] > 0 ? (double)(fabsl(s1[j]) / std::sqrt((double)s2[j])) : 0;
+      char name[64];
+      std::snprintf(name, sizeof(name), "mean %s kind%d", forms[j], kind);
+      bad += report(name, NP, sigma <= 5, sigma);
+    }
+  }
+  return bad;
+}
+
+// A negated operand gives the negated result to the bit.
+template <int NP> static int odd() {
+  const Basis B = make(NP);
+  int differ = 0;
+  for (int it = 0; it < 40000; ++it) {
+    double x[NP], y[NP], k[NP], v[NP], a[NP], b[NP];
+    const double m = 1e-5 * uni(), wide = it % 2 ? 20 : 0;
+    for (int i = 0; i < NP; ++i) {
+      x[i] = (2 * uni() - 1) * std::ldexp(1.0, (int)(wide * uni()));
+      y[i] = -x[i];
+      k[i] = 1e-4 * (1 + uni());
+      v[i] = 2 * uni() - 1;
+    }
+    const FixScale c = fix_scale(1 + uni());
+    FixFlux<NP> f, g;
+    FixDeriv<NP> d;
+    FixSums<NP> r, s;
+    line_rows<NP>(B, c, x, a);
+    line_rows<NP>(B, c, y, b);
+    for (int i = 0; i < NP; ++i) differ += a[i] != -b[i];
+    flux_line<NP>(B, x, k, f);
+    flux_line<NP>(B, y, k, g);
+    deriv_line<NP>(B, v, d);
+    differ += (f.t0 != -g.t0) + (f.tL != -g.tL);
+    auto compare = [&](auto units) {
+      constexpr int U = decltype(units)::value;
+      for (int i = 0; i < NP; ++i) {
+        const int j = (i + 1) % NP;
+        differ += node_total<U>(r.G[i], r.e, r.G[j], r.e, m, 1) != -node_total<U>(s.G[i], s.e, s.G[j], s.e, -m, 1);
+      }
+    };
+    row_sums<NP>(B, f, m, -m, x[0] * m, m, r);
+    row_sums<NP>(B, g, -m, m, y[0] * m, -m, s);
+    compare(std::integral_constant<int, 59>());
+    row_products<NP>(f, d, m, x[0] * m, r);
+    row_products<NP>(g, d, -m, y[0] * m, s);
+    compare(std::integral_constant<int, 60>());
+    row_scaled<NP, true>(B, c, x, r);
+    row_add_ends<NP>(r, m, x[0] * m);
+    row_scaled<NP, true>(B, c, y, s);
+    row_add_ends<NP>(s, -m, y[0] * m);
+    compare(std::integral_constant<int, 60>());
+  }
+  return report("odd", NP, differ == 0, differ);
+}
+
 template <int NP> static int run_one(const char* name) {
   if (!std::strcmp(name, "flux_range")) return flux_range<NP>();
+  if (!std::strcmp(name, "mean")) return mean<NP>();
+  if (!std::strcmp(name, "odd")) return odd<NP>();
   return 1;
 }
 
