@@ -340,6 +340,27 @@ __device__ __forceinline__ bool zero(double v) { return (((unsigned)abs_hi(v)) |
 __device__ __forceinline__ bool plain_coef(int k_hi) { return (unsigned)(k_hi - (523 << 20)) < (unsigned)(1000 << 20); }
 }  // namespace fix
 
+// The flux at one end of a line; k is the coefficient there. It depends on nothing else, so that both sides of a face hold
+// the same bits.
+template <int NP, class BASIS>
+__device__ __forceinline__ double flux_end(const BASIS& B, bool last, const double* x, double k) {
+  const int m = fix::max_hi<NP>(x), ke = fix::abs_hi(k);
+  const int ex = max(m >> 20, fix::E_MIN), e = ex + B.fD.s - 1022 + (ke >> 20);
+  if (fix::out_of_range<NP>(m, x) || !fix::plain_coef(ke) || (unsigned)(e - fix::E_FLUX) >= (unsigned)(fix::E_MAX - fix::E_FLUX)) {
+    double s = 0.0;
+#pragma unroll
+    for (int j = 0; j < NP; ++j) s = fma(last ? B.D[NP - 1][j] : B.D[0][j], x[j], s);
+    return s * k;
+  }
+  fix::Limb X[NP];
+#pragma unroll
+  for (int j = 0; j < NP; ++j) X[j] = fix::limbs(x[j], ex);
+  const long long G = fix::line_sum<NP>(
+      X, [&](int j) { return fix::Limb{last ? B.fD.h[NP - 1][j] : B.fD.h[0][j], last ? B.fD.l[NP - 1][j] : B.fD.l[0][j]}; },
+      [](int) { return true; }, 0);
+  return fix::to_double(fix::times(G, fix::mantissa(k)), e);
+}
+
 template <int NP, class BASIS>
 __device__ __forceinline__ void flux_line(const BASIS& B, const double* x, const double* k, FixFlux<NP>& f) {
   const int m = fix::max_hi<NP>(x);
@@ -363,11 +384,10 @@ __device__ __forceinline__ void flux_line(const BASIS& B, const double* x, const
       double g = 0.0;
 #pragma unroll
       for (int j = 0; j < NP; ++j) if (!fix::skip<NP>(i, j)) g = fma(B.D[i][j], x[j], g);
-      g *= k[i];
-      if (i == 0) f.t0 = g;
-      if (i == NP - 1) f.tL = g;
-      f.P[i] = __double_as_longlong(g);
+      f.P[i] = __double_as_longlong(g * k[i]);
     }
+    f.t0 = flux_end<NP>(B, false, x, k[0]);
+    f.tL = flux_end<NP>(B, true, x, k[NP - 1]);
     return;
   }
   f.e = m == 0 ? 0 : eg + (km >> 20);
@@ -395,26 +415,6 @@ __device__ __forceinline__ void flux_line(const BASIS& B, const double* x, const
 #pragma unroll
   for (int i = 0; i < NP; ++i) f.P[i] = (long long)((unsigned long long)f.P[i] << z);
   if (m != 0) f.e += 2 - z;
-}
-
-// The flux at one end of a line, with the bits of flux_line's t0 / tL; k is the coefficient there.
-template <int NP, class BASIS>
-__device__ __forceinline__ double flux_end(const BASIS& B, bool last, const double* x, double k) {
-  const int m = fix::max_hi<NP>(x), ke = fix::abs_hi(k);
-  const int ex = max(m >> 20, fix::E_MIN), e = ex + B.fD.s - 1022 + (ke >> 20);
-  if (fix::out_of_range<NP>(m, x) || !fix::plain_coef(ke) || (unsigned)(e - fix::E_FLUX) >= (unsigned)(fix::E_MAX - fix::E_FLUX)) {
-    double s = 0.0;
-#pragma unroll
-    for (int j = 0; j < NP; ++j) s = fma(last ? B.D[NP - 1][j] : B.D[0][j], x[j], s);
-    return s * k;
-  }
-  fix::Limb X[NP];
-#pragma unroll
-  for (int j = 0; j < NP; ++j) X[j] = fix::limbs(x[j], ex);
-  const long long G = fix::line_sum<NP>(
-      X, [&](int j) { return fix::Limb{last ? B.fD.h[NP - 1][j] : B.fD.h[0][j], last ? B.fD.l[NP - 1][j] : B.fD.l[0][j]}; },
-      [](int) { return true; }, 0);
-  return fix::to_double(fix::times(G, fix::mantissa(k)), e);
 }
 
 // Sums in units of 2^59 / 2^(e - 1022); e < 0: the bits of doubles (FP64 lines).

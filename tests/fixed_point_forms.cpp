@@ -124,6 +124,22 @@ template <int NP> static int mean() {
   return bad;
 }
 
+// Both sides of a face hold the same end flux, whatever the other coefficients of either line are.
+template <int NP> static int face_sides() {
+  const Basis B = make(NP);
+  int differ = 0;
+  for (int it = 0; it < 20000; ++it) {
+    double x[NP], k[NP];
+    for (int i = 0; i < NP; ++i) { x[i] = (2 * uni() - 1) * std::ldexp(1.0, it % 3 == 0 ? (int)(12 * uni()) : 0); k[i] = 1e-4 * (1 + uni()); }
+    k[it % NP] *= it % 2 ? std::ldexp(1.0, (int)(1200 * uni()) - 600) : 0.0;
+    FixFlux<NP> f;
+    flux_line<NP>(B, x, k, f);
+    const double h0 = flux_end<NP>(B, false, x, k[0]), hL = flux_end<NP>(B, true, x, k[NP - 1]);
+    differ += std::memcmp(&h0, &f.t0, 8) != 0 || std::memcmp(&hL, &f.tL, 8) != 0;
+  }
+  return report("face_sides", NP, differ == 0, differ);
+}
+
 // A negated operand gives the negated result to the bit.
 template <int NP> static int odd() {
   const Basis B = make(NP);
@@ -174,6 +190,7 @@ template <int NP> static int run_one(const char* name) {
   if (!std::strcmp(name, "flux_range")) return flux_range<NP>();
   if (!std::strcmp(name, "mean")) return mean<NP>();
   if (!std::strcmp(name, "odd")) return odd<NP>();
+  if (!std::strcmp(name, "face_sides")) return face_sides<NP>();
   return 1;
 }
 
