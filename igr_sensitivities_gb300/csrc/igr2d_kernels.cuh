@@ -636,7 +636,7 @@ __device__ __forceinline__ void dg_stage(const PH& ph, const BasisDev& B, const 
 #pragma unroll
       for (int k = 0; k < NP; ++k) f[k] = flux(v, e, at + k * st);
       FixSums<NP> r;
-      row_scaled<NP, false>(B, c, f, r);
+      row_scaled<NP, false>(B, c, f, r, raw);
 #pragma unroll
       for (int k = 0; k < NP; ++k) sm.k[dir][v][e][at + k * st] = r.G[k];
       sm.ke[dir][v][e][t] = r.e;

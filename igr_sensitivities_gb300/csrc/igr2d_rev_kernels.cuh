@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(2 * Tiling2D<NP>::NH, NP == 4 ? 7 : 1) k2_appl
 #pragma unroll
       for (int i = 0; i < NP; ++i) { s_u[e][at + i] = u[i]; s_v[e][at + i] = v[i]; }
     }
-    flux_line<NP>(B, u, k, f);
+    flux_line<NP, true>(B, u, k, f);
     deriv_line<NP>(B, v, d);
     s_t[dir][e][t][0] = f.t0; s_t[dir][e][t][1] = f.tL;
     u0 = u[0]; uL = u[L]; v0 = v[0]; vL = v[L]; k0 = k[0]; kL = k[L];

@@ -32,6 +32,8 @@
 // but subnormal-range values (below 2^-894), take the FP64 chain, as before. A
 // line of zeros gives zeros, a negated line the negated result to the bit (but for a
 // tie of 32 low bits).
+// Lines in which an interior node leads too far take the chain for the rows that
+// leave it out (fix::leads).
 #pragma once
 #include <cmath>
 
@@ -189,6 +191,26 @@ __device__ __forceinline__ int max_hi(const double* v) {
   return m;
 }
 
+// A row of D or D^T leaves out its own interior node. Where that node exceeds all others by too much, units that go by the
+// line's largest value are too coarse for that row on its own, and the FP64 chain runs. Up to these bounds (differences of high
+// words: a factor of about 2 or 3 for rows of D, 8 for D itself unscaled and for D^T) the integer row's rms error is at most the chain's;
+// at 2^4 a row of D has two to three times the chain's, and it doubles with every further power of two
+// (tests/fixed_point_forms.cpp, leading).
+template <int NP>
+constexpr int LEAD = NP == 3 ? 1 << 20 : 3 << 19;
+constexpr int LEAD_T = 3 << 20;
+template <int NP, int BY>
+__device__ __forceinline__ bool leads(const double* v) {
+  int big = abs_hi(v[1]), next = max(abs_hi(v[0]), abs_hi(v[NP - 1]));
+#pragma unroll
+  for (int k = 2; k < NP - 1; ++k) {
+    const int a = abs_hi(v[k]);
+    next = max(next, min(big, a));
+    big = max(big, a);
+  }
+  return big - next > BY;
+}
+
 constexpr long long HALF = 1LL << 31;  // M / 2^31 is added as 2 (M >> 32): rounded to nearest by this
 
 // One sum of a line: coefficient (h, l)[k] by index function cf(k) -> Limb, over the terms keep(k) lets through
@@ -257,15 +279,18 @@ __device__ __forceinline__ void line_op(const FixMat& F, const MAT& A, const Fix
   }
   const int e = max(max(m >> 20, (ma >> 20) - up), fix::E_MIN);
   if (SCALED) slow |= (unsigned)(e + up - 64) >= (unsigned)(fix::E_MAX - 64);
+  auto row_fp64 = [&](int i, double s) {
+#pragma unroll
+    for (int k = 0; k < NP; ++k) {
+      if (SKIP && fix::skip<NP>(i, k)) continue;
+      s = fma(T ? A[k][i] : A[i][k], v[k], s);
+    }
+    return s;
+  };
   if (slow) {
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
-      double s = (has(i) && !SCALED) ? acc[i] : 0.0;
-#pragma unroll
-      for (int k = 0; k < NP; ++k) {
-        if (SKIP && fix::skip<NP>(i, k)) continue;
-        s = fma(T ? A[k][i] : A[i][k], v[k], s);
-      }
+      const double s = row_fp64(i, (has(i) && !SCALED) ? acc[i] : 0.0);
       out[i] = SCALED ? (has(i) ? fma(c->d, s, acc[i]) : c->d * s) : s;
     }
     return;
@@ -281,6 +306,14 @@ __device__ __forceinline__ void line_op(const FixMat& F, const MAT& A, const Fix
         [&](int k) { return !(SKIP && fix::skip<NP>(i, k)); }, SCALED ? 0 : A0);
     if (SCALED) G = fix::times(G, c->m, A0);
     out[i] = fix::to_double(G, e + up - (SCALED ? 0 : 1));
+  }
+  if (fix::leads<NP, T ? fix::LEAD_T : fix::LEAD<NP>>(v)) {
+#pragma unroll
+    for (int i = 1; i < NP - 1; ++i) {
+      if (fix::abs_hi(v[i]) != m) continue;
+      const double s = row_fp64(i, 0.0), a = has(i) ? acc[i] : 0.0;
+      out[i] = SCALED ? fma(c->d, s, a) : s + a;
+    }
   }
 }
 
@@ -361,7 +394,10 @@ __device__ __forceinline__ double flux_end(const BASIS& B, bool last, const doub
   return fix::to_double(fix::times(G, fix::mantissa(k)), e);
 }
 
-template <int NP, class BASIS>
+// ROWS: the fluxes serve by themselves (products). The operator's sums need no such care with x: each of them holds a flux of
+// another node, whose FP64 form carries the rounding of a leading x too (measured at factors up to 2^12: 0.5 to 0.6 of the
+// chain's error); a leading coefficient matters from 2^4 on.
+template <int NP, bool ROWS = false, class BASIS>
 __device__ __forceinline__ void flux_line(const BASIS& B, const double* x, const double* k, FixFlux<NP>& f) {
   const int m = fix::max_hi<NP>(x);
   int ke[NP], km = 0, kn = 0x7fffffff;
@@ -376,7 +412,8 @@ __device__ __forceinline__ void flux_line(const BASIS& B, const double* x, const
   const int ex = max(m >> 20, fix::E_MIN);
   const int eg = ex + B.fD.s - 1022;  // P_i before alignment has exponent eg + ke_i
   // Every P_i, and the line's after its shift by up to 30 below, stays where to_double's exponent cannot pass below zero.
-  f.slow = fix::out_of_range<NP>(m, x) || !ok || eg + (kn >> 20) < fix::E_FLUX || eg + (km >> 20) >= fix::E_MAX;
+  f.slow = fix::out_of_range<NP>(m, x) || !ok || eg + (kn >> 20) < fix::E_FLUX || eg + (km >> 20) >= fix::E_MAX ||
+           (ROWS && fix::leads<NP, fix::LEAD<NP>>(x)) || (km - kn > (4 << 20) && fix::leads<NP, 4 << 20>(k));
   if (f.slow) {
     f.e = 0;
 #pragma unroll
@@ -491,7 +528,7 @@ struct FixDeriv { long long G[NP]; int e; bool slow; };
 template <int NP, class BASIS>
 __device__ __forceinline__ void deriv_line(const BASIS& B, const double* v, FixDeriv<NP>& d) {
   const int m = fix::max_hi<NP>(v);
-  d.slow = fix::out_of_range<NP>(m, v);
+  d.slow = fix::out_of_range<NP>(m, v) || fix::leads<NP, fix::LEAD_T>(v);
   d.e = 0;
   if (d.slow) {
 #pragma unroll
@@ -607,10 +644,11 @@ __device__ __forceinline__ double node_blend(long long r, int er, long long c, i
 // A scaled line derivative (or its transpose, T) kept as integers, c (D v), with row_add_ends' terms at its end nodes,
 // in units of 2^60 / 2^(e - 1022); r.e < 0: the bits of doubles (FP64 lines). node_total and node_blend end the sums.
 // ---------------------------------------------------------------------------
+// rows: the sums serve by themselves, not as a small addition to the node's value (see fix::leads)
 template <int NP, bool T, class BASIS>
-__device__ __forceinline__ bool scaled_line(const BASIS& B, const FixScale& c, const double* v, FixSums<NP>& r) {
+__device__ __forceinline__ bool scaled_line(const BASIS& B, const FixScale& c, const double* v, bool rows, FixSums<NP>& r) {
   const int m = fix::max_hi<NP>(v);
-  if (fix::out_of_range<NP>(m, v) || (unsigned)(c.e - 1022 + 256) > 512u) return false;
+  if (fix::out_of_range<NP>(m, v) || (rows && fix::leads<NP, T ? fix::LEAD_T : fix::LEAD<NP>>(v)) || (unsigned)(c.e - 1022 + 256) > 512u) return false;
   const int ex = max(m >> 20, fix::E_MIN), e = ex + B.fD.s + c.e - 1022;
   if ((unsigned)(e - 64) >= (unsigned)(fix::E_MAX - 64)) return false;
   fix::Limb X[NP];
@@ -635,8 +673,8 @@ __device__ __forceinline__ void scaled_line_fp64(const BASIS& B, const FixScale&
   }
 }
 template <int NP, bool T, class BASIS>
-__device__ __forceinline__ void row_scaled(const BASIS& B, const FixScale& c, const double* v, FixSums<NP>& r) {
-  if (scaled_line<NP, T>(B, c, v, r)) return;
+__device__ __forceinline__ void row_scaled(const BASIS& B, const FixScale& c, const double* v, FixSums<NP>& r, bool rows = true) {
+  if (scaled_line<NP, T>(B, c, v, rows, r)) return;
   double s[NP];
   scaled_line_fp64<NP, T>(B, c, v, s);
   r.e = -1;

@@ -64,6 +64,77 @@ static Full full(int np) {
   return F;
 }
 
+// One interior value (or coefficient) larger than the others by 2^g: its own row, which leaves it out, is as exact relative to
+// its own terms as the FP64 chain's, in rms over random lines.
+template <int NP> static int leading() {
+  if (NP == 2) return 0;
+  const Full B = full(NP);
+  int bad = 0;
+  const char* forms[] = {"rows", "cols", "w2_cols", "w2_rows", "dr_cols", "scaled", "deriv", "flux", "div", "div_coef"};
+  for (int form = 0; form < 10; ++form)
+    for (int g8 = 0; g8 <= 160; g8 += g8 < 32 ? 2 : 16) {
+      double si = 0, sf = 0;
+      for (int it = 0; it < 20000; ++it) {
+        const int at = 1 + (int)(uni() * (NP - 2));
+        double v[NP], k[NP], out[NP];
+        for (int i = 0; i < NP; ++i) { v[i] = (uni() < 0.5 ? -1 : 1) * (1 + uni()); k[i] = 1e-4 * (1 + uni()); }
+        const double s = std::exp2(g8 / 8.0);
+        (form == 9 ? k : v)[at] *= s;
+        const FixScale c = fix_scale((1 + uni()) * 8);
+        const bool T = form == 1 || form == 2 || form >= 4 && form != 6 && form != 7;
+        const double (*A)[FIX_MAXNP] = form == 4 ? B.Dr : (form == 2 || form == 3 ? B.W2 : B.D);
+        auto none = [](int) { return false; };
+        FixSums<NP> r;
+        if (form == 0) line_op<NP, false, true, true>(B.fD, B.D, &c, v, nullptr, none, out);
+        if (form == 1) line_op<NP, true, true, true>(B.fD, B.D, &c, v, nullptr, none, out);
+        if (form == 2) line_op<NP, true, false, true>(B.fW2, B.W2, &c, v, nullptr, none, out);
+        if (form == 3) line_op<NP, false, false, true>(B.fW2, B.W2, &c, v, nullptr, none, out);
+        if (form == 4) line_op<NP, true, true, true>(B.fDr, B.Dr, &c, v, nullptr, none, out);
+        if (form == 5) { row_scaled<NP, true>(B, c, v, r); for (int i = 0; i < NP; ++i) out[i] = sums_at<NP>(r, i); }
+        if (form == 6) { FixDeriv<NP> d; deriv_line<NP>(B, v, d); for (int i = 0; i < NP; ++i) out[i] = deriv_at<NP>(d, i); }
+        if (form >= 7) {
+          FixFlux<NP> f;
+          if (form == 7) flux_line<NP, true>(B, v, k, f);
+          else flux_line<NP>(B, v, k, f);
+          for (int i = 0; i < NP; ++i) out[i] = flux_at<NP>(f, i);
+          if (form >= 8) {
+            row_sums<NP>(B, f, 0.0, 0.0, 0.0, 0.0, r);
+            for (int i = 0; i < NP; ++i) out[i] = node_total<59>(r.G[i], r.e, 0, 0, 0.0, 1);
+          }
+        }
+        long double ref = 0, mag = 0;
+        double f64 = 0;
+        if (form < 8) {
+          for (int j = 0; j < NP; ++j) {
+            if (j == at) continue;
+            const double a = T ? A[j][at] : A[at][j];
+            ref += (long double)a * v[j]; mag += fabsl((long double)a * v[j]); f64 = std::fma(a, v[j], f64);
+          }
+          const double cc = form == 7 ? k[at] : (form == 6 ? 1.0 : c.d);
+          ref *= cc; mag *= cc; f64 *= cc;
+        } else {
+          for (int i = 0; i < NP; ++i) {
+            if (i == at) continue;
+            long double G = 0, H = 0;
+            double h = 0;
+            for (int j = 0; j < NP; ++j) {
+              if (fix::skip<NP>(i, j)) continue;
+              G += (long double)B.D[i][j] * v[j]; H += fabsl((long double)B.D[i][j] * v[j]); h = std::fma(B.D[i][j], v[j], h);
+            }
+            ref += B.D[i][at] * (G * k[i]); mag += fabs(B.D[i][at]) * (H * k[i]); f64 = std::fma(B.D[i][at], h * k[i], f64);
+          }
+        }
+        const long double ei = (out[at] - ref) / mag, ef = (f64 - ref) / mag;
+        si += (double)(ei * ei); sf += (double)(ef * ef);
+      }
+      const double ratio = std::sqrt(si / sf);
+      char name[64];
+      std::snprintf(name, sizeof(name), "leading %s 2^%.2f", forms[form], g8 / 8.0);
+      bad += report(name, NP, ratio <= 1.001, ratio);  // 1 where the chain runs or both round once, the same sums
+    }
+  return bad;
+}
+
 // No result is high or low on average: the mean error over random lines stays within five standard errors of zero.
 template <int NP> static int mean() {
   if (NP == 2) return 0;
@@ -188,6 +259,7 @@ template <int NP> static int odd() {
 
 template <int NP> static int run_one(const char* name) {
   if (!std::strcmp(name, "flux_range")) return flux_range<NP>();
+  if (!std::strcmp(name, "leading")) return leading<NP>();
   if (!std::strcmp(name, "mean")) return mean<NP>();
   if (!std::strcmp(name, "odd")) return odd<NP>();
   if (!std::strcmp(name, "face_sides")) return face_sides<NP>();
