@@ -567,18 +567,17 @@ __device__ __forceinline__ double flux_at(const FixFlux<NP>& f, int i) {
 }
 
 // The products flux_i (D v)_i, with z0 and zL added at the end nodes, in units of 2^60 / 2^(r.e - 1022) (r.e < 0: the
-// bits of doubles); need: the largest exponent of what the caller adds. The products go by the line's largest flux and
-// derivative and are not aligned to the operator's sums.
+// bits of doubles). They go by the line's largest flux and derivative and are not aligned to the operator's sums.
 template <int NP>
-__device__ __forceinline__ bool product_line(const FixFlux<NP>& f, const FixDeriv<NP>& d, double z0, double zL, int need,
-                                             bool all_zero, FixSums<NP>& r) {
+__device__ __forceinline__ bool product_line(const FixFlux<NP>& f, const FixDeriv<NP>& d, double z0, double zL,
+                                             FixSums<NP>& r) {
   const int mz = max(fix::abs_hi(z0), fix::abs_hi(zL)) >> 20;
   const bool none = f.e == 0 || d.e == 0;
   const int ep = none ? 0 : f.e + d.e - 1022;
-  int e = max(max(ep, mz), need);
+  int e = max(ep, mz);
   if (f.slow || d.slow || e >= fix::E_MAX || (!none && ep < 64)) return false;
   if (e < 128) {
-    if (!none || !fix::zero(z0) || !fix::zero(zL) || !all_zero) return false;
+    if (!none || !fix::zero(z0) || !fix::zero(zL)) return false;
     e = 128;
   }
   r.e = e;
@@ -596,7 +595,7 @@ __device__ __forceinline__ bool product_line(const FixFlux<NP>& f, const FixDeri
 template <int NP>
 __device__ __forceinline__ void row_products(const FixFlux<NP>& f, const FixDeriv<NP>& d, double z0, double zL,
                                              FixSums<NP>& r) {
-  if (product_line<NP>(f, d, z0, zL, 0, true, r)) return;
+  if (product_line<NP>(f, d, z0, zL, r)) return;
   r.e = -1;
 #pragma unroll
   for (int i = 0; i < NP; ++i) {

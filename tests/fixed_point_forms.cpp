@@ -211,6 +211,108 @@ template <int NP> static int face_sides() {
   return report("face_sides", NP, differ == 0, differ);
 }
 
+// The forms that the kernels use, over the kinds of lines of fixed_point_check.cpp: scaled sums with the matrices Dr and W2 and
+// with end terms, against long double. The rms error is at most the FP64 chain's, with three standard errors of it (both may
+// end in one rounding of the same size); single errors stay below 8e-16 of the largest term, also where the chain runs.
+template <int NP> static int forms() {
+  const Full B = full(NP);
+  int bad = 0;
+  const char* names[] = {"dr_cols_ends", "w2_cols_ends", "w2_rows_ends", "stage_line", "transposes"};
+  for (int form = 0; form < 5; ++form)
+    for (int kind = 0; kind <= 8; ++kind) {
+      double si = 0, sf = 0, worst = 0;
+      bool ok = true;
+      for (int it = 0; it < 4000; ++it) {
+        double v[NP], out[NP];
+        for (int i = 0; i < NP; ++i) v[i] = value(kind);
+        const double big = std::ldexp(1.0, (int)(40 * uni()) - 20);
+        const double a0 = kind == 6 ? 0.0 : value(kind) * (kind < 4 ? big : 1), aL = kind == 6 ? 0.0 : value(kind) * (kind < 4 ? big : 1);
+        const FixScale c = fix_scale((uni() < 0.5 ? -1 : 1) * std::ldexp(1 + uni(), (int)(8 * uni()) - 8));
+        const bool T = form == 0 || form == 1 || form == 4;
+        const FixMat& F = form == 0 ? B.fDr : (form < 3 ? B.fW2 : B.fD);
+        const double (*A)[FIX_MAXNP] = form == 0 ? B.Dr : (form < 3 ? B.W2 : B.D);
+        auto ends = [](int k) { return k == 0 || k == NP - 1; };
+        double acc[NP] = {};
+        acc[0] = form == 4 ? 0.0 : a0;
+        acc[NP - 1] = form == 4 ? 0.0 : aL;
+        FixSums<NP> r;
+        if (form == 0) line_op<NP, true, true, true>(F, A, &c, v, acc, ends, out);
+        if (form == 1) line_op<NP, true, false, true>(F, A, &c, v, acc, ends, out);
+        if (form == 2) line_op<NP, false, false, true>(F, A, &c, v, acc, ends, out);
+        if (form == 3) { row_scaled<NP, false>(B, c, v, r); row_add_ends<NP>(r, a0, aL); }
+        if (form == 4) row_scaled<NP, true>(B, c, v, r);
+        if (form >= 3) for (int i = 0; i < NP; ++i) out[i] = node_total<60>(r.G[i], r.e, 0, 0, 0.0, 1);
+        long double top = std::fmax(std::fabs(acc[0]), std::fabs(acc[NP - 1]));
+        for (int i = 0; i < NP; ++i) top = fmaxl(top, ldexpl(fabsl((long double)v[i] * c.d), F.s));
+        for (int i = 0; i < NP; ++i) {
+          long double s = 0;
+          double f64 = 0;
+          for (int k = 0; k < NP; ++k) {
+            if ((form == 0 || form >= 3) && fix::skip<NP>(i, k)) continue;
+            const double m = T ? A[k][i] : A[i][k];
+            s += (long double)m * v[k];
+            f64 = std::fma(m, v[k], f64);
+          }
+          s = s * c.d + acc[i];
+          f64 = std::fma(c.d, f64, acc[i]);
+          if (!std::isfinite(f64) || fabsl(s) > 1.7e308L || top > 1e307L) continue;
+          if (top == 0) { ok &= out[i] == 0; continue; }
+          const long double ei = (out[i] - s) / top, ef = (f64 - s) / top;
+          worst = std::fmax(worst, (double)(fabsl(out[i] - s) / (top * 8e-16L + 1e-321L)));
+          si += (double)(ei * ei); sf += (double)(ef * ef);
+        }
+      }
+      const double ratio = NP > 2 && kind < 7 && kind != 4 && sf > 0 ? std::sqrt(si / sf) : 0;
+      char name[64];
+      std::snprintf(name, sizeof(name), "forms %s kind%d", names[form], kind);
+      bad += report(name, NP, ok && worst <= 1 && ratio <= 1 + 3 / std::sqrt(4000.0 * NP), std::fmax(worst, ratio));
+    }
+  return bad;
+}
+
+// Infinities and NaN come out as not finite wherever the FP64 chain has them, in the same forms and in the operator's lines.
+template <int NP> static int nonfinite() {
+  const Full B = full(NP);
+  int wrong = 0;
+  const double inf = std::numeric_limits<double>::infinity();
+  for (double bad : {inf, -inf, std::numeric_limits<double>::quiet_NaN()})
+    for (int at = 0; at < NP + 2; ++at) {  // NP, NP + 1: an end term
+      double v[NP], k[NP], acc[NP] = {}, out[NP];
+      for (int i = 0; i < NP; ++i) { v[i] = 0.5 + i; k[i] = 1e-4 * (1 + i); }
+      acc[0] = 0.25; acc[NP - 1] = -0.5;
+      if (at < NP) v[at] = bad;
+      else acc[at == NP ? 0 : NP - 1] = bad;
+      const FixScale c = fix_scale(-1.5);
+      auto ends = [](int i) { return i == 0 || i == NP - 1; };
+      auto chain = [&](const double (*A)[FIX_MAXNP], bool T, bool skip, int i) {
+        double s = 0;
+        for (int j = 0; j < NP; ++j) if (!(skip && fix::skip<NP>(i, j))) s = std::fma(T ? A[j][i] : A[i][j], v[j], s);
+        return std::fma(c.d, s, acc[i]);
+      };
+      line_op<NP, true, true, true>(B.fDr, B.Dr, &c, v, acc, ends, out);
+      for (int i = 0; i < NP; ++i) wrong += std::isfinite(out[i]) != std::isfinite(chain(B.Dr, true, true, i));
+      line_op<NP, true, false, true>(B.fW2, B.W2, &c, v, acc, ends, out);
+      for (int i = 0; i < NP; ++i) wrong += std::isfinite(out[i]) != std::isfinite(chain(B.W2, true, false, i));
+      FixSums<NP> r;
+      row_scaled<NP, false>(B, c, v, r);
+      row_add_ends<NP>(r, acc[0], acc[NP - 1]);
+      for (int i = 0; i < NP; ++i)
+        wrong += std::isfinite(node_total<60>(r.G[i], r.e, 0, 0, 1.0, 1)) != std::isfinite(chain(B.D, false, true, i));
+      FixFlux<NP> f;
+      FixDeriv<NP> d;
+      flux_line<NP>(B, v, k, f);
+      deriv_line<NP>(B, v, d);
+      row_products<NP>(f, d, 0.0, 0.0, r);
+      for (int i = 0; i < NP; ++i) {
+        const bool fine = at >= NP || fix::skip<NP>(i, at);
+        wrong += std::isfinite(deriv_at<NP>(d, i)) != fine;
+        wrong += std::isfinite(flux_at<NP>(f, i)) != fine;
+        wrong += std::isfinite(node_total<60>(r.G[i], r.e, 0, 0, 1.0, -1)) != fine;
+      }
+    }
+  return report("nonfinite", NP, wrong == 0, wrong);
+}
+
 // A negated operand gives the negated result to the bit.
 template <int NP> static int odd() {
   const Basis B = make(NP);
@@ -263,6 +365,8 @@ template <int NP> static int run_one(const char* name) {
   if (!std::strcmp(name, "mean")) return mean<NP>();
   if (!std::strcmp(name, "odd")) return odd<NP>();
   if (!std::strcmp(name, "face_sides")) return face_sides<NP>();
+  if (!std::strcmp(name, "forms")) return forms<NP>();
+  if (!std::strcmp(name, "nonfinite")) return nonfinite<NP>();
   return 1;
 }
 

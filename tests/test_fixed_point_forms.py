@@ -15,7 +15,7 @@ def exe(tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("name", ["flux_range", "mean", "odd", "face_sides", "leading"])
+@pytest.mark.parametrize("name", ["flux_range", "mean", "odd", "face_sides", "leading", "forms", "nonfinite"])
 def test_form(exe, name):
     r = subprocess.run([exe, name], capture_output=True, text=True)
     bad = [ln for ln in r.stdout.splitlines() if " ok " not in ln]
