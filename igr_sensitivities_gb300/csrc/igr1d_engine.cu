@@ -79,11 +79,9 @@ long long forward1d_scratch_fields(const Inst1DDesc&, int) { return E1_FIELDS + 
 // it is chosen for speed. One CTA advances an instance at one element per
 // thread; its SM's FP64 rate bounds it (a 256-element Jacobi iteration: ~6 us).
 // Small batches of instances with at least T1 elements therefore spread each
-// over a cluster of up to 16 SMs (at least 16 elements per CTA); below T1
-// elements the cluster barrier costs more than it saves (measured on GB300:
-// N_e = 64 and 128 run 10-20% faster on one CTA), and batches that fill the
-// GPU use one CTA per instance. For everything between, the cluster size is
-// the one with the shortest estimate of a solver iteration, in rounds of one
+// over a cluster of up to 16 SMs (at least 16 elements per CTA). For all other
+// batches, small or filling the GPU, the cluster size is the one with the
+// shortest estimate of a solver iteration, in rounds of one
 // warp of elements per SM sub-partition: the longest instance (its rounds per
 // CTA plus the barriers, 0.8 for a CTA's and 1.6 for a cluster's; half a round
 // where the iterate fits shared memory, d1_local_ok), the batch's CTAs over the
@@ -92,7 +90,12 @@ long long forward1d_scratch_fields(const Inst1DDesc&, int) { return E1_FIELDS + 
 // Measured (two steps of the adjoint, ms, 1 / chosen): 256 instances of
 // 64..1024 elements, PCG 102: 94 / 73 (2 CTAs); 40 of 25..400, PCG 30: 11.7 /
 // 7.5 (4); 8 of 56..900, PCG 30: 23.2 / 7.5 (8); 150 of 12..200: one CTA, 7.7
-// (8.0 with 2). A context setting overrides the choice, and autotuning replaces
+// (8.0 with 2). Single instances keep one CTA up to 128 elements and with PCG
+// below T1 (its inner products add cluster barriers). With 129 to 255 elements
+// Jacobi and Chebyshev take 8 (P3), 4 (P1) or 16 CTAs (P4): P3 forward, 40 steps,
+// Jacobi 50, 160 / 200 / 255 elements: 25.8 / 32.1 / 37.0 ms on one CTA, 15.4 / 15.6 /
+// 15.6 on 8; adjoint, 10 steps, Chebyshev 5: 5.2 / 6.5 / 7.5 and 4.2 / 4.3 / 4.3; the least
+// gain is 1.05 (P1 adjoint, 160 elements). A context setting overrides the choice, and autotuning replaces
 // it with a measurement (cluster_size).
 static int cluster_heuristic(Ctx& c, const Plan1D& P, int solver) {
   int sms = 0;

@@ -586,9 +586,12 @@ __device__ void d1_stage_rev(const View1<NP>& v, const BasisDev& B, int solver, 
 // The adjoint kernel. Scratch per instance (fields of N doubles):
 //   state X (3), 1/rho, Sigma chain (2), step work, reverse buffers,
 //   three stage tapes, `seg` step snapshots (level 2) and ceil(n_steps/seg)
-//   segment snapshots (level 1). The forward runs once storing level-1
-//   snapshots; each segment is re-run storing every step's state, and each
-//   step is re-run once more with full stage tapes before its reverse.
+//   segment snapshots (level 1). The forward runs once and stores a level-1
+//   snapshot per segment, but for the last segment: of that it stores every
+//   step's state (level 2), and of the last step the stage tapes, which the
+//   reverse starts with. The segments before are re-run storing every step's
+//   state, and every step but the last is run once more with full stage tapes
+//   before its reverse.
 // ---------------------------------------------------------------------------
 enum : int {
   A1_X = 0, A1_IR = 3, A1_SA = 4, A1_SB = 5, A1_WK = 6,

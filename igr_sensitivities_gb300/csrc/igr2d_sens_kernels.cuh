@@ -12,7 +12,9 @@
 // The tangent LLF flux uses the primal wave speed (sensitivity_llf_flux_x/_y,
 // sensitivity.jl:85-118: no d lambda term); it is read from the face-node wave
 // speeds the primal k2_hyp_rk of the same stage wrote.
-// Same thread mapping as the primal kernels (one thread per element line).
+// k2_sens_hyp_rk is the primal stage with other physics (dg_stage: rows and
+// columns side by side); k2_sens_rhs runs rows, then columns, on one thread per
+// element line.
 #pragma once
 #include "igr2d_kernels.cuh"
 

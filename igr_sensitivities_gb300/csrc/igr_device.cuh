@@ -312,6 +312,7 @@ __device__ __forceinline__ void chained_start() {
 // above that they all ask for nearly everything by themselves and a larger L1 is worth more. P3 gradients, ms, driver's
 // split / 100 KB / all shared: 64^2 (256 tiles) 4.68 / 3.94 / 4.03, 40^2 3.12 / 3.04 / 3.07, 76^2 5.57 / 5.34 / 5.31; 8 x 128^2
 // (8192 tiles) 43.1 / 47.8 / 43.5.
+// 152 is the GB300's SM count, the only chip this is built for; the attribute is a hint and results do not depend on it.
 constexpr int SMALL_GRID = 3 * 152;
 constexpr unsigned SMALL_GRID_CARVEOUT = 44;  // percent of 228 KB
 template <class... P, class... A>
