@@ -39,18 +39,18 @@ METRIC = "2D P3 128Â² adjoint gradients/s: batched vs plain, same GPU, rel err â
 # (2 DFMA + DADD + DMUL) of one ncu capture divided by the launch's nodes
 # (profiles/adjoint2d_kernels_128.md). Used for the live roofline. The line
 # contractions run as integer sums and are not in these counts.
-FLOPS_PER_NODE = {0: 28.3, 1: 14.5, 2: 67.8, 3: 116.0, 4: 25.1, 5: 46.6}
+FLOPS_PER_NODE = {0: 32.4, 1: 14.5, 2: 76.8, 3: 127.9, 4: 25.1, 5: 46.6}
 # Algorithmic FP64 bytes per node per launch: one read of every live field and
 # one write of every output field (halo re-reads excluded), for the HBM fraction.
 BYTES_PER_NODE = {0: 8 * 11, 1: 8 * 13, 2: 8 * 17, 3: 8 * 35, 4: 8 * 23, 5: 8 * 19}
 # DRAM bytes per node of one launch of each family, measured with ncu on an
 # 8-instance case whose fields exceed L2 (profiles/adjoint2d_kernels_128.md);
 # scaled by the launch's node count for `roofline.traffic`.
-TRAFFIC_PER_NODE = {0: 59.1, 1: 89.7, 2: 126.9, 3: 222.8, 4: 151.6, 5: 140.4}
+TRAFFIC_PER_NODE = {0: 58.9, 1: 90.1, 2: 127.1, 3: 222.9, 4: 151.8, 5: 140.8}
 # FP64 instructions per node (DFMA + DADD + DMUL thread instructions of the same
 # captures): the issue-rate view of the FP64 roof, whose peak is half the DFMA
 # probe's flop rate (one DFMA = 2 flops).
-INST_PER_NODE = {0: 21.3, 1: 11.5, 2: 50.8, 3: 85.0, 4: 19.3, 5: 35.1}
+INST_PER_NODE = {0: 23.3, 1: 11.5, 2: 56.5, 3: 91.1, 4: 19.3, 5: 35.1}
 FAMILY = {0: "k2_setup", 1: "k2_apply", 2: "k2_hyp_rk", 3: "k2_hyp_rev", 4: "k2_apply_rev", 5: "k2_setup_rev"}
 # Algorithmic FP64 operations per node: the reference's arithmetic as restated in the oracle, counted with an
 # operation-counting scalar (+ - * / sqrt |x| max = 1 each, a multiply-add = 2), and its reverse by the

@@ -160,7 +160,8 @@ struct SetupArgs2D {
 // What bounds it: FP64 issue, at a third of the FP64 instructions of its FP64-contraction form: the velocity derivatives
 // and both diagonal contractions (with their scales and the face terms) are integer line operations, and the face
 // constants are tabulated once per CTA. Rows and columns run side by side like the operator's, between two pointwise
-// passes. 8 x 128^2 P3: 259 us with FP64 contractions, 113 us with integer ones, 103 us in halves; 64^2: 16.5, 13.9, 12.4.
+// passes. 8 x 128^2 P3: 259 us with FP64 contractions, 113 us with integer ones, 103 us in halves, 110 us with IEEE 1/x again
+// (restarts to the bit) and sums without a mean error. 64^2: 16.5, 13.9, 12.4.
 template <int NP>
 __global__ void __launch_bounds__(2 * Tiling2D<NP>::NH) k2_setup(SetupArgs2D a) {
   using TL = Tiling2D<NP>;
@@ -343,9 +344,9 @@ struct ApplySmem {
 // line's chain of loads, integer sums and FP64 faces is all that a warp runs before the CTA meets, and the epilogue is
 // pointwise over all threads with coalesced accesses. PCG's direction update p_k = M^-1 r_k + beta p_{k-1} is pointwise
 // too and is formed once per node, in front of the lines.
-// What bounds it: FP64 issue (68% busy), the integer ALU (59%) and L2 latency, with 32 warps per SM. 8 x 128^2 P3,
+// What bounds it: the integer ALU (65% busy), FP64 issue (61%) and L2 latency, with 32 warps per SM. 8 x 128^2 P3,
 // Chebyshev: 127 us with FP64 contractions; 79 us with integer ones and one thread per pair of lines (18 warps); 69 us in
-// halves; 65 us with the pointwise loads ahead of its stores. 64^2: 12.3, 11.3, 10.2, 9.9.
+// halves; 65 us with the pointwise loads ahead of its stores; 68 us with sums without a mean error. 64^2: 12.3, 11.3, 10.2, 9.9.
 template <int NP, int EPI>
 __device__ __forceinline__ double apply_tile(const ApplyArgs2D& a, const Tile2D tl, const Inst2D& I, ApplySmem<NP>& sm) {
   using TL = Tiling2D<NP>;
@@ -583,8 +584,9 @@ struct StageSmem {
 // What bounds it: FP64 issue. Volume terms, their scaling, the row and column parts and the stage combination's sum are
 // integer work (igr_fix.cuh); the stage coefficient is folded into the scale of the derivatives and face terms, so that
 // q_out = c0 q^n + c1 q_s + [c2 dt k] is one rounded sum and k itself is never formed. Euler, 8 x 128^2 P3: 427 us with
-// FP64 contractions and IEEE square roots, 248 us now (FP64 pipe 80% busy; 252 with the state weights in FP64); 64^2: 24.9,
-// 22.4 with one thread per pair of lines, 18.6 in halves.
+// FP64 contractions, 248 us with integer ones (252 with the state weights in FP64) and 1/x and square roots of FP32 seeds, 274 us
+// with the IEEE ones again and sums without a mean error (FP64 pipe 72% busy); 64^2: 24.9, 22.4 with one thread per pair
+// of lines, 18.6 in halves, 18.7 now.
 template <int NP, bool AUX, class PH>
 __device__ __forceinline__ void dg_stage(const PH& ph, const BasisDev& B, const Tile2D tl, const Inst2D& I, double c0, double c1,
                                          double c2, bool raw, StageSmem<NP, AUX>& sm) {

@@ -246,7 +246,8 @@ __device__ __forceinline__ AdjFlux pde_adjoint_flux(double g, double mx, double 
 
 // What bounds it: FP64 issue (adjoint fluxes, sources, faces). Volume terms and the nonlocal source's derivatives are
 // integer line operations; the faces take f_partner - f_own - lambda (a_L - a_R) (see llf_jump). 8 x 128^2 P3: 793 us with
-// FP64 contractions, 544 us now; k2_pde_prep and k2_pde_b together 285 and 165 us per launch.
+// FP64 contractions, 544 us with integer ones, 595 us with sums without a mean error and the leading-node checks; k2_pde_prep
+// and k2_pde_b together 285, 165 and 170 us per launch on average.
 template <int NP>
 __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_pde_rk(PdeRkArgs2D a) {
   using TL = Tiling2D<NP>;

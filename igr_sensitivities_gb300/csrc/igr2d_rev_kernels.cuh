@@ -110,8 +110,8 @@ struct HypRevArgs2D {
 // Rows and columns run side by side, one half of the CTA each; the node work (flux reverse, combination) is spread over
 // all threads. What bounds it: FP64 issue. The transposed volume terms run on the integer pipes with the stage
 // coefficient and the own side of the face corrections in their matrix; a face takes 5 FP64 instructions per component.
-// 8 x 128^2 P3: 680 us with FP64 contractions; 442 with integer ones; 390 with the shorter faces and node reverse (191
-// FP64 instructions per warp of half the lines, pipe 84% busy). 64^2: 40.8, 37.8, and 23.6 in halves.
+// 8 x 128^2 P3: 680 us with FP64 contractions; 442 with integer ones; 360 with the shorter faces and node reverse; 394 with
+// IEEE divides again (pipe 84% busy). 64^2: 40.8, 37.8, and 23.6 in halves.
 template <int NP>
 __global__ void __launch_bounds__(2 * Tiling2D<NP>::NH) k2_hyp_rev(HypRevArgs2D a) {
   using TL = Tiling2D<NP>;
@@ -319,9 +319,10 @@ struct ApplyRevArgs2D {
 struct Partner2 { double u, v, t, ir; };
 
 // Rows and columns run side by side, one half of the CTA each, and the outputs are pointwise over all threads (see
-// k2_apply). What bounds it: FP64 issue (67% busy) and the integer ALU (54%). 8 x 128^2 P3, Chebyshev: 226 us with FP64
+// k2_apply). What bounds it: FP64 issue (60% busy) and the integer ALU (56%). 8 x 128^2 P3, Chebyshev: 226 us with FP64
 // contractions; 140 us with integer ones and one thread per pair of lines; in halves, with the pointwise loads ahead of
-// its stores, 114 us at seven CTAs per SM (72 registers; 137 us at the 80 the compiler takes). 64^2: 18.9, 17.4, 12.4.
+// its stores, 114 us at seven CTAs per SM (72 registers; 137 us at the 80 the compiler takes); 126 us with sums without a
+// mean error and the leading-node checks. 64^2: 18.9, 17.4, 12.4.
 template <int NP, int SREV>
 __global__ void __launch_bounds__(2 * Tiling2D<NP>::NH, NP == 4 ? 7 : 1) k2_apply_rev(ApplyRevArgs2D a) {
   using TL = Tiling2D<NP>;
@@ -507,8 +508,8 @@ struct SetupRevArgs2D {
 
 // What bounds it: FP64 issue. All derivatives, transposes and diagonal contractions are integer line operations; the two
 // transposes of a node meet as integers. Rows and columns run side by side, between pointwise passes whose loads
-// come before any store. 8 x 128^2 P3: 409 us with FP64 contractions, 196 us with integer ones, 158 us in halves; 64^2: 22.8,
-// 22.7, 14.9.
+// come before any store. 8 x 128^2 P3: 409 us with FP64 contractions, 196 us with integer ones, 167 us in halves, 177 us with sums
+// without a mean error and the leading-node checks; 64^2: 22.8, 22.7, 14.9.
 template <int NP>
 __global__ void __launch_bounds__(2 * Tiling2D<NP>::NH) k2_setup_rev(SetupRevArgs2D a) {
   using TL = Tiling2D<NP>;

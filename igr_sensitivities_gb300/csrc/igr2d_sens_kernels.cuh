@@ -35,7 +35,7 @@ struct SensRhsArgs2D {
 };
 
 // What bounds it: FP64 issue; the twelve line derivatives are integer work in rolled loops over the fields. With
-// k2_sens_hyp_rk 393 us per launch on average with FP64 contractions, 199 us now (2 x 256^2 P3).
+// k2_sens_hyp_rk 393 us per launch on average with FP64 contractions, 189 us now (122 and 279 us, 2 x 256^2 P3).
 template <int NP>
 __global__ void __launch_bounds__(Tiling2D<NP>::NT) k2_sens_rhs(SensRhsArgs2D a) {
   using TL = Tiling2D<NP>;
