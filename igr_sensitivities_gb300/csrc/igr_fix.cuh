@@ -567,7 +567,8 @@ __device__ __forceinline__ double flux_at(const FixFlux<NP>& f, int i) {
 }
 
 // The products flux_i (D v)_i, with z0 and zL added at the end nodes, in units of 2^60 / 2^(r.e - 1022) (r.e < 0: the
-// bits of doubles). They go by the line's largest flux and derivative and are not aligned to the operator's sums.
+// bits of doubles). They go by the line's largest flux and derivative and are not aligned to the operator's sums: exact by the
+// line's norm (0.1 to 0.9 of the FP64 chain's rms error), not for a node far below it in both factors.
 template <int NP>
 __device__ __forceinline__ bool product_line(const FixFlux<NP>& f, const FixDeriv<NP>& d, double z0, double zL,
                                              FixSums<NP>& r) {
